@@ -65,6 +65,19 @@ __device__ __forceinline__ void tmem_cp_sf(uint32_t taddr, uint32_t smem_addr) {
     const uint64_t desc = (uint64_t) ((smem_addr >> 4) & 0x3fff) | ((uint64_t) (128 >> 4) << 32) | ((uint64_t) 1 << 46);
     asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
 }
+// tensor memory <- registers: thread i of the warp writes N consecutive 32-bit columns of lane (its quarter's base + i)
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint4 (&v)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0].x),
+                 "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w), "r"(v[2].x), "r"(v[2].y), "r"(v[2].z),
+                 "r"(v[2].w), "r"(v[3].x), "r"(v[3].y), "r"(v[3].z), "r"(v[3].w)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint4 (&v)[2]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0].x), "r"(v[0].y), "r"(v[0].z),
+                 "r"(v[0].w), "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // instruction descriptor: E2M1 x E2M1, UE4M3 scales, both operands K-major, M = 128, N = n (a multiple of 8)
 __host__ __device__ constexpr uint32_t umma_idesc_fp4(int n) { return (1u << 7) | (1u << 10) | ((uint32_t) (n >> 3) << 17) | ((128u >> 4) << 24); }
 // byte offset of the 4 scale bytes of row r (0..127) inside the 512-byte scale tile of one K = 64 step
@@ -307,7 +320,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
     uint8_t * tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
     uint8_t * acts = tiles + (size_t) TS * C::STAGE;
     uint8_t * raws = acts + (size_t) AS * C::ACT_STAGE;
-    __shared__ uint64_t raw_full[RS], raw_empty[RS], tile_full[TS], tile_empty[TS], act_full[AS], act_empty[AS], acc_full[2], acc_empty[2];
+    __shared__ uint64_t raw_full[RS], raw_empty[RS], tile_full[TS], tile_empty[TS], act_full[AS], act_empty[AS], acc_full[2], acc_empty[2], sfx_full[2];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
 
@@ -316,7 +329,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
         for (int i = 0; i < RS; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 8); }
         for (int i = 0; i < TS; ++i) { mbar_init(&tile_full[i], 256); mbar_init(&tile_empty[i], 1); }
         for (int i = 0; i < AS; ++i) { mbar_init(&act_full[i], 1); mbar_init(&act_empty[i], 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); mbar_init(&sfx_full[i], 4); }
         mbar_fence_init();
         s_abort = 0;
     }
@@ -427,17 +440,11 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                         const uint32_t sbase = smem_u32(tiles + (size_t) tile.stage * C::STAGE);
                         const uint32_t abase = smem_u32(acts + (size_t) act.stage * C::ACT_STAGE);
                         const uint32_t da = DESC_LO | (sbase >> 4), db = DESC_LO | (abase >> 4);
-                        // The scale copies are issued by this thread, in front of the instructions that read them: tcgen05.cp and tcgen05.mma
-                        // of one thread run in order.  Issued by a thread of their own (with a commit on an mbarrier between) they
-                        // were 15 % faster on the whole kernel, but now and then an instruction read a scale that was not in place.
-                        const uint32_t sf_set = tmem + C::SF_COL + 48 * (uint32_t) tile.stage;
+                        const uint32_t sf_set = tmem + C::SF_COL + 48 * (uint32_t) tile.stage;   // [tile 0][tile 1][planes], 4 x 4 columns each
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk) {   // 4 x K64 = 256; 32 bytes (2 units) further along the 128-byte row each
-                            const uint32_t t_sfa0 = sf_set + 12 * kk, t_sfa1 = t_sfa0 + 4, t_sfb = t_sfa0 + 8;
+                            const uint32_t t_sfa0 = sf_set + 4 * kk, t_sfa1 = t_sfa0 + 16, t_sfb = t_sfa0 + 32;
                             const bool accum = kc != 0 || kk != 0;
-                            tmem_cp_sf(t_sfa0, sbase + OFF_SFA + kk * 512);
-                            tmem_cp_sf(t_sfa1, sbase + OFF_SFA + FP4_SF_TILE + kk * 512);
-                            tmem_cp_sf(t_sfb, abase + OFF_SFB + kk * 512);
                             umma_fp4(d0, da + 2 * kk, db + 2 * kk, DESC_HI, idesc, t_sfa0, t_sfb, accum);
                             umma_fp4(d1, da + (OFF_A1 >> 4) + 2 * kk, db + 2 * kk, DESC_HI, idesc, t_sfa1, t_sfb, accum);
                         }
@@ -512,7 +519,8 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
         for (int c = 0; c < 8; ++c) a_off[c] = tsel * C::A_TILE + sw128_offset(trow, c);
         const uint32_t sf_off = OFF_SFA + tsel * FP4_SF_TILE + sf_tile_offset(trow);
         const uint32_t raw_off = (uint32_t) dq * GEMM_RAW_ROW;
-        Ring raw, tile;
+        const uint32_t quarter = (uint32_t) ((warp & 3) * 32) << 16;   // the lanes of tensor memory this warp may write
+        Ring raw, tile, act, sfx;
         FP4_PROF_DECL();
         for (int u = blockIdx.x; u < n_units && !s_abort; u += gridDim.x) {
             {
@@ -534,16 +542,11 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&raw_empty[raw.stage]);
                     raw.template advance<RS>();
-                    {
-                        FP4_PROF_T0();
-                        if (!__all_sync(0xffffffffu, wait_or_abort(&tile_empty[tile.stage], tile.phase ^ 1u, &s_abort, p.err))) break;
-                        FP4_PROF_ADD(1);
-                    }
+                    // Scale words of the tile's 128 rows, exchanged between its four warps: lane l of every warp needs those of rows
+                    // l, l + 32, l + 64 and l + 96 (one 16-byte read per K = 64 step).
                     uint8_t * st = tiles + (size_t) tile.stage * C::STAGE;
 #pragma unroll
                     for (int kb = 0; kb < 4; ++kb) {
-                        *reinterpret_cast<uint4 *>(st + a_off[2 * kb]) = make_uint4(R[9 * kb + 1], R[9 * kb + 2], R[9 * kb + 3], R[9 * kb + 4]);
-                        *reinterpret_cast<uint4 *>(st + a_off[2 * kb + 1]) = make_uint4(R[9 * kb + 5], R[9 * kb + 6], R[9 * kb + 7], R[9 * kb + 8]);
                         // The reference reads scale bytes through ggml_ue4m3_to_fp32: bit 7 ignored, 0x7f decodes to zero; to the tensor
                         // core 0x7f is NaN.  Clear bit 7 and turn 0x7f into 0 (t <= 0x7f per byte, so t + 1 carries into bit 7 only
                         // for 0x7f and never into the next byte).
@@ -551,6 +554,41 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                         const uint32_t nan1 = ((t + 0x01010101u) >> 7) & 0x01010101u;
                         *reinterpret_cast<uint32_t *>(st + sf_off + kb * 512) = t & ~((nan1 << 7) - nan1);
                     }
+                    // The next write to this stage's words comes two rounds later, behind the exchange of the round between.  (An mbarrier and
+                    // not a named barrier: a warp that gives up must not leave the others of its tile waiting without limit.)
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sfx_full[tsel]);
+                    if (!__all_sync(0xffffffffu, wait_or_abort(&sfx_full[tsel], sfx.phase, &s_abort, p.err))) break;
+                    sfx.template advance<1>();
+                    uint4 sfa[4], sfb[2];
+#pragma unroll
+                    for (int kb = 0; kb < 4; ++kb) sfa[kb] = *reinterpret_cast<const uint4 *>(st + OFF_SFA + tsel * FP4_SF_TILE + kb * 512 + lane * 16);
+                    {
+                        FP4_PROF_T0();
+                        if (!__all_sync(0xffffffffu, wait_or_abort(&act_full[act.stage], act.phase, &s_abort, p.err))) break;
+                        FP4_PROF_ADD(2);
+                    }
+                    // the planes' scales: tile 0's warps move those of the first two K = 64 steps, tile 1's those of the last two
+                    const uint8_t * sfb_src = acts + (size_t) act.stage * C::ACT_STAGE + OFF_SFB + tsel * 1024 + lane * 16;
+                    sfb[0] = *reinterpret_cast<const uint4 *>(sfb_src);
+                    sfb[1] = *reinterpret_cast<const uint4 *>(sfb_src + 512);
+                    act.template advance<AS>();
+                    {
+                        FP4_PROF_T0();
+                        if (!__all_sync(0xffffffffu, wait_or_abort(&tile_empty[tile.stage], tile.phase ^ 1u, &s_abort, p.err))) break;
+                        FP4_PROF_ADD(1);
+                    }
+                    tc_fence_after();
+                    const uint32_t sf_set = tmem + C::SF_COL + 48 * (uint32_t) tile.stage + quarter;
+                    tmem_st16(sf_set + 16 * tsel, sfa);
+                    tmem_st8(sf_set + 32 + 8 * tsel, sfb);
+#pragma unroll
+                    for (int kb = 0; kb < 4; ++kb) {
+                        *reinterpret_cast<uint4 *>(st + a_off[2 * kb]) = make_uint4(R[9 * kb + 1], R[9 * kb + 2], R[9 * kb + 3], R[9 * kb + 4]);
+                        *reinterpret_cast<uint4 *>(st + a_off[2 * kb + 1]) = make_uint4(R[9 * kb + 5], R[9 * kb + 6], R[9 * kb + 7], R[9 * kb + 8]);
+                    }
+                    tmem_wait_st();
+                    tc_fence_before();
                     // every writer orders its own stores against the tensor core's (async proxy) reads and then arrives itself
                     fence_async_smem();
                     mbar_arrive(&tile_full[tile.stage]);
@@ -558,7 +596,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                 }
             }
         }
-        if (tid == 256) FP4_PROF_STORE(10, 2);
+        if (tid == 256) FP4_PROF_STORE(10, 3);
     }
 
     // ---- teardown: everyone meets here (all waits above are bounded), then tensor memory goes back
