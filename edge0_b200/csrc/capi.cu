@@ -22,6 +22,7 @@
 #include "expert_gemm_tm.cuh"
 #include "expert_gemv.cuh"
 #include "expert_mma.cuh"
+#include "expert_mma_q3k.cuh"
 #include "fp4_probe.cuh"
 #include "graph_ops.cuh"
 #include "requant_fixup.cuh"
@@ -366,6 +367,45 @@ int launch_gemv(b200moe_ctx * ctx, int wtype, int k, const GemvParams & p, int n
     CASE(TYPE_Q3_K, 256) CASE(TYPE_Q3_K, 512) CASE(TYPE_Q3_K, 768) CASE(TYPE_Q3_K, 2048)
 #undef CASE
     return fail(ctx, B200MOE_ERR_UNSUPPORTED, "no expert kernel for type %d width %d", wtype, k);
+}
+
+// Q3_K on the int8 matrix instruction (expert_mma_q3k.cuh): the same bits as the integer GEMV.
+template <int K, bool DUAL>
+int launch_q3k_mma_t(b200moe_ctx * ctx, const GemvParams & p, cudaStream_t st) {
+    using C = Q3kMmaCfg<K, DUAL>;
+    static_assert(C::SMEM <= 220 * 1024, "operand buffers do not fit shared memory");
+    auto kern = expert_mma_q3k_kernel<K, DUAL>;
+    static bool configured[MAX_DEVICE_ORDINALS] = {};  // per instantiation and device
+    if (int rc = raise_smem_limit(ctx, kern, C::SMEM, configured)) return rc;
+    b200moe_ctx::Timed tm{};
+    if (ctx->timing) {
+        CUDA_TRY(ctx, cudaEventCreate(&tm.beg));
+        CUDA_TRY(ctx, cudaEventCreate(&tm.end));
+        tm.kind = DUAL ? 0 : ctx->dense_now ? 2 : 1;
+        CUDA_TRY(ctx, cudaEventRecord(tm.beg, st));
+    }
+    kern<<<ctx->sm_count, 256, C::SMEM, st>>>(p);
+    if (ctx->timing) {
+        CUDA_TRY(ctx, cudaEventRecord(tm.end, st));
+        ctx->timed.push_back(tm);
+    }
+    return check_launch(ctx, "expert_mma_q3k");
+}
+
+bool q3k_on_mma(int wtype, int64_t rows, int n_groups) { return wtype == TYPE_Q3_K && rows >= (int64_t) Q3K_MMA_MIN_ROWS * n_groups; }
+
+// the integer product of grouped rows: `rows` routed rows in up to n_groups groups
+template <bool DUAL>
+int launch_integer(b200moe_ctx * ctx, int wtype, int k, const GemvParams & p, int64_t rows, int n_groups, int nt, cudaStream_t st) {
+    if (q3k_on_mma(wtype, rows, n_groups)) {
+        switch (k) {
+            case 256: return launch_q3k_mma_t<256, DUAL>(ctx, p, st);
+            case 512: return launch_q3k_mma_t<512, DUAL>(ctx, p, st);
+            case 768: return launch_q3k_mma_t<768, DUAL>(ctx, p, st);
+            case 2048: return launch_q3k_mma_t<2048, DUAL>(ctx, p, st);
+        }
+    }
+    return launch_gemv<DUAL>(ctx, wtype, k, p, nt, st);
 }
 
 // ---- tensor maps for the warp-specialised grouped GEMM (the encoder is a host-side driver entry point; looked up
@@ -825,8 +865,8 @@ int dense_matvec(b200moe_ctx * ctx, int wtype, const void * w, const float * sca
     if ((rc = launch_group(ctx, p.one_group_ids, groups, T, st))) return rc;
     GemvParams g = gemv_params(ctx, w, w1, nullptr, nullptr, xq, y, n_out, 1, 1, groups);
     g.w_stride = 0;
-    if (w1) return launch_gemv<true>(ctx, wtype, k, g, 4, st);
-    if ((rc = launch_gemv<false>(ctx, wtype, k, g, 4, st))) return rc;
+    if (w1) return launch_integer<true>(ctx, wtype, k, g, T, groups, 4, st);
+    if ((rc = launch_integer<false>(ctx, wtype, k, g, T, groups, 4, st))) return rc;
     if (scale) {
         const size_t n = (size_t) T * n_out;
         scale_rows_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(y, scale, n);
@@ -1036,7 +1076,7 @@ int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const 
         if ((rc = tm_gu ? launch_gemm_tm<true>(ctx, n_in, m, rows, st) : launch_gemm<true>(ctx, n_in, m, rows, small_tiles, st))) return rc;
     } else {
         GemvParams gu = gemv_params(ctx, l->gate, l->up, l->gate_scale, l->up_scale, xq, p.hid, l->n_ff, k, 1, l->n_expert);
-        if ((rc = launch_gemv<true>(ctx, l->wtype, n_in, gu, nt, st))) return rc;
+        if ((rc = launch_integer<true>(ctx, l->wtype, n_in, gu, rows, l->n_expert, nt, st))) return rc;
     }
     if (fixup && (rc = launch_requant_fixup(ctx, l, xq, rows, n_in, k, fp4_gu, st))) return rc;
     // the integer down kernel quantises `hidden` itself while staging it (NVFP4 / Q8_0); otherwise a separate pass
@@ -1052,7 +1092,7 @@ int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const 
     } else {
         GemvParams dn = gemv_params(ctx, l->down, nullptr, l->down_scale, nullptr, p.hq, y, n_in, k, k, l->n_expert);
         if (fused_quant) dn.act_f32 = p.hid;
-        if ((rc = launch_gemv<false>(ctx, l->wtype, l->n_ff, dn, nt, st))) return rc;
+        if ((rc = launch_integer<false>(ctx, l->wtype, l->n_ff, dn, rows, l->n_expert, nt, st))) return rc;
     }
     if (!y_direct) {
         dim3 grid((n_in / 4 + 255) / 256, T);
@@ -1484,7 +1524,7 @@ int b200moe_mul_mat_id(b200moe_ctx * ctx, int wtype, const void * as, int64_t ne
     if ((rc = check_launch(ctx, "count_ids"))) return rc;
     if ((rc = launch_group(ctx, p.ids, (int) n_as, rows, st))) return rc;
     GemvParams g = gemv_params(ctx, as, nullptr, nullptr, nullptr, p.hq, dst, (int) ne01, (int) n_ids, (int) ne11, (int) n_as);
-    return launch_gemv<false>(ctx, wtype, (int) ne00, g, tokens_per_pass(rows, (int) n_as), st);
+    return launch_integer<false>(ctx, wtype, (int) ne00, g, rows, (int) n_as, tokens_per_pass(rows, (int) n_as), st);
 }
 
 int b200moe_mul_mat(b200moe_ctx * ctx, int wtype, const void * w, int64_t ne00, int64_t ne01, const float * x, int64_t T, const float * scale,
