@@ -158,7 +158,10 @@ void carve(Plan & p, uint8_t * base) {
     p.outb = c.take<float>(T * H);
     p.one_group_ids = c.take<int>(T);
     p.afp16 = c.take<__half>(2 * std::max<size_t>(std::max(R, T), 64) * std::max({kin, I, H, Ish}));   // hi plane, then lo plane
-    p.asf_bytes = (std::min(E, std::max(R, T)) + std::max(R, T) / FP4_RPT + 1) * ((std::max({kin, I, H, Ish}) + 255) / 256) * FP4_SF_TILE;
+    // scale tiles: at most one partial token tile per expert, whatever the tile size
+    const size_t sf_stage = std::max((std::min(E, std::max(R, T)) + std::max(R, T) / FP4_RPT_SMALL + 1) * fp4_sfb_bytes(FP4_RPT_SMALL),
+                                     (std::min(E, std::max(R, T)) + std::max(R, T) / FP4_RPT_LARGE + 1) * fp4_sfb_bytes(FP4_RPT_LARGE));
+    p.asf_bytes = sf_stage * ((std::max({kin, I, H, Ish}) + 255) / 256);
     p.asf = c.take<uint8_t>(p.asf_bytes);
     p.arow_scale = c.take<float>(std::max(R, T));
     if (Ish) {
@@ -212,6 +215,8 @@ constexpr float FIX_STEP_MARGIN = 0.015f;  // quantisation steps; largest GEMM e
 constexpr float FIX_REL_MARGIN = 1.2e-4f;  // of the block maximum; largest error measured: 3.0e-5 of it
 // after the block-scaled FP4 GEMM (exact digit planes; only fp32 accumulation differs):
 constexpr float FIX_STEP_MARGIN_FP4 = 2.5e-3f;  // largest error measured: 2.3e-4 steps (p99.99: 1.0e-4)
+constexpr int FP4_LARGE_TILE_ROWS = 24;    // routed rows per expert from which the FP4 kernels take the large token tile
+
 constexpr float FIX_REL_MARGIN_FP4 = 2.0e-5f;   // largest error measured: 1.8e-6 of the block maximum
 
 // need_router / need_experts: which weight pointers the entry point is going to read
@@ -528,10 +533,11 @@ int launch_gemm(b200moe_ctx * ctx, int k, const MmaParams & p, int rows, bool sm
 }
 
 // block-scaled FP4 grouped GEMM (expert_gemm_fp4.cuh): digit planes of the routed rows, then the GEMM
-template <int K, bool DUAL>
+template <int K, bool DUAL, int RPT>
 int launch_gemm_fp4_t(b200moe_ctx * ctx, const Fp4Params & fp, const void * w0, const void * w1, const uint8_t * planes, int rows, cudaStream_t st) {
-    using C = Fp4Cfg<K>;
-    auto kern = expert_gemm_fp4_kernel<K, DUAL>;
+    using C = Fp4Cfg<K, RPT>;
+    static_assert(C::SMEM <= 226 * 1024, "rings do not fit shared memory");
+    auto kern = expert_gemm_fp4_kernel<K, DUAL, RPT>;
     static bool configured[MAX_DEVICE_ORDINALS] = {};  // per instantiation and device
     if (int rc = raise_smem_limit(ctx, kern, C::SMEM, configured)) return rc;
     constexpr uint64_t ROW_BYTES = K / 64 * 36;
@@ -544,8 +550,8 @@ int launch_gemm_fp4_t(b200moe_ctx * ctx, const Fp4Params & fp, const void * w0, 
     } else {
         mw1 = mw0;
     }
-    const uint64_t prows = std::max<uint64_t>((uint64_t) rows * FP4_PLANES, FP4_NROW);
-    if ((rc = make_map_2d(ctx, &mpl, CU_TENSOR_MAP_DATA_TYPE_UINT8, planes, K / 2, prows, K / 2, 128, FP4_NROW, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
+    const uint64_t prows = std::max<uint64_t>((uint64_t) rows * FP4_PLANES, C::NROW);
+    if ((rc = make_map_2d(ctx, &mpl, CU_TENSOR_MAP_DATA_TYPE_UINT8, planes, K / 2, prows, K / 2, 128, C::NROW, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
     b200moe_ctx::Timed tm{};
     if (ctx->timing) {
         CUDA_TRY(ctx, cudaEventCreate(&tm.beg));
@@ -585,7 +591,8 @@ int launch_gemm_fp4_t(b200moe_ctx * ctx, const Fp4Params & fp, const void * w0, 
 
 template <bool DUAL>
 int launch_gemm_fp4(b200moe_ctx * ctx, int k, const Fp4Params & fp, const void * w0, const void * w1, const uint8_t * planes, int rows, cudaStream_t st) {
-#define GEMM_CASE(KK) case KK: return launch_gemm_fp4_t<KK, DUAL>(ctx, fp, w0, w1, planes, rows, st);
+#define GEMM_CASE(KK) case KK: return ctx->plan.groups.tile_rows == FP4_RPT_LARGE ? launch_gemm_fp4_t<KK, DUAL, FP4_RPT_LARGE>(ctx, fp, w0, w1, planes, rows, st) \
+                                                                          : launch_gemm_fp4_t<KK, DUAL, FP4_RPT_SMALL>(ctx, fp, w0, w1, planes, rows, st);
     switch (k) { GEMM_CASE(256) GEMM_CASE(512) GEMM_CASE(768) GEMM_CASE(1024) GEMM_CASE(2048) GEMM_CASE(4096) }
 #undef GEMM_CASE
     return fail(ctx, B200MOE_ERR_UNSUPPORTED, "no FP4 tensor-core expert kernel for width %d", k);
@@ -602,7 +609,7 @@ bool fp4_supported(int wtype, int n_in, int n_ff) { return wtype == TYPE_NVFP4 &
 int launch_act_planes(b200moe_ctx * ctx, ActQuant act, const float * src, const int32_t * ids, int rows, int k, int n_ids, int ne11, int n_as,
                       cudaStream_t st, ActQuant emit = ActQuant{}, int64_t src_stride = 0) {
     Plan & p = ctx->plan;
-    PlaneOut po{ reinterpret_cast<uint8_t *>(p.afp16), p.asf, p.arow_scale, p.groups.pos /* free once the rows are grouped */ };
+    PlaneOut po{ reinterpret_cast<uint8_t *>(p.afp16), p.asf, p.arow_scale, p.groups.pos /* free once the rows are grouped */, p.groups.tile_rows };
     const int * tiles = p.groups.cost + 3 * (n_as + 1);
     if (src_stride == 0) src_stride = k;
     if (src && (((uintptr_t) src & 15) || src_stride % 4)) return fail(ctx, B200MOE_ERR_INVALID_ARG, "fp32 activation rows must be 16-byte aligned");
@@ -705,9 +712,14 @@ int launch_front(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T
     return T <= 8 ? launch_front_t<1, XT>(ctx, l, x, T, st) : launch_front_t<4, XT>(ctx, l, x, T, st);
 }
 
+// Routed rows per token tile of the FP4 kernels for `rows` rows in up to n_groups groups; kept in the plan from the grouping to the
+// kernels that walk the tiles.
+int token_tile_rows(int64_t rows, int n_groups) { return rows >= (int64_t) FP4_LARGE_TILE_ROWS * n_groups ? FP4_RPT_LARGE : FP4_RPT_SMALL; }
+
 int launch_select_group(b200moe_ctx * ctx, const b200moe_layer * l, int T, float * probs, cudaStream_t st) {
     Plan & p = ctx->plan;
     const int E = l->n_expert, K = l->n_expert_used;
+    p.groups.tile_rows = token_tile_rows((int64_t) T * K, E);
     const size_t sh = (size_t) (3 * E + 1) * sizeof(int);
 #define SELG(EPL) launch_k(ctx, route_select_group_kernel<EPL>, dim3(1), dim3(1024), sh, st, p.logits, E, K, T, p.ids, p.wts, probs, p.groups, ctx->d_err)
     if (E <= 32) SELG(1);
@@ -738,6 +750,7 @@ int launch_select(b200moe_ctx * ctx, const b200moe_layer * l, int T, int32_t * i
 
 int launch_group(b200moe_ctx * ctx, const int32_t * ids, int E, int rows, cudaStream_t st, bool allow_empty = false) {
     Plan & p = ctx->plan;
+    p.groups.tile_rows = token_tile_rows(rows, E);
     const size_t sh = (size_t) (3 * E + 1) * sizeof(int);
     launch_k(ctx, group_scan_kernel, dim3(1), dim3(1024), sh, st, p.groups, ids, E, rows, ctx->d_err, allow_empty ? 1 : 0);
     return check_launch(ctx, "group_scan");
@@ -890,6 +903,8 @@ int dense_matmul_fp4(b200moe_ctx * ctx, const void * w, const float * scale, con
                      bool exact_requant, ActQuant xq, void * list_room, size_t list_room_bytes, const void * w1) {
     Plan & p = ctx->plan;
     int rc;
+    // a dense product has one group: the large tile once its units fill the GPU
+    p.groups.tile_rows = (int64_t) ((T + FP4_RPT_LARGE - 1) / FP4_RPT_LARGE) * (n_out / (w1 ? 128 : 256)) >= ctx->sm_count ? FP4_RPT_LARGE : FP4_RPT_SMALL;
     one_group_kernel<<<(T + 255) / 256, 256, 0, st>>>(p.groups, p.one_group_ids, T);
     if ((rc = check_launch(ctx, "one_group"))) return rc;
     // the fix-up recomputes with the quantised activations: have the plane kernel leave them in xq
@@ -1037,8 +1052,7 @@ int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const 
     switch (path) {
         case 0:
             if (rows <= 16) break;                           // one or two tokens: the small integer kernel, bit-identical
-            if (can_fp4 && few_rows) { fp4_gu = fp4_down = true; fixup = latent; }
-            else if (can_mma && rows >= 2 * l->n_expert) { mma_gu = true; mma_down = !latent; fixup = rows > 4096 || latent; }
+            if (can_fp4) { fp4_gu = true; fp4_down = few_rows || !latent; fixup = latent || (!few_rows && rows > 4096); }
             break;
         case 1: break;
         case 2: mma_gu = mma_down = can_mma; break;

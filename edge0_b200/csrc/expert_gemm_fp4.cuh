@@ -42,10 +42,12 @@
 namespace b200moe {
 
 constexpr int FP4_PLANES = 7;
-constexpr int FP4_RPT = TOKEN_TILE_ROWS;          // 14 routed rows per token tile
-constexpr int FP4_NROW = FP4_PLANES * FP4_RPT;    // 98 plane rows per token tile
-constexpr int FP4_NCOL = 104;                     // accumulator columns per weight tile: N of the instruction is a multiple of 8
+// Routed rows per token tile: 14 for batched decode (two accumulator buffers, so the epilogue runs beside the next unit), 27 for
+// prefill (N = 192 fills tensor memory with one buffer; a weight tile is repacked and fetched half as often per routed row).
+constexpr int FP4_RPT_SMALL = TOKEN_TILE_SMALL, FP4_RPT_LARGE = TOKEN_TILE_LARGE;
 constexpr int FP4_SF_TILE = 4 * 512;              // scale factors of 128 rows for the four K = 64 steps of a stage
+// bytes of one token tile's scale factors per K = 256 stage: one block of 128 plane rows, or two
+__host__ __device__ constexpr int fp4_sfb_bytes(int rpt) { return (FP4_PLANES * rpt + 127) / 128 * FP4_SF_TILE; }
 constexpr int FP4_THREADS = 512;
 
 __device__ __forceinline__ void umma_fp4(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t sfa, uint32_t sfb,
@@ -102,20 +104,22 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 // ---- activation planes ---------------------------------------------------------------------------------------------------
 // Expert-sorted routed row i -> seven plane rows 7i .. 7i+6 of `planes` (K/2 bytes each, ggml nibble order inside every
 // 16-block), its scale bytes in the scale tiles of its token tile, and the power of two the epilogue multiplies with.
-//   tile_of_expert[e]: index of expert e's first token tile (prefix of ceil(rows_e / 14)); tile_expert[tile]: the inverse
-//   sf tiles: [tile][K / 256][4 steps][512 bytes], byte for (plane row n of the tile, 16-block g of the step) at sf_tile_offset(n) + g
+//   tile_of_expert[e]: index of expert e's first token tile (prefix of ceil(rows_e / rpt)); tile_expert[tile]: the inverse
+//   sf tiles: [tile][K / 256][4 steps][1 or 2 blocks of 128 plane rows][512 bytes], byte for (plane row n of the block, 16-block g of
+//   the step) at sf_tile_offset(n) + g
 struct PlaneOut {
     uint8_t * planes;       // [rows * 7][K / 2]
     uint8_t * sf;           // [tiles][K / 256][2048]
     float *   row_scale;    // [rows] by sorted position
     int *     tile_expert;  // [tiles] expert of every token tile
+    int       rpt;          // routed rows per token tile
 };
 
 // digits, codes and scale bytes of one quad: 16-block g, bytes j0 .. j0+3 (elements 16g + j and 16g + j + 8) with int8 values lo[], hi[]
 // and the fp32 bits of the block scale d (an fp16 number: d = M * 2^(exp8 - 137) with M the top 11 bits of the significand).
 // The four code bytes of every plane leave as one 32-bit store.
 __device__ __forceinline__ void plane_quad(const int (&lo)[4], const int (&hi)[4], uint32_t dbits, int E_row, int g, int j0, int K, int in_tile,
-                                           uint8_t * __restrict__ prow, uint8_t * __restrict__ sft) {
+                                           int sfb_bytes, uint8_t * __restrict__ prow, uint8_t * __restrict__ sft) {
     const bool nz = (dbits & 0x7fffffffu) != 0;
     const int M = nz ? (int) (((dbits & 0x7fffffu) | 0x800000u) >> 13) : 0;
     const int s = nz ? (int) ((dbits >> 23) & 0xff) - 137 - E_row + 8 : -100;           // scale exponent, at most 8
@@ -149,9 +153,12 @@ __device__ __forceinline__ void plane_quad(const int (&lo)[4], const int (&hi)[4
     if (j0 == 0) {
         // UE4M3 byte of 2^s: normal for s >= -6, the three power-of-two subnormals below, zero when flushed
         const uint32_t sb = s >= -6 ? (uint32_t) (s + 7) << 3 : s == -7 ? 4u : s == -8 ? 2u : s == -9 ? 1u : 0u;
-        uint8_t * dst = sft + (size_t) (g >> 4) * FP4_SF_TILE + ((g >> 2) & 3) * 512 + (g & 3);
+        uint8_t * dst = sft + (size_t) (g >> 4) * sfb_bytes + ((g >> 2) & 3) * (sfb_bytes / 4) + (g & 3);
 #pragma unroll
-        for (int p = 0; p < FP4_PLANES; ++p) dst[sf_tile_offset(in_tile * FP4_PLANES + p)] = (uint8_t) sb;
+        for (int p = 0; p < FP4_PLANES; ++p) {
+            const int n = in_tile * FP4_PLANES + p;
+            dst[(n >> 7) * 512 + sf_tile_offset(n & 127)] = (uint8_t) sb;
+        }
     }
 }
 
@@ -183,8 +190,8 @@ __global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const flo
         int e = ids[r];
         e = e < 0 ? 0 : (e >= n_as ? n_as - 1 : e);    // bad ids were reported by the grouping kernels; stay inside the tables
         const int row_beg = offsets[e];
-        in_tile = (i - row_beg) % FP4_RPT;
-        tile = tile_of_expert[e] + (i - row_beg) / FP4_RPT;
+        in_tile = (i - row_beg) % out.rpt;
+        tile = tile_of_expert[e] + (i - row_beg) / out.rpt;
         if (in_tile == 0 && t_in == 0) out.tile_expert[tile] = e;
     }
     const int nb32 = K / 32;
@@ -246,12 +253,13 @@ __global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const flo
     const int E_row = s_E[lrow];
     if (t_in == 0) out.row_scale[i] = E_row > -1000 ? __uint_as_float((uint32_t) (E_row - 8 + 127) << 23) : 0.0f;   // 2^(E_row - 8): far from the fp32 limits
     uint8_t * prow = out.planes + (size_t) i * FP4_PLANES * (K / 2);
-    uint8_t * sft = out.sf + (size_t) tile * (K / 256) * FP4_SF_TILE;
+    const int sfb_bytes = fp4_sfb_bytes(out.rpt);
+    uint8_t * sft = out.sf + (size_t) tile * (K / 256) * sfb_bytes;
 #pragma unroll
     for (int u = 0; u < MAX_QUADS; ++u)
         if (u < qpt) {
             const int qd = t_in + tpr * u;
-            plane_quad(lo[u], hi[u], db[u], E_row, qd >> 1, (qd & 1) * 4, K, in_tile, prow, sft);
+            plane_quad(lo[u], hi[u], db[u], E_row, qd >> 1, (qd & 1) * 4, K, in_tile, sfb_bytes, prow, sft);
         }
 }
 
@@ -286,20 +294,27 @@ struct Fp4Params {
     long long * prof;       // development builds only
 };
 
-template <int K>
+template <int K, int RPT>
 struct Fp4Cfg {
+    static constexpr int NROW = FP4_PLANES * RPT;                    // plane rows of a token tile (98, 189)
+    static constexpr int NCOL = (NROW + 7) / 8 * 8;                  // accumulator columns per weight tile: N of the instruction is a multiple of 8
+    static constexpr int NACC = RPT == FP4_RPT_SMALL ? 2 : 1;        // accumulator buffers
+    static constexpr int NBLK = (NROW + 127) / 128;                  // blocks of 128 plane rows in the scale tile
     static constexpr int A_TILE = 128 * 128;                         // 128 weight rows x 256 K as fp4
-    static constexpr int B_BYTES = FP4_NROW * 128;                   // 98 plane rows arrive per stage
-    static constexpr int B_TILE = 13 * 1024;                         // their room (rows 98..103 of an N = 104 instruction read what lies there: columns nobody uses)
-    static constexpr int STAGE = 2 * A_TILE + 2 * FP4_SF_TILE;      // repacked weights of both tiles, then their scale tiles
-    static constexpr int ACT_STAGE = B_TILE + FP4_SF_TILE;           // digit planes, then their scale tile
+    static constexpr int B_BYTES = NROW * 128;                       // plane rows that arrive per stage
+    static constexpr int B_TILE = (NCOL * 128 + 1023) / 1024 * 1024; // their room (rows beyond NROW are read by the instruction: columns nobody uses)
+    static constexpr int SFB = fp4_sfb_bytes(RPT);
+    static constexpr int STAGE = 2 * A_TILE;                         // repacked weights of both tiles
+    static constexpr int ACT_STAGE = B_TILE + SFB;                   // digit planes, then their scale tile
     static constexpr int RAW_STAGE = 256 * GEMM_RAW_ROW;
-    static constexpr int RS = 3;
+    static constexpr int RS = RPT == FP4_RPT_SMALL ? 3 : 2;
     static constexpr int TS = 2;
     static constexpr int AS = 3;                                      // plane tiles come from L2 with ~1 us latency: fetched three stages ahead
-    static constexpr uint32_t TMEM_COLS = 512;                        // 2 buffers x 2 accumulators x 104 columns, then two sets of scale factors
-    static constexpr uint32_t SF_COL = 4 * FP4_NCOL;                  // 416; 48 columns per set
-    static_assert(TS == 2 && B_TILE >= B_BYTES + 6 * 128, "one scale-factor set per operand stage");
+    static constexpr uint32_t TMEM_COLS = 512;                        // NACC buffers x 2 accumulators, then two sets of scale factors
+    static constexpr uint32_t SF_COL = NACC * 2 * NCOL;
+    static constexpr uint32_t SF_SET = 32 + 16 * NBLK;                // [tile 0][tile 1][planes]: 4 columns per K = 64 step and 128 rows
+    static_assert(SF_COL + TS * SF_SET <= TMEM_COLS, "accumulators and one scale-factor set per operand stage fit tensor memory");
+    static_assert(NROW <= 256 && B_TILE >= B_BYTES, "plane rows fit one box and their room");
     static_assert(STAGE % 1024 == 0 && ACT_STAGE % 1024 == 0, "stages keep the 1024-byte alignment of swizzled tiles");
     static_assert(K % GEMM_RAW_K == 0, "K must be a multiple of 256");
     static constexpr size_t SMEM = (size_t) TS * STAGE + (size_t) AS * ACT_STAGE + (size_t) RS * RAW_STAGE + 1024;
@@ -307,12 +322,12 @@ struct Fp4Cfg {
 
 // DUAL: tile 0 = gate rows f .. f+127, tile 1 = up rows of the same features; epilogue = SwiGLU; 128 features per item.
 // single: tiles 0 and 1 = 256 consecutive rows of the one tensor; 256 features per item.
-template <int K, bool DUAL>
+template <int K, bool DUAL, int RPT>
 __global__ void __launch_bounds__(FP4_THREADS, 1)
 expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1,
                        const __grid_constant__ CUtensorMap map_planes) {
-    using C = Fp4Cfg<K>;
-    constexpr int TS = C::TS, RS = C::RS, AS = C::AS;
+    using C = Fp4Cfg<K, RPT>;
+    constexpr int TS = C::TS, RS = C::RS, AS = C::AS, NACC = C::NACC;
     constexpr int KC = K / GEMM_RAW_K;
     constexpr int FEAT = DUAL ? 128 : 256;
 
@@ -320,7 +335,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
     uint8_t * tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
     uint8_t * acts = tiles + (size_t) TS * C::STAGE;
     uint8_t * raws = acts + (size_t) AS * C::ACT_STAGE;
-    __shared__ uint64_t raw_full[RS], raw_empty[RS], tile_full[TS], tile_empty[TS], act_full[AS], act_empty[AS], acc_full[2], acc_empty[2], sfx_full[2];
+    __shared__ uint64_t raw_full[RS], raw_empty[RS], tile_full[TS], tile_empty[TS], act_full[AS], act_empty[AS], acc_full[NACC], acc_empty[NACC], sfx_full[2];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
 
@@ -329,7 +344,8 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
         for (int i = 0; i < RS; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 8); }
         for (int i = 0; i < TS; ++i) { mbar_init(&tile_full[i], 256); mbar_init(&tile_empty[i], 1); }
         for (int i = 0; i < AS; ++i) { mbar_init(&act_full[i], 1); mbar_init(&act_empty[i], 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); mbar_init(&sfx_full[i], 4); }
+        for (int i = 0; i < NACC; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
+        for (int i = 0; i < 2; ++i) mbar_init(&sfx_full[i], 4);
         mbar_fence_init();
         s_abort = 0;
     }
@@ -358,13 +374,13 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
         w.tile = u / f_tiles;
         w.ft = u - w.tile * f_tiles;
         w.e = p.tile_expert[w.tile];
-        const int row_beg = p.offsets[w.e], t0 = (w.tile - p.tile_of_expert[w.e]) * FP4_RPT;
+        const int row_beg = p.offsets[w.e], t0 = (w.tile - p.tile_of_expert[w.e]) * RPT;
         w.row0 = row_beg + t0;                                   // first expert-sorted row of the token tile
-        w.nt = min(FP4_RPT, p.offsets[w.e + 1] - w.row0);
+        w.nt = min(RPT, p.offsets[w.e + 1] - w.row0);
         return w;
     };
-    // weight stage: [A0][A1][SFA0][SFA1]; activation stage: [B][SFB]
-    constexpr uint32_t OFF_A1 = C::A_TILE, OFF_SFA = 2 * C::A_TILE, OFF_SFB = C::B_TILE;
+    // weight stage: [A0][A1]; activation stage: [B][SFB]
+    constexpr uint32_t OFF_A1 = C::A_TILE, OFF_SFB = C::B_TILE;
 
     if (warp == 0) {
         // ---------------------------------------------------------------- raw weight producer
@@ -395,15 +411,15 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
             FP4_PROF_DECL();
             for (int u = blockIdx.x; u < n_units && !s_abort; u += gridDim.x) {
                 const Unit w = unit_at(u);
-                const uint8_t * sft = p.sf + (size_t) w.tile * KC * FP4_SF_TILE;
+                const uint8_t * sft = p.sf + (size_t) w.tile * KC * C::SFB;
                 for (int kc = 0; kc < KC; ++kc) {
                     FP4_PROF_T0();
                     if (!wait_or_abort<100>(&act_empty[act.stage], act.phase ^ 1u, &s_abort, p.err)) break;
                     FP4_PROF_ADD(0);
                     uint8_t * st = acts + (size_t) act.stage * C::ACT_STAGE;
-                    mbar_arrive_expect_tx(&act_full[act.stage], C::B_BYTES + FP4_SF_TILE);
+                    mbar_arrive_expect_tx(&act_full[act.stage], C::B_BYTES + C::SFB);
                     tma_load_2d(st, &map_planes, kc * 128, FP4_PLANES * w.row0, &act_full[act.stage]);
-                    bulk_g2s(st + OFF_SFB, sft + (size_t) kc * FP4_SF_TILE, FP4_SF_TILE, &act_full[act.stage]);
+                    bulk_g2s(st + OFF_SFB, sft + (size_t) kc * C::SFB, C::SFB, &act_full[act.stage]);
                     act.template advance<AS>();
                 }
             }
@@ -424,7 +440,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                         FP4_PROF_ADD(0);
                     }
                     tc_fence_after();
-                    const uint32_t d0 = tmem + (uint32_t) acc.stage * (2 * FP4_NCOL), d1 = d0 + FP4_NCOL;
+                    const uint32_t d0 = tmem + (uint32_t) acc.stage * (2 * C::NCOL), d1 = d0 + C::NCOL;
                     for (int kc = 0; kc < KC; ++kc) {
                         {
                             FP4_PROF_T0();
@@ -440,10 +456,10 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                         const uint32_t sbase = smem_u32(tiles + (size_t) tile.stage * C::STAGE);
                         const uint32_t abase = smem_u32(acts + (size_t) act.stage * C::ACT_STAGE);
                         const uint32_t da = DESC_LO | (sbase >> 4), db = DESC_LO | (abase >> 4);
-                        const uint32_t sf_set = tmem + C::SF_COL + 48 * (uint32_t) tile.stage;   // [tile 0][tile 1][planes], 4 x 4 columns each
+                        const uint32_t sf_set = tmem + C::SF_COL + C::SF_SET * (uint32_t) tile.stage;   // [tile 0][tile 1][planes]
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk) {   // 4 x K64 = 256; 32 bytes (2 units) further along the 128-byte row each
-                            const uint32_t t_sfa0 = sf_set + 4 * kk, t_sfa1 = t_sfa0 + 16, t_sfb = t_sfa0 + 32;
+                            const uint32_t t_sfa0 = sf_set + 4 * kk, t_sfa1 = t_sfa0 + 16, t_sfb = sf_set + 32 + 4 * C::NBLK * kk;
                             const bool accum = kc != 0 || kk != 0;
                             umma_fp4(d0, da + 2 * kk, db + 2 * kk, DESC_HI, idesc, t_sfa0, t_sfb, accum);
                             umma_fp4(d1, da + (OFF_A1 >> 4) + 2 * kk, db + 2 * kk, DESC_HI, idesc, t_sfa1, t_sfb, accum);
@@ -454,7 +470,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                         act.template advance<AS>();
                     }
                     umma_commit(&acc_full[acc.stage]);
-                    acc.template advance<2>();
+                    acc.template advance<NACC>();
                 }
             }
             FP4_PROF_STORE(4, 3);
@@ -469,45 +485,51 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
             const float sc0 = p.scale0 ? p.scale0[w.e] : 1.0f;
             const float sc1 = DUAL ? (p.scale1 ? p.scale1[w.e] : 1.0f) : sc0;
             const int feature = w.ft * FEAT + q * 32 + lane;
+            // lane i holds the routed row and the power of two of the tile's row i (a tile has at most 27)
+            const int my_row = lane < w.nt ? p.perm[w.row0 + lane] : 0;
+            const float my_rs = lane < w.nt ? p.row_scale[w.row0 + lane] : 0.0f;
+            // lanes leave the polling loop one by one: the vote reconverges the warp (tcgen05.ld below needs all of it)
             {
-                const int nt = w.nt;
-                // lanes leave the polling loop one by one: the vote reconverges the warp (tcgen05.ld below needs all of it)
-                {
-                    FP4_PROF_T0();
-                    if (!__all_sync(0xffffffffu, wait_or_abort<200>(&acc_full[acc.stage], acc.phase, &s_abort, p.err))) break;
-                    FP4_PROF_ADD(0);
-                }
-                tc_fence_after();
-                const uint32_t d0 = tmem + (uint32_t) acc.stage * (2 * FP4_NCOL) + ((uint32_t) (q * 32) << 16);
-                for (int g = 0; g < nt; g += 4) {          // four routed rows = 28 plane columns per load (the last load of a full tile reads past its 98)
-                    float v0[32], v1[32];
-                    tmem_ld32(d0 + FP4_PLANES * g, v0);
-                    tmem_ld32(d0 + FP4_NCOL + FP4_PLANES * g, v1);
-#pragma unroll
-                    for (int rr = 0; rr < 4; ++rr) {
-                        if (g + rr < nt) {
-                            const int i = w.row0 + g + rr;
-                            const float rs = p.row_scale[i];
-                            // sum_p 8^p * plane_p, highest plane first
-                            float x0 = v0[7 * rr + 6], x1 = v1[7 * rr + 6];
-#pragma unroll
-                            for (int pl = 5; pl >= 0; --pl) {
-                                x0 = __fmaf_rn(x0, 8.0f, v0[7 * rr + pl]);
-                                x1 = __fmaf_rn(x1, 8.0f, v1[7 * rr + pl]);
-                            }
-                            x0 = __fmul_rn(__fmul_rn(x0, rs), sc0);
-                            x1 = __fmul_rn(__fmul_rn(x1, rs), sc1);
-                            float * orow = p.out + (size_t) p.perm[i] * p.n_out;
-                            if (DUAL) orow[feature] = __fmul_rn(ggml_silu(x0), x1);
-                            else { orow[feature] = x0; orow[feature + 128] = x1; }
-                        }
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[acc.stage]);
-                acc.template advance<2>();
+                FP4_PROF_T0();
+                if (!__all_sync(0xffffffffu, wait_or_abort<200>(&acc_full[acc.stage], acc.phase, &s_abort, p.err))) break;
+                FP4_PROF_ADD(0);
             }
+            tc_fence_after();
+            const uint32_t d0 = tmem + (uint32_t) acc.stage * (2 * C::NCOL) + ((uint32_t) (q * 32) << 16);
+            // The planes of every routed row are folded first and the accumulators given back before anything else is done with the
+            // sums: with a single accumulator buffer the next unit's instructions wait for this loop.
+            float x0[RPT], x1[RPT];
+#pragma unroll
+            for (int g = 0; g < RPT; g += 4)              // four routed rows = 28 plane columns per load (the last load may read past the tile's columns)
+                if (g < w.nt) {
+                    auto fold = [&](uint32_t col, float (&x)[RPT]) {
+                        float v[32];
+                        tmem_ld32(col, v);
+#pragma unroll
+                        for (int rr = 0; rr < 4; ++rr)
+                            if (g + rr < RPT) {
+                                float a = v[7 * rr + 6];     // sum_p 8^p * plane_p, highest plane first
+#pragma unroll
+                                for (int pl = 5; pl >= 0; --pl) a = __fmaf_rn(a, 8.0f, v[7 * rr + pl]);
+                                x[g + rr] = a;
+                            }
+                    };
+                    fold(d0 + FP4_PLANES * g, x0);
+                    fold(d0 + C::NCOL + FP4_PLANES * g, x1);
+                }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[acc.stage]);
+            acc.template advance<NACC>();
+#pragma unroll
+            for (int i = 0; i < RPT; ++i)
+                if (i < w.nt) {
+                    const float rs = __shfl_sync(0xffffffffu, my_rs, i);
+                    float * orow = p.out + (size_t) __shfl_sync(0xffffffffu, my_row, i) * p.n_out;
+                    const float v0 = __fmul_rn(__fmul_rn(x0[i], rs), sc0), v1 = __fmul_rn(__fmul_rn(x1[i], rs), sc1);
+                    if (DUAL) orow[feature] = __fmul_rn(ggml_silu(v0), v1);
+                    else { orow[feature] = v0; orow[feature + 128] = v1; }
+                }
         }
         if (warp == 4 && lane == 0) FP4_PROF_STORE(8, 1);
     } else if (warp >= 8) {
@@ -517,7 +539,6 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
         uint32_t a_off[8];
 #pragma unroll
         for (int c = 0; c < 8; ++c) a_off[c] = tsel * C::A_TILE + sw128_offset(trow, c);
-        const uint32_t sf_off = OFF_SFA + tsel * FP4_SF_TILE + sf_tile_offset(trow);
         const uint32_t raw_off = (uint32_t) dq * GEMM_RAW_ROW;
         const uint32_t quarter = (uint32_t) ((warp & 3) * 32) << 16;   // the lanes of tensor memory this warp may write
         Ring raw, tile, act, sfx;
@@ -539,12 +560,10 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                             R[4 * i] = v.x; R[4 * i + 1] = v.y; R[4 * i + 2] = v.z; R[4 * i + 3] = v.w;
                         }
                     }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&raw_empty[raw.stage]);
-                    raw.template advance<RS>();
-                    // Scale words of the tile's 128 rows, exchanged between its four warps: lane l of every warp needs those of rows
-                    // l, l + 32, l + 64 and l + 96 (one 16-byte read per K = 64 step).
-                    uint8_t * st = tiles + (size_t) tile.stage * C::STAGE;
+                    // Scale words of the tile's 128 rows, exchanged between its four warps: lane l of every warp needs those of rows l, l + 32,
+                    // l + 64 and l + 96.  A row's four words go into the first 16 bytes of its own raw row, which this thread has just
+                    // read.  (An mbarrier and not a named barrier: a warp that gives up must not leave the others waiting without limit.)
+                    uint32_t S[4];
 #pragma unroll
                     for (int kb = 0; kb < 4; ++kb) {
                         // The reference reads scale bytes through ggml_ue4m3_to_fp32: bit 7 ignored, 0x7f decodes to zero; to the tensor
@@ -552,26 +571,34 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                         // for 0x7f and never into the next byte).
                         const uint32_t t = R[9 * kb] & 0x7f7f7f7fu;
                         const uint32_t nan1 = ((t + 0x01010101u) >> 7) & 0x01010101u;
-                        *reinterpret_cast<uint32_t *>(st + sf_off + kb * 512) = t & ~((nan1 << 7) - nan1);
+                        S[kb] = t & ~((nan1 << 7) - nan1);
                     }
-                    // The next write to this stage's words comes two rounds later, behind the exchange of the round between.  (An mbarrier and
-                    // not a named barrier: a warp that gives up must not leave the others of its tile waiting without limit.)
+                    uint8_t * const raw_tile = raws + (size_t) raw.stage * C::RAW_STAGE + (size_t) tsel * 128 * GEMM_RAW_ROW;
+                    *reinterpret_cast<uint4 *>(raw_tile + trow * GEMM_RAW_ROW) = make_uint4(S[0], S[1], S[2], S[3]);
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&sfx_full[tsel]);
                     if (!__all_sync(0xffffffffu, wait_or_abort(&sfx_full[tsel], sfx.phase, &s_abort, p.err))) break;
                     sfx.template advance<1>();
-                    uint4 sfa[4], sfb[2];
+                    uint4 sfr[4];                  // [row l + 32 j][K = 64 step]
 #pragma unroll
-                    for (int kb = 0; kb < 4; ++kb) sfa[kb] = *reinterpret_cast<const uint4 *>(st + OFF_SFA + tsel * FP4_SF_TILE + kb * 512 + lane * 16);
+                    for (int j = 0; j < 4; ++j) sfr[j] = *reinterpret_cast<const uint4 *>(raw_tile + (32 * j + lane) * GEMM_RAW_ROW);
+                    fence_async_smem();            // the next copy into this stage comes behind the words written above
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&raw_empty[raw.stage]);
+                    raw.template advance<RS>();
+                    const uint4 sfa[4] = { make_uint4(sfr[0].x, sfr[1].x, sfr[2].x, sfr[3].x), make_uint4(sfr[0].y, sfr[1].y, sfr[2].y, sfr[3].y),
+                                           make_uint4(sfr[0].z, sfr[1].z, sfr[2].z, sfr[3].z), make_uint4(sfr[0].w, sfr[1].w, sfr[2].w, sfr[3].w) };
+                    uint8_t * st = tiles + (size_t) tile.stage * C::STAGE;
                     {
                         FP4_PROF_T0();
                         if (!__all_sync(0xffffffffu, wait_or_abort(&act_full[act.stage], act.phase, &s_abort, p.err))) break;
                         FP4_PROF_ADD(2);
                     }
                     // the planes' scales: tile 0's warps move those of the first two K = 64 steps, tile 1's those of the last two
-                    const uint8_t * sfb_src = acts + (size_t) act.stage * C::ACT_STAGE + OFF_SFB + tsel * 1024 + lane * 16;
-                    sfb[0] = *reinterpret_cast<const uint4 *>(sfb_src);
-                    sfb[1] = *reinterpret_cast<const uint4 *>(sfb_src + 512);
+                    const uint8_t * sfb_src = acts + (size_t) act.stage * C::ACT_STAGE + OFF_SFB + tsel * (C::SFB / 2) + lane * 16;
+                    uint4 sfb[2 * C::NBLK];
+#pragma unroll
+                    for (int i = 0; i < 2 * C::NBLK; ++i) sfb[i] = *reinterpret_cast<const uint4 *>(sfb_src + 512 * i);
                     act.template advance<AS>();
                     {
                         FP4_PROF_T0();
@@ -579,9 +606,10 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                         FP4_PROF_ADD(1);
                     }
                     tc_fence_after();
-                    const uint32_t sf_set = tmem + C::SF_COL + 48 * (uint32_t) tile.stage + quarter;
+                    const uint32_t sf_set = tmem + C::SF_COL + C::SF_SET * (uint32_t) tile.stage + quarter;
                     tmem_st16(sf_set + 16 * tsel, sfa);
-                    tmem_st8(sf_set + 32 + 8 * tsel, sfb);
+                    if constexpr (C::NBLK == 2) tmem_st16(sf_set + 32 + 16 * tsel, sfb);
+                    else tmem_st8(sf_set + 32 + 8 * tsel, sfb);
 #pragma unroll
                     for (int kb = 0; kb < 4; ++kb) {
                         *reinterpret_cast<uint4 *>(st + a_off[2 * kb]) = make_uint4(R[9 * kb + 1], R[9 * kb + 2], R[9 * kb + 3], R[9 * kb + 4]);

@@ -486,7 +486,8 @@ __global__ void __launch_bounds__(256) route_select_kernel(const float * __restr
 //   offsets[e]   first slot of expert e in perm, offsets[E] = total rows
 //   perm[i]      routed row index (token*K + slot) placed i-th
 //   active[a]    a-th expert that has at least one row; n_active in meta[0], total rows in meta[1]
-constexpr int TOKEN_TILE_ROWS = 14;   // routed rows per token tile of the FP4 tensor-core kernels (7 digit planes each)
+// routed rows per token tile of the FP4 tensor-core kernels (7 digit planes each): batched decode, prefill
+constexpr int TOKEN_TILE_SMALL = 14, TOKEN_TILE_LARGE = 27;
 
 struct Groups {
     int * counts;   // [E]
@@ -496,7 +497,8 @@ struct Groups {
     int * active;   // [E]
     int * meta;     // [4]
     int * cost;     // [4][E+1]: rows 0-2: prefix over active experts of the work per weight row for the nt = 1, 2, 4 kernels;
-                    // row 3, indexed by EXPERT id: index of the expert's first token tile (prefix of ceil(rows / TOKEN_TILE_ROWS))
+                    // row 3, indexed by EXPERT id: index of the expert's first token tile (prefix of ceil(rows / tile_rows))
+    int tile_rows;  // TOKEN_TILE_SMALL or TOKEN_TILE_LARGE
 };
 
 // Block-wide: counts must be final and visible to this block.
@@ -516,7 +518,7 @@ __device__ __forceinline__ void group_scan_body(Groups g, const int32_t * __rest
             const int n = e < E ? cnt[e] : 0;
             // work per weight row: nt=1 kernels: one pass per routed row; nt=4 kernels: 3 per pass (decode) + 2 per routed row
             int incl = n, w2 = (n + 1) / 2, w4 = 3 * ((n + 3) / 4) + 2 * n;
-            int i2 = w2, i4 = w4, it = (n + TOKEN_TILE_ROWS - 1) / TOKEN_TILE_ROWS;
+            int i2 = w2, i4 = w4, it = (n + g.tile_rows - 1) / g.tile_rows;
             const int wt = it;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -574,7 +576,7 @@ __global__ void __launch_bounds__(256) one_group_kernel(Groups g, int32_t * __re
         g.cost[0] = 0; g.cost[1] = T;
         g.cost[2] = 0; g.cost[3] = (T + 1) / 2;
         g.cost[4] = 0; g.cost[5] = 3 * ((T + 3) / 4) + 2 * T;
-        g.cost[6] = 0; g.cost[7] = (T + TOKEN_TILE_ROWS - 1) / TOKEN_TILE_ROWS;
+        g.cost[6] = 0; g.cost[7] = (T + g.tile_rows - 1) / g.tile_rows;
     }
 }
 
