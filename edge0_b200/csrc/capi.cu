@@ -59,6 +59,7 @@ struct Plan {  // carved out of the scratch arena for one (layer shape, max_toke
     __half * afp16 = nullptr;       // [T*k][max(n_in, n_ff)] expert-sorted fp16 activations of the tensor-core path (or the FP4 digit planes)
     uint8_t * asf = nullptr;        // scale tiles of the FP4 digit planes: [token tiles][K / 256][2048]
     size_t asf_bytes = 0;
+    int * tile_expert = nullptr;    // expert of every token tile of the FP4 kernels
     float * arow_scale = nullptr;   // [T*k] power of two per expert-sorted routed row (FP4 digit planes)
     float * sh_a = nullptr;         // [T][n_ff_sh] shared expert: gate product, then silu(gate) * up
     float * sh_b = nullptr;         // [T][n_ff_sh] shared expert: up product
@@ -164,6 +165,7 @@ void carve(Plan & p, uint8_t * base) {
     p.asf_bytes = sf_stage * ((std::max({kin, I, H, Ish}) + 255) / 256);
     p.asf = c.take<uint8_t>(p.asf_bytes);
     p.arow_scale = c.take<float>(std::max(R, T));
+    p.tile_expert = c.take<int>(std::min(E, std::max(R, T)) + std::max(R, T) / FP4_RPT_SMALL + 1);
     if (Ish) {
         p.sh_a = c.take<float>(T * Ish);
         p.sh_b = c.take<float>(T * Ish);
@@ -609,14 +611,15 @@ bool fp4_supported(int wtype, int n_in, int n_ff) { return wtype == TYPE_NVFP4 &
 int launch_act_planes(b200moe_ctx * ctx, ActQuant act, const float * src, const int32_t * ids, int rows, int k, int n_ids, int ne11, int n_as,
                       cudaStream_t st, ActQuant emit = ActQuant{}, int64_t src_stride = 0) {
     Plan & p = ctx->plan;
-    PlaneOut po{ reinterpret_cast<uint8_t *>(p.afp16), p.asf, p.arow_scale, p.groups.pos /* free once the rows are grouped */, p.groups.tile_rows };
+    PlaneOut po{ reinterpret_cast<uint8_t *>(p.afp16), p.asf, p.arow_scale, p.tile_expert, p.groups.tile_rows };
     const int * tiles = p.groups.cost + 3 * (n_as + 1);
     if (src_stride == 0) src_stride = k;
     if (src && (((uintptr_t) src & 15) || src_stride % 4)) return fail(ctx, B200MOE_ERR_INVALID_ARG, "fp32 activation rows must be 16-byte aligned");
     const int rows_per_block = 256 / std::min(256, k / 8);
-    const unsigned blocks = (unsigned) ((rows + rows_per_block - 1) / rows_per_block);
-    if (src) act_planes_kernel<true><<<blocks, 256, 0, st>>>(act, src, src_stride, p.groups.perm, ids, p.groups.offsets, tiles, p.groups.meta, rows, k, n_ids, ne11, n_as, po, emit);
-    else act_planes_kernel<false><<<blocks, 256, 0, st>>>(act, nullptr, 0, p.groups.perm, ids, p.groups.offsets, tiles, p.groups.meta, rows, k, n_ids, ne11, n_as, po, ActQuant{});
+    const int act_rows = rows / n_ids * ne11;
+    const unsigned blocks = (unsigned) ((act_rows + rows_per_block - 1) / rows_per_block);
+    if (src) act_planes_kernel<true><<<blocks, 256, 0, st>>>(act, src, src_stride, p.groups.pos, ids, p.groups.offsets, tiles, act_rows, k, n_ids, ne11, n_as, po, emit);
+    else act_planes_kernel<false><<<blocks, 256, 0, st>>>(act, nullptr, 0, p.groups.pos, ids, p.groups.offsets, tiles, act_rows, k, n_ids, ne11, n_as, po, ActQuant{});
     return check_launch(ctx, "act_planes");
 }
 
@@ -624,7 +627,7 @@ Fp4Params fp4_params(b200moe_ctx * ctx, const float * s0, const float * s1, floa
     Plan & p = ctx->plan;
     Fp4Params f{};
     f.scale0 = s0; f.scale1 = s1; f.sf = p.asf; f.row_scale = p.arow_scale; f.offsets = p.groups.offsets; f.perm = p.groups.perm;
-    f.active = p.groups.active; f.meta = p.groups.meta; f.tile_of_expert = p.groups.cost + 3 * (n_as + 1); f.tile_expert = p.groups.pos; f.out = out; f.n_out = n_out;
+    f.active = p.groups.active; f.meta = p.groups.meta; f.tile_of_expert = p.groups.cost + 3 * (n_as + 1); f.tile_expert = p.tile_expert; f.out = out; f.n_out = n_out;
     f.n_as = n_as; f.err = ctx->d_err; f.prof = nullptr;
     return f;
 }

@@ -115,11 +115,10 @@ struct PlaneOut {
     int       rpt;          // routed rows per token tile
 };
 
-// digits, codes and scale bytes of one quad: 16-block g, bytes j0 .. j0+3 (elements 16g + j and 16g + j + 8) with int8 values lo[], hi[]
-// and the fp32 bits of the block scale d (an fp16 number: d = M * 2^(exp8 - 137) with M the top 11 bits of the significand).
-// The four code bytes of every plane leave as one 32-bit store.
-__device__ __forceinline__ void plane_quad(const int (&lo)[4], const int (&hi)[4], uint32_t dbits, int E_row, int g, int j0, int K, int in_tile,
-                                           int sfb_bytes, uint8_t * __restrict__ prow, uint8_t * __restrict__ sft) {
+// digits and codes of one quad: 16-block g, bytes j0 .. j0+3 (elements 16g + j and 16g + j + 8) with int8 values lo[], hi[] and the
+// fp32 bits of the block scale d (an fp16 number: d = M * 2^(exp8 - 137) with M the top 11 bits of the significand).  words[p]: the
+// four code bytes of plane p; returned: the UE4M3 byte of the block's scale.
+__device__ __forceinline__ uint8_t plane_quad(const int (&lo)[4], const int (&hi)[4], uint32_t dbits, int E_row, uint32_t (&words)[FP4_PLANES]) {
     const bool nz = (dbits & 0x7fffffffu) != 0;
     const int M = nz ? (int) (((dbits & 0x7fffffu) | 0x800000u) >> 13) : 0;
     const int s = nz ? (int) ((dbits >> 23) & 0xff) - 137 - E_row + 8 : -100;           // scale exponent, at most 8
@@ -127,7 +126,6 @@ __device__ __forceinline__ void plane_quad(const int (&lo)[4], const int (&hi)[4
     int p0[4], p1[4];
 #pragma unroll
     for (int m = 0; m < 4; ++m) { p0[m] = lo[m] * Ms; p1[m] = hi[m] * Ms; }
-    uint32_t * pw = reinterpret_cast<uint32_t *>(prow + 8 * g + j0);
     // Balanced radix-8 digits, lowest first: digit = ((p + 4) & 7) - 4 and carry (p + 4) >> 3.  The digit's E2M1 code comes from
     // a table indexed by p & 7 (residues 0..3 are the digits 0..3, residues 4..7 the digits -4..-1): codes 0,2,4,5 and, with the
     // sign bit, E,D,C,A.  The top plane takes what is left (|p| <= 4) through the magnitude table 0,2,4,5,6.
@@ -148,52 +146,48 @@ __device__ __forceinline__ void plane_quad(const int (&lo)[4], const int (&hi)[4
             }
             word |= (c0 | (c1 << 4)) << (8 * m);
         }
-        pw[(size_t) p * (K / 8)] = word;
+        words[p] = word;
     }
-    if (j0 == 0) {
-        // UE4M3 byte of 2^s: normal for s >= -6, the three power-of-two subnormals below, zero when flushed
-        const uint32_t sb = s >= -6 ? (uint32_t) (s + 7) << 3 : s == -7 ? 4u : s == -8 ? 2u : s == -9 ? 1u : 0u;
-        uint8_t * dst = sft + (size_t) (g >> 4) * sfb_bytes + ((g >> 2) & 3) * (sfb_bytes / 4) + (g & 3);
-#pragma unroll
-        for (int p = 0; p < FP4_PLANES; ++p) {
-            const int n = in_tile * FP4_PLANES + p;
-            dst[(n >> 7) * 512 + sf_tile_offset(n & 127)] = (uint8_t) sb;
-        }
-    }
+    // normal for s >= -6, the three power-of-two subnormals below, zero when flushed
+    return (uint8_t) (s >= -6 ? (uint32_t) (s + 7) << 3 : s == -7 ? 4u : s == -8 ? 2u : s == -9 ? 1u : 0u);
 }
 
-// K / 8 threads per expert-sorted routed row (at most 256: a block holds 256 * 8 / K rows, and a thread two quads when K = 4096).
+// K / 8 threads per ACTIVATION row (at most 256: a block holds 256 * 8 / K rows, and a thread two quads when K = 4096).  The digits of
+// a row are worked out once and stored for each of the n_ids / ne11 routed rows that read it (gate/up: the k experts of a token).
 // SRC_F32 = false: the row's activations are already quantised (ActQuant planes, Q8_0).
 // SRC_F32 = true: they are fp32 (`src`, rows `src_stride` floats apart) and are quantised here exactly as quantize_q8_0_block
 // does it (d = half(amax / 127), q = rint(v * (127 / amax))), which saves the separate quantisation pass; `emit`, when it has
 // planes, receives that quantised form as well (row index as in `src`).
+// Bound by the stores: 3.5 bytes per routed value.
 template <bool SRC_F32>
 __global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const float * __restrict__ src, int64_t src_stride,
-                                                        const int * __restrict__ perm, const int32_t * __restrict__ ids,
+                                                        const int * __restrict__ pos, const int32_t * __restrict__ ids,
                                                         const int * __restrict__ offsets, const int * __restrict__ tile_of_expert,
-                                                        const int * __restrict__ meta, int rows, int K, int n_ids, int ne11, int n_as,
-                                                        PlaneOut out, ActQuant emit) {
+                                                        int act_rows, int K, int n_ids, int ne11, int n_as, PlaneOut out, ActQuant emit) {
     constexpr int MAX_QUADS = 2;
     __shared__ int s_E[8];
+    __shared__ int s_at[8][32], s_tile[8][32], s_in[8][32];   // sorted position, token tile and row in it of every routed row of a block row
     const int tid = threadIdx.x, lane = tid & 31;
     const int tpr = min(256, K / 8), rpb = 256 / tpr, qpt = (K / 8) / tpr;
     const int lrow = tid / tpr, t_in = tid % tpr;
-    const int i = blockIdx.x * rpb + lrow;          // sorted position
+    const int arow = blockIdx.x * rpb + lrow;
+    const int n_dst = n_ids / ne11;
     if (tid < 8) s_E[tid] = -1000;
-    __syncthreads();
-    // meta[1]: rows that are in a group (fewer than `rows` when slots are empty); threads beyond the block's last whole row idle (K = 768)
-    const bool live = lrow < rpb && i < rows && i < meta[1];
-    int arow = 0, in_tile = 0, tile = 0;
-    if (live) {
-        const int r = perm[i];
-        arow = (r / n_ids) * ne11 + (r % n_ids) % ne11;
-        int e = ids[r];
-        e = e < 0 ? 0 : (e >= n_as ? n_as - 1 : e);    // bad ids were reported by the grouping kernels; stay inside the tables
-        const int row_beg = offsets[e];
-        in_tile = (i - row_beg) % out.rpt;
-        tile = tile_of_expert[e] + (i - row_beg) / out.rpt;
-        if (in_tile == 0 && t_in == 0) out.tile_expert[tile] = e;
+    const bool live = lrow < rpb && arow < act_rows;   // threads beyond the block's last whole row idle (K = 768)
+    if (live && t_in < n_dst) {
+        const int r = (arow / ne11) * n_ids + arow % ne11 + ne11 * t_in;
+        const int e = ids[r];
+        int at = -1, tile = 0, in_tile = 0;            // an id of -1 is an empty slot; other bad ids were reported by the grouping kernels
+        if (e >= 0 && e < n_as) {
+            const int in_e = pos[r];
+            at = offsets[e] + in_e;
+            tile = tile_of_expert[e] + in_e / out.rpt;
+            in_tile = in_e % out.rpt;
+            if (in_tile == 0) out.tile_expert[tile] = e;
+        }
+        s_at[lrow][t_in] = at; s_tile[lrow][t_in] = tile; s_in[lrow][t_in] = in_tile;
     }
+    __syncthreads();
     const int nb32 = K / 32;
     int lo[MAX_QUADS][4], hi[MAX_QUADS][4];
     uint32_t db[MAX_QUADS];
@@ -251,15 +245,28 @@ __global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const flo
     __syncthreads();
     if (!live) return;
     const int E_row = s_E[lrow];
-    if (t_in == 0) out.row_scale[i] = E_row > -1000 ? __uint_as_float((uint32_t) (E_row - 8 + 127) << 23) : 0.0f;   // 2^(E_row - 8): far from the fp32 limits
-    uint8_t * prow = out.planes + (size_t) i * FP4_PLANES * (K / 2);
+    if (t_in < n_dst && s_at[lrow][t_in] >= 0)
+        out.row_scale[s_at[lrow][t_in]] = E_row > -1000 ? __uint_as_float((uint32_t) (E_row - 8 + 127) << 23) : 0.0f;   // 2^(E_row - 8): far from the fp32 limits
     const int sfb_bytes = fp4_sfb_bytes(out.rpt);
-    uint8_t * sft = out.sf + (size_t) tile * (K / 256) * sfb_bytes;
 #pragma unroll
     for (int u = 0; u < MAX_QUADS; ++u)
         if (u < qpt) {
-            const int qd = t_in + tpr * u;
-            plane_quad(lo[u], hi[u], db[u], E_row, qd >> 1, (qd & 1) * 4, K, in_tile, sfb_bytes, prow, sft);
+            const int qd = t_in + tpr * u, g = qd >> 1;
+            uint32_t words[FP4_PLANES];
+            const uint8_t sb = plane_quad(lo[u], hi[u], db[u], E_row, words);
+            for (int j = 0; j < n_dst; ++j) {
+                const int at = s_at[lrow][j];
+                if (at < 0) continue;
+                uint32_t * pw = reinterpret_cast<uint32_t *>(out.planes + (size_t) at * FP4_PLANES * (K / 2)) + qd;
+#pragma unroll
+                for (int p = 0; p < FP4_PLANES; ++p) pw[(size_t) p * (K / 8)] = words[p];
+                if ((qd & 1) == 0) {
+                    uint8_t * dst = out.sf + ((size_t) s_tile[lrow][j] * (K / 256) + (g >> 4)) * sfb_bytes + ((g >> 2) & 3) * (sfb_bytes / 4) + (g & 3);
+                    const int n0 = s_in[lrow][j] * FP4_PLANES;
+#pragma unroll
+                    for (int p = 0; p < FP4_PLANES; ++p) dst[((n0 + p) >> 7) * 512 + sf_tile_offset((n0 + p) & 127)] = sb;
+                }
+            }
         }
 }
 

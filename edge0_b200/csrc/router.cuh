@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(256) one_group_kernel(Groups g, int32_t * __re
     pdl_wait();
     pdl_launch_dependents();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < T) { ids[t] = 0; g.perm[t] = t; }
+    if (t < T) { ids[t] = 0; g.perm[t] = t; g.pos[t] = t; }
     if (t == 0) {
         g.counts[0] = T;
         g.offsets[0] = 0; g.offsets[1] = T;
