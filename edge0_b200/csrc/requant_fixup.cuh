@@ -56,10 +56,10 @@ __global__ void __launch_bounds__(256) requant_mark_kernel(const float * __restr
     pdl_launch_dependents();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     const int chunks = n_ff / 128;
-    if (warp >= rows * chunks || warp % rows >= meta[1]) return;
-    const int c = warp / rows, r = perm[warp % rows];
+    const bool live = warp < rows * chunks && warp % rows < meta[1];     // the whole block meets at the barriers below
+    const int c = live ? warp / rows : 0, r = live ? perm[warp % rows] : 0;
     const int f0 = c * 128 + lane * 4;
-    const float4 v4 = *reinterpret_cast<const float4 *>(hid + (size_t) r * n_ff + f0);
+    const float4 v4 = live ? *reinterpret_cast<const float4 *>(hid + (size_t) r * n_ff + f0) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     const float a[4] = { fabsf(v4.x), fabsf(v4.y), fabsf(v4.z), fabsf(v4.w) };
     float amax = fmaxf(fmaxf(a[0], a[1]), fmaxf(a[2], a[3]));
 #pragma unroll
@@ -89,16 +89,26 @@ __global__ void __launch_bounds__(256) requant_mark_kernel(const float * __restr
         const int up = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += up;
     }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    if (total == 0) return;
-    int base = 0;
-    if (lane == 0) {
-        base = atomicAdd(list.count, total);
-        const int over = base + total - max(base, list.capacity);
-        if (over > 0 && list.overflow) atomicAdd(list.overflow, (unsigned long long) over);
+    // one atomic per block: with one per warp the counter's line was what the kernel waited for
+    __shared__ int s_total[8], s_base;
+    const int wib = threadIdx.x >> 5;
+    if (lane == 31) s_total[wib] = incl;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int total = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) total += s_total[w];
+        int base = 0;
+        if (total) {
+            base = atomicAdd(list.count, total);
+            const int over = base + total - max(base, list.capacity);
+            if (over > 0 && list.overflow) atomicAdd(list.overflow, (unsigned long long) over);
+        }
+        s_base = base;
     }
-    base = __shfl_sync(0xffffffffu, base, 0);
-    int slot = base + incl - n_mine;
+    __syncthreads();
+    int slot = s_base + incl - n_mine;
+    for (int w = 0; w < wib; ++w) slot += s_total[w];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
         if (risky[j]) {
