@@ -656,37 +656,49 @@ int launch_quantize(b200moe_ctx * ctx, const XT * src, int64_t stride, ActQuant 
     return check_launch(ctx, "quantize_act");
 }
 
-template <int WE, int WT, typename XT>
+// quant.q != null: further blocks quantise x on the way (kind as in quantize_act_kernel)
+template <int WE, int WT, int RT, typename XT>
 int launch_logits_smem(b200moe_ctx * ctx, const float * w, const float * bias, const XT * x, float * logits, int H, int E, int T, int * zero_buf,
-                       int zero_n, cudaStream_t st) {
-    auto kern = router_logits_smem_kernel<WE, WT, XT>;
-    constexpr size_t smem = router_smem_bytes<WE, WT, XT>();
+                       int zero_n, ActQuant quant, int kind, cudaStream_t st) {
+    auto kern = router_logits_smem_kernel<WE, WT, RT, XT>;
+    constexpr size_t smem = router_smem_bytes<WE, WT, RT, XT>();
     static bool configured[MAX_DEVICE_ORDINALS] = {};
     if (int rc = raise_smem_limit(ctx, kern, smem, configured)) return rc;
-    const int blocks = ((E + 8 * WE - 1) / (8 * WE)) * ((T + 8 * WT - 1) / (8 * WT));
-    kern<<<blocks, WE * WT * 32, smem, st>>>(w, bias, x, logits, H, E, T, zero_buf, zero_n);
+    const int blocks = ((E + 8 * WE - 1) / (8 * WE)) * ((T + RT * WT - 1) / (RT * WT));
+    // few blocks that loop: each holds the shared memory of a tile, and thousands of short ones took twice the time of the logits
+    const int qblocks = quant.q ? (int) std::min<int64_t>(2 * ctx->sm_count, ((int64_t) T * (H / (kind ? 256 : 32)) + WE * WT - 1) / (WE * WT)) : 0;
+    launch_k(ctx, kern, dim3(blocks + qblocks), dim3(WE * WT * 32), smem, st, w, bias, x, logits, H, E, T, zero_buf, zero_n, blocks, quant, kind);
     return check_launch(ctx, "router_logits");
 }
 
 // F32 matrix times a batch in the reference's summation order: logits [T][E] = W [E][H] . x [T][H] (+ bias)
 template <typename XT>
 int launch_logits_any(b200moe_ctx * ctx, const float * w, const float * bias, const XT * x, float * logits, int H, int E, int T, int * zero_buf,
-                      int zero_n, cudaStream_t st) {
-    const bool staged = T >= 16 && H % ROUTER_KC == 0 && (((uintptr_t) w | (uintptr_t) x) & 15) == 0;
-    if (staged) {   // shared-memory tiles: 32 experts x 16 tokens when that fills the GPU, else 16 x 8
+                      int zero_n, cudaStream_t st, ActQuant quant = ActQuant{}, int kind = 0) {
+    const bool staged = T >= 16 && E >= 8 && H % ROUTER_KC == 0 && (((uintptr_t) w | (uintptr_t) x) & 15) == 0;
+    if (staged) {
+        // shared-memory tiles: 32 experts x 16 tokens (8 warps) when there are two of them per SM, else 16 x 8 (4 warps)
         const int big = ((E + 31) / 32) * ((T + 15) / 16);
-        if (big >= ctx->sm_count) return launch_logits_smem<4, 2, XT>(ctx, w, bias, x, logits, H, E, T, zero_buf, zero_n, st);
-        return launch_logits_smem<2, 1, XT>(ctx, w, bias, x, logits, H, E, T, zero_buf, zero_n, st);
+        if (big >= 2 * ctx->sm_count) return launch_logits_smem<4, 2, 8, XT>(ctx, w, bias, x, logits, H, E, T, zero_buf, zero_n, quant, kind, st);
+        return launch_logits_smem<2, 2, 4, XT>(ctx, w, bias, x, logits, H, E, T, zero_buf, zero_n, quant, kind, st);
     }
-    if (T >= 16) {   // batches: 4 experts x 8 tokens per warp
+    // few tokens or a single row: one warp per (expert, token) with deep load prefetch; otherwise 4 tokens share each weight load
+    const int tt = T <= 8 || E < 8 ? 1 : 4;
+    const int lblocks = (int) (((int64_t) E * ((T + tt - 1) / tt) + 7) / 8);
+    if (quant.q) {
+        const int qblocks = (int) (((int64_t) T * (H / (kind ? 256 : 32)) + 7) / 8);
+        if (tt == 1) launch_k(ctx, route_front_kernel<1, XT>, dim3(lblocks + qblocks), dim3(256), 0, st, w, bias, x, logits, H, E, T, zero_buf, zero_n, lblocks, quant, kind);
+        else launch_k(ctx, route_front_kernel<4, XT>, dim3(lblocks + qblocks), dim3(256), 0, st, w, bias, x, logits, H, E, T, zero_buf, zero_n, lblocks, quant, kind);
+        return check_launch(ctx, "route_front");
+    }
+    if (T >= 16 && E >= 8) {   // batches whose rows cannot be staged: 4 experts x 8 tokens per warp
         constexpr int TE = 4, TT = 8;
         const int64_t warps = (int64_t) ((E + TE - 1) / TE) * ((T + TT - 1) / TT);
         router_logits_tiled_kernel<TE, TT, XT><<<(unsigned) ((warps * 32 + 255) / 256), 256, 0, st>>>(w, bias, x, logits, H, E, T, zero_buf, zero_n);
         return check_launch(ctx, "router_logits");
     }
-    constexpr int TT = 4;
-    const int64_t warps = (int64_t) E * ((T + TT - 1) / TT);
-    router_logits_kernel<TT, XT><<<(unsigned) ((warps * 32 + 255) / 256), 256, 0, st>>>(w, bias, x, logits, H, E, T, zero_buf, zero_n);
+    if (tt == 1) launch_k(ctx, router_logits_kernel<1, XT>, dim3(lblocks), dim3(256), 0, st, w, bias, x, logits, H, E, T, zero_buf, zero_n);
+    else launch_k(ctx, router_logits_kernel<4, XT>, dim3(lblocks), dim3(256), 0, st, w, bias, x, logits, H, E, T, zero_buf, zero_n);
     return check_launch(ctx, "router_logits");
 }
 
@@ -696,23 +708,12 @@ int launch_logits(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int 
     return launch_logits_any<XT>(ctx, l->router_w, l->router_bias, x, p.logits, l->n_embd, l->n_expert, T, p.groups.counts, l->n_expert, st);
 }
 
-template <int TT, typename XT>
-int launch_front_t(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T, cudaStream_t st) {
-    Plan & p = ctx->plan;
-    const int64_t lwarps = (int64_t) l->n_expert * ((T + TT - 1) / TT);
-    const int lblocks = (int) ((lwarps * 32 + 255) / 256);
-    const int kind = l->wtype == TYPE_Q3_K ? 1 : 0;
-    const int64_t qwarps = (int64_t) T * (kind ? l->n_embd / 256 : l->n_embd / 32);
-    const int qblocks = (int) ((qwarps * 32 + 255) / 256);
-    launch_k(ctx, route_front_kernel<TT, XT>, dim3(lblocks + qblocks), dim3(256), 0, st, l->router_w, l->router_bias, x, p.logits, l->n_embd,
-             l->n_expert, T, p.groups.counts, l->n_expert, lblocks, p.xq, kind);
-    return check_launch(ctx, "route_front");
-}
-
+// router logits, and the activations quantised into the plan's xq by further blocks of the same launch
 template <typename XT>
 int launch_front(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T, cudaStream_t st) {
-    // few tokens: one warp per (expert, token) with deep load prefetch; otherwise 4 tokens share each weight load
-    return T <= 8 ? launch_front_t<1, XT>(ctx, l, x, T, st) : launch_front_t<4, XT>(ctx, l, x, T, st);
+    Plan & p = ctx->plan;
+    return launch_logits_any<XT>(ctx, l->router_w, l->router_bias, x, p.logits, l->n_embd, l->n_expert, T, p.groups.counts, l->n_expert, st, p.xq,
+                                 l->wtype == TYPE_Q3_K ? 1 : 0);
 }
 
 // Routed rows per token tile of the FP4 kernels for `rows` rows in up to n_groups groups; kept in the plan from the grouping to the
@@ -1146,10 +1147,7 @@ int shared_expert_impl(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x,
         xf32 = p.xf;
     }
     // logit of the gate: the reference's F32 dot product, lane chains as in the router
-    constexpr int TT = 4;
-    const int64_t warps = (T + TT - 1) / TT;
-    router_logits_kernel<TT, float><<<(unsigned) ((warps * 32 + 255) / 256), 256, 0, st>>>(l->gate_inp_shexp, nullptr, xf32, p.sh_gate, H, 1, T, nullptr, 0);
-    if ((rc = check_launch(ctx, "shexp_gate_logit"))) return rc;
+    if ((rc = launch_logits_any<float>(ctx, l->gate_inp_shexp, nullptr, xf32, p.sh_gate, H, 1, T, nullptr, 0, st))) return rc;
     if ((rc = dense_matvec(ctx, l->wtype, l->gate_shexp, nullptr, xf32, p.xq, H, Is, T, p.sh_a, st, false, l->up_shexp, p.sh_b))) return rc;
     if ((rc = dense_matvec(ctx, l->wtype, l->down_shexp, nullptr, p.sh_a, p.shq, Is, H, T, p.sh_out, st))) return rc;
     dim3 grid((H + 255) / 256, T);
@@ -1162,8 +1160,8 @@ int layer_impl(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T, 
     Plan & p = ctx->plan;
     const int k = l->n_expert_used;
     int rc;
-    const bool fused_front = !l->n_latent && T <= 128;  // decode-sized batches: 2 launches instead of 4
-    if (fused_front) {
+    if (!l->n_latent) {   // x feeds the experts: quantised in the router's launch
+
         if ((rc = launch_front<XT>(ctx, l, x, T, st))) return rc;
         float * probs = (ob && ob->ffn_moe_probs) ? ob->ffn_moe_probs : nullptr;
         if (T <= 32) {   // one warp per token fits one block: selection and grouping in a single launch
@@ -1176,14 +1174,12 @@ int layer_impl(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T, 
             CUDA_TRY(ctx, cudaMemcpyAsync(ob->ffn_moe_logits, p.logits, sizeof(float) * (size_t) T * l->n_expert, cudaMemcpyDeviceToDevice, st));
     } else {
         if ((rc = route_impl<XT>(ctx, l, x, T, p.ids, p.wts, ob, true, st))) return rc;
-        if (!l->n_latent && (rc = launch_group(ctx, p.ids, l->n_expert, T * k, st))) return rc;
     }
     if (ob && ob->ffn_moe_topk) CUDA_TRY(ctx, cudaMemcpyAsync(ob->ffn_moe_topk, p.ids, sizeof(int32_t) * (size_t) T * k, cudaMemcpyDeviceToDevice, st));
     if (ob && ob->ffn_moe_weights_norm)
         CUDA_TRY(ctx, cudaMemcpyAsync(ob->ffn_moe_weights_norm, p.wts, sizeof(float) * (size_t) T * k, cudaMemcpyDeviceToDevice, st));
 
     if (!l->n_latent) {
-        if (!fused_front && (rc = launch_quantize<XT>(ctx, x, l->n_embd, p.xq, T, l->n_embd, l->wtype, st))) return rc;
         rc = experts_impl(ctx, l, p.xq, p.ids, p.wts, T, out, ob, st);
         if (!rc && l->gate_shexp) rc = shared_expert_impl<XT>(ctx, l, x, T, out, ob, st);
         account(ctx, l, T);

@@ -25,35 +25,37 @@ struct ActQuant {
 // i.e. chain i%32, with FMAs in increasing i.  The cross-chain reduction follows GGML_F32x8_REDUCE:
 // (a0+a2),(a1+a3) -> sum -> lanes j+(j+4) -> two horizontal adds.
 template <int TT, typename XT>
-__global__ void __launch_bounds__(256) router_logits_kernel(const float * __restrict__ W, const float * __restrict__ bias,
-                                                           const XT * __restrict__ x, float * __restrict__ logits, int H,
-                                                           int E, int T, int * __restrict__ zero_buf, int zero_n) {
-    pdl_wait();
-    pdl_launch_dependents();
-
-    // block 0 also clears the per-expert counters the selection kernel accumulates into
-    if (blockIdx.x == 0)
-        for (int i = threadIdx.x; i < zero_n; i += blockDim.x) zero_buf[i] = 0;
-
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+__device__ __forceinline__ void router_warp(const float * __restrict__ W, const float * __restrict__ bias, const XT * __restrict__ x,
+                                            float * __restrict__ logits, int H, int E, int T, int warp, int lane) {
     const int n_tt = (T + TT - 1) / TT;
     if (warp >= E * n_tt) return;
     const int e = warp % E;
     const int t0 = (warp / E) * TT;
-
     float acc[TT];
 #pragma unroll
     for (int i = 0; i < TT; ++i) acc[i] = 0.0f;
     const float * w = W + (size_t) e * H;
-    for (int j = lane; j < H; j += 32) {
-        const float wv = __ldg(w + j);
+    // The FMA chain of a lane is sequential by definition of the reference's order, but its loads are not:
+    // fetch CH steps of weights and activations at once, then run the chain over them.
+    constexpr int CH = TT == 1 ? 32 : 8;
+    for (int j0 = lane; j0 < H; j0 += 32 * CH) {
+        float wv[CH], xv[TT][CH];
 #pragma unroll
-        for (int i = 0; i < TT; ++i) {
-            const int t = min(t0 + i, T - 1);
-            const float xv = (float) x[(size_t) t * H + j];
-            acc[i] = __fmaf_rn(wv, xv, acc[i]);
+        for (int c = 0; c < CH; ++c) {
+            const int j = j0 + 32 * c;
+            wv[c] = j < H ? __ldg(w + j) : 0.0f;
+#pragma unroll
+            for (int i = 0; i < TT; ++i) {
+                const int t = min(t0 + i, T - 1);
+                xv[i][c] = j < H ? (float) x[(size_t) t * H + j] : 0.0f;
+            }
         }
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+            if (j0 + 32 * c < H) {
+#pragma unroll
+                for (int i = 0; i < TT; ++i) acc[i] = __fmaf_rn(wv[c], xv[i][c], acc[i]);
+            }
     }
 #pragma unroll
     for (int i = 0; i < TT; ++i) {
@@ -68,6 +70,19 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const float * __rest
             logits[(size_t) (t0 + i) * E + e] = v;
         }
     }
+}
+
+template <int TT, typename XT>
+__global__ void __launch_bounds__(256) router_logits_kernel(const float * __restrict__ W, const float * __restrict__ bias,
+                                                           const XT * __restrict__ x, float * __restrict__ logits, int H,
+                                                           int E, int T, int * __restrict__ zero_buf, int zero_n) {
+    pdl_wait();
+    pdl_launch_dependents();
+
+    // block 0 also clears the per-expert counters the selection kernel accumulates into
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < zero_n; i += blockDim.x) zero_buf[i] = 0;
+    router_warp<TT, XT>(W, bias, x, logits, H, E, T, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, threadIdx.x & 31);
 }
 
 // Register-tiled form for batches: one warp per (TE experts x TT tokens).  Every (expert, token) pair still runs the reference's
@@ -122,99 +137,6 @@ __global__ void __launch_bounds__(256) router_logits_tiled_kernel(const float * 
             if (lane == 0 && e0 + a < E && t0 + b < T) {
                 if (bias) v = __fadd_rn(v, bias[e0 + a]);
                 logits[(size_t) (t0 + b) * E + e0 + a] = v;
-            }
-        }
-}
-
-// Shared-memory form for larger batches: a block owns (8 WE experts) x (8 WT tokens); weight and activation rows arrive in
-// 128-element pieces through a three-deep cp.async ring, and every warp runs an 8 x 8 register tile out of shared memory.  The
-// chains are the reference's (lane l owns elements l, l + 32, ... in increasing order), so the logits keep its bits; what changes is
-// that global loads are 16 bytes wide, issued two pieces ahead, and shared by the whole tile.
-// Needs H to be a multiple of 128 and 16-byte aligned rows.
-constexpr int ROUTER_KC = 128, ROUTER_ST = 3;
-template <int WE, int WT, typename XT>
-constexpr size_t router_smem_bytes() { return (size_t) ROUTER_ST * ROUTER_KC * (8 * WE * sizeof(float) + 8 * WT * sizeof(XT)); }
-
-__device__ __forceinline__ void cp_async16(void * smem, const void * gmem) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t) __cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-template <int WE, int WT, typename XT>
-__global__ void __launch_bounds__(WE * WT * 32) router_logits_smem_kernel(const float * __restrict__ W, const float * __restrict__ bias,
-                                                                         const XT * __restrict__ x, float * __restrict__ logits, int H, int E, int T,
-                                                                         int * __restrict__ zero_buf, int zero_n) {
-    constexpr int EB = 8 * WE, TB = 8 * WT, KC = ROUTER_KC, ST = ROUTER_ST, NTHR = WE * WT * 32;
-    constexpr int XP = 16 / sizeof(XT);   // activation elements per 16-byte piece
-    extern __shared__ __align__(16) uint8_t router_smem[];
-    float (*ws)[EB][KC] = reinterpret_cast<float (*)[EB][KC]>(router_smem);
-    XT (*xs)[TB][KC] = reinterpret_cast<XT (*)[TB][KC]>(router_smem + (size_t) ST * EB * KC * sizeof(float));
-    pdl_wait();
-    pdl_launch_dependents();
-    if (blockIdx.x == 0)
-        for (int i = threadIdx.x; i < zero_n; i += NTHR) zero_buf[i] = 0;
-    const int n_eb = (E + EB - 1) / EB;
-    const int e0 = (blockIdx.x % n_eb) * EB, t0 = (blockIdx.x / n_eb) * TB;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int we = (warp % WE) * 8, wt = (warp / WE) * 8;
-    const int n_chunks = H / KC;
-
-    auto load_chunk = [&](int c) {
-        const int s = c % ST;
-        for (int i = threadIdx.x; i < EB * (KC / 4); i += NTHR) {
-            const int r = i / (KC / 4), q = i % (KC / 4);
-            cp_async16(&ws[s][r][q * 4], W + (size_t) min(e0 + r, E - 1) * H + (size_t) c * KC + q * 4);
-        }
-        for (int i = threadIdx.x; i < TB * (KC / XP); i += NTHR) {
-            const int r = i / (KC / XP), q = i % (KC / XP);
-            cp_async16(&xs[s][r][q * XP], x + (size_t) min(t0 + r, T - 1) * H + (size_t) c * KC + q * XP);
-        }
-    };
-    float acc[8][8];
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-        for (int b = 0; b < 8; ++b) acc[a][b] = 0.0f;
-#pragma unroll
-    for (int c = 0; c < ST - 1; ++c) {
-        if (c < n_chunks) load_chunk(c);
-        cp_async_commit();
-    }
-    for (int c = 0; c < n_chunks; ++c) {
-        cp_async_wait<ST - 2>();   // piece c has landed (one younger group may still be in flight)
-        __syncthreads();           // ... for every thread, and everybody is done with the stage the next load overwrites
-        if (c + ST - 1 < n_chunks) load_chunk(c + ST - 1);
-        cp_async_commit();
-        const int s = c % ST;
-#pragma unroll
-        for (int kk = 0; kk < KC / 32; ++kk) {
-            float wv[8], xv[8];
-#pragma unroll
-            for (int a = 0; a < 8; ++a) wv[a] = ws[s][we + a][kk * 32 + lane];
-#pragma unroll
-            for (int b = 0; b < 8; ++b) xv[b] = (float) xs[s][wt + b][kk * 32 + lane];
-#pragma unroll
-            for (int a = 0; a < 8; ++a)
-#pragma unroll
-                for (int b = 0; b < 8; ++b) acc[a][b] = __fmaf_rn(wv[a], xv[b], acc[a][b]);
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < 8; ++a)
-#pragma unroll
-        for (int b = 0; b < 8; ++b) {
-            float v = acc[a][b];
-            v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 16));
-            v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 8));
-            v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 4));
-            v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
-            v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 2));
-            const int e = e0 + we + a, t = t0 + wt + b;
-            if (lane == 0 && e < E && t < T) {
-                if (bias) v = __fadd_rn(v, bias[e]);
-                logits[(size_t) t * E + e] = v;
             }
         }
 }
@@ -303,7 +225,18 @@ __global__ void __launch_bounds__(256) quantize_act_kernel(const XT * __restrict
     }
 }
 
-// Router logits and activation quantisation in one launch (decode path): blocks [0, n_logit_blocks) compute logits,
+// The warps of the quantising blocks share the activation blocks of the expert matmuls (kind: 0 = Q8_0, 1 = Q8_K) in strides.
+template <typename XT>
+__device__ __forceinline__ void quantize_warps(const XT * __restrict__ x, const ActQuant & dst, int H, int T, int kind, int warp, int n_warps, int lane) {
+    const int nb = H / (kind ? 256 : 32);
+    for (int i = warp; i < T * nb; i += n_warps) {
+        const int r = i / nb, b = i % nb;
+        if (kind == 0) quantize_q8_0_block(x + (size_t) r * H + b * 32, dst.q + (size_t) r * H + b * 32, dst.d + (size_t) r * nb + b, lane);
+        else quantize_q8_K_block(x + (size_t) r * H + b * 256, dst.q + (size_t) r * H + b * 256, dst.d + (size_t) r * nb + b, dst.bsum + (size_t) r * (H / 16) + b * 16, lane);
+    }
+}
+
+// Router logits and activation quantisation in one launch (few tokens): blocks [0, n_logit_blocks) compute logits,
 // the rest quantise x for the expert matmuls.  Both only read x.
 template <int TT, typename XT>
 __global__ void __launch_bounds__(256) route_front_kernel(const float * __restrict__ W, const float * __restrict__ bias,
@@ -313,70 +246,114 @@ __global__ void __launch_bounds__(256) route_front_kernel(const float * __restri
     pdl_wait();
     pdl_launch_dependents();
 
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if ((int) blockIdx.x < n_logit_blocks) {
         if (blockIdx.x == 0)
             for (int i = threadIdx.x; i < zero_n; i += blockDim.x) zero_buf[i] = 0;
-        const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-        const int lane = threadIdx.x & 31;
-        const int n_tt = (T + TT - 1) / TT;
-        if (warp >= E * n_tt) return;
-        const int e = warp % E;
-        const int t0 = (warp / E) * TT;
-        float acc[TT];
-#pragma unroll
-        for (int i = 0; i < TT; ++i) acc[i] = 0.0f;
-        const float * w = W + (size_t) e * H;
-        // The FMA chain of a lane is sequential by definition of the reference's order, but its loads are not:
-        // fetch CH steps of weights and activations at once, then run the chain over them.
-        constexpr int CH = TT == 1 ? 32 : 8;
-        for (int j0 = lane; j0 < H; j0 += 32 * CH) {
-            float wv[CH], xv[TT][CH];
-#pragma unroll
-            for (int c = 0; c < CH; ++c) {
-                const int j = j0 + 32 * c;
-                wv[c] = j < H ? __ldg(w + j) : 0.0f;
-#pragma unroll
-                for (int i = 0; i < TT; ++i) {
-                    const int t = min(t0 + i, T - 1);
-                    xv[i][c] = j < H ? (float) x[(size_t) t * H + j] : 0.0f;
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < CH; ++c)
-                if (j0 + 32 * c < H) {
-#pragma unroll
-                    for (int i = 0; i < TT; ++i) acc[i] = __fmaf_rn(wv[c], xv[i][c], acc[i]);
-                }
+        router_warp<TT, XT>(W, bias, x, logits, H, E, T, (int) blockIdx.x * 8 + wib, lane);
+        return;
+    }
+    quantize_warps<XT>(x, dst, H, T, kind, ((int) blockIdx.x - n_logit_blocks) * 8 + wib, ((int) gridDim.x - n_logit_blocks) * 8, lane);
+}
+
+// Shared-memory form for larger batches: a block owns (8 WE experts) x (RT WT tokens); weight and activation rows arrive in
+// 128-element pieces through a three-deep cp.async ring, and every warp runs an 8 x RT register tile out of shared memory.  Blocks from
+// n_logit_blocks on quantise x for the expert matmuls instead (dst.q null: there are none).  The
+// chains are the reference's (lane l owns elements l, l + 32, ... in increasing order), so the logits keep its bits; what changes is
+// that global loads are 16 bytes wide, issued two pieces ahead, and shared by the whole tile.
+// Needs H to be a multiple of 128 and 16-byte aligned rows.
+constexpr int ROUTER_KC = 128, ROUTER_ST = 3;
+template <int WE, int WT, int RT, typename XT>
+constexpr size_t router_smem_bytes() { return (size_t) ROUTER_ST * ROUTER_KC * (8 * WE * sizeof(float) + RT * WT * sizeof(XT)); }
+
+__device__ __forceinline__ void cp_async16(void * smem, const void * gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t) __cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+template <int WE, int WT, int RT, typename XT>
+__global__ void __launch_bounds__(WE * WT * 32) router_logits_smem_kernel(const float * __restrict__ W, const float * __restrict__ bias,
+                                                                         const XT * __restrict__ x, float * __restrict__ logits, int H, int E, int T,
+                                                                         int * __restrict__ zero_buf, int zero_n, int n_logit_blocks, ActQuant dst,
+                                                                         int kind) {
+    constexpr int EB = 8 * WE, TB = RT * WT, KC = ROUTER_KC, ST = ROUTER_ST, NTHR = WE * WT * 32;
+    constexpr int XP = 16 / sizeof(XT);   // activation elements per 16-byte piece
+    extern __shared__ __align__(16) uint8_t router_smem[];
+    float (*ws)[EB][KC] = reinterpret_cast<float (*)[EB][KC]>(router_smem);
+    XT (*xs)[TB][KC] = reinterpret_cast<XT (*)[TB][KC]>(router_smem + (size_t) ST * EB * KC * sizeof(float));
+    pdl_wait();
+    pdl_launch_dependents();
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < zero_n; i += NTHR) zero_buf[i] = 0;
+    if ((int) blockIdx.x >= n_logit_blocks) {
+        quantize_warps<XT>(x, dst, H, T, kind, ((int) blockIdx.x - n_logit_blocks) * (NTHR / 32) + (int) (threadIdx.x >> 5),
+                           ((int) gridDim.x - n_logit_blocks) * (NTHR / 32), threadIdx.x & 31);
+        return;
+    }
+    const int n_eb = (E + EB - 1) / EB;
+    const int e0 = (blockIdx.x % n_eb) * EB, t0 = (blockIdx.x / n_eb) * TB;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int we = (warp % WE) * 8, wt = (warp / WE) * RT;
+    const int n_chunks = H / KC;
+
+    auto load_chunk = [&](int c) {
+        const int s = c % ST;
+        for (int i = threadIdx.x; i < EB * (KC / 4); i += NTHR) {
+            const int r = i / (KC / 4), q = i % (KC / 4);
+            cp_async16(&ws[s][r][q * 4], W + (size_t) min(e0 + r, E - 1) * H + (size_t) c * KC + q * 4);
         }
+        for (int i = threadIdx.x; i < TB * (KC / XP); i += NTHR) {
+            const int r = i / (KC / XP), q = i % (KC / XP);
+            cp_async16(&xs[s][r][q * XP], x + (size_t) min(t0 + r, T - 1) * H + (size_t) c * KC + q * XP);
+        }
+    };
+    float acc[8][RT];
 #pragma unroll
-        for (int i = 0; i < TT; ++i) {
-            float v = acc[i];
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+        for (int b = 0; b < RT; ++b) acc[a][b] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < ST - 1; ++c) {
+        if (c < n_chunks) load_chunk(c);
+        cp_async_commit();
+    }
+    for (int c = 0; c < n_chunks; ++c) {
+        cp_async_wait<ST - 2>();   // piece c has landed (one younger group may still be in flight)
+        __syncthreads();           // ... for every thread, and everybody is done with the stage the next load overwrites
+        if (c + ST - 1 < n_chunks) load_chunk(c + ST - 1);
+        cp_async_commit();
+        const int s = c % ST;
+#pragma unroll
+        for (int kk = 0; kk < KC / 32; ++kk) {
+            float wv[8], xv[RT];
+#pragma unroll
+            for (int a = 0; a < 8; ++a) wv[a] = ws[s][we + a][kk * 32 + lane];
+#pragma unroll
+            for (int b = 0; b < RT; ++b) xv[b] = (float) xs[s][wt + b][kk * 32 + lane];
+#pragma unroll
+            for (int a = 0; a < 8; ++a)
+#pragma unroll
+                for (int b = 0; b < RT; ++b) acc[a][b] = __fmaf_rn(wv[a], xv[b], acc[a][b]);
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+        for (int b = 0; b < RT; ++b) {
+            float v = acc[a][b];
             v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 16));
             v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 8));
             v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 4));
             v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
             v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 2));
-            if (lane == 0 && t0 + i < T) {
+            const int e = e0 + we + a, t = t0 + wt + b;
+            if (lane == 0 && e < E && t < T) {
                 if (bias) v = __fadd_rn(v, bias[e]);
-                logits[(size_t) (t0 + i) * E + e] = v;
+                logits[(size_t) t * E + e] = v;
             }
         }
-        return;
-    }
-    const int warp = (((int) blockIdx.x - n_logit_blocks) * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (kind == 0) {
-        const int nb = H / 32;
-        if (warp >= T * nb) return;
-        const int r = warp / nb, b = warp % nb;
-        quantize_q8_0_block(x + (size_t) r * H + b * 32, dst.q + (size_t) r * H + b * 32, dst.d + (size_t) r * nb + b, lane);
-    } else {
-        const int nb = H / 256;
-        if (warp >= T * nb) return;
-        const int r = warp / nb, b = warp % nb;
-        quantize_q8_K_block(x + (size_t) r * H + b * 256, dst.q + (size_t) r * H + b * 256, dst.d + (size_t) r * nb + b,
-                            dst.bsum + (size_t) r * (H / 16) + b * 16, lane);
-    }
 }
 
 // ---- K1: softmax + top-k + renormalise, one warp per token ---------------------------------------------
