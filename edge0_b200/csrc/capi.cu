@@ -307,7 +307,7 @@ int check_launch(b200moe_ctx * ctx, const char * what) {
 // ---- kernel dispatch -----------------------------------------------------------------------------------
 template <int WT, int K, bool DUAL, int NT>
 int launch_gemv_t(b200moe_ctx * ctx, const GemvParams & p, cudaStream_t st) {
-    constexpr int GEMV_STAGES = gemv_stages<WT, K, DUAL>();
+    constexpr int GEMV_STAGES = gemv_stages<WT, K, DUAL, NT>();
     constexpr size_t smem = gemv_smem_bytes<WT, K, DUAL, NT, GEMV_STAGES>();
     static_assert(smem <= 227 * 1024, "ring does not fit shared memory");
     auto kern = expert_gemv_kernel<WT, K, DUAL, NT, GEMV_STAGES>;
@@ -320,7 +320,7 @@ int launch_gemv_t(b200moe_ctx * ctx, const GemvParams & p, cudaStream_t st) {
         tm.kind = DUAL ? 0 : ctx->dense_now ? 2 : 1;
         CUDA_TRY(ctx, cudaEventRecord(tm.beg, st));
     }
-    launch_k(ctx, kern, dim3(ctx->sm_count), dim3(GemvCfg<WT, K>::NWARPS * 32), smem, st, p);
+    launch_k(ctx, kern, dim3(ctx->sm_count * gemv_ctas<WT, K, DUAL, NT>()), dim3(GemvCfg<WT, K>::NWARPS * 32), smem, st, p);
     if (ctx->timing) {
         CUDA_TRY(ctx, cudaEventRecord(tm.end, st));
         ctx->timed.push_back(tm);

@@ -387,7 +387,25 @@ struct ChunkWalker {
 };
 
 template <int WT, int K, bool DUAL, int NT, int STAGES, int NW = 8>
-__global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 4) expert_gemv_kernel(const GemvParams p) {
+constexpr size_t gemv_smem_bytes() {
+    return (size_t) STAGES * GemvCfg<WT, K, NW>::TENSOR_STAGE_BYTES * (DUAL ? 2 : 1) + NT * GemvCfg<WT, K, NW>::ACT_TOKEN_BYTES + STAGES * 8 +
+           256 * 4 + 64;
+}
+
+// CTAs per SM: the kernel waits on the latency of its own lane chains, so two CTAs (16 warps) beat one with a deeper ring; two
+// whenever two stages and the activations fit twice.  Ring depth: what fits then, up to four stages.
+template <int WT, int K, bool DUAL, int NT>
+constexpr int gemv_ctas() { return 2 * (gemv_smem_bytes<WT, K, DUAL, NT, 2>() + 1024 + 128) <= 228 * 1024 ? 2 : 1; }
+template <int WT, int K, bool DUAL, int NT>
+constexpr int gemv_stages() {
+    if (gemv_ctas<WT, K, DUAL, NT>() == 2)
+        return 2 * (gemv_smem_bytes<WT, K, DUAL, NT, 4>() + 1024 + 128) <= 228 * 1024 ? 4 : 2 * (gemv_smem_bytes<WT, K, DUAL, NT, 3>() + 1024 + 128) <= 228 * 1024 ? 3 : 2;
+    constexpr int stage = GemvCfg<WT, K>::TENSOR_STAGE_BYTES * (DUAL ? 2 : 1);
+    return (4 * stage <= 190 * 1024) ? 4 : (3 * stage <= 190 * 1024) ? 3 : 2;
+}
+
+template <int WT, int K, bool DUAL, int NT, int STAGES, int NW = 8>
+__global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>() : 4) expert_gemv_kernel(const GemvParams p) {
     using C = GemvCfg<WT, K, NW>;
     constexpr int NTENS = DUAL ? 2 : 1;
     constexpr int STAGE_BYTES = C::TENSOR_STAGE_BYTES * NTENS;
@@ -590,19 +608,6 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : 4) expert_gemv_kernel(c
         // bounded drain of copies still in flight before the block (and its shared memory) goes away
         for (int k = ci; k < issued; ++k) mbar_wait_bounded(&full[k % STAGES], (uint32_t) (k / STAGES) & 1u, 200000000ull);
     }
-}
-
-// ring depth: four stages unless that would not fit in shared memory
-template <int WT, int K, bool DUAL>
-constexpr int gemv_stages() {
-    constexpr int stage = GemvCfg<WT, K>::TENSOR_STAGE_BYTES * (DUAL ? 2 : 1);
-    return (4 * stage <= 190 * 1024) ? 4 : (3 * stage <= 190 * 1024) ? 3 : 2;
-}
-
-template <int WT, int K, bool DUAL, int NT, int STAGES, int NW = 8>
-constexpr size_t gemv_smem_bytes() {
-    return (size_t) STAGES * GemvCfg<WT, K, NW>::TENSOR_STAGE_BYTES * (DUAL ? 2 : 1) + NT * GemvCfg<WT, K, NW>::ACT_TOKEN_BYTES + STAGES * 8 +
-           256 * 4 + 64;
 }
 
 // ---- weighted combine: out[t][i] = sum over slots in slot order of y[t*k+s][i] * w[t][s] (forward.cpp:308-310)
