@@ -724,7 +724,7 @@ int launch_select_group(b200moe_ctx * ctx, const b200moe_layer * l, int T, float
     Plan & p = ctx->plan;
     const int E = l->n_expert, K = l->n_expert_used;
     p.groups.tile_rows = token_tile_rows((int64_t) T * K, E);
-    const size_t sh = (size_t) (3 * E + 1) * sizeof(int);
+    const size_t sh = (size_t) E * sizeof(int);
 #define SELG(EPL) launch_k(ctx, route_select_group_kernel<EPL>, dim3(1), dim3(1024), sh, st, p.logits, E, K, T, p.ids, p.wts, probs, p.groups, ctx->d_err)
     if (E <= 32) SELG(1);
     else if (E <= 64) SELG(2);
@@ -755,8 +755,9 @@ int launch_select(b200moe_ctx * ctx, const b200moe_layer * l, int T, int32_t * i
 int launch_group(b200moe_ctx * ctx, const int32_t * ids, int E, int rows, cudaStream_t st, bool allow_empty = false) {
     Plan & p = ctx->plan;
     p.groups.tile_rows = token_tile_rows(rows, E);
-    const size_t sh = (size_t) (3 * E + 1) * sizeof(int);
-    launch_k(ctx, group_scan_kernel, dim3(1), dim3(1024), sh, st, p.groups, ids, E, rows, ctx->d_err, allow_empty ? 1 : 0);
+    const size_t sh = (size_t) E * sizeof(int);
+    const int blocks = std::min(32, std::max(1, rows / 1024));
+    launch_k(ctx, group_scan_kernel, dim3(blocks), dim3(1024), sh, st, p.groups, ids, E, rows, ctx->d_err, allow_empty ? 1 : 0);
     return check_launch(ctx, "group_scan");
 }
 

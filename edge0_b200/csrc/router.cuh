@@ -385,22 +385,41 @@ __device__ __forceinline__ void route_select_token(const float * __restrict__ lo
         const int e = lane * EPL + i;
         p[i] = e < E ? ggml_expf(__fsub_rn(p[i], mx)) : 0.0f;
     }
-    // group-of-8 sums in the reference's order, then the double accumulation over groups in index order
-    double sum = 0.0;
-    for (int g = 0; g < E / 8; ++g) {
-        float v[8];
+    // group-of-8 sums in the reference's order, then the double accumulation over groups in index order.  A group's values v0..v7 sit in
+    // one lane (EPL >= 8) or in 8 / EPL neighbouring lanes, so each step of ((v0+v4)+(v2+v6))+((v1+v5)+(v3+v7)) is an addition inside the lane
+    // or one exchange with the lane that holds the partner (addition commutes: both ends get the same bits).
+    constexpr int GPL = EPL >= 8 ? EPL / 8 : 1;   // groups a lane holds
+    float gs[GPL];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int e = g * 8 + j;
-            const int owner = e / EPL, slot = e % EPL;
-            float val = 0.0f;
+    for (int q = 0; q < GPL; ++q) {
+        constexpr int N = EPL < 8 ? EPL : 8;
+        float v[N];
 #pragma unroll
-            for (int i = 0; i < EPL; ++i)
-                if (i == slot) val = p[i];
-            v[j] = __shfl_sync(0xffffffffu, val, owner);
+        for (int i = 0; i < N; ++i) v[i] = p[8 * q + i];
+#pragma unroll
+        for (int step = 4; step > 0; step >>= 1) {
+            if (step >= N) {
+#pragma unroll
+                for (int i = 0; i < N; ++i) v[i] = __fadd_rn(v[i], __shfl_xor_sync(0xffffffffu, v[i], step / N));
+            } else {
+#pragma unroll
+                for (int i = 0; i < N; ++i)
+                    if (i < step) v[i] = __fadd_rn(v[i], v[i + step]);
+            }
         }
-        const float r0 = __fadd_rn(v[4], v[0]), r1 = __fadd_rn(v[5], v[1]), r2 = __fadd_rn(v[6], v[2]), r3 = __fadd_rn(v[7], v[3]);
-        sum += (double) __fadd_rn(__fadd_rn(r0, r2), __fadd_rn(r1, r3));
+        gs[q] = v[0];
+    }
+    double sum = 0.0;
+    if (EPL >= 8) {
+        for (int o = 0; o * EPL < E; ++o) {
+#pragma unroll
+            for (int q = 0; q < GPL; ++q) {
+                const float g = __shfl_sync(0xffffffffu, gs[q], o);
+                if (o * EPL + 8 * q < E) sum += (double) g;
+            }
+        }
+    } else {
+        for (int g = 0; g < E / 8; ++g) sum += (double) __shfl_sync(0xffffffffu, gs[0], g * (8 / (EPL < 8 ? EPL : 8)));
     }
     const float inv = (float) (1.0 / sum);
 #pragma unroll
@@ -423,12 +442,11 @@ __device__ __forceinline__ void route_select_token(const float * __restrict__ lo
             const int e = lane * EPL + i;
             if (e < E && !((taken >> i) & 1u) && p[i] > best) { best = p[i]; best_e = e; }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-            if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
-        }
+        // candidates are not negative, so their bits order as they do; 0 marks a lane without one (all taken, or NaN)
+        const uint32_t key = best >= 0.0f ? __float_as_uint(fabsf(best)) + 1u : 0u;
+        const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+        best_e = (int) __reduce_min_sync(0xffffffffu, key == top ? (uint32_t) best_e : 0x7fffffffu);
+        best = top ? __uint_as_float(top - 1u) : -1.0f;
         if (best_e / EPL == lane) taken |= 1u << (best_e % EPL);
         if (lane == k) { sel_p = best; sel_e = best_e; }
         wsum += (double) best;  // sum_rows accumulates in double in slot order (ggml-cpu/vec.h:1495-1505)
@@ -478,59 +496,70 @@ struct Groups {
     int tile_rows;  // TOKEN_TILE_SMALL or TOKEN_TILE_LARGE
 };
 
-// Block-wide: counts must be final and visible to this block.
+// Block-wide: counts must be final and visible to this block.  With several blocks every one scans the counts for itself (a
+// microsecond) and fills its share of perm, which is what takes long with thousands of rows; block 0 writes the tables.
 // allow_empty: ids equal to -1 mark routed rows that do not exist (empty slots of an expert-parallel exchange): they are in no group.
-__device__ __forceinline__ void group_scan_body(Groups g, const int32_t * __restrict__ ids, int E, int rows, int * err, int * sh, bool allow_empty = false) {
-    int * off = sh;
-    int * act = sh + (E + 1);  // act[a] = a-th active expert (also written to g.active)
-    int * cnt = sh + (2 * E + 1);  // counts, fetched by the whole block at once (the scan below would wait for memory 32 at a time)
-    const int tid = threadIdx.x;
-    for (int e = tid; e < E; e += blockDim.x) cnt[e] = g.counts[e];
-    __syncthreads();
-    if (tid < 32) {
-        // warp 0: exclusive scan of counts, compaction of active experts and the three work prefixes, 32 experts a step
-        int run = 0, na = 0, c1 = 0, c2 = 0, c4 = 0, tl = 0;
-        for (int base = 0; base < E; base += 32) {
-            const int e = base + tid;
-            const int n = e < E ? cnt[e] : 0;
-            // work per weight row: nt=1 kernels: one pass per routed row; nt=4 kernels: 3 per pass (decode) + 2 per routed row
-            int incl = n, w2 = (n + 1) / 2, w4 = 3 * ((n + 3) / 4) + 2 * n;
-            int i2 = w2, i4 = w4, it = (n + g.tile_rows - 1) / g.tile_rows;
-            const int wt = it;
+__device__ __forceinline__ void group_scan_body(Groups g, const int32_t * __restrict__ ids, int E, int rows, int * err, int * sh, bool allow_empty = false,
+                                                int block = 0, int n_blocks = 1) {
+    // thread = expert (the launchers use 1024 threads, the largest expert count): a scan per warp, then one over the warps' totals
+    int * off = sh;                      // [E]
+    __shared__ int s_tot[6][32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int n = tid < E ? g.counts[tid] : 0;
+    // rows; active experts; work per weight row: nt=1 kernels: one pass per routed row; nt=2; nt=4 kernels: 3 per pass (decode) + 2 per
+    // routed row; token tiles
+    const int own[5] = { n, n > 0 ? 1 : 0, (n + 1) / 2, 3 * ((n + 3) / 4) + 2 * n, (n + g.tile_rows - 1) / g.tile_rows };
+    int v[5];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int a = __shfl_up_sync(0xffffffffu, incl, o), b = __shfl_up_sync(0xffffffffu, i2, o), c = __shfl_up_sync(0xffffffffu, i4, o);
-                const int d = __shfl_up_sync(0xffffffffu, it, o);
-                if (tid >= o) { incl += a; i2 += b; i4 += c; it += d; }
-            }
-            if (e < E) { off[e] = run + incl - n; g.cost[3 * (E + 1) + e] = tl + it - wt; }
-            const unsigned m = __ballot_sync(0xffffffffu, n > 0);
-            if (n > 0) {
-                const int a = na + __popc(m & ((1u << tid) - 1));
-                act[a] = e;
-                g.active[a] = e;
-                g.cost[a] = c1 + incl - n;
-                g.cost[(E + 1) + a] = c2 + i2 - w2;
-                g.cost[2 * (E + 1) + a] = c4 + i4 - w4;
-            }
-            run += __shfl_sync(0xffffffffu, incl, 31);
-            c1 += __shfl_sync(0xffffffffu, incl, 31);
-            c2 += __shfl_sync(0xffffffffu, i2, 31);
-            c4 += __shfl_sync(0xffffffffu, i4, 31);
-            tl += __shfl_sync(0xffffffffu, it, 31);
-            na += __popc(m);
+    for (int i = 0; i < 5; ++i) v[i] = own[i];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const int up = __shfl_up_sync(0xffffffffu, v[i], o);
+            if (lane >= o) v[i] += up;
         }
-        if (tid == 0) {
-            off[E] = run;
-            g.cost[na] = c1; g.cost[(E + 1) + na] = c2; g.cost[2 * (E + 1) + na] = c4; g.cost[3 * (E + 1) + E] = tl;
-            g.meta[0] = na;
-            g.meta[1] = run;
-            if (allow_empty ? run > rows : run != rows) report_error(err, DEV_ERR_BAD_SHAPE);
+    if (lane == 31)
+#pragma unroll
+        for (int i = 0; i < 5; ++i) s_tot[i][warp] = v[i];
+    __syncthreads();
+    if (warp < 5) {
+        const int own_t = lane < (int) (blockDim.x >> 5) ? s_tot[warp][lane] : 0;
+        int t = own_t;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, t, o);
+            if (lane >= o) t += up;
         }
+        s_tot[warp][lane] = t - own_t;
+        if (lane == 31) s_tot[5][warp] = t;
     }
     __syncthreads();
-    for (int e = tid; e <= E; e += blockDim.x) g.offsets[e] = off[e];
-    for (int r = tid; r < rows; r += blockDim.x) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) v[i] += s_tot[i][warp] - own[i];     // exclusive prefixes
+    if (tid < E) {
+        off[tid] = v[0];
+        if (block == 0) {
+            g.offsets[tid] = v[0];
+            g.cost[3 * (E + 1) + tid] = v[4];
+            if (n > 0) {
+                g.active[v[1]] = tid;
+                g.cost[v[1]] = v[0];
+                g.cost[(E + 1) + v[1]] = v[2];
+                g.cost[2 * (E + 1) + v[1]] = v[3];
+            }
+        }
+    }
+    if (tid == 0 && block == 0) {
+        const int run = s_tot[5][0], na = s_tot[5][1];
+        g.offsets[E] = run;
+        g.cost[na] = run; g.cost[(E + 1) + na] = s_tot[5][2]; g.cost[2 * (E + 1) + na] = s_tot[5][3]; g.cost[3 * (E + 1) + E] = s_tot[5][4];
+        g.meta[0] = na;
+        g.meta[1] = run;
+        if (allow_empty ? run > rows : run != rows) report_error(err, DEV_ERR_BAD_SHAPE);
+    }
+    __syncthreads();
+    for (int r = block * blockDim.x + tid; r < rows; r += n_blocks * blockDim.x) {
         const int e = ids[r];
         if (allow_empty && e == -1) continue;
         if (e < 0 || e >= E) { report_error(err, DEV_ERR_BAD_EXPERT_ID); continue; }
@@ -557,13 +586,13 @@ __global__ void __launch_bounds__(256) one_group_kernel(Groups g, int32_t * __re
     }
 }
 
-// Single block.  counts must be final (selection kernel finished).
+// counts must be final (selection kernel finished).
 __global__ void __launch_bounds__(1024) group_scan_kernel(Groups g, const int32_t * __restrict__ ids, int E, int rows, int * err, int allow_empty) {
     pdl_wait();
     pdl_launch_dependents();
 
-    extern __shared__ int sh[];  // [E+1] offsets, [E] active experts, [E] counts
-    group_scan_body(g, ids, E, rows, err, sh, allow_empty != 0);
+    extern __shared__ int sh[];  // [E] offsets
+    group_scan_body(g, ids, E, rows, err, sh, allow_empty != 0, blockIdx.x, gridDim.x);
 }
 
 // Small batches: selection for every token and the grouping in ONE single-block launch (one warp per token, looping).
