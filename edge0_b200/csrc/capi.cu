@@ -789,28 +789,12 @@ GemvParams gemv_params(b200moe_ctx * ctx, const void * w0, const void * w1, cons
 // one-or-two-token kernel
 int tokens_per_pass(int rows, int n_as) { return rows <= 16 ? -rows : rows <= n_as ? (rows <= 32 ? 1 : 4) : 4; }
 
-__global__ void scale_rows_kernel(float * v, const float * s, size_t n) {
-    pdl_wait();
-    pdl_launch_dependents();
-
-    const size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) v[i] = __fmul_rn(v[i], s[0]);
-}
-
 __global__ void bf16_to_f32_kernel(const __nv_bfloat16 * src, float * dst, size_t n) {
     pdl_wait();
     pdl_launch_dependents();
 
     const size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = __bfloat162float(src[i]);
-}
-
-// token t belongs to group t / group_size
-__global__ void fill_group_ids_kernel(int * ids, int T, int group_size) {
-    pdl_wait();
-    pdl_launch_dependents();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < T) ids[t] = t / group_size;
 }
 
 // Dense quantised matvec y[T][n_out] = W[n_out][k] . x[T][k] on the indexed-matmul kernel: the tokens are cut into up to 32
@@ -869,28 +853,20 @@ int dense_matvec(b200moe_ctx * ctx, int wtype, const void * w, const float * sca
         silu_mul_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(y, y1_tmp, n);
         return check_launch(ctx, "silu_mul");
     }
-    if ((rc = launch_quantize<float>(ctx, x, k, xq, T, k, wtype, st))) return rc;
+    // few tokens of an NVFP4 product: the kernel quantises the rows while it stages them
+    const bool fused_quant = wtype == TYPE_NVFP4 && T < 4 && !((uintptr_t) x & 15);
+    if (!fused_quant && (rc = launch_quantize<float>(ctx, x, k, xq, T, k, wtype, st))) return rc;
     const int G = std::max(1, std::min({32, T / 8, p.n_expert}));
     const int gsize = (T + G - 1) / G;
     const int groups = (T + gsize - 1) / gsize;
-    fill_group_ids_kernel<<<(T + 255) / 256, 256, 0, st>>>(p.one_group_ids, T, gsize);
-    if ((rc = check_launch(ctx, "fill_group_ids"))) return rc;
-    CUDA_TRY(ctx, cudaMemsetAsync(p.groups.counts, 0, sizeof(int) * std::max(groups, 8), st));
-    count_ids_kernel<<<(T + 255) / 256, 256, 0, st>>>(p.one_group_ids, 1, 1, T, groups, p.groups.perm /*scratch: compact ids*/, p.groups.counts,
-                                                      p.groups.pos, ctx->d_err);
-    if ((rc = check_launch(ctx, "count_ids"))) return rc;
-    // perm is about to be overwritten by the scan: read the ids from one_group_ids
-    if ((rc = launch_group(ctx, p.one_group_ids, groups, T, st))) return rc;
-    GemvParams g = gemv_params(ctx, w, w1, nullptr, nullptr, xq, y, n_out, 1, 1, groups);
+    p.groups.tile_rows = FP4_RPT_SMALL;
+    dense_groups_kernel<<<(T + 256) / 256, 256, 0, st>>>(p.groups, p.one_group_ids, T, gsize);
+    if ((rc = check_launch(ctx, "dense_groups"))) return rc;
+    GemvParams g = gemv_params(ctx, w, w1, scale, nullptr, xq, y, n_out, 1, 1, groups);
     g.w_stride = 0;
+    if (fused_quant) g.act_f32 = x;
     if (w1) return launch_integer<true>(ctx, wtype, k, g, T, groups, 4, st);
-    if ((rc = launch_integer<false>(ctx, wtype, k, g, T, groups, 4, st))) return rc;
-    if (scale) {
-        const size_t n = (size_t) T * n_out;
-        scale_rows_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(y, scale, n);
-        if ((rc = check_launch(ctx, "scale_rows"))) return rc;
-    }
-    return B200MOE_OK;
+    return launch_integer<false>(ctx, wtype, k, g, T, groups, 4, st);
 }
 
 // The same product on the FP4 tensor-core kernel: the matrix is the single "expert" of a one-group routing, the tokens its routed
@@ -910,8 +886,8 @@ int dense_matmul_fp4(b200moe_ctx * ctx, const void * w, const float * scale, con
     int rc;
     // a dense product has one group: the large tile once its units fill the GPU
     p.groups.tile_rows = (int64_t) ((T + FP4_RPT_LARGE - 1) / FP4_RPT_LARGE) * (n_out / (w1 ? 128 : 256)) >= ctx->sm_count ? FP4_RPT_LARGE : FP4_RPT_SMALL;
-    one_group_kernel<<<(T + 255) / 256, 256, 0, st>>>(p.groups, p.one_group_ids, T);
-    if ((rc = check_launch(ctx, "one_group"))) return rc;
+    dense_groups_kernel<<<(T + 256) / 256, 256, 0, st>>>(p.groups, p.one_group_ids, T, T);
+    if ((rc = check_launch(ctx, "dense_groups"))) return rc;
     // the fix-up recomputes with the quantised activations: have the plane kernel leave them in xq
     if ((rc = launch_act_planes(ctx, ActQuant{}, x, p.one_group_ids, T, k, 1, 1, 1, st, exact_requant ? xq : ActQuant{}))) return rc;
     if (w1) return launch_gemm_fp4<true>(ctx, k, fp4_params(ctx, nullptr, nullptr, y, n_out, 1), w, w1, reinterpret_cast<const uint8_t *>(p.afp16), T, st);
@@ -922,7 +898,6 @@ int dense_matmul_fp4(b200moe_ctx * ctx, const void * w, const float * scale, con
     list.count = p.groups.meta + 2;
     list.capacity = (int) std::min<size_t>(list_room_bytes / sizeof(int2), (size_t) T * n_out / 4);
     list.overflow = reinterpret_cast<unsigned long long *>(ctx->d_err + 2);
-    CUDA_TRY(ctx, cudaMemsetAsync(list.count, 0, sizeof(int), st));
     const int64_t warps = (int64_t) T * (n_out / 128);
     requant_mark_kernel<<<(unsigned) ((warps * 32 + 255) / 256), 256, 0, st>>>(y, p.groups.perm, p.groups.meta, T, n_out, FIX_STEP_MARGIN_FP4, FIX_REL_MARGIN_FP4, list);
     if ((rc = check_launch(ctx, "requant_mark"))) return rc;
@@ -998,7 +973,6 @@ int launch_requant_fixup(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq
     more.count = p.groups.meta + 3;
     more.capacity = (int) (room - room * 3 / 4);
     more.overflow = list.overflow;
-    CUDA_TRY(ctx, cudaMemsetAsync(list.count, 0, 2 * sizeof(int), st));
     const int64_t warps = (int64_t) rows * (l->n_ff / 128);
     launch_k(ctx, requant_mark_kernel, dim3((unsigned) ((warps * 32 + 255) / 256)), dim3(256), 0, st, (const float *) p.hid,
              (const int *) p.groups.perm, (const int *) p.groups.meta, rows, l->n_ff, after_fp4 ? FIX_STEP_MARGIN_FP4 : FIX_STEP_MARGIN, after_fp4 ? FIX_REL_MARGIN_FP4 : FIX_REL_MARGIN, list);
@@ -1161,8 +1135,21 @@ int layer_impl(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T, 
     Plan & p = ctx->plan;
     const int k = l->n_expert_used;
     int rc;
-    if (!l->n_latent) {   // x feeds the experts: quantised in the router's launch
-
+    if (l->n_latent) {
+        // the dense projections use the plan's grouping buffers: the down-projection runs before the routing that is grouped into them
+        const float * xf32;
+        if (std::is_same<XT, float>::value) {
+            xf32 = reinterpret_cast<const float *>(x);
+        } else {
+            const size_t n = (size_t) T * l->n_embd;
+            bf16_to_f32_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16 *>(x), p.xf, n);
+            if ((rc = check_launch(ctx, "bf16_to_f32"))) return rc;
+            xf32 = p.xf;
+        }
+        // the latent row is re-quantised for the experts: keep its quantised form the reference's (exact fix-up behind the FP4 engine)
+        if ((rc = dense_matvec(ctx, l->wtype, l->lat_down, l->lat_down_scale, xf32, p.xq, l->n_embd, l->n_latent, T, p.xl, st, true))) return rc;
+        if ((rc = route_impl<XT>(ctx, l, x, T, p.ids, p.wts, ob, true, st))) return rc;
+    } else {              // x feeds the experts: quantised in the router's launch
         if ((rc = launch_front<XT>(ctx, l, x, T, st))) return rc;
         float * probs = (ob && ob->ffn_moe_probs) ? ob->ffn_moe_probs : nullptr;
         if (T <= 32) {   // one warp per token fits one block: selection and grouping in a single launch
@@ -1173,8 +1160,6 @@ int layer_impl(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T, 
         }
         if (ob && ob->ffn_moe_logits)
             CUDA_TRY(ctx, cudaMemcpyAsync(ob->ffn_moe_logits, p.logits, sizeof(float) * (size_t) T * l->n_expert, cudaMemcpyDeviceToDevice, st));
-    } else {
-        if ((rc = route_impl<XT>(ctx, l, x, T, p.ids, p.wts, ob, true, st))) return rc;
     }
     if (ob && ob->ffn_moe_topk) CUDA_TRY(ctx, cudaMemcpyAsync(ob->ffn_moe_topk, p.ids, sizeof(int32_t) * (size_t) T * k, cudaMemcpyDeviceToDevice, st));
     if (ob && ob->ffn_moe_weights_norm)
@@ -1186,23 +1171,6 @@ int layer_impl(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T, 
         account(ctx, l, T);
         return rc;
     }
-    // latent: routing was grouped into the plan's Groups, but the dense projections reuse the same Groups
-    // buffers, so run the down-projection first and regroup afterwards.
-    const float * xf32;
-    if (std::is_same<XT, float>::value) {
-        xf32 = reinterpret_cast<const float *>(x);
-    } else {
-        const size_t n = (size_t) T * l->n_embd;
-        bf16_to_f32_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16 *>(x), p.xf, n);
-        if ((rc = check_launch(ctx, "bf16_to_f32"))) return rc;
-        xf32 = p.xf;
-    }
-    // the latent row is re-quantised for the experts: keep its quantised form the reference's (exact fix-up behind the FP4 engine)
-    if ((rc = dense_matvec(ctx, l->wtype, l->lat_down, l->lat_down_scale, xf32, p.xq, l->n_embd, l->n_latent, T, p.xl, st, true))) return rc;
-    // regroup the expert routing
-    CUDA_TRY(ctx, cudaMemsetAsync(p.groups.counts, 0, sizeof(int) * l->n_expert, st));
-    count_ids_kernel<<<(T * k + 255) / 256, 256, 0, st>>>(p.ids, k, k, T, l->n_expert, p.groups.perm, p.groups.counts, p.groups.pos, ctx->d_err);
-    if ((rc = check_launch(ctx, "count_ids"))) return rc;
     if ((rc = launch_group(ctx, p.ids, l->n_expert, T * k, st))) return rc;
     if ((rc = experts_impl(ctx, l, p.xlq, p.ids, p.wts, T, p.moe, ob, st, nullptr, p.xl, l->n_latent))) return rc;
     rc = dense_matvec(ctx, l->wtype, l->lat_up, l->lat_up_scale, p.moe, p.moq, l->n_latent, l->n_embd, T, out, st);

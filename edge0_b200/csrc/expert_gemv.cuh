@@ -506,8 +506,9 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
         const int e = p.active[ck.a];
         const int row_beg = p.offsets[e], n_e = p.offsets[e + 1] - row_beg;
         const uint8_t * st = ring + (size_t) stage * STAGE_BYTES;
-        const float sc0 = p.scale0 ? p.scale0[e] : 1.0f;
-        const float sc1 = (DUAL && p.scale1) ? p.scale1[e] : 1.0f;
+        const int se = p.w_stride ? e : 0;      // every group of a dense product has the one matrix and its scale
+        const float sc0 = p.scale0 ? p.scale0[se] : 1.0f;
+        const float sc1 = (DUAL && p.scale1) ? p.scale1[se] : 1.0f;
 
         // Routed rows of this expert are taken NT at a time; a remainder of 1 or 2 runs the narrower chains instead of
         // padding to NT (the weight decode is shared by the rows of a pass, the per-row work is not).

@@ -279,8 +279,9 @@ __global__ void __launch_bounds__(256, 1) expert_mma_q3k_kernel(const GemvParams
         }
         if (failed) break;
         // hsum_float_8 of every value, scales, SwiGLU, scatter
-        const float sc0 = p.scale0 ? p.scale0[cur.e] : 1.0f;
-        const float sc1 = (DUAL && p.scale1) ? p.scale1[cur.e] : 1.0f;
+        const int se = p.w_stride ? cur.e : 0;   // every group of a dense product has the one matrix and its scale
+        const float sc0 = p.scale0 ? p.scale0[se] : 1.0f;
+        const float sc1 = (DUAL && p.scale1) ? p.scale1[se] : 1.0f;
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll

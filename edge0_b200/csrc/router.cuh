@@ -490,7 +490,7 @@ struct Groups {
     int * pos;      // [rows]
     int * perm;     // [rows]
     int * active;   // [E]
-    int * meta;     // [4]
+    int * meta;     // [4]: number of active experts, rows in a group, two counters of the re-quantisation fix-up (cleared by the grouping)
     int * cost;     // [4][E+1]: rows 0-2: prefix over active experts of the work per weight row for the nt = 1, 2, 4 kernels;
                     // row 3, indexed by EXPERT id: index of the expert's first token tile (prefix of ceil(rows / tile_rows))
     int tile_rows;  // TOKEN_TILE_SMALL or TOKEN_TILE_LARGE
@@ -556,6 +556,7 @@ __device__ __forceinline__ void group_scan_body(Groups g, const int32_t * __rest
         g.cost[na] = run; g.cost[(E + 1) + na] = s_tot[5][2]; g.cost[2 * (E + 1) + na] = s_tot[5][3]; g.cost[3 * (E + 1) + E] = s_tot[5][4];
         g.meta[0] = na;
         g.meta[1] = run;
+        g.meta[2] = g.meta[3] = 0;       // the counters of the re-quantisation fix-up
         if (allow_empty ? run > rows : run != rows) report_error(err, DEV_ERR_BAD_SHAPE);
     }
     __syncthreads();
@@ -567,23 +568,25 @@ __device__ __forceinline__ void group_scan_body(Groups g, const int32_t * __rest
     }
 }
 
-// The grouping of a dense product: every one of the T rows belongs to the single group 0 (one launch instead of the
-// count / scan pair; same tables as group_scan_body leaves for E = 1).
-__global__ void __launch_bounds__(256) one_group_kernel(Groups g, int32_t * __restrict__ ids, int T) {
+// The grouping of a dense product: rows in order, gsize of them to a group (one launch instead of fill, count and scan; the same tables
+// as group_scan_body leaves).
+__global__ void __launch_bounds__(256) dense_groups_kernel(Groups g, int32_t * __restrict__ ids, int T, int gsize) {
     pdl_wait();
     pdl_launch_dependents();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < T) { ids[t] = 0; g.perm[t] = t; g.pos[t] = t; }
-    if (t == 0) {
-        g.counts[0] = T;
-        g.offsets[0] = 0; g.offsets[1] = T;
-        g.active[0] = 0;
-        g.meta[0] = 1; g.meta[1] = T;
-        g.cost[0] = 0; g.cost[1] = T;
-        g.cost[2] = 0; g.cost[3] = (T + 1) / 2;
-        g.cost[4] = 0; g.cost[5] = 3 * ((T + 3) / 4) + 2 * T;
-        g.cost[6] = 0; g.cost[7] = (T + g.tile_rows - 1) / g.tile_rows;
+    if (t < T) { ids[t] = t / gsize; g.perm[t] = t; g.pos[t] = t % gsize; }
+    const int G = (T + gsize - 1) / gsize;
+    if (t <= G) {
+        // prefixes over t groups: all of gsize rows but for the last group
+        const int last = T - (G - 1) * gsize, full = min(t, G - 1), tail = t == G ? 1 : 0;
+        g.offsets[t] = full * gsize + tail * last;
+        g.cost[t] = full * gsize + tail * last;
+        g.cost[(G + 1) + t] = full * ((gsize + 1) / 2) + tail * ((last + 1) / 2);
+        g.cost[2 * (G + 1) + t] = full * (3 * ((gsize + 3) / 4) + 2 * gsize) + tail * (3 * ((last + 3) / 4) + 2 * last);
+        g.cost[3 * (G + 1) + t] = full * ((gsize + g.tile_rows - 1) / g.tile_rows) + tail * ((last + g.tile_rows - 1) / g.tile_rows);
+        if (t < G) g.active[t] = t;
     }
+    if (t == 0) { g.meta[0] = G; g.meta[1] = T; g.meta[2] = g.meta[3] = 0; }
 }
 
 // counts must be final (selection kernel finished).
