@@ -497,11 +497,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
     while (cons.next(ck)) {
         const int stage = ci % STAGES;
         const uint32_t parity = (uint32_t) (ci / STAGES) & 1u;
-        if (!mbar_wait_bounded(&full[stage], parity)) {
-            report_error(p.err, DEV_ERR_BARRIER_TIMEOUT);
-            s_abort = 1;
-        }
-        if (__syncthreads_or(s_abort)) { failed = true; break; }
+        bool landed = false;    // the weights are waited for behind the loads of the first pass's activations
 
         const int e = p.active[ck.a];
         const int row_beg = p.offsets[e], n_e = p.offsets[e + 1] - row_beg;
@@ -562,6 +558,14 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
                 loaded_e = e;
                 loaded_tc = tc;
             }
+            if (!landed) {
+                if (!mbar_wait_bounded(&full[stage], parity)) {
+                    report_error(p.err, DEV_ERR_BARRIER_TIMEOUT);
+                    s_abort = 1;
+                }
+                if (__syncthreads_or(s_abort)) { failed = true; break; }
+                landed = true;
+            }
 #pragma unroll 1
             for (int ps = 0; ps < C::PASSES; ++ps) {
                 const int lr = (ps * C::NWARPS + warp) * C::RPP + rgrp;  // row within the stage
@@ -597,6 +601,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
             }
             t0 += ntc;
         }
+        if (failed) break;
         __syncthreads();  // everyone is done reading this stage
         if (tid == 0) {
             Chunk c;
