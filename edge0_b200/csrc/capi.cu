@@ -146,6 +146,7 @@ void carve(Plan & p, uint8_t * base) {
     p.groups.active = c.take<int>(E);
     p.groups.meta = c.take<int>(4);
     p.groups.cost = c.take<int>(4 * (E + 1));
+    p.groups.done = c.take<int>(kin);   // at most 16 tokens of kin / 16 chunks each
     p.xq = c.act(T, std::max(H, kin));
     p.xlq = c.act(T, kin);
     p.hq = c.act(R, I);
@@ -724,6 +725,7 @@ int launch_select_group(b200moe_ctx * ctx, const b200moe_layer * l, int T, float
     Plan & p = ctx->plan;
     const int E = l->n_expert, K = l->n_expert_used;
     p.groups.tile_rows = token_tile_rows((int64_t) T * K, E);
+    p.groups.n_done = T * K <= 16 ? p.n_in : 0;
     const size_t sh = (size_t) E * sizeof(int);
 #define SELG(EPL) launch_k(ctx, route_select_group_kernel<EPL>, dim3(1), dim3(1024), sh, st, p.logits, E, K, T, p.ids, p.wts, probs, p.groups, ctx->d_err)
     if (E <= 32) SELG(1);
@@ -755,6 +757,7 @@ int launch_select(b200moe_ctx * ctx, const b200moe_layer * l, int T, int32_t * i
 int launch_group(b200moe_ctx * ctx, const int32_t * ids, int E, int rows, cudaStream_t st, bool allow_empty = false) {
     Plan & p = ctx->plan;
     p.groups.tile_rows = token_tile_rows(rows, E);
+    p.groups.n_done = rows <= 16 ? p.n_in : 0;
     const size_t sh = (size_t) E * sizeof(int);
     const int blocks = std::min(32, std::max(1, rows / 1024));
     launch_k(ctx, group_scan_kernel, dim3(blocks), dim3(1024), sh, st, p.groups, ids, E, rows, ctx->d_err, allow_empty ? 1 : 0);
@@ -1072,8 +1075,11 @@ int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const 
         if ((rc = launch_integer<true>(ctx, l->wtype, n_in, gu, rows, l->n_expert, nt, st))) return rc;
     }
     if (fixup && (rc = launch_requant_fixup(ctx, l, xq, rows, n_in, k, fp4_gu, st))) return rc;
-    // the integer down kernel quantises `hidden` itself while staging it (NVFP4 / Q8_0); otherwise a separate pass
-    const bool fused_quant = !mma_down && !fp4_down && l->wtype == TYPE_NVFP4;
+    // The integer down kernel quantises `hidden` itself while staging it (NVFP4 / Q8_0; Q3_K / Q8_K for the few rows of one or two
+    // tokens); otherwise a separate pass.  With so few rows it also sums a token's rows (GemvParams::comb_out).
+    const bool tiny_down = !mma_down && !fp4_down && nt < 0 && !q3k_on_mma(l->wtype, rows, l->n_expert);
+    const bool fused_quant = !mma_down && !fp4_down && (l->wtype == TYPE_NVFP4 || tiny_down);
+    const bool fused_combine = tiny_down && !y_direct;
     if (!fused_quant && !fp4_down && (rc = launch_quantize<float>(ctx, p.hid, l->n_ff, p.hq, rows, l->n_ff, l->wtype, st))) return rc;
     if (fp4_down) {
         if ((rc = launch_act_planes(ctx, p.hq, p.hid, p.ids, rows, l->n_ff, k, k, l->n_expert, st))) return rc;   // quantises `hidden` itself
@@ -1085,9 +1091,10 @@ int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const 
     } else {
         GemvParams dn = gemv_params(ctx, l->down, nullptr, l->down_scale, nullptr, p.hq, y, n_in, k, k, l->n_expert);
         if (fused_quant) dn.act_f32 = p.hid;
+        if (fused_combine) { dn.comb_out = out; dn.comb_w = wts; dn.comb_cnt = p.groups.done; }
         if ((rc = launch_integer<false>(ctx, l->wtype, l->n_ff, dn, rows, l->n_expert, nt, st))) return rc;
     }
-    if (!y_direct) {
+    if (!y_direct && !fused_combine) {
         dim3 grid((n_in / 4 + 255) / 256, T);
         launch_k(ctx, combine_kernel, grid, dim3(256), 0, st, y, wts, out, n_in, k, T);
         if ((rc = check_launch(ctx, "combine"))) return rc;

@@ -33,7 +33,7 @@ struct GemvParams {
     const float * scale0; // per-expert fp32 scale applied to w0's result (or null)
     const float * scale1;
     ActQuant act;         // quantised activation planes, row index = (row / n_ids) * ne11 + (row % n_ids) % ne11
-    const float * act_f32; // or (NVFP4 only): the fp32 activations [rows][K], quantised to Q8_0 while they are staged (act unused)
+    const float * act_f32; // or: the fp32 activations [rows][K], quantised (Q8_0 or Q8_K) while they are staged (act unused)
     const int * offsets;  // [n_as + 1]
     const int * perm;     // [rows]
     const int * active;   // [n_as]
@@ -44,6 +44,9 @@ struct GemvParams {
     int n_ids;
     int ne11;
     int n_as;
+    float * comb_out;     // one-or-two-token kernel only, or null: the weighted sum over a token's rows goes here ([tokens][n_out])
+    const float * comb_w; // [rows] combine weights
+    int * comb_cnt;       // [tokens][n_out / 16] rows of `out` finished so far, cleared by the grouping
     int w_stride;         // rows between consecutive experts' matrices: n_out, or 0 when every group uses the same matrix
     int * err;
 };
@@ -416,7 +419,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
     uint8_t * acts = smem + STAGES * STAGE_BYTES;                                 // NT * ACT_TOKEN_BYTES (16-byte aligned)
     uint64_t * full = reinterpret_cast<uint64_t *>(acts + NT * C::ACT_TOKEN_BYTES);  // STAGES barriers
     float * ue_tab = reinterpret_cast<float *>(full + STAGES);                    // 256 floats (NVFP4 only)
-    __shared__ int s_abort;
+    __shared__ int s_abort, s_last;
     __shared__ int s_span[2];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -548,6 +551,15 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
                                 if ((i & 7) == 0) dd[(size_t) (i >> 3) * NT + t] = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
                             }
                         }
+                    } else if (WT == TYPE_Q3_K && p.act_f32) {
+                        for (int b = warp; b < K / 256; b += C::NWARPS) {      // a warp quantises one 256-block
+                            uint32_t q[2] = { 0u, 0u };
+                            float d = 0.0f;
+                            if (r >= 0) q8_K_words(p.act_f32 + (size_t) arow * K + b * 256 + lane * 8, lane, q, d);
+                            dq[(size_t) (b * 64 + lane * 2) * NT + t] = q[0];
+                            dq[(size_t) (b * 64 + lane * 2 + 1) * NT + t] = q[1];
+                            if (lane == 0) dd[(size_t) b * NT + t] = d;
+                        }
                     } else {
                         const uint32_t * srcq = reinterpret_cast<const uint32_t *>(p.act.q + (size_t) arow * K);
                         for (int i = tid; i < K / 4; i += NTHREADS) dq[(size_t) i * NT + t] = r >= 0 ? __ldg(srcq + i) : 0u;
@@ -602,6 +614,28 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
             t0 += ntc;
         }
         if (failed) break;
+        if (NW != 8 && !DUAL && p.comb_out) {
+            // The rows of this chunk are finished for every routed row of this expert.  The CTA that finishes the last of a token's
+            // rows sums them - in slot order, so which CTA that is does not show - and saves the combine its launch.
+            __threadfence();
+            __syncthreads();
+            for (int i = 0; i < n_e; ++i) {
+                const int tok = p.perm[row_beg + i] / p.n_ids;
+                if (tid == 0) s_last = atomicAdd(&p.comb_cnt[tok * (p.n_out / 16) + ck.r0 / 16], 1) == p.n_ids - 1;
+                __syncthreads();
+                if (s_last) {
+                    __threadfence();
+                    const float * wr = p.comb_w + (size_t) tok * p.n_ids;
+                    for (int j = tid; j < ck.n; j += NTHREADS) {
+                        const float * y = p.out + (size_t) tok * p.n_ids * p.n_out + ck.r0 + j;
+                        float a = __fmul_rn(__ldcg(y), wr[0]);
+                        for (int s = 1; s < p.n_ids; ++s) a = __fadd_rn(a, __fmul_rn(__ldcg(y + (size_t) s * p.n_out), wr[s]));
+                        p.comb_out[(size_t) tok * p.n_out + ck.r0 + j] = a;
+                    }
+                }
+                __syncthreads();
+            }
+        }
         __syncthreads();  // everyone is done reading this stage
         if (tid == 0) {
             Chunk c;

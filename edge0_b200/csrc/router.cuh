@@ -161,15 +161,15 @@ __device__ __forceinline__ void quantize_q8_0_block(const XT * __restrict__ src,
 // Q8_K as quantize_row_q8_K_ref (ggml-quants.c:2768-2805): the FIRST element with the largest |x| sets
 // iscale = -127/x; q = min(127, nearest_int(iscale*x)); d = 1/iscale; bsums over 16.
 // One warp per 256-element block, 8 elements per lane (lane owns elements 8*lane .. 8*lane+7).
+// src: the lane's eight values; q: its eight bytes; d: the block's scale, the same in every lane
 template <typename XT>
-__device__ __forceinline__ void quantize_q8_K_block(const XT * __restrict__ src, int8_t * __restrict__ q, float * __restrict__ d,
-                                                   int16_t * __restrict__ bsum, int lane) {
+__device__ __forceinline__ void q8_K_words(const XT * __restrict__ src, int lane, uint32_t (&q)[2], float & d) {
     float v[8];
     float amax = 0.0f, mx = 0.0f;
     int arg = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        v[i] = (float) src[lane * 8 + i];
+        v[i] = (float) src[i];
         const float a = fabsf(v[i]);
         if (a > amax) { amax = a; mx = v[i]; arg = lane * 8 + i; }
     }
@@ -180,25 +180,25 @@ __device__ __forceinline__ void quantize_q8_K_block(const XT * __restrict__ src,
         const int oi = __shfl_xor_sync(0xffffffffu, arg, o);
         if (oa > amax || (oa == amax && oi < arg)) { amax = oa; mx = om; arg = oi; }
     }
-    if (amax == 0.0f) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) q[lane * 8 + i] = 0;
-        if ((lane & 1) == 0) bsum[lane >> 1] = 0;
-        if (lane == 0) *d = 0.0f;
-        return;
-    }
+    q[0] = q[1] = 0u;
+    d = 0.0f;
+    if (amax == 0.0f) return;
     const float iscale = __fdiv_rn(-127.0f, mx);
-    int s = 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        int qi = __float2int_rn(__fmul_rn(iscale, v[i]));
-        qi = min(127, qi);
-        q[lane * 8 + i] = (int8_t) qi;
-        s += qi;
-    }
+    for (int i = 0; i < 8; ++i) q[i >> 2] |= ((uint32_t) min(127, __float2int_rn(__fmul_rn(iscale, v[i]))) & 0xffu) << (8 * (i & 3));
+    d = __fdiv_rn(1.0f, iscale);
+}
+template <typename XT>
+__device__ __forceinline__ void quantize_q8_K_block(const XT * __restrict__ src, int8_t * __restrict__ q, float * __restrict__ d,
+                                                   int16_t * __restrict__ bsum, int lane) {
+    uint32_t w[2];
+    float dd;
+    q8_K_words(src + lane * 8, lane, w, dd);
+    *reinterpret_cast<uint2 *>(q + lane * 8) = make_uint2(w[0], w[1]);
+    int s = dot4((int) w[0], 0x01010101, dot4((int) w[1], 0x01010101, 0));
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     if ((lane & 1) == 0) bsum[lane >> 1] = (int16_t) s;
-    if (lane == 0) *d = __fdiv_rn(1.0f, iscale);
+    if (lane == 0) *d = dd;
 }
 
 // rows x K activations -> ActQuant planes.  kind: 0 = Q8_0 (32-blocks), 1 = Q8_K (256-blocks).
@@ -494,6 +494,8 @@ struct Groups {
     int * cost;     // [4][E+1]: rows 0-2: prefix over active experts of the work per weight row for the nt = 1, 2, 4 kernels;
                     // row 3, indexed by EXPERT id: index of the expert's first token tile (prefix of ceil(rows / tile_rows))
     int tile_rows;  // TOKEN_TILE_SMALL or TOKEN_TILE_LARGE
+    int * done;     // [n_done] arrival counters of the one-or-two-token down kernel (GemvParams::comb_cnt), cleared by the grouping
+    int n_done;
 };
 
 // Block-wide: counts must be final and visible to this block.  With several blocks every one scans the counts for itself (a
@@ -501,6 +503,8 @@ struct Groups {
 // allow_empty: ids equal to -1 mark routed rows that do not exist (empty slots of an expert-parallel exchange): they are in no group.
 __device__ __forceinline__ void group_scan_body(Groups g, const int32_t * __restrict__ ids, int E, int rows, int * err, int * sh, bool allow_empty = false,
                                                 int block = 0, int n_blocks = 1) {
+    if (block == 0)
+        for (int i = threadIdx.x; i < g.n_done; i += blockDim.x) g.done[i] = 0;
     // thread = expert (the launchers use 1024 threads, the largest expert count): a scan per warp, then one over the warps' totals
     int * off = sh;                      // [E]
     __shared__ int s_tot[6][32];
