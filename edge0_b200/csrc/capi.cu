@@ -647,13 +647,17 @@ int launch_sorted_act(b200moe_ctx * ctx, ActQuant act, int rows, int k, int n_id
     return check_launch(ctx, "sorted_act_fp16");
 }
 
+// whether a warp may take 256 values of a row at a time (see quantize_warp)
+template <typename XT>
+bool quant_spans(const XT * src, int64_t stride, int k) { return k % 256 == 0 && ((uintptr_t) src & 15) == 0 && stride * sizeof(XT) % 16 == 0; }
+
 template <typename XT>
 int launch_quantize(b200moe_ctx * ctx, const XT * src, int64_t stride, ActQuant dst, int rows, int k, int wtype, cudaStream_t st) {
-    const int kind = wtype == TYPE_Q3_K ? 1 : 0;
-    const int64_t warps = (int64_t) rows * (kind ? k / 256 : k / 32);
+    const int kind = wtype == TYPE_Q3_K ? 1 : 0, spans = quant_spans(src, stride, k) ? 1 : 0;
+    const int64_t warps = (int64_t) rows * (kind || spans ? k / 256 : k / 32);
     if (warps == 0) return B200MOE_OK;
     const int blocks = (int) ((warps * 32 + 255) / 256);
-    launch_k(ctx, quantize_act_kernel<XT>, dim3(blocks), dim3(256), 0, st, src, stride, dst, rows, k, kind);
+    launch_k(ctx, quantize_act_kernel<XT>, dim3(blocks), dim3(256), 0, st, src, stride, dst, rows, k, kind, spans);
     return check_launch(ctx, "quantize_act");
 }
 
@@ -667,8 +671,9 @@ int launch_logits_smem(b200moe_ctx * ctx, const float * w, const float * bias, c
     if (int rc = raise_smem_limit(ctx, kern, smem, configured)) return rc;
     const int blocks = ((E + 8 * WE - 1) / (8 * WE)) * ((T + RT * WT - 1) / (RT * WT));
     // few blocks that loop: each holds the shared memory of a tile, and thousands of short ones took twice the time of the logits
-    const int qblocks = quant.q ? (int) std::min<int64_t>(2 * ctx->sm_count, ((int64_t) T * (H / (kind ? 256 : 32)) + WE * WT - 1) / (WE * WT)) : 0;
-    launch_k(ctx, kern, dim3(blocks + qblocks), dim3(WE * WT * 32), smem, st, w, bias, x, logits, H, E, T, zero_buf, zero_n, blocks, quant, kind);
+    const int spans = quant_spans(x, H, H) ? 1 : 0;
+    const int qblocks = quant.q ? (int) std::min<int64_t>(2 * ctx->sm_count, ((int64_t) T * (H / (kind || spans ? 256 : 32)) + WE * WT - 1) / (WE * WT)) : 0;
+    launch_k(ctx, kern, dim3(blocks + qblocks), dim3(WE * WT * 32), smem, st, w, bias, x, logits, H, E, T, zero_buf, zero_n, blocks, quant, kind, spans);
     return check_launch(ctx, "router_logits");
 }
 
@@ -678,18 +683,19 @@ int launch_logits_any(b200moe_ctx * ctx, const float * w, const float * bias, co
                       int zero_n, cudaStream_t st, ActQuant quant = ActQuant{}, int kind = 0) {
     const bool staged = T >= 16 && E >= 8 && H % ROUTER_KC == 0 && (((uintptr_t) w | (uintptr_t) x) & 15) == 0;
     if (staged) {
-        // shared-memory tiles: 32 experts x 16 tokens (8 warps) when there are two of them per SM, else 16 x 8 (4 warps)
+        // shared-memory tiles: 32 experts x 16 tokens (8 warps) when they fill the GPU, else 16 x 8 (4 warps)
         const int big = ((E + 31) / 32) * ((T + 15) / 16);
-        if (big >= 2 * ctx->sm_count) return launch_logits_smem<4, 2, 8, XT>(ctx, w, bias, x, logits, H, E, T, zero_buf, zero_n, quant, kind, st);
+        if (big >= ctx->sm_count) return launch_logits_smem<4, 2, 8, XT>(ctx, w, bias, x, logits, H, E, T, zero_buf, zero_n, quant, kind, st);
         return launch_logits_smem<2, 2, 4, XT>(ctx, w, bias, x, logits, H, E, T, zero_buf, zero_n, quant, kind, st);
     }
     // few tokens or a single row: one warp per (expert, token) with deep load prefetch; otherwise 4 tokens share each weight load
     const int tt = T <= 8 || E < 8 ? 1 : 4;
     const int lblocks = (int) (((int64_t) E * ((T + tt - 1) / tt) + 7) / 8);
     if (quant.q) {
-        const int qblocks = (int) (((int64_t) T * (H / (kind ? 256 : 32)) + 7) / 8);
-        if (tt == 1) launch_k(ctx, route_front_kernel<1, XT>, dim3(lblocks + qblocks), dim3(256), 0, st, w, bias, x, logits, H, E, T, zero_buf, zero_n, lblocks, quant, kind);
-        else launch_k(ctx, route_front_kernel<4, XT>, dim3(lblocks + qblocks), dim3(256), 0, st, w, bias, x, logits, H, E, T, zero_buf, zero_n, lblocks, quant, kind);
+        const int spans = quant_spans(x, H, H) ? 1 : 0;
+        const int qblocks = (int) (((int64_t) T * (H / (kind || spans ? 256 : 32)) + 7) / 8);
+        if (tt == 1) launch_k(ctx, route_front_kernel<1, XT>, dim3(lblocks + qblocks), dim3(256), 0, st, w, bias, x, logits, H, E, T, zero_buf, zero_n, lblocks, quant, kind, spans);
+        else launch_k(ctx, route_front_kernel<4, XT>, dim3(lblocks + qblocks), dim3(256), 0, st, w, bias, x, logits, H, E, T, zero_buf, zero_n, lblocks, quant, kind, spans);
         return check_launch(ctx, "route_front");
     }
     if (T >= 16 && E >= 8) {   // batches whose rows cannot be staged: 4 experts x 8 tokens per warp
@@ -713,8 +719,12 @@ int launch_logits(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int 
 template <typename XT>
 int launch_front(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T, cudaStream_t st) {
     Plan & p = ctx->plan;
-    return launch_logits_any<XT>(ctx, l->router_w, l->router_bias, x, p.logits, l->n_embd, l->n_expert, T, p.groups.counts, l->n_expert, st, p.xq,
-                                 l->wtype == TYPE_Q3_K ? 1 : 0);
+    // beyond a few waves of logit tiles the quantising blocks only hold shared memory back from them (4096 tokens: 156 us in one
+    // launch, 99 + 39 in two before the quantiser took eight values a lane)
+    const bool fused = T <= 256;
+    const int rc = launch_logits_any<XT>(ctx, l->router_w, l->router_bias, x, p.logits, l->n_embd, l->n_expert, T, p.groups.counts, l->n_expert, st,
+                                         fused ? p.xq : ActQuant{}, l->wtype == TYPE_Q3_K ? 1 : 0);
+    return rc || fused ? rc : launch_quantize<XT>(ctx, x, l->n_embd, p.xq, T, l->n_embd, l->wtype, st);
 }
 
 // Routed rows per token tile of the FP4 kernels for `rows` rows in up to n_groups groups; kept in the plan from the grouping to the

@@ -628,8 +628,19 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
                     const float * wr = p.comb_w + (size_t) tok * p.n_ids;
                     for (int j = tid; j < ck.n; j += NTHREADS) {
                         const float * y = p.out + (size_t) tok * p.n_ids * p.n_out + ck.r0 + j;
-                        float a = __fmul_rn(__ldcg(y), wr[0]);
-                        for (int s = 1; s < p.n_ids; ++s) a = __fadd_rn(a, __fmul_rn(__ldcg(y + (size_t) s * p.n_out), wr[s]));
+                        float a = 0.0f;
+                        for (int s0 = 0; s0 < p.n_ids; s0 += 8) {          // eight rows' loads in flight, added in slot order
+                            float v[8], w[8];
+#pragma unroll
+                            for (int s = 0; s < 8; ++s) {
+                                const bool in = s0 + s < p.n_ids;
+                                v[s] = in ? __ldcg(y + (size_t) (s0 + s) * p.n_out) : 0.0f;
+                                w[s] = in ? wr[s0 + s] : 0.0f;
+                            }
+#pragma unroll
+                            for (int s = 0; s < 8; ++s)
+                                if (s0 + s < p.n_ids) a = s0 + s == 0 ? __fmul_rn(v[s], w[s]) : __fadd_rn(a, __fmul_rn(v[s], w[s]));
+                        }
                         p.comb_out[(size_t) tok * p.n_out + ck.r0 + j] = a;
                     }
                 }

@@ -161,6 +161,36 @@ __device__ __forceinline__ void quantize_q8_0_block(const XT * __restrict__ src,
 // Q8_K as quantize_row_q8_K_ref (ggml-quants.c:2768-2805): the FIRST element with the largest |x| sets
 // iscale = -127/x; q = min(127, nearest_int(iscale*x)); d = 1/iscale; bsums over 16.
 // One warp per 256-element block, 8 elements per lane (lane owns elements 8*lane .. 8*lane+7).
+// The same for eight blocks at a time: a lane holds eight neighbouring values, four lanes one block.  src 16-byte aligned.  (A lane
+// per value moved 16 MB of a 4096-token prompt in 39 us.)
+__device__ __forceinline__ void load8(const float * __restrict__ src, float (&v)[8]) {
+    const float4 a = *reinterpret_cast<const float4 *>(src), b = *reinterpret_cast<const float4 *>(src + 4);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void load8(const __nv_bfloat16 * __restrict__ src, float (&v)[8]) {
+    const uint4 a = *reinterpret_cast<const uint4 *>(src);
+    const uint32_t w[4] = { a.x, a.y, a.z, a.w };
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+}
+template <typename XT>
+__device__ __forceinline__ void quantize_q8_0_span(const XT * __restrict__ src, int8_t * __restrict__ q, float * __restrict__ d, int lane) {
+    float v[8];
+    load8(src + lane * 8, v);
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    const float dd = __fdiv_rn(amax, 127.0f);
+    const float id = amax != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+    uint32_t w[2] = { 0u, 0u };
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i >> 2] |= ((uint32_t) __float2int_rn(__fmul_rn(v[i], id)) & 0xffu) << (8 * (i & 3));
+    *reinterpret_cast<uint2 *>(q + lane * 8) = make_uint2(w[0], w[1]);
+    if ((lane & 3) == 0) d[lane >> 2] = __half2float(__float2half_rn(dd));
+}
+
 // src: the lane's eight values; q: its eight bytes; d: the block's scale, the same in every lane
 template <typename XT>
 __device__ __forceinline__ void q8_K_words(const XT * __restrict__ src, int lane, uint32_t (&q)[2], float & d) {
@@ -203,37 +233,28 @@ __device__ __forceinline__ void quantize_q8_K_block(const XT * __restrict__ src,
 
 // rows x K activations -> ActQuant planes.  kind: 0 = Q8_0 (32-blocks), 1 = Q8_K (256-blocks).
 // src row r starts at src + r*src_stride.
+// spans: K is a multiple of 256 and the rows are 16-byte aligned, so a warp takes 256 values of either kind at a time
 template <typename XT>
-__global__ void __launch_bounds__(256) quantize_act_kernel(const XT * __restrict__ src, int64_t src_stride, ActQuant dst, int rows,
-                                                          int K, int kind) {
-    pdl_wait();
-    pdl_launch_dependents();
-
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (kind == 0) {
-        const int nb = K / 32;
-        if (warp >= rows * nb) return;
-        const int r = warp / nb, b = warp % nb;
-        quantize_q8_0_block(src + (size_t) r * src_stride + b * 32, dst.q + (size_t) r * K + b * 32, dst.d + (size_t) r * nb + b, lane);
-    } else {
-        const int nb = K / 256;
-        if (warp >= rows * nb) return;
-        const int r = warp / nb, b = warp % nb;
-        quantize_q8_K_block(src + (size_t) r * src_stride + b * 256, dst.q + (size_t) r * K + b * 256, dst.d + (size_t) r * nb + b,
-                            dst.bsum + (size_t) r * (K / 16) + b * 16, lane);
+__device__ __forceinline__ void quantize_warp(const XT * __restrict__ src, int64_t src_stride, const ActQuant & dst, int rows, int K, int kind, bool spans,
+                                              int warp, int n_warps, int lane) {
+    const int nb = K / (kind == 0 && !spans ? 32 : 256);
+    for (int i = warp; i < rows * nb; i += n_warps) {
+        const int r = i / nb, b = i % nb;
+        const XT * row = src + (size_t) r * src_stride;
+        int8_t * q = dst.q + (size_t) r * K;
+        if (kind) quantize_q8_K_block(row + b * 256, q + b * 256, dst.d + (size_t) r * nb + b, dst.bsum + (size_t) r * (K / 16) + b * 16, lane);
+        else if (spans) quantize_q8_0_span(row + b * 256, q + b * 256, dst.d + (size_t) r * (K / 32) + b * 8, lane);
+        else quantize_q8_0_block(row + b * 32, q + b * 32, dst.d + (size_t) r * nb + b, lane);
     }
 }
 
-// The warps of the quantising blocks share the activation blocks of the expert matmuls (kind: 0 = Q8_0, 1 = Q8_K) in strides.
 template <typename XT>
-__device__ __forceinline__ void quantize_warps(const XT * __restrict__ x, const ActQuant & dst, int H, int T, int kind, int warp, int n_warps, int lane) {
-    const int nb = H / (kind ? 256 : 32);
-    for (int i = warp; i < T * nb; i += n_warps) {
-        const int r = i / nb, b = i % nb;
-        if (kind == 0) quantize_q8_0_block(x + (size_t) r * H + b * 32, dst.q + (size_t) r * H + b * 32, dst.d + (size_t) r * nb + b, lane);
-        else quantize_q8_K_block(x + (size_t) r * H + b * 256, dst.q + (size_t) r * H + b * 256, dst.d + (size_t) r * nb + b, dst.bsum + (size_t) r * (H / 16) + b * 16, lane);
-    }
+__global__ void __launch_bounds__(256) quantize_act_kernel(const XT * __restrict__ src, int64_t src_stride, ActQuant dst, int rows,
+                                                          int K, int kind, int spans) {
+    pdl_wait();
+    pdl_launch_dependents();
+    quantize_warp<XT>(src, src_stride, dst, rows, K, kind, spans != 0, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
+                      threadIdx.x & 31);
 }
 
 // Router logits and activation quantisation in one launch (few tokens): blocks [0, n_logit_blocks) compute logits,
@@ -242,7 +263,7 @@ template <int TT, typename XT>
 __global__ void __launch_bounds__(256) route_front_kernel(const float * __restrict__ W, const float * __restrict__ bias,
                                                          const XT * __restrict__ x, float * __restrict__ logits, int H, int E, int T,
                                                          int * __restrict__ zero_buf, int zero_n, int n_logit_blocks, ActQuant dst,
-                                                         int kind) {
+                                                         int kind, int spans) {
     pdl_wait();
     pdl_launch_dependents();
 
@@ -253,7 +274,7 @@ __global__ void __launch_bounds__(256) route_front_kernel(const float * __restri
         router_warp<TT, XT>(W, bias, x, logits, H, E, T, (int) blockIdx.x * 8 + wib, lane);
         return;
     }
-    quantize_warps<XT>(x, dst, H, T, kind, ((int) blockIdx.x - n_logit_blocks) * 8 + wib, ((int) gridDim.x - n_logit_blocks) * 8, lane);
+    quantize_warp<XT>(x, H, dst, T, H, kind, spans != 0, ((int) blockIdx.x - n_logit_blocks) * 8 + wib, ((int) gridDim.x - n_logit_blocks) * 8, lane);
 }
 
 // Shared-memory form for larger batches: a block owns (8 WE experts) x (RT WT tokens); weight and activation rows arrive in
@@ -277,7 +298,7 @@ template <int WE, int WT, int RT, typename XT>
 __global__ void __launch_bounds__(WE * WT * 32) router_logits_smem_kernel(const float * __restrict__ W, const float * __restrict__ bias,
                                                                          const XT * __restrict__ x, float * __restrict__ logits, int H, int E, int T,
                                                                          int * __restrict__ zero_buf, int zero_n, int n_logit_blocks, ActQuant dst,
-                                                                         int kind) {
+                                                                         int kind, int spans) {
     constexpr int EB = 8 * WE, TB = RT * WT, KC = ROUTER_KC, ST = ROUTER_ST, NTHR = WE * WT * 32;
     constexpr int XP = 16 / sizeof(XT);   // activation elements per 16-byte piece
     extern __shared__ __align__(16) uint8_t router_smem[];
@@ -288,8 +309,8 @@ __global__ void __launch_bounds__(WE * WT * 32) router_logits_smem_kernel(const 
     if (blockIdx.x == 0)
         for (int i = threadIdx.x; i < zero_n; i += NTHR) zero_buf[i] = 0;
     if ((int) blockIdx.x >= n_logit_blocks) {
-        quantize_warps<XT>(x, dst, H, T, kind, ((int) blockIdx.x - n_logit_blocks) * (NTHR / 32) + (int) (threadIdx.x >> 5),
-                           ((int) gridDim.x - n_logit_blocks) * (NTHR / 32), threadIdx.x & 31);
+        quantize_warp<XT>(x, H, dst, T, H, kind, spans != 0, ((int) blockIdx.x - n_logit_blocks) * (NTHR / 32) + (int) (threadIdx.x >> 5),
+                          ((int) gridDim.x - n_logit_blocks) * (NTHR / 32), threadIdx.x & 31);
         return;
     }
     const int n_eb = (E + EB - 1) / EB;
