@@ -17,20 +17,26 @@
 // product inside the tensor core is exact, and the result differs from the integer path only by fp32 accumulation.
 //
 // Operand roles: D[feature, plane] = W[feature, k] * P[plane, k].  M = 128 weight rows, N = 7 planes x up to 14 routed rows
-// (N = 8 .. 104), K = 64 per instruction.  The seven plane columns of a routed row sit next to each other in one lane of tensor
+// (N = 8 .. 104; prefill: up to 27 rows, N = 192), K = 64 per instruction.  The seven plane columns of a routed row sit next to each other in one lane of tensor
 // memory, so the epilogue recombines them with a Horner chain in registers and stores 32 consecutive features per warp.
 // Two weight tiles are in flight per stage with an accumulator each (gate and up rows of the same 128 features, or two
 // consecutive 128-row tiles of `down`): dependent MMAs on one accumulator issue every ~190-230 cycles, MMAs that alternate
 // between two accumulators every ~116 (measured with the probe kernel in fp4_probe.cuh).
 //
 // Roles (every wait bounded, as in expert_gemm.cuh):
-//   warp 0      raw-weight producer: tiled TMA of [128 rows][144 bytes] boxes (K = 256 per row) of both tiles
-//   warp 1      activation producer: one tiled TMA box [98 plane rows][128 bytes] + one bulk copy of the 2 KB scale tile, into a
-//               ring of its own that runs three stages ahead (the planes come from L2 with about a microsecond of latency)
-//   warp 2      MMA issuer: per K = 64 step three tcgen05.cp (scales of tile 0, tile 1, planes) and two tcgen05.mma
-//   warp 3      owns tensor memory
-//   warps 4-7   epilogue
-//   warps 8-15  repack: thread = one weight row of one tile; 9 x 16-byte loads, 8 x 16-byte stores, 4 scale words
+//   warp 0       raw-weight producer: tiled TMA of [128 rows][144 bytes] boxes (K = 256 per row) of both tiles
+//   warp 1       activation producer: one tiled TMA box of the token tile's plane rows (128 bytes each) + one bulk copy of its scale
+//                tile, into a ring of its own that runs three stages ahead (the planes come from L2 with about a microsecond of latency)
+//   warp 2       MMA issuer: two tcgen05.mma per K = 64 step
+//   warp 3       owns tensor memory
+//   warps 4-7    epilogue
+//   warps 8-15   repack: thread = one weight row of one tile; 9 x 16-byte loads, 8 x 16-byte stores, the row's scale words set aside
+//   warps 16-19  scale factors: from shared memory through registers into tensor memory (tcgen05.st)
+// The scales go through registers because a tcgen05.cp holds its issuing thread ~80 cycles: twelve per stage in front of the MMAs cost
+// 15-20 % of the kernel, and from a thread of their own an instruction now and then read a scale that was not in place.  The exchange
+// between rows and lanes and the waits of tcgen05.st have warps of their own because the repack warps' chain is the longest of a stage: with
+// both in the repack warps gate/up of 64 tokens over 512 experts (1024 -> 1024) took 107 us, like this 98; sixteen repack warps
+// that take the stages in turn gained nothing more and cost the prefill tile its registers (4096 tokens: 481 -> 685 us).
 #pragma once
 #include <cuda.h>
 
@@ -48,7 +54,7 @@ constexpr int FP4_RPT_SMALL = TOKEN_TILE_SMALL, FP4_RPT_LARGE = TOKEN_TILE_LARGE
 constexpr int FP4_SF_TILE = 4 * 512;              // scale factors of 128 rows for the four K = 64 steps of a stage
 // bytes of one token tile's scale factors per K = 256 stage: one block of 128 plane rows, or two
 __host__ __device__ constexpr int fp4_sfb_bytes(int rpt) { return (FP4_PLANES * rpt + 127) / 128 * FP4_SF_TILE; }
-constexpr int FP4_THREADS = 512;
+constexpr int FP4_THREADS = 640;
 
 __device__ __forceinline__ void umma_fp4(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t sfa, uint32_t sfb,
                                          bool accumulate) {
@@ -72,11 +78,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint4 (&v)[4]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0].x),
                  "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w), "r"(v[2].x), "r"(v[2].y), "r"(v[2].z),
                  "r"(v[2].w), "r"(v[3].x), "r"(v[3].y), "r"(v[3].z), "r"(v[3].w)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint4 (&v)[2]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0].x), "r"(v[0].y), "r"(v[0].z),
-                 "r"(v[0].w), "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w)
                  : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -342,17 +343,16 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
     uint8_t * tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
     uint8_t * acts = tiles + (size_t) TS * C::STAGE;
     uint8_t * raws = acts + (size_t) AS * C::ACT_STAGE;
-    __shared__ uint64_t raw_full[RS], raw_empty[RS], tile_full[TS], tile_empty[TS], act_full[AS], act_empty[AS], acc_full[NACC], acc_empty[NACC], sfx_full[2];
+    __shared__ uint64_t raw_full[RS], raw_empty[RS], tile_full[TS], tile_empty[TS], act_full[AS], act_empty[AS], acc_full[NACC], acc_empty[NACC], sf_ready[RS];
     __shared__ uint32_t s_tmem;
     __shared__ volatile int s_abort;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
-        for (int i = 0; i < RS; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 8); }
-        for (int i = 0; i < TS; ++i) { mbar_init(&tile_full[i], 256); mbar_init(&tile_empty[i], 1); }
+        for (int i = 0; i < RS; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4); mbar_init(&sf_ready[i], 8); }
+        for (int i = 0; i < TS; ++i) { mbar_init(&tile_full[i], 256 + 4); mbar_init(&tile_empty[i], 1); }
         for (int i = 0; i < AS; ++i) { mbar_init(&act_full[i], 1); mbar_init(&act_empty[i], 1); }
         for (int i = 0; i < NACC; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
-        for (int i = 0; i < 2; ++i) mbar_init(&sfx_full[i], 4);
         mbar_fence_init();
         s_abort = 0;
     }
@@ -386,6 +386,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
         w.nt = min(RPT, p.offsets[w.e + 1] - w.row0);
         return w;
     };
+    const int my_stages = n_units > (int) blockIdx.x ? (n_units - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x * KC : 0;
     // weight stage: [A0][A1]; activation stage: [B][SFB]
     constexpr uint32_t OFF_A1 = C::A_TILE, OFF_SFB = C::B_TILE;
 
@@ -539,99 +540,116 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                 }
         }
         if (warp == 4 && lane == 0) FP4_PROF_STORE(8, 1);
-    } else if (warp >= 8) {
+    } else if (warp >= 8 && warp < 16) {
         // ---------------------------------------------------------------- repack: strip the scale bytes, keep everything else
         const int dq = tid - 256;
         const int trow = dq & 127, tsel = dq >> 7;
-        uint32_t a_off[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) a_off[c] = tsel * C::A_TILE + sw128_offset(trow, c);
+        const uint32_t a_off = tsel * C::A_TILE + sw128_offset(trow, 0);   // 16-byte chunk c of the row lies at a_off ^ (16 c)
         const uint32_t raw_off = (uint32_t) dq * GEMM_RAW_ROW;
-        const uint32_t quarter = (uint32_t) ((warp & 3) * 32) << 16;   // the lanes of tensor memory this warp may write
-        Ring raw, tile, act, sfx;
+        Ring raw, tile;
         FP4_PROF_DECL();
-        for (int u = blockIdx.x; u < n_units && !s_abort; u += gridDim.x) {
+        for (int i = 0; i < my_stages && !s_abort; ++i) {
             {
-                for (int kc = 0; kc < KC && !s_abort; ++kc) {
-                    {
-                        FP4_PROF_T0();
-                        if (!__all_sync(0xffffffffu, wait_or_abort(&raw_full[raw.stage], raw.phase, &s_abort, p.err))) break;
-                        FP4_PROF_ADD(0);
-                    }
-                    uint32_t R[36];                // 4 blocks of [scale word][8 code words]
-                    {
-                        const uint4 * src = reinterpret_cast<const uint4 *>(raws + (size_t) raw.stage * C::RAW_STAGE + raw_off);
-#pragma unroll
-                        for (int i = 0; i < 9; ++i) {
-                            const uint4 v = src[i];
-                            R[4 * i] = v.x; R[4 * i + 1] = v.y; R[4 * i + 2] = v.z; R[4 * i + 3] = v.w;
-                        }
-                    }
-                    // Scale words of the tile's 128 rows, exchanged between its four warps: lane l of every warp needs those of rows l, l + 32,
-                    // l + 64 and l + 96.  A row's four words go into the first 16 bytes of its own raw row, which this thread has just
-                    // read.  (An mbarrier and not a named barrier: a warp that gives up must not leave the others waiting without limit.)
-                    uint32_t S[4];
-#pragma unroll
-                    for (int kb = 0; kb < 4; ++kb) {
-                        // The reference reads scale bytes through ggml_ue4m3_to_fp32: bit 7 ignored, 0x7f decodes to zero; to the tensor
-                        // core 0x7f is NaN.  Clear bit 7 and turn 0x7f into 0 (t <= 0x7f per byte, so t + 1 carries into bit 7 only
-                        // for 0x7f and never into the next byte).
-                        const uint32_t t = R[9 * kb] & 0x7f7f7f7fu;
-                        const uint32_t nan1 = ((t + 0x01010101u) >> 7) & 0x01010101u;
-                        S[kb] = t & ~((nan1 << 7) - nan1);
-                    }
-                    uint8_t * const raw_tile = raws + (size_t) raw.stage * C::RAW_STAGE + (size_t) tsel * 128 * GEMM_RAW_ROW;
-                    *reinterpret_cast<uint4 *>(raw_tile + trow * GEMM_RAW_ROW) = make_uint4(S[0], S[1], S[2], S[3]);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&sfx_full[tsel]);
-                    if (!__all_sync(0xffffffffu, wait_or_abort(&sfx_full[tsel], sfx.phase, &s_abort, p.err))) break;
-                    sfx.template advance<1>();
-                    uint4 sfr[4];                  // [row l + 32 j][K = 64 step]
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) sfr[j] = *reinterpret_cast<const uint4 *>(raw_tile + (32 * j + lane) * GEMM_RAW_ROW);
-                    fence_async_smem();            // the next copy into this stage comes behind the words written above
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&raw_empty[raw.stage]);
-                    raw.template advance<RS>();
-                    const uint4 sfa[4] = { make_uint4(sfr[0].x, sfr[1].x, sfr[2].x, sfr[3].x), make_uint4(sfr[0].y, sfr[1].y, sfr[2].y, sfr[3].y),
-                                           make_uint4(sfr[0].z, sfr[1].z, sfr[2].z, sfr[3].z), make_uint4(sfr[0].w, sfr[1].w, sfr[2].w, sfr[3].w) };
-                    uint8_t * st = tiles + (size_t) tile.stage * C::STAGE;
-                    {
-                        FP4_PROF_T0();
-                        if (!__all_sync(0xffffffffu, wait_or_abort(&act_full[act.stage], act.phase, &s_abort, p.err))) break;
-                        FP4_PROF_ADD(2);
-                    }
-                    // the planes' scales: tile 0's warps move those of the first two K = 64 steps, tile 1's those of the last two
-                    const uint8_t * sfb_src = acts + (size_t) act.stage * C::ACT_STAGE + OFF_SFB + tsel * (C::SFB / 2) + lane * 16;
-                    uint4 sfb[2 * C::NBLK];
-#pragma unroll
-                    for (int i = 0; i < 2 * C::NBLK; ++i) sfb[i] = *reinterpret_cast<const uint4 *>(sfb_src + 512 * i);
-                    act.template advance<AS>();
-                    {
-                        FP4_PROF_T0();
-                        if (!__all_sync(0xffffffffu, wait_or_abort(&tile_empty[tile.stage], tile.phase ^ 1u, &s_abort, p.err))) break;
-                        FP4_PROF_ADD(1);
-                    }
-                    tc_fence_after();
-                    const uint32_t sf_set = tmem + C::SF_COL + C::SF_SET * (uint32_t) tile.stage + quarter;
-                    tmem_st16(sf_set + 16 * tsel, sfa);
-                    if constexpr (C::NBLK == 2) tmem_st16(sf_set + 32 + 16 * tsel, sfb);
-                    else tmem_st8(sf_set + 32 + 8 * tsel, sfb);
-#pragma unroll
-                    for (int kb = 0; kb < 4; ++kb) {
-                        *reinterpret_cast<uint4 *>(st + a_off[2 * kb]) = make_uint4(R[9 * kb + 1], R[9 * kb + 2], R[9 * kb + 3], R[9 * kb + 4]);
-                        *reinterpret_cast<uint4 *>(st + a_off[2 * kb + 1]) = make_uint4(R[9 * kb + 5], R[9 * kb + 6], R[9 * kb + 7], R[9 * kb + 8]);
-                    }
-                    tmem_wait_st();
-                    tc_fence_before();
-                    // every writer orders its own stores against the tensor core's (async proxy) reads and then arrives itself
-                    fence_async_smem();
-                    mbar_arrive(&tile_full[tile.stage]);
-                    tile.template advance<TS>();
-                }
+                FP4_PROF_T0();
+                if (!__all_sync(0xffffffffu, wait_or_abort(&raw_full[raw.stage], raw.phase, &s_abort, p.err))) break;
+                FP4_PROF_ADD(0);
             }
+            uint4 * const src = reinterpret_cast<uint4 *>(raws + (size_t) raw.stage * C::RAW_STAGE + raw_off);
+            uint32_t R[36];                // 4 blocks of [scale word][8 code words]
+#pragma unroll
+            for (int j = 0; j < 9; ++j) {
+                const uint4 v = src[j];
+                R[4 * j] = v.x; R[4 * j + 1] = v.y; R[4 * j + 2] = v.z; R[4 * j + 3] = v.w;
+            }
+            // the row's four scale words, for the scale warps, into the first 16 bytes of the raw row, which this thread has just read
+            uint32_t S[4];
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb) {
+                // The reference reads scale bytes through ggml_ue4m3_to_fp32: bit 7 ignored, 0x7f decodes to zero; to the tensor
+                // core 0x7f is NaN.  Clear bit 7 and turn 0x7f into 0 (t <= 0x7f per byte, so t + 1 carries into bit 7 only
+                // for 0x7f and never into the next byte).
+                const uint32_t t = R[9 * kb] & 0x7f7f7f7fu;
+                const uint32_t nan1 = ((t + 0x01010101u) >> 7) & 0x01010101u;
+                S[kb] = t & ~((nan1 << 7) - nan1);
+            }
+            *src = make_uint4(S[0], S[1], S[2], S[3]);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sf_ready[raw.stage]);
+            raw.template advance<RS>();
+            {
+                FP4_PROF_T0();
+                if (!__all_sync(0xffffffffu, wait_or_abort(&tile_empty[tile.stage], tile.phase ^ 1u, &s_abort, p.err))) break;
+                FP4_PROF_ADD(1);
+            }
+            uint8_t * st = tiles + (size_t) tile.stage * C::STAGE;
+#pragma unroll
+            for (int kb = 0; kb < 4; ++kb) {
+                *reinterpret_cast<uint4 *>(st + (a_off ^ (32 * kb))) = make_uint4(R[9 * kb + 1], R[9 * kb + 2], R[9 * kb + 3], R[9 * kb + 4]);
+                *reinterpret_cast<uint4 *>(st + (a_off ^ (32 * kb + 16))) = make_uint4(R[9 * kb + 5], R[9 * kb + 6], R[9 * kb + 7], R[9 * kb + 8]);
+            }
+            // every writer orders its own stores against the tensor core's (async proxy) reads and then arrives itself
+            fence_async_smem();
+            mbar_arrive(&tile_full[tile.stage]);
+            tile.template advance<TS>();
         }
-        if (tid == 256) FP4_PROF_STORE(10, 3);
+        if (tid == 256) FP4_PROF_STORE(10, 2);
+    } else if (warp >= 16) {
+        // ---------------------------------------------------------------- scale factors: registers -> tensor memory
+        // One warp per lane quarter of tensor memory; each writes all of a stage's scales to its quarter.  Lane l holds those of rows l,
+        // l + 32, l + 64 and l + 96 of either weight tile (what tcgen05.cp 32x128b.warpx4 would put there) and of the planes.
+        const uint32_t quarter = (uint32_t) ((warp & 3) * 32) << 16;
+        Ring raw, tile, act;
+        FP4_PROF_DECL();
+        for (int i = 0; i < my_stages && !s_abort; ++i) {
+            {
+                FP4_PROF_T0();
+                if (!__all_sync(0xffffffffu, wait_or_abort<20>(&sf_ready[raw.stage], raw.phase, &s_abort, p.err))) break;
+                FP4_PROF_ADD(0);
+            }
+            const uint8_t * rows = raws + (size_t) raw.stage * C::RAW_STAGE + lane * GEMM_RAW_ROW;
+            uint4 a[2][4];
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                uint4 r[4];                // [row l + 32 j][K = 64 step]
+#pragma unroll
+                for (int j = 0; j < 4; ++j) r[j] = *reinterpret_cast<const uint4 *>(rows + (128 * t + 32 * j) * GEMM_RAW_ROW);
+                a[t][0] = make_uint4(r[0].x, r[1].x, r[2].x, r[3].x);
+                a[t][1] = make_uint4(r[0].y, r[1].y, r[2].y, r[3].y);
+                a[t][2] = make_uint4(r[0].z, r[1].z, r[2].z, r[3].z);
+                a[t][3] = make_uint4(r[0].w, r[1].w, r[2].w, r[3].w);
+            }
+            fence_async_smem();            // the next copy into this stage comes behind the words written to it
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&raw_empty[raw.stage]);
+            raw.template advance<RS>();
+            {
+                FP4_PROF_T0();
+                if (!__all_sync(0xffffffffu, wait_or_abort<20>(&act_full[act.stage], act.phase, &s_abort, p.err))) break;
+                FP4_PROF_ADD(1);
+            }
+            const uint8_t * sfb = acts + (size_t) act.stage * C::ACT_STAGE + OFF_SFB + lane * 16;
+            uint4 b[C::NBLK][4];
+#pragma unroll
+            for (int j = 0; j < 4 * C::NBLK; ++j) b[j >> 2][j & 3] = *reinterpret_cast<const uint4 *>(sfb + 512 * j);
+            act.template advance<AS>();
+            {
+                FP4_PROF_T0();
+                if (!__all_sync(0xffffffffu, wait_or_abort<20>(&tile_empty[tile.stage], tile.phase ^ 1u, &s_abort, p.err))) break;
+                FP4_PROF_ADD(2);
+            }
+            tc_fence_after();
+            const uint32_t sf_set = tmem + C::SF_COL + C::SF_SET * (uint32_t) tile.stage + quarter;
+            tmem_st16(sf_set, a[0]);
+            tmem_st16(sf_set + 16, a[1]);
+#pragma unroll
+            for (int n = 0; n < C::NBLK; ++n) tmem_st16(sf_set + 32 + 16 * n, b[n]);
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tile_full[tile.stage]);
+            tile.template advance<TS>();
+        }
+        if (tid == 512) FP4_PROF_STORE(13, 3);
     }
 
     // ---- teardown: everyone meets here (all waits above are bounded), then tensor memory goes back
