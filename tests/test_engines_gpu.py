@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from edge0_b200 import moe
+from edge0_b200 import workloads as W
 from edge0_b200.capi import TYPE_NVFP4, TYPE_Q3_K
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +62,59 @@ def test_q3k_matrix_instruction_keeps_the_bits(K, N, counts, ne11, gpu_ctx, chec
         aq = checker.quantize_activation(TYPE_Q3_K, b[t, 0])
         r = int(rng.integers(0, N))
         assert float(got[t, 0, r]) == checker.vec_dot(TYPE_Q3_K, K, w[rows[t, 0], r], aq)
+
+
+@pytest.mark.parametrize("T,n_ff,shape", [(96, 256, (512, 8, 2)), (108, 512, (256, 8, 2)), (109, 768, (768, 8, 2)), (433, 256, (512, 8, 2))])
+def test_fp4_large_token_tile(T, n_ff, shape, gpu_ctx):
+    """From 24 routed rows per expert on the FP4 kernels take tiles of 27 rows (N = 192, two blocks of plane scales): full, ragged and
+    one-row tiles.  With the fix-up and the integer down kernel the layer keeps the integer engine's bits; without them `hidden` stays
+    within the engine's fp32 accumulation error, 5e-5 of RMS."""
+    n_embd, n_expert, top_k = shape
+    cfg = W.small_config(TYPE_NVFP4, n_embd=n_embd, n_expert=n_expert, top_k=top_k, n_ff=n_ff, seed=T)
+    layer = W.make_layer(cfg).to_device(gpu_ctx)
+    x = torch.from_numpy(W.make_tokens(cfg, T)).cuda()
+    got = {}
+    try:
+        for path in (1, 6, 7):
+            gpu_ctx.set_expert_path(path)
+            out, ob = layer.forward(x, observe=True)
+            gpu_ctx.synchronize()
+            got[path] = (out.clone(), ob.hidden.clone())
+    finally:
+        gpu_ctx.set_expert_path(0)
+    assert torch.equal(got[7][0], got[1][0])
+    want = got[1][1]
+    assert float((got[6][1] - want).abs().max() / want.pow(2).mean().sqrt()) <= 5e-5
+
+
+@pytest.mark.parametrize("T,top_k", [(1, 1), (1, 16), (2, 8), (16, 1), (5, 3)])
+@pytest.mark.parametrize("wtype", [TYPE_NVFP4, TYPE_Q3_K])
+def test_few_rows_summed_in_the_down_kernel(T, top_k, wtype, gpu_ctx, checker):
+    """Up to 16 routed rows the CTA that finishes a token's last row sums them: the reference's bits, repeatedly."""
+    cfg = W.small_config(wtype, n_embd=512, n_expert=16, top_k=top_k, n_ff=256, seed=T * 32 + top_k)
+    layer = W.make_layer(cfg, quantize_q3k=(lambda w: checker.quantize(TYPE_Q3_K, w)) if wtype == TYPE_Q3_K else None)
+    x = W.make_tokens(cfg, T)
+    want = checker.moe_layer(x=x, **layer.checker_kwargs()).out
+    dl = layer.to_device(gpu_ctx)
+    for _ in range(3):
+        out = dl.forward(torch.from_numpy(x).cuda())
+        gpu_ctx.synchronize()
+        assert np.array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("E,top_k", [(8, 2), (40, 4), (200, 8), (512, 10), (1000, 6)])
+def test_routing_does_not_depend_on_the_batch(E, top_k, gpu_ctx):
+    """Logits, probabilities, choice and weights of a token are the same bits whatever kernel and tile its batch takes (few-token chains,
+    16 x 8 and 32 x 16 tiles, ragged edges, one block or several for the grouping), for fp32 and bf16 tokens."""
+    rng = np.random.default_rng(E)
+    none = np.zeros((E, 256, 144), np.uint8)
+    layer = moe.MoeLayer(gpu_ctx, wtype=TYPE_NVFP4, top_k=top_k, router_w=rng.normal(0, 0.05, (E, 256)).astype(np.float32), gate=none, up=none, down=none)
+    for dtype in (torch.float32, torch.bfloat16):
+        x = torch.from_numpy(rng.normal(0, 1, (1201, 256)).astype(np.float32)).cuda().to(dtype)
+        whole = None
+        for n in (1201, 1, 2, 9, 17, 33, 130, 300):
+            _, ob = layer.forward(x[:n].contiguous(), observe=True)
+            gpu_ctx.synchronize()
+            now = [ob.logits.clone(), ob.probs.clone(), ob.topk.clone(), ob.weights_norm.clone()]
+            whole = whole or now
+            assert all(torch.equal(a, b[:n]) for a, b in zip(now, whole)), n
