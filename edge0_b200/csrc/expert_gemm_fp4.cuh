@@ -29,7 +29,7 @@
 //                tile, into a ring of its own that runs three stages ahead (the planes come from L2 with about a microsecond of latency)
 //   warp 2       MMA issuer: two tcgen05.mma per K = 64 step
 //   warp 3       owns tensor memory
-//   warps 4-7    epilogue
+//   warps 4-7, 20-23  epilogue
 //   warps 8-15   repack: thread = one weight row of one tile; 9 x 16-byte loads, 8 x 16-byte stores, the row's scale words set aside
 //   warps 16-19  scale factors: from shared memory through registers into tensor memory (tcgen05.st)
 // The scales go through registers because a tcgen05.cp holds its issuing thread ~80 cycles: twelve per stage in front of the MMAs cost
@@ -54,7 +54,7 @@ constexpr int FP4_RPT_SMALL = TOKEN_TILE_SMALL, FP4_RPT_LARGE = TOKEN_TILE_LARGE
 constexpr int FP4_SF_TILE = 4 * 512;              // scale factors of 128 rows for the four K = 64 steps of a stage
 // bytes of one token tile's scale factors per K = 256 stage: one block of 128 plane rows, or two
 __host__ __device__ constexpr int fp4_sfb_bytes(int rpt) { return (FP4_PLANES * rpt + 127) / 128 * FP4_SF_TILE; }
-constexpr int FP4_THREADS = 640;
+constexpr int FP4_THREADS = 768;
 
 __device__ __forceinline__ void umma_fp4(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t sfa, uint32_t sfb,
                                          bool accumulate) {
@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const flo
     const int lrow = tid / tpr, t_in = tid % tpr;
     const int arow = blockIdx.x * rpb + lrow;
     const int n_dst = n_ids / ne11;
+    const int dst_step = gridDim.y, dst0 = blockIdx.y;    // few rows: the blocks of a column store every dst_step-th routed row each
     if (tid < 8) s_E[tid] = -1000;
     const bool live = lrow < rpb && arow < act_rows;   // threads beyond the block's last whole row idle (K = 768)
     if (live && t_in < n_dst) {
@@ -352,7 +353,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
         for (int i = 0; i < RS; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4); mbar_init(&sf_ready[i], 8); }
         for (int i = 0; i < TS; ++i) { mbar_init(&tile_full[i], 256 + 4); mbar_init(&tile_empty[i], 1); }
         for (int i = 0; i < AS; ++i) { mbar_init(&act_full[i], 1); mbar_init(&act_empty[i], 1); }
-        for (int i = 0; i < NACC; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
+        for (int i = 0; i < NACC; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
         mbar_fence_init();
         s_abort = 0;
     }
@@ -400,7 +401,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                 const int row0 = w.e * p.n_out + w.ft * FEAT;
                 for (int kc = 0; kc < KC; ++kc) {
                     FP4_PROF_T0();
-                    if (!wait_or_abort<200>(&raw_empty[raw.stage], raw.phase ^ 1u, &s_abort, p.err)) break;
+                    if (!wait_or_abort<40>(&raw_empty[raw.stage], raw.phase ^ 1u, &s_abort, p.err)) break;
                     FP4_PROF_ADD(0);
                     uint8_t * dst = raws + (size_t) raw.stage * C::RAW_STAGE;
                     mbar_arrive_expect_tx(&raw_full[raw.stage], C::RAW_STAGE);
@@ -422,7 +423,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                 const uint8_t * sft = p.sf + (size_t) w.tile * KC * C::SFB;
                 for (int kc = 0; kc < KC; ++kc) {
                     FP4_PROF_T0();
-                    if (!wait_or_abort<100>(&act_empty[act.stage], act.phase ^ 1u, &s_abort, p.err)) break;
+                    if (!wait_or_abort<40>(&act_empty[act.stage], act.phase ^ 1u, &s_abort, p.err)) break;
                     FP4_PROF_ADD(0);
                     uint8_t * st = acts + (size_t) act.stage * C::ACT_STAGE;
                     mbar_arrive_expect_tx(&act_full[act.stage], C::B_BYTES + C::SFB);
@@ -483,11 +484,14 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
             }
             FP4_PROF_STORE(4, 3);
         }
-    } else if (warp >= 4 && warp < 8) {
+    } else if ((warp >= 4 && warp < 8) || warp >= 20) {
         // ---------------------------------------------------------------- epilogue
         Ring acc;
         FP4_PROF_DECL();
         const int q = warp & 3;                 // TMEM lane quarter this warp may read
+        // two warps per quarter: the first takes the tile's first rows, the second the rest
+        constexpr int HALF = (RPT + 7) / 8 * 4;
+        const int first = warp >= 20 ? HALF : 0;
         for (int u = blockIdx.x; u < n_units && !s_abort; u += gridDim.x) {
             const Unit w = unit_at(u);
             const float sc0 = p.scale0 ? p.scale0[w.e] : 1.0f;
@@ -506,34 +510,33 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
             const uint32_t d0 = tmem + (uint32_t) acc.stage * (2 * C::NCOL) + ((uint32_t) (q * 32) << 16);
             // The planes of every routed row are folded first and the accumulators given back before anything else is done with the
             // sums: with a single accumulator buffer the next unit's instructions wait for this loop.
-            float x0[RPT], x1[RPT];
+            float x0[HALF], x1[HALF];
 #pragma unroll
-            for (int g = 0; g < RPT; g += 4)              // four routed rows = 28 plane columns per load (the last load may read past the tile's columns)
-                if (g < w.nt) {
-                    auto fold = [&](uint32_t col, float (&x)[RPT]) {
+            for (int j = 0; j < HALF; j += 4)             // four routed rows = 28 plane columns per load (the last load may read past the tile's columns)
+                if (first + j < w.nt) {
+                    auto fold = [&](uint32_t col, float (&x)[HALF]) {
                         float v[32];
                         tmem_ld32(col, v);
 #pragma unroll
-                        for (int rr = 0; rr < 4; ++rr)
-                            if (g + rr < RPT) {
-                                float a = v[7 * rr + 6];     // sum_p 8^p * plane_p, highest plane first
+                        for (int rr = 0; rr < 4; ++rr) {
+                            float a = v[7 * rr + 6];     // sum_p 8^p * plane_p, highest plane first
 #pragma unroll
-                                for (int pl = 5; pl >= 0; --pl) a = __fmaf_rn(a, 8.0f, v[7 * rr + pl]);
-                                x[g + rr] = a;
-                            }
+                            for (int pl = 5; pl >= 0; --pl) a = __fmaf_rn(a, 8.0f, v[7 * rr + pl]);
+                            x[j + rr] = a;
+                        }
                     };
-                    fold(d0 + FP4_PLANES * g, x0);
-                    fold(d0 + C::NCOL + FP4_PLANES * g, x1);
+                    fold(d0 + FP4_PLANES * (first + j), x0);
+                    fold(d0 + C::NCOL + FP4_PLANES * (first + j), x1);
                 }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[acc.stage]);
             acc.template advance<NACC>();
 #pragma unroll
-            for (int i = 0; i < RPT; ++i)
-                if (i < w.nt) {
-                    const float rs = __shfl_sync(0xffffffffu, my_rs, i);
-                    float * orow = p.out + (size_t) __shfl_sync(0xffffffffu, my_row, i) * p.n_out;
+            for (int i = 0; i < HALF; ++i)
+                if (first + i < w.nt) {
+                    const float rs = __shfl_sync(0xffffffffu, my_rs, first + i);
+                    float * orow = p.out + (size_t) __shfl_sync(0xffffffffu, my_row, first + i) * p.n_out;
                     const float v0 = __fmul_rn(__fmul_rn(x0[i], rs), sc0), v1 = __fmul_rn(__fmul_rn(x1[i], rs), sc1);
                     if (DUAL) orow[feature] = __fmul_rn(ggml_silu(v0), v1);
                     else { orow[feature] = v0; orow[feature + 128] = v1; }
@@ -593,7 +596,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
             tile.template advance<TS>();
         }
         if (tid == 256) FP4_PROF_STORE(10, 2);
-    } else if (warp >= 16) {
+    } else if (warp >= 16 && warp < 20) {
         // ---------------------------------------------------------------- scale factors: registers -> tensor memory
         // One warp per lane quarter of tensor memory; each writes all of a stage's scales to its quarter.  Lane l holds those of rows l,
         // l + 32, l + 64 and l + 96 of either weight tile (what tcgen05.cp 32x128b.warpx4 would put there) and of the planes.
