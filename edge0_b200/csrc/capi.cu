@@ -618,7 +618,9 @@ int launch_act_planes(b200moe_ctx * ctx, ActQuant act, const float * src, const 
     if (src && (((uintptr_t) src & 15) || src_stride % 4)) return fail(ctx, B200MOE_ERR_INVALID_ARG, "fp32 activation rows must be 16-byte aligned");
     const int rows_per_block = 256 / std::min(256, k / 8);
     const int act_rows = rows / n_ids * ne11;
-    const unsigned blocks = (unsigned) ((act_rows + rows_per_block - 1) / rows_per_block);
+    // few rows (8 tokens: 8 blocks): the routed rows of a token are shared out over further blocks, which work the digits out again
+    const int bx = (act_rows + rows_per_block - 1) / rows_per_block;
+    const dim3 blocks((unsigned) bx, (unsigned) std::max(1, std::min(n_ids / ne11, 2 * ctx->sm_count / std::max(1, bx))));
     if (src) act_planes_kernel<true><<<blocks, 256, 0, st>>>(act, src, src_stride, p.groups.pos, ids, p.groups.offsets, tiles, act_rows, k, n_ids, ne11, n_as, po, emit);
     else act_planes_kernel<false><<<blocks, 256, 0, st>>>(act, nullptr, 0, p.groups.pos, ids, p.groups.offsets, tiles, act_rows, k, n_ids, ne11, n_as, po, ActQuant{});
     return check_launch(ctx, "act_planes");

@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const flo
                     hi[u][m] = __float2int_rn(__fmul_rn(vb[m], id));
                 }
                 db[u] = __float_as_uint(d);
-                if (emit.q) {
+                if (emit.q && blockIdx.y == 0) {
                     int8_t * qo = emit.q + (size_t) arow * K + 16 * g + j0;
                     *reinterpret_cast<uint32_t *>(qo) = (uint32_t) (lo[u][0] & 0xff) | ((uint32_t) (lo[u][1] & 0xff) << 8) |
                                                         ((uint32_t) (lo[u][2] & 0xff) << 16) | ((uint32_t) (lo[u][3] & 0xff) << 24);
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const flo
             const int qd = t_in + tpr * u, g = qd >> 1;
             uint32_t words[FP4_PLANES];
             const uint8_t sb = plane_quad(lo[u], hi[u], db[u], E_row, words);
-            for (int j = 0; j < n_dst; ++j) {
+            for (int j = dst0; j < n_dst; j += dst_step) {
                 const int at = s_at[lrow][j];
                 if (at < 0) continue;
                 uint32_t * pw = reinterpret_cast<uint32_t *>(out.planes + (size_t) at * FP4_PLANES * (K / 2)) + qd;
