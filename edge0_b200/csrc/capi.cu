@@ -1030,13 +1030,14 @@ int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const 
     //   integer kernels   reproduce the reference's fp32 summation order: bit-identical to the CPU path; cost grows with the rows an
     //                     expert receives
     //   FP4 tensor cores  (tcgen05 kind::mxf4nvf4, expert_gemm_fp4.cuh): NVFP4 rows as they lie in HBM, activations as exact digit
-    //                     planes, 14 routed rows per pass over an expert; error = fp32 accumulation only (~5e-6 of RMS on `hidden`)
+    //                     planes, 14 or 27 routed rows per pass over an expert; error = fp32 accumulation only (~5e-6 of RMS on `hidden`)
     //   f16 tensor cores  (tcgen05 kind::f16, expert_gemm.cuh): weights dequantised to fp16, activations as fp16 hi + lo, up to 128
-    //                     routed rows per pass (~1.4e-4 of RMS on `hidden`): the prefill engine
+    //                     routed rows per pass (~1.4e-4 of RMS on `hidden`); only behind the paths that name it: with its wider fix-up
+    //                     margin a 4096-token prompt took 4.75 ms on it against 1.57 ms on the FP4 engine (777 tokens: 952 and 409 us)
     // After `down` nothing is re-quantised, so a tensor-core `down` only adds its own ~1e-5 to the output.  A tensor-core gate/up
     // moves a few values of `hidden` across int8 rounding boundaries of the reference's re-quantisation; the exact fix-up
-    // (requant_fixup.cuh) removes those flips where the bar needs it: beyond 4096 routed rows on the f16 engine, and on latent
-    // layers, which re-quantise once more after `down`.
+    // (requant_fixup.cuh) removes those flips where the bar needs it: beyond 4096 routed rows of a prompt, and on latent layers,
+    // which re-quantise once more after `down` (and keep `down` on the integer kernels at prompt sizes).
     const bool can_mma = mma_supported(l->wtype, n_in, l->n_ff) && mma_supported(l->wtype, l->n_ff, n_in);
     const bool can_fp4 = fp4_supported(l->wtype, n_in, l->n_ff);
     const int path = ctx->expert_path;

@@ -17,6 +17,9 @@
 // one table look-up per (row, sub-block) gives the eight possible products as 8 bytes and one byte permute picks four of
 // them.  Decode of step s + 1 and the copies of its activations run beside the matrix work of step s (two operand buffers, one
 // barrier per super-block); the raw rows of the next unit arrive by bulk copy meanwhile.
+// What it waits for is its own decode and shared memory at two warps per scheduler (0.32 instructions per cycle); sixteen warps of half
+// the tile were no faster (581 against 537 us), the A fragments then being read twice as often.  1001 tokens, 128 experts: gate/up
+// 2823 -> 537 us, down 1986 -> 305 us.
 // Operand rows are 272 bytes apart (256 + 16), which makes the 16-byte fragment loads conflict-free.
 #pragma once
 #include "common.cuh"
@@ -26,7 +29,10 @@
 
 namespace b200moe {
 
-constexpr int Q3K_MMA_MIN_ROWS = 8;   // routed rows per expert from which this kernel is used
+// Routed rows per expert (on average) from which this kernel replaces the GEMV, whose time grows with them while this one's does not up
+// to 64.  Gate/up (2048 -> 768), 128 experts: 4 rows GEMV 217 us, this 357; 8 rows 369 and 337; 16 rows 741 and 352; 63 rows 2825 and 537.
+// 16 experts: 8 rows 76 and 90 us, 16 rows 135 and 75.
+constexpr int Q3K_MMA_MIN_ROWS = 12;
 
 template <int K, bool DUAL>
 struct Q3kMmaCfg {
