@@ -218,7 +218,10 @@ constexpr float FIX_STEP_MARGIN = 0.015f;  // quantisation steps; largest GEMM e
 constexpr float FIX_REL_MARGIN = 1.2e-4f;  // of the block maximum; largest error measured: 3.0e-5 of it
 // after the block-scaled FP4 GEMM (exact digit planes; only fp32 accumulation differs):
 constexpr float FIX_STEP_MARGIN_FP4 = 2.5e-3f;  // largest error measured: 2.3e-4 steps (p99.99: 1.0e-4)
-constexpr int FP4_LARGE_TILE_ROWS = 24;    // routed rows per expert from which the FP4 kernels take the large token tile
+// Routed rows per expert (on average) from which the FP4 kernels take the large token tile: from there an expert's rows spill over into a
+// second small tile and its weights are repacked again.  128 experts, 2048 -> 768, gate/up and down in us, small tile against large: 8 rows
+// 64 + 37 and 74 + 39, 12 rows 70 + 43 and 74 + 41, 16 rows 84 + 52 and 76 + 41, 32 rows 127 + 78 and 104 + 57.
+constexpr int FP4_LARGE_TILE_ROWS = 14;
 
 constexpr float FIX_REL_MARGIN_FP4 = 2.0e-5f;   // largest error measured: 1.8e-6 of the block maximum
 

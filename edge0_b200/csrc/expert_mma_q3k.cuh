@@ -30,8 +30,8 @@
 namespace b200moe {
 
 // Routed rows per expert (on average) from which this kernel replaces the GEMV, whose time grows with them while this one's does not up
-// to 64.  Gate/up (2048 -> 768), 128 experts: 4 rows GEMV 217 us, this 357; 8 rows 369 and 337; 16 rows 741 and 352; 63 rows 2825 and 537.
-// 16 experts: 8 rows 76 and 90 us, 16 rows 135 and 75.
+// to 64.  Gate/up (2048 -> 768), 128 experts: 4 rows GEMV 217 us, this 357; 8 rows 369 and 366; 16 rows 741 and 362; 63 rows 2825 and 537.
+// 16 experts: 8 rows 76 and 110 us, 16 rows 135 and 110.
 constexpr int Q3K_MMA_MIN_ROWS = 12;
 
 template <int K, bool DUAL>

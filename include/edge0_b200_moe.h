@@ -122,20 +122,22 @@ B200MOE_API int  b200moe_synchronize(b200moe_ctx * ctx, void * stream); /* ggml_
 
 /* Which kernels run the expert matmuls (reference: model option switches such as `routing` / `experts`,
  * edge0-infer/docs/configuration.md:62-72; plain struct-style option, no environment variables).  Three engines exist:
- *   integer   dp4a kernels that follow the reference's fp32 summation order: bit-identical to the CPU path
+ *   integer   kernels that follow the reference's fp32 summation order: bit-identical to the CPU path (dp4a; Q3_K from 8 routed rows
+ *             per expert on the int8 matrix instruction)
  *   FP4       tcgen05 kind::mxf4nvf4 (block-scaled FP4 MMA, UE4M3 scale per 16): NVFP4 rows exactly as they lie in memory,
  *             activations as exact digit planes of the reference's int8 grid; differs from the integer engine only by fp32
- *             accumulation (~5e-6 of RMS on `hidden`); one pass over an expert's weights per 14 routed rows: batched decode
+ *             accumulation (~5e-6 of RMS on `hidden`); one pass over an expert's weights per 14 routed rows (batched decode) or
+ *             27 (from 14 routed rows per expert on average)
  *   f16       tcgen05 kind::f16: weights dequantised to fp16, activations as fp16 hi + lo (~1.4e-4 of RMS on `hidden`); one pass
- *             per 128 routed rows: prefill
+ *             per 128 routed rows; only behind the paths that name it
  * The reference re-quantises `hidden` to int8 before `down`, which turns a tensor-core gate/up's error into a few flipped
  * values; the "fix-up" recomputes every value of `hidden` within a safe margin of a rounding boundary or of its block's maximum
  * with the integer engine's arithmetic, so the quantised `hidden` is the reference's own.
- *   0  default.  Up to 16 routed rows (one or two tokens at top-8): integer (bit-identical).  Fewer than 24 routed rows per
- *      expert on average: FP4 for gate/up and down (output within ~3e-3 of RMS at 256 tokens; latent layers, which re-quantise
- *      once more after `down`, add the fix-up).  More: f16 for gate/up and down, with the fix-up beyond 4096 routed rows;
- *      latent layers add the fix-up and keep `down` on the integer engine.  Types or widths an engine has no kernel for
- *      (Q3_K; n_ff not a multiple of 128; n_in not a multiple of 256 for FP4, of 128 for f16) fall back to integer.
+ *   0  default.  Up to 16 routed rows (one or two tokens at top-8): integer (bit-identical).  More, NVFP4: FP4 for gate/up and
+ *      down (output within ~3e-3 of RMS at 256 tokens); the fix-up is added on latent layers, which re-quantise once more after
+ *      `down`, and beyond 4096 routed rows when experts see 24 or more on average; latent layers with that many keep `down` on the
+ *      integer engine.  Types or widths an engine has no kernel for (Q3_K; n_ff not a multiple of 128; n_in not a multiple of
+ *      256) fall back to integer.
  *      Dense products (b200moe_mul_mat, the latent projections) of NVFP4 matrices with at least 4 tokens use the FP4 engine
  *      under paths 0, 2, 3, 4, 6 and 8, the integer engine otherwise.
  *   1  integer everywhere: the whole layer is bit-identical to the reference CPU path

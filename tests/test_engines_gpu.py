@@ -66,7 +66,7 @@ def test_q3k_matrix_instruction_keeps_the_bits(K, N, counts, ne11, gpu_ctx, chec
 
 @pytest.mark.parametrize("T,n_ff,shape", [(96, 256, (512, 8, 2)), (108, 512, (256, 8, 2)), (109, 768, (768, 8, 2)), (433, 256, (512, 8, 2))])
 def test_fp4_large_token_tile(T, n_ff, shape, gpu_ctx):
-    """From 24 routed rows per expert on the FP4 kernels take tiles of 27 rows (N = 192, two blocks of plane scales): full, ragged and
+    """From 14 routed rows per expert on the FP4 kernels take tiles of 27 rows (N = 192, two blocks of plane scales): full, ragged and
     one-row tiles.  With the fix-up and the integer down kernel the layer keeps the integer engine's bits; without them `hidden` stays
     within the engine's fp32 accumulation error, 5e-5 of RMS."""
     n_embd, n_expert, top_k = shape
