@@ -740,7 +740,7 @@ int launch_select_group(b200moe_ctx * ctx, const b200moe_layer * l, int T, float
     Plan & p = ctx->plan;
     const int E = l->n_expert, K = l->n_expert_used;
     p.groups.tile_rows = token_tile_rows((int64_t) T * K, E);
-    p.groups.n_done = T * K <= 16 ? p.n_in : 0;
+    p.groups.n_done = T * K <= 16 ? T * (p.n_in / 16) : 0;
     const size_t sh = (size_t) E * sizeof(int);
 #define SELG(EPL) launch_k(ctx, route_select_group_kernel<EPL>, dim3(1), dim3(1024), sh, st, p.logits, E, K, T, p.ids, p.wts, probs, p.groups, ctx->d_err)
     if (E <= 32) SELG(1);
