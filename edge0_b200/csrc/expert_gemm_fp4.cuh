@@ -1,11 +1,11 @@
 // Grouped expert GEMM on the block-scaled FP4 tensor-core instruction (tcgen05.mma kind::mxf4nvf4, one UE4M3 scale per 16
-// elements, fp32 accumulators in tensor memory) for NVFP4 experts in batched decode.
+// elements, fp32 accumulators in tensor memory) for NVFP4 experts in batched decode and prefill.
 //
 // Why it fits: ggml's block_nvfp4 IS the operand format of that instruction - E2M1 codes, one UE4M3 scale per 16 elements
 // (ggml-common.h:221-227; the doubled code table and the halved scale decode of ggml-impl.h:514-527 cancel).  A weight row
 // needs no arithmetic at all before the MMA: the 4 scale bytes in front of every 32 code bytes are stripped while the row moves
-// from the raw TMA stage into the 128B-swizzled K-major operand tile, and collected as the scale-factor tile that tcgen05.cp
-// copies into tensor memory.  Element order inside a 16-block does not matter as long as both operands agree on it, so the
+// from the raw TMA stage into the 128B-swizzled K-major operand tile, and go to tensor memory as the instruction's scale
+// factors.  Element order inside a 16-block does not matter as long as both operands agree on it, so the
 // activations are simply stored in ggml's nibble order (byte j = elements j and j+8 of the block).
 //
 // Activations stay on the reference's int8 grid (q * d with d an fp16 number per 32 elements, the Q8_0 rows the CPU path
@@ -48,8 +48,8 @@
 namespace b200moe {
 
 constexpr int FP4_PLANES = 7;
-// Routed rows per token tile: 14 for batched decode (two accumulator buffers, so the epilogue runs beside the next unit), 27 for
-// prefill (N = 192 fills tensor memory with one buffer; a weight tile is repacked and fetched half as often per routed row).
+// Routed rows per token tile: 14 for few rows per expert (two accumulator buffers, so the epilogue runs beside the next unit), 27 for
+// more (N = 192 fills tensor memory with one buffer; a weight tile is repacked and fetched half as often per routed row).
 constexpr int FP4_RPT_SMALL = TOKEN_TILE_SMALL, FP4_RPT_LARGE = TOKEN_TILE_LARGE;
 constexpr int FP4_SF_TILE = 4 * 512;              // scale factors of 128 rows for the four K = 64 steps of a stage
 // bytes of one token tile's scale factors per K = 256 stage: one block of 128 plane rows, or two

@@ -43,11 +43,11 @@ class LayerConfig:
 CONFIGS = {
     # Q3_K decode
     "c1_q3k": LayerConfig("c1_q3k", TYPE_Q3_K, seed=101),
-    # configs[1]: NVFP4 batched decode
+    # NVFP4 batched decode
     "c2_nvfp4": LayerConfig("c2_nvfp4", TYPE_NVFP4, seed=102),
-    # configs[2]: NVFP4 prefill with per-expert logit bias
+    # NVFP4 prefill with per-expert logit bias
     "c3_nvfp4_prefill": LayerConfig("c3_nvfp4_prefill", TYPE_NVFP4, router_bias=True, seed=103),
-    # configs[4]: latent expert-parallel layer
+    # latent expert-parallel layer
     "c5_latent": LayerConfig("c5_latent", TYPE_NVFP4, n_embd=4096, n_latent=1024, n_expert=512, top_k=10, n_ff=1024, seed=105),
 }
 
