@@ -189,9 +189,9 @@ template <typename XT>
 __device__ __forceinline__ void quantize_q8_0_span(const XT * __restrict__ src, int8_t * __restrict__ q, float * __restrict__ d, int lane) {
     float v[8];
     load8(src + lane * 8, v);
-    float amax = 0.0f;
+    float amax = fabsf(v[0]);    // not zero: a block of nothing but NaN must come out with a NaN scale, as it does a value a lane
 #pragma unroll
-    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    for (int i = 1; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
     const float dd = __fdiv_rn(amax, 127.0f);

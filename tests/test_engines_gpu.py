@@ -118,3 +118,24 @@ def test_routing_does_not_depend_on_the_batch(E, top_k, gpu_ctx):
             now = [ob.logits.clone(), ob.probs.clone(), ob.topk.clone(), ob.weights_norm.clone()]
             whole = whole or now
             assert all(torch.equal(a, b[:n]) for a, b in zip(now, whole)), n
+
+
+@pytest.mark.parametrize("K", [256, 2048])
+def test_block_of_nan_keeps_its_nan(K, gpu_ctx):
+    """A block of 32 activations that are all NaN gets a NaN scale (a NaN among numbers is passed over), whether the quantiser takes one
+    value or eight values per lane: 16-byte aligned rows against the same rows four bytes further on."""
+    rng = np.random.default_rng(K)
+    E, N, T = 4, 32, 24
+    w = nvfp4_matrix(rng, E, N, K)
+    ids = torch.from_numpy(rng.integers(0, E, (T, 1)).astype(np.int32)).cuda()
+    flat = torch.from_numpy(rng.normal(0, 1, T * K + 4).astype(np.float32)).cuda()
+    got = []
+    for off in (0, 1):
+        b = flat[off:off + T * K].view(T, 1, K)
+        b.copy_(torch.from_numpy(np.random.default_rng(K + 1).normal(0, 1, (T, 1, K)).astype(np.float32)))
+        b[3, 0, 32:64] = float("nan")
+        b[5, 0, 7] = float("nan")
+        got.append(gpu_ctx.mul_mat_id(TYPE_NVFP4, w, b, ids, K))
+        gpu_ctx.synchronize()
+    assert bool(torch.isnan(got[0][3]).all()) and int(torch.isnan(got[0]).sum()) == N
+    assert torch.equal(torch.nan_to_num(got[0], nan=7.0), torch.nan_to_num(got[1], nan=7.0))
