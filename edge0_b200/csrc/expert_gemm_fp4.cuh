@@ -203,9 +203,9 @@ __global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const flo
                 const float * xrow = src + (size_t) arow * src_stride + 16 * g + j0;
                 const float4 a = *reinterpret_cast<const float4 *>(xrow), b = *reinterpret_cast<const float4 *>(xrow + 8);
                 const float va[4] = { a.x, a.y, a.z, a.w }, vb[4] = { b.x, b.y, b.z, b.w };
-                float amax = 0.0f;
+                float amax = fmaxf(fabsf(va[0]), fabsf(vb[0]));   // NaN only for a block of nothing else
 #pragma unroll
-                for (int m = 0; m < 4; ++m) amax = fmaxf(amax, fmaxf(fabsf(va[m]), fabsf(vb[m])));
+                for (int m = 1; m < 4; ++m) amax = fmaxf(amax, fmaxf(fabsf(va[m]), fabsf(vb[m])));
                 // the four quads of a 32-block sit in four consecutive lanes (all live or none: a row never splits a warp)
                 amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
                 amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
@@ -248,7 +248,9 @@ __global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const flo
     if (!live) return;
     const int E_row = s_E[lrow];
     if (t_in < n_dst && s_at[lrow][t_in] >= 0)
-        out.row_scale[s_at[lrow][t_in]] = E_row > -1000 ? __uint_as_float((uint32_t) (E_row - 8 + 127) << 23) : 0.0f;   // 2^(E_row - 8): far from the fp32 limits
+        // 2^(E_row - 8): far from the fp32 limits.  A block scale that is infinite or NaN has no digits: the row's results are NaN, which is
+        // what 0 * inf makes of them on the other engines (and in the reference).
+        out.row_scale[s_at[lrow][t_in]] = E_row == 255 - 137 ? __uint_as_float(0x7fc00000u) : E_row > -1000 ? __uint_as_float((uint32_t) (E_row - 8 + 127) << 23) : 0.0f;
     const int sfb_bytes = fp4_sfb_bytes(out.rpt);
 #pragma unroll
     for (int u = 0; u < MAX_QUADS; ++u)

@@ -139,3 +139,30 @@ def test_block_of_nan_keeps_its_nan(K, gpu_ctx):
         gpu_ctx.synchronize()
     assert bool(torch.isnan(got[0][3]).all()) and int(torch.isnan(got[0]).sum()) == N
     assert torch.equal(torch.nan_to_num(got[0], nan=7.0), torch.nan_to_num(got[1], nan=7.0))
+
+
+@pytest.mark.parametrize("T", [8, 120])     # token tiles of 14 and of 27 rows
+@pytest.mark.parametrize("path", [0, 6, 7, 8])
+def test_fp4_engine_keeps_what_is_not_finite(T, path, gpu_ctx):
+    """An infinite activation, one whose block scale overflows fp16 (above 8.3e6) and a block of NaN have no digits in the planes: those
+    tokens' outputs are not finite where the integer engine's are not, and the other tokens' outputs do not change."""
+    cfg = W.small_config(TYPE_NVFP4, n_embd=512, n_expert=16, top_k=4, n_ff=256, seed=5)
+    layer = W.make_layer(cfg).to_device(gpu_ctx)
+    rng = np.random.default_rng(T)
+    ids = torch.from_numpy(np.stack([rng.permutation(16)[:4] for _ in range(T)]).astype(np.int32)).cuda()
+    w = torch.full((T, 4), 0.25, device="cuda")
+    x = torch.from_numpy(W.make_tokens(cfg, T)).cuda()
+    bad = x.clone()
+    bad[1, 7], bad[3, 100], bad[5, 64:96] = float("inf"), 1e7, float("nan")
+    got = {}
+    try:
+        for p, tokens in ((1, bad), (path, bad), (path, x)):
+            gpu_ctx.set_expert_path(p)
+            got[p, tokens is bad] = layer.ffn(tokens, ids, w)
+            gpu_ctx.synchronize()
+    finally:
+        gpu_ctx.set_expert_path(0)
+    assert not torch.isfinite(got[1, True][[1, 3, 5]]).any()
+    assert torch.equal(torch.isfinite(got[path, True]), torch.isfinite(got[1, True]))
+    good = [t for t in range(T) if t not in (1, 3, 5)]
+    assert torch.equal(got[path, True][good], got[path, False][good])
