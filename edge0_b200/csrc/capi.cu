@@ -1010,6 +1010,7 @@ int launch_requant_fixup(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq
             case 768: rc = launch_fix_t<768>(ctx, *pass, st); break;
             case 1024: rc = launch_fix_t<1024>(ctx, *pass, st); break;
             case 2048: rc = launch_fix_t<2048>(ctx, *pass, st); break;
+            case 4096: rc = launch_fix_t<4096>(ctx, *pass, st); break;
             default: return fail(ctx, B200MOE_ERR_UNSUPPORTED, "no re-quantisation fix-up for width %d", n_in);
         }
         if (rc) return rc;

@@ -166,3 +166,20 @@ def test_fp4_engine_keeps_what_is_not_finite(T, path, gpu_ctx):
     assert torch.equal(torch.isfinite(got[path, True]), torch.isfinite(got[1, True]))
     good = [t for t in range(T) if t not in (1, 3, 5)]
     assert torch.equal(got[path, True][good], got[path, False][good])
+
+
+@pytest.mark.parametrize("T,bar", [(512, 1e-2), (513, 2e-4)])
+def test_width_4096_on_both_sides_of_the_fixup(T, bar, gpu_ctx, checker):
+    """A plain layer of the widest rows at 4096 routed rows (the last size without the re-quantisation fix-up: the stated bar of the path)
+    and beyond it (fix-up, then a tensor-core `down`: 2e-4 of RMS, the bar of its other tests).  Tokens are independent of each other, so
+    the first and last few stand for all."""
+    cfg = W.small_config(TYPE_NVFP4, n_embd=4096, n_expert=16, top_k=8, n_ff=256, seed=T)
+    layer = W.make_layer(cfg)
+    x = W.make_tokens(cfg, T)
+    out, ob = layer.to_device(gpu_ctx).forward(torch.from_numpy(x).cuda(), observe=True)
+    gpu_ctx.synchronize()
+    some = [0, 1, 2, T - 3, T - 2, T - 1]
+    want = checker.moe_layer(x=x[some], **layer.checker_kwargs())
+    for got, ref, limit in ((ob.hidden, want.hidden, 5e-5), (out, want.out, bar)):
+        got = got[some].cpu().numpy().astype(np.float64)
+        assert np.abs(got - ref).max() / np.sqrt((ref.astype(np.float64) ** 2).mean()) <= limit
