@@ -79,6 +79,7 @@ SIGNATURES = {
     "b200moe_ep_pack": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int64,
                                   C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "b200moe_ep_expert_rows": (C.c_int, [C.c_void_p, C.POINTER(Layer), C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]),
+    "b200moe_ep_expert_rows_expected": (C.c_int, [C.c_void_p, C.POINTER(Layer), C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]),
     "b200moe_ep_combine": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64,
                                      C.c_void_p, C.c_void_p]),
     "b200moe_ffn": (C.c_int, [C.c_void_p, C.POINTER(Layer), C.c_void_p, C.c_int, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p,

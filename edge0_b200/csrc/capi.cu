@@ -769,9 +769,10 @@ int launch_select(b200moe_ctx * ctx, const b200moe_layer * l, int T, int32_t * i
     return check_launch(ctx, "route_select");
 }
 
-int launch_group(b200moe_ctx * ctx, const int32_t * ids, int E, int rows, cudaStream_t st, bool allow_empty = false) {
+// expected_rows: how many of the `rows` slots are taken, about, where an exchange leaves some empty (sizes the token tile)
+int launch_group(b200moe_ctx * ctx, const int32_t * ids, int E, int rows, cudaStream_t st, bool allow_empty = false, int64_t expected_rows = -1) {
     Plan & p = ctx->plan;
-    p.groups.tile_rows = token_tile_rows(rows, E);
+    p.groups.tile_rows = token_tile_rows(expected_rows >= 0 ? expected_rows : rows, E);
     p.groups.n_done = rows <= 16 ? p.n_in : 0;
     const size_t sh = (size_t) E * sizeof(int);
     const int blocks = std::min(32, std::max(1, rows / 1024));
@@ -1022,12 +1023,15 @@ int launch_requant_fixup(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq
 // y_direct != null: the per-row results of `down` go there ([rows][n_in]) and the weighted combine is left to the caller
 // x_src != null: the activations are still fp32 (rows x_src_stride floats apart, indexed like xq's rows) and xq is only room for
 // their quantised form: the engine that runs gate/up quantises them on its way in
+// expected_rows: as for launch_group; it chooses among kernels with the same results, the engine is chosen by all rows
 int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const int32_t * ids, const float * wts, int T, float * out,
-                 const b200moe_observe * ob, cudaStream_t st, float * y_direct = nullptr, const float * x_src = nullptr, int64_t x_src_stride = 0) {
+                 const b200moe_observe * ob, cudaStream_t st, float * y_direct = nullptr, const float * x_src = nullptr, int64_t x_src_stride = 0,
+                 int64_t expected_rows = -1) {
     Plan & p = ctx->plan;
     float * const y = y_direct ? y_direct : p.y;
     const int n_in = l->n_latent ? l->n_latent : l->n_embd;
     const int k = l->n_expert_used, rows = T * k;
+    const int64_t likely_rows = expected_rows >= 0 ? expected_rows : rows;
     const int nt = tokens_per_pass(rows, l->n_expert);
     int rc;
     // Which engine runs which matmul (b200moe_set_expert_path documents the paths).
@@ -1089,12 +1093,12 @@ int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const 
         if ((rc = tm_gu ? launch_gemm_tm<true>(ctx, n_in, m, rows, st) : launch_gemm<true>(ctx, n_in, m, rows, small_tiles, st))) return rc;
     } else {
         GemvParams gu = gemv_params(ctx, l->gate, l->up, l->gate_scale, l->up_scale, xq, p.hid, l->n_ff, k, 1, l->n_expert);
-        if ((rc = launch_integer<true>(ctx, l->wtype, n_in, gu, rows, l->n_expert, nt, st))) return rc;
+        if ((rc = launch_integer<true>(ctx, l->wtype, n_in, gu, likely_rows, l->n_expert, nt, st))) return rc;
     }
     if (fixup && (rc = launch_requant_fixup(ctx, l, xq, rows, n_in, k, fp4_gu, st))) return rc;
     // The integer down kernel quantises `hidden` itself while staging it (NVFP4 / Q8_0; Q3_K / Q8_K for the few rows of one or two
     // tokens); otherwise a separate pass.  With so few rows it also sums a token's rows (GemvParams::comb_out).
-    const bool tiny_down = !mma_down && !fp4_down && nt < 0 && !q3k_on_mma(l->wtype, rows, l->n_expert);
+    const bool tiny_down = !mma_down && !fp4_down && nt < 0 && !q3k_on_mma(l->wtype, likely_rows, l->n_expert);
     const bool fused_quant = !mma_down && !fp4_down && (l->wtype == TYPE_NVFP4 || tiny_down);
     const bool fused_combine = tiny_down && !y_direct;
     if (!fused_quant && !fp4_down && (rc = launch_quantize<float>(ctx, p.hid, l->n_ff, p.hq, rows, l->n_ff, l->wtype, st))) return rc;
@@ -1109,7 +1113,7 @@ int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const 
         GemvParams dn = gemv_params(ctx, l->down, nullptr, l->down_scale, nullptr, p.hq, y, n_in, k, k, l->n_expert);
         if (fused_quant) dn.act_f32 = p.hid;
         if (fused_combine) { dn.comb_out = out; dn.comb_w = wts; dn.comb_cnt = p.groups.done; }
-        if ((rc = launch_integer<false>(ctx, l->wtype, l->n_ff, dn, rows, l->n_expert, nt, st))) return rc;
+        if ((rc = launch_integer<false>(ctx, l->wtype, l->n_ff, dn, likely_rows, l->n_expert, nt, st))) return rc;
     }
     if (!y_direct && !fused_combine) {
         dim3 grid((n_in / 4 + 255) / 256, T);
@@ -1701,11 +1705,17 @@ int b200moe_ep_pack(b200moe_ctx * ctx, const float * rows, const int32_t * ids, 
 }
 
 int b200moe_ep_expert_rows(b200moe_ctx * ctx, const b200moe_layer * l, const void * slots, int64_t n_slots, float * y, void * stream) {
+    return b200moe_ep_expert_rows_expected(ctx, l, slots, n_slots, n_slots, y, stream);
+}
+
+int b200moe_ep_expert_rows_expected(b200moe_ctx * ctx, const b200moe_layer * l, const void * slots, int64_t n_slots, int64_t expected_rows, float * y,
+                                    void * stream) {
     int rc = validate_layer(ctx, l, false, true);
     if (rc) return rc;
     if (l->n_latent) return fail(ctx, B200MOE_ERR_INVALID_ARG, "the owner's layer is the plain expert layer of the exchanged width");
     if (n_slots == 0) return B200MOE_OK;
     if (!slots || !y || n_slots < 0 || n_slots > (1 << 30)) return fail(ctx, B200MOE_ERR_INVALID_ARG, "null pointer or bad slot count");
+    if (expected_rows < 0 || expected_rows > n_slots) return fail(ctx, B200MOE_ERR_INVALID_ARG, "expected rows outside 0 .. slots");
     if ((uintptr_t) slots & 15) return fail(ctx, B200MOE_ERR_INVALID_ARG, "slots must be 16-byte aligned");
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     ctx->overlap_now = false;
@@ -1719,9 +1729,9 @@ int b200moe_ep_expert_rows(b200moe_ctx * ctx, const b200moe_layer * l, const voi
     CUDA_TRY(ctx, cudaMemsetAsync(p.groups.counts, 0, sizeof(int) * l->n_expert, st));
     count_ids_kernel<<<(R + 255) / 256, 256, 0, st>>>(ids, slot_words, 1, R, l->n_expert, p.ids, p.groups.counts, p.groups.pos, ctx->d_err, 1);
     if ((rc = check_launch(ctx, "count_ids"))) return rc;
-    if ((rc = launch_group(ctx, p.ids, l->n_expert, R, st, true))) return rc;
+    if ((rc = launch_group(ctx, p.ids, l->n_expert, R, st, true, expected_rows))) return rc;
     // the slots' rows are quantised by whichever engine runs gate/up (empty slots hold garbage nobody reads)
-    rc = experts_impl(ctx, l, p.xq, p.ids, nullptr, R, nullptr, nullptr, st, y, rows, slot_words);
+    rc = experts_impl(ctx, l, p.xq, p.ids, nullptr, R, nullptr, nullptr, st, y, rows, slot_words, expected_rows);
     account(ctx, l, 0);
     return rc;
 }

@@ -166,7 +166,7 @@ class CudaBackend:
     def __init__(self, ctx, host_layer, rank: int = 0, world: int = 1):
         from . import moe
         cfg = host_layer.cfg
-        self.ctx, self.cfg = ctx, cfg
+        self.ctx, self.cfg, self.world = ctx, cfg, world
         if cfg.n_latent:
             # The owner of an expert sees a plain layer of the latent width and cannot know that its rows are re-quantised
             # again by the up-projection on the token's rank: pin what the library does by default for a latent layer it sees
@@ -241,7 +241,8 @@ class CudaBackend:
 
     def expert_rows(self, slots):
         y = self._get("y", (slots.shape[0], self.cfg.n_in), torch.float32, zero=True)
-        return self.local.ep_expert_rows(slots, y)
+        # every peer's slots are sized for all of its rows going to one owner; evenly routed, one in `world` is taken
+        return self.local.ep_expert_rows(slots, y, expected_rows=-(-slots.shape[0] // self.world))
 
     def combine(self, back, slot_of, w):
         return self.ctx.ep_combine(back, slot_of, w)

@@ -376,13 +376,15 @@ class MoeLayer:
         c.check(c.lib.b200moe_latent_up(c.handle, C.byref(self.desc), _ptr(m), T, _ptr(out), c._stream()))
         return out
 
-    def ep_expert_rows(self, slots: torch.Tensor, y: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """slots uint8 [n_slots, slot_bytes] as received from the exchange -> float32 [n_slots, n_in] (rows of empty slots untouched)."""
+    def ep_expert_rows(self, slots: torch.Tensor, y: Optional[torch.Tensor] = None, expected_rows: Optional[int] = None) -> torch.Tensor:
+        """slots uint8 [n_slots, slot_bytes] as received from the exchange -> float32 [n_slots, n_in] (rows of empty slots untouched).
+        expected_rows: about how many slots are taken (default: all); results do not depend on it."""
         n_slots = slots.numel() // slots.shape[-1]
         if y is None:
             y = torch.zeros((n_slots, self.n_in), dtype=torch.float32, device=slots.device)
         c = self.ctx
-        c.check(c.lib.b200moe_ep_expert_rows(c.handle, C.byref(self.desc), _ptr(slots), n_slots, _ptr(y), c._stream()))
+        c.check(c.lib.b200moe_ep_expert_rows_expected(c.handle, C.byref(self.desc), _ptr(slots), n_slots,
+                                                      n_slots if expected_rows is None else expected_rows, _ptr(y), c._stream()))
         return y
 
     def forward(self, x: torch.Tensor, observe: bool = False, out: Optional[torch.Tensor] = None):

@@ -267,6 +267,11 @@ B200MOE_API int b200moe_ep_pack(b200moe_ctx * ctx, const float * rows, const int
  * the arithmetic of b200moe_ffn with one slot of weight 1.  y F32 [width, n_slots]; rows of empty slots are left untouched. */
 B200MOE_API int b200moe_ep_expert_rows(b200moe_ctx * ctx, const b200moe_layer * layer, const void * slots, int64_t n_slots, float * y,
                                        void * stream);
+/* The same for a caller that knows about how many slots are taken (n_slots / N after an exchange among N ranks, whose slots are
+ * sized for the case that every row goes to one of them).  The number only chooses among kernels with the same results, by the rows an
+ * expert is likely to have; b200moe_ep_expert_rows takes every slot for a row.  0 <= expected_rows <= n_slots. */
+B200MOE_API int b200moe_ep_expert_rows_expected(b200moe_ctx * ctx, const b200moe_layer * layer, const void * slots, int64_t n_slots,
+                                                int64_t expected_rows, float * y, void * stream);
 /* Back on the token's rank: out[:, t] = sum over s = 0..k-1, in that order, of back[:, slot_of[s, t]] * weights[s, t]
  * (the tail of Builder::ffn, forward.cpp:308-310, behind an index).  back F32 [width, n_slots]. */
 B200MOE_API int b200moe_ep_combine(b200moe_ctx * ctx, const float * back, int64_t n_slots, const int32_t * slot_of, const float * weights,

@@ -1,4 +1,6 @@
 """Kernels at the sizes where they can go wrong: edges of tiles, remainders, the ends of the range of a dispatch rule."""
+import re
+
 import numpy as np
 import pytest
 import torch
@@ -6,6 +8,7 @@ import torch
 from edge0_b200 import moe
 from edge0_b200 import workloads as W
 from edge0_b200.capi import TYPE_NVFP4, TYPE_Q3_K
+from edge0_b200.expert_parallel import SLOT_EXTRA_WORDS
 
 pytestmark = pytest.mark.gpu
 
@@ -183,3 +186,48 @@ def test_width_4096_on_both_sides_of_the_fixup(T, bar, gpu_ctx, checker):
     for got, ref, limit in ((ob.hidden, want.hidden, 5e-5), (out, want.out, bar)):
         got = got[some].cpu().numpy().astype(np.float64)
         assert np.abs(got - ref).max() / np.sqrt((ref.astype(np.float64) ** 2).mean()) <= limit
+
+
+@pytest.mark.parametrize("wtype", [TYPE_NVFP4, TYPE_Q3_K])
+def test_expert_parallel_kernels_follow_the_rows_that_exist(wtype, gpu_ctx):
+    """The owner of 16 of 128 experts receives 8 x 80 slots of which 80 hold a row: five rows per expert, not forty.  The FP4 kernels take the
+    tile of few rows and Q3_K the integer GEMV, as they do for 80 rows that come without empty slots; the results are the same bits
+    whatever the expected number of rows."""
+    cfg = W.small_config(wtype, n_embd=512, n_expert=16, top_k=1, n_ff=256, seed=8)
+    rng = np.random.default_rng(8)
+    none = np.zeros((16, 512), np.float32)
+    if wtype == TYPE_NVFP4:
+        mats = [nvfp4_matrix(rng, 16, r, c) for r, c in ((256, 512), (256, 512), (512, 256))]
+    else:
+        mats = []
+        for r, c in ((256, 512), (256, 512), (512, 256)):
+            m = rng.integers(0, 256, (16, r, c // 256, 110), dtype=np.uint8)
+            m[..., 108:110] = rng.normal(0, 1e-4, (16, r, c // 256, 1)).astype(np.float16).view(np.uint8)
+            mats.append(torch.from_numpy(m.reshape(16, r, -1)).cuda())
+    layer = moe.MoeLayer(gpu_ctx, wtype=wtype, top_k=1, router_w=none, gate=mats[0], up=mats[1], down=mats[2])
+    world, cap = 8, 80
+    words = np.zeros((world, cap, cfg.n_embd + SLOT_EXTRA_WORDS), np.float32)
+    words[..., :cfg.n_embd] = rng.normal(0, 1, (world, cap, cfg.n_embd))
+    ids = np.full((world, cap), -1, np.int32)
+    ids[:, :10] = rng.permutation(np.repeat(np.arange(16), 5)).reshape(world, 10)
+    words.view(np.int32)[..., cfg.n_embd] = ids
+    slots = torch.from_numpy(words.reshape(world * cap, -1).view(np.uint8)).cuda()
+    taken = slots[torch.from_numpy(ids.reshape(-1) >= 0).cuda()].contiguous()
+    few = "expert_gemm_fp4_kernel.*(14>|Li14E)" if wtype == TYPE_NVFP4 else "expert_gemv_kernel"
+    many = "expert_gemm_fp4_kernel.*(27>|Li27E)" if wtype == TYPE_NVFP4 else "expert_mma_q3k_kernel"
+    got = {}
+    gpu_ctx.set_expert_path(8 if wtype == TYPE_NVFP4 else 0)
+    try:
+        for name, s, expected, want in (("all", slots, None, many), ("few", slots, cap, few), ("packed", taken, None, few)):
+            layer.ep_expert_rows(s, expected_rows=expected)
+            gpu_ctx.synchronize()
+            with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+                got[name] = layer.ep_expert_rows(s, expected_rows=expected)
+                gpu_ctx.synchronize()
+            kernels = [e.key for e in prof.key_averages()]
+            for pattern in (few, many):
+                assert any(re.search(pattern, k) for k in kernels) == (pattern == want), (name, kernels)
+    finally:
+        gpu_ctx.set_expert_path(0)
+    assert torch.equal(got["all"], got["few"])
+    assert torch.equal(got["few"][torch.from_numpy(ids.reshape(-1) >= 0).cuda()], got["packed"])
