@@ -682,6 +682,11 @@ int launch_logits_smem(b200moe_ctx * ctx, const float * w, const float * bias, c
     return check_launch(ctx, "router_logits");
 }
 
+// Values of an F32 matrix from which it streams from HBM (beyond the 126 MB L2): half the loads in flight per lane and half as many warps
+// again on an SM.  Eight steps and four, 2 and 8 tokens, us: 8192 x 4096 (134 MB) 55, 92 and 57, 98; 16384 x 3072 (201 MB) 74, 125 and 64, 113;
+// 131072 x 2048 (1 GB) 295, 573 and 254, 483.
+constexpr int64_t ROUTER_STREAMED = 40 << 20;
+
 // F32 matrix times a batch in the reference's summation order: logits [T][E] = W [E][H] . x [T][H] (+ bias)
 template <typename XT>
 int launch_logits_any(b200moe_ctx * ctx, const float * w, const float * bias, const XT * x, float * logits, int H, int E, int T, int * zero_buf,
@@ -693,8 +698,11 @@ int launch_logits_any(b200moe_ctx * ctx, const float * w, const float * bias, co
         if (big >= ctx->sm_count) return launch_logits_smem<4, 2, 8, XT>(ctx, w, bias, x, logits, H, E, T, zero_buf, zero_n, quant, kind, st);
         return launch_logits_smem<2, 2, 4, XT>(ctx, w, bias, x, logits, H, E, T, zero_buf, zero_n, quant, kind, st);
     }
-    // few tokens or a single row: one warp per (expert, token) with deep load prefetch; otherwise 4 tokens share each weight load
-    const int tt = T <= 8 || E < 8 ? 1 : 4;
+    // few tokens or a single row: one warp per (expert, token) with deep load prefetch; otherwise 4 tokens share each weight load.  The
+    // lone tokens read the matrix again for each of them, which pays while about all their warps are resident together.  fp32, a token
+    // and four tokens to a warp, us: 512 x 4096, 8 tokens 16.4 and 24.6; 2048 x 2048, 4 tokens 16.4 and 18.4, 8 tokens 23.5 and 18.4;
+    // 8192 x 2048, 2 tokens 30.7 and 32.8, 4 tokens 45 and 35; 32768 x 2048, 2 tokens 98 and 74, 8 tokens 332 and 137.
+    const int tt = T == 1 || E < 8 || (T <= 8 && (int64_t) E * (T - 1) <= 64 * ctx->sm_count) ? 1 : 4;
     const int lblocks = (int) (((int64_t) E * ((T + tt - 1) / tt) + 7) / 8);
     if (quant.q) {
         const int spans = quant_spans(x, H, H) ? 1 : 0;
@@ -710,6 +718,7 @@ int launch_logits_any(b200moe_ctx * ctx, const float * w, const float * bias, co
         return check_launch(ctx, "router_logits");
     }
     if (tt == 1) launch_k(ctx, router_logits_kernel<1, XT>, dim3(lblocks), dim3(256), 0, st, w, bias, x, logits, H, E, T, zero_buf, zero_n);
+    else if ((int64_t) E * H >= ROUTER_STREAMED) launch_k(ctx, router_logits_kernel<4, XT, 4>, dim3(lblocks), dim3(256), 0, st, w, bias, x, logits, H, E, T, zero_buf, zero_n);
     else launch_k(ctx, router_logits_kernel<4, XT>, dim3(lblocks), dim3(256), 0, st, w, bias, x, logits, H, E, T, zero_buf, zero_n);
     return check_launch(ctx, "router_logits");
 }

@@ -28,7 +28,8 @@ struct ActQuant {
 // shared memory as fp32 - 32 two-byte loads per lane cost more than the weights (one token over 128 experts 7.0 -> 6.2 us, three tokens
 // over 512 experts 13 -> 11 us).  fp32 rows are read directly (3.9 us; staged, four layers of one token took 6 us more).
 constexpr int ROUTER_ROW = 4096;
-template <int TT, typename XT>
+// CH: steps of a lane's chain whose loads are in flight together
+template <int TT, typename XT, int CH = TT == 1 ? 32 : 8>
 __device__ __forceinline__ void router_warp(const float * __restrict__ W, const float * __restrict__ bias, const XT * __restrict__ x,
                                             float * __restrict__ logits, int H, int E, int T, int warp, int lane) {
     constexpr bool STAGE = TT == 1 && sizeof(XT) == 2;
@@ -49,7 +50,6 @@ __device__ __forceinline__ void router_warp(const float * __restrict__ W, const 
     const float * w = W + (size_t) e * H;
     // The FMA chain of a lane is sequential by definition of the reference's order, but its loads are not:
     // fetch CH steps of weights and activations at once, then run the chain over them.
-    constexpr int CH = TT == 1 ? 32 : 8;
     for (int j0 = lane; j0 < H; j0 += 32 * CH) {
         float wv[CH], xv[TT][CH];
 #pragma unroll
@@ -84,7 +84,7 @@ __device__ __forceinline__ void router_warp(const float * __restrict__ W, const 
     }
 }
 
-template <int TT, typename XT>
+template <int TT, typename XT, int CH = TT == 1 ? 32 : 8>
 __global__ void __launch_bounds__(256) router_logits_kernel(const float * __restrict__ W, const float * __restrict__ bias,
                                                            const XT * __restrict__ x, float * __restrict__ logits, int H,
                                                            int E, int T, int * __restrict__ zero_buf, int zero_n) {
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const float * __rest
     // block 0 also clears the per-expert counters the selection kernel accumulates into
     if (blockIdx.x == 0)
         for (int i = threadIdx.x; i < zero_n; i += blockDim.x) zero_buf[i] = 0;
-    router_warp<TT, XT>(W, bias, x, logits, H, E, T, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, threadIdx.x & 31);
+    router_warp<TT, XT, CH>(W, bias, x, logits, H, E, T, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, threadIdx.x & 31);
 }
 
 // Register-tiled form for batches: one warp per (TE experts x TT tokens).  Every (expert, token) pair still runs the reference's

@@ -231,3 +231,26 @@ def test_expert_parallel_kernels_follow_the_rows_that_exist(wtype, gpu_ctx):
         gpu_ctx.set_expert_path(0)
     assert torch.equal(got["all"], got["few"])
     assert torch.equal(got["few"][torch.from_numpy(ids.reshape(-1) >= 0).cuda()], got["packed"])
+
+
+@pytest.mark.parametrize("E,H", [(1200, 64), (4100, 96), (20000, 2112)])    # all warps resident; not; a matrix beyond the L2
+def test_f32_product_of_few_tokens(E, H, gpu_ctx):
+    """The F32 matmul gives a token the same bits in any batch, and a matrix that many warps share is read once for four tokens, not once
+    for each (by the kernel that runs)."""
+    gen = torch.Generator(device="cuda").manual_seed(E)
+    w, x = torch.randn((E, H), generator=gen, device="cuda"), torch.randn((9, H), generator=gen, device="cuda")
+
+    def product(n):
+        d = torch.empty((n, E), device="cuda")
+        gpu_ctx.check(gpu_ctx.lib.b200moe_op_mul_mat_f32(gpu_ctx.handle, w.data_ptr(), H, E, x.data_ptr(), n, d.data_ptr(), gpu_ctx._stream()))
+        gpu_ctx.synchronize()
+        return d
+
+    whole = product(9)
+    assert float((whole.double() - x.double() @ w.double().T).abs().max()) <= 1e-6 * H    # 32 chains of H / 32 fp32 steps of size ~1
+    for n in (1, 2, 3, 4, 5, 8):
+        assert torch.equal(product(n), whole[:n]), n
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        product(8)
+    kernels = [e.key for e in prof.key_averages() if "router_logits" in e.key]
+    assert kernels and all(bool(re.search("<4|ILi4E", k)) == (E > 1200) for k in kernels), kernels
