@@ -580,6 +580,9 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
             }
 #pragma unroll 1
             for (int ps = 0; ps < C::PASSES; ++ps) {
+                // A warp without rows leaves the pass out: with two CTAs on the SM its idle chains would hold up the other's (8 experts,
+                // 256 -> 512, 400 rows each: 1020 us with them, 547 without; one CTA per SM 906 and 547).
+                if ((ps * C::NWARPS + warp) * C::RPP >= ck.n) break;
                 const int lr = (ps * C::NWARPS + warp) * C::RPP + rgrp;  // row within the stage
                 const bool row_ok = lr < ck.n;
                 const uint8_t * wrow = st + (size_t) (row_ok ? lr : 0) * C::ROW_BYTES;

@@ -254,3 +254,19 @@ def test_f32_product_of_few_tokens(E, H, gpu_ctx):
         product(8)
     kernels = [e.key for e in prof.key_averages() if "router_logits" in e.key]
     assert kernels and all(bool(re.search("<4|ILi4E", k)) == (E > 1200) for k in kernels), kernels
+
+
+@pytest.mark.parametrize("K", [256, 2048])      # four passes of 32 weight rows to a stage, and one
+@pytest.mark.parametrize("E,N", [(1, 8), (1, 64), (8, 512), (13, 728), (16, 768)])
+def test_integer_gemv_leaves_no_weight_row_out(K, E, N, gpu_ctx):
+    """A warp that has no weight rows in a pass leaves it out.  From a row or two per CTA over half-filled passes to ragged chunks, the bits
+    are those of a token at a time (the one-or-two-token kernel)."""
+    T = 30
+    rng = np.random.default_rng(E + N)
+    w = nvfp4_matrix(rng, E, N, K)
+    b = torch.from_numpy(rng.normal(0, 1, (T, 1, K)).astype(np.float32)).cuda()
+    ids = torch.from_numpy(np.tile(np.arange(T)[:, None] % E, (1, 2)).astype(np.int32)).cuda()
+    got = gpu_ctx.mul_mat_id(TYPE_NVFP4, w, b, ids, K)
+    one = torch.cat([gpu_ctx.mul_mat_id(TYPE_NVFP4, w, b[t:t + 1], ids[t:t + 1], K) for t in range(T)])
+    gpu_ctx.synchronize()
+    assert torch.equal(got, one)
