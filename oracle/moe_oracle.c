@@ -602,7 +602,7 @@ static int layer_once(const orc_moe_args * a) {
     float * dn     = (float *) malloc(sizeof(float) * (size_t) L * K);
     float * moe    = (float *) malloc(sizeof(float) * L);
     void  * actx   = malloc((size_t) big * 2 + 1024);
-    void  * acth   = malloc((size_t) big * 2 + 1024);
+    void  * acth   = malloc((size_t) I * 2 + 1024);
     int32_t * ids  = (int32_t *) malloc(sizeof(int32_t) * K);
     float * wts    = (float *) malloc(sizeof(float) * K);
 
