@@ -1,4 +1,5 @@
 """Kernels at the sizes where they can go wrong: edges of tiles, remainders, the ends of the range of a dispatch rule."""
+import ctypes as C
 import re
 
 import numpy as np
@@ -65,6 +66,37 @@ def test_q3k_matrix_instruction_keeps_the_bits(K, N, counts, ne11, gpu_ctx, chec
         aq = checker.quantize_activation(TYPE_Q3_K, b[t, 0])
         r = int(rng.integers(0, N))
         assert float(got[t, 0, r]) == checker.vec_dot(TYPE_Q3_K, K, w[rows[t, 0], r], aq)
+
+
+@pytest.mark.parametrize("n_embd,n_ff", [(256, 256), (512, 768), (768, 512), (2048, 768)])
+def test_q3k_matrix_instruction_gate_up(n_embd, n_ff, gpu_ctx):
+    """The gate/up form in a layer with given routing: an expert of three 64-row tiles, ragged ones of 33, 9 and 1 rows and an idle one (one
+    super-block to a row at 256 columns: the operand buffers change hands at every unit).  `hidden`, `down` and the output are those of a
+    token at a time, on the integer GEMV."""
+    counts = (130, 33, 0, 9, 1)
+    rng = np.random.default_rng(n_embd + n_ff)
+    E, T = len(counts), sum(counts)
+    mats = []
+    for r, c in ((n_ff, n_embd), (n_ff, n_embd), (n_embd, n_ff)):
+        m = rng.integers(0, 256, (E, r, c // 256, 110), dtype=np.uint8)
+        m[..., 108:110] = rng.normal(0, 3e-4, (E, r, c // 256, 1)).astype(np.float16).view(np.uint8)
+        mats.append(m.reshape(E, r, -1))
+    layer = moe.MoeLayer(gpu_ctx, wtype=TYPE_Q3_K, top_k=1, router_w=np.zeros((E, n_embd), np.float32), gate=mats[0], up=mats[1], down=mats[2])
+    x = torch.from_numpy(rng.normal(0, 1, (T, n_embd)).astype(np.float32)).cuda()
+    ids = torch.from_numpy(rng.permutation(np.repeat(np.arange(E), counts)).astype(np.int32).reshape(T, 1)).cuda()
+    w = torch.from_numpy(rng.uniform(0.1, 1, (T, 1)).astype(np.float32)).cuda()
+
+    def run(a, b):
+        s, ob = layer._observe(b - a, x.device)
+        out = torch.empty((b - a, n_embd), device="cuda")
+        gpu_ctx.check(gpu_ctx.lib.b200moe_ffn(gpu_ctx.handle, C.byref(layer.desc), x[a:].data_ptr(), 0, b - a, ids[a:].data_ptr(), w[a:].data_ptr(),
+                                              out.data_ptr(), C.byref(s), gpu_ctx._stream()))
+        gpu_ctx.synchronize()
+        return ob.hidden, ob.down, out
+
+    whole = run(0, T)
+    one = [torch.cat(t) for t in zip(*(run(t, t + 1) for t in range(T)))]
+    assert bool(torch.isfinite(whole[2]).all()) and all(torch.equal(a, b) for a, b in zip(whole, one))
 
 
 @pytest.mark.parametrize("T,n_ff,shape", [(96, 256, (512, 8, 2)), (108, 512, (256, 8, 2)), (109, 768, (768, 8, 2)), (433, 256, (512, 8, 2))])

@@ -3,13 +3,14 @@
 * Routing (logits, probabilities, ids, weights) is bit-exact.
 * The integer expert kernels follow the reference's fp32 summation order: with them (expert path 1) `hidden`, `down` and
   the layer output are BIT-IDENTICAL to the CPU path, for NVFP4 and Q3_K, plain and latent layers, 1 to 4096 tokens.
-* The default path keeps everything on the integer kernels below two routed rows per expert (bit-identical).  Above that
-  `down` goes to the tcgen05 grouped GEMM (`down`/output differ by the tensor core's accumulation error: bar here 2e-4 of
-  RMS, measured ~3e-5) and, up to 4096 routed rows, so does gate/up: then `hidden` carries that error too, the reference's
-  re-quantisation of `hidden` amplifies it, and the outputs are held to the stated bar of the path, max-abs <= 1e-2 * RMS.
-* Expert path 2 forces the f16 tensor-core engine wherever the shape allows; path 3 keeps gate/up on the integer kernels.
-* Expert paths 6-8 are the block-scaled FP4 tensor-core engine (exact digit planes of the int8 grid): `hidden` within 5e-5 of RMS;
-  with the fix-up and an integer `down` (path 7) the layer is bit-identical again.
+* The default path keeps Q3_K, and NVFP4 up to 16 routed rows, on the integer kernels (bit-identical).  NVFP4 above that takes the
+  block-scaled FP4 tensor-core engine (exact digit planes of the int8 grid) for gate/up and down: `hidden` within 5e-5 of RMS, the
+  reference's re-quantisation of `hidden` amplifies that, and the outputs are held to the stated bar of the path, max-abs <= 1e-2 * RMS.
+  From 24 routed rows per expert on and beyond 4096 routed rows the exact re-quantisation fix-up follows gate/up: `down` and the output
+  then differ by the tensor core's accumulation error alone (bar 2e-4 of RMS).  Latent layers always have the fix-up, and an integer
+  `down` from 24 rows per expert on.
+* Expert path 2 forces the f16 tensor-core engine wherever the shape allows (`hidden` within 5e-4); path 3 keeps gate/up on the integer kernels.
+* Expert paths 6-8 pin the FP4 engine; with the fix-up and an integer `down` (path 7) the layer is bit-identical again.
 * Latent layers under a path that lets dense products use the FP4 engine carry its accumulation error through three
   re-quantisations: they are held to the stated bar on the output, max-abs <= 1e-2 * RMS.
 """
@@ -51,11 +52,8 @@ def expected_engines(cfg, T, path):
     if path == 0:
         if rows <= 16:
             return False, False, False
-        if can_fp4 and rows < 24 * cfg.n_expert:
-            return True, True, latent
-        if can_f16 and rows >= 2 * cfg.n_expert:
-            return True, not latent, rows > 4096 or latent
-        return False, False, False
+        few_rows = rows < 24 * cfg.n_expert
+        return (True, few_rows or not latent, latent or (not few_rows and rows > 4096)) if can_fp4 else (False, False, False)
     table = {1: (False, False, False), 2: (can_f16, can_f16, False), 3: (False, can_f16, False), 4: (can_f16, can_f16, can_f16),
              5: (can_f16, False, can_f16), 6: (True, True, False), 7: (True, False, True), 8: (True, True, True)}
     return table[path]
@@ -81,7 +79,7 @@ def run_and_compare(gpu_ctx, checker, layer, x_np, bf16, path=0):
     errs = dict(hidden=rel_err(hidden, r.hidden), down=rel_err(down, r.down_out), out=rel_err(o, r.out))
     T = x_np.shape[0]
     gu_tensor, down_tensor, fix = expected_engines(layer.cfg, T, path)
-    fp4 = path in (6, 7, 8) or (path == 0 and gu_tensor and T * layer.cfg.top_k < 24 * layer.cfg.n_expert)
+    fp4 = path in (6, 7, 8) or (path == 0 and gu_tensor)
     dense_fp4 = bool(layer.cfg.n_latent) and layer.cfg.wtype == TYPE_NVFP4 and T >= 4 and path not in (1, 5, 7)
     if dense_fp4:
         # the latent input already differs by the FP4 engine's accumulation error and is re-quantised: everything behind it is
@@ -176,6 +174,16 @@ def test_c3_nvfp4_prefill_with_logit_bias(gpu_ctx, checker):
     errs = run_and_compare(gpu_ctx, checker, layer, x_np, bf16=True, path=0)
     print("c3 T=%d default-path errors" % T, errs)
     run_and_compare(gpu_ctx, checker, layer, x_np[:512], bf16=True, path=1)
+
+
+@pytest.mark.parametrize("T,shape", [(8, (256, 8, 2, 4096)), (20, (256, 8, 2, 4096)), (512, (256, 8, 8, 256)), (513, (256, 8, 8, 256))])
+def test_default_engine_at_its_edges(T, shape, gpu_ctx, checker):
+    """The widest `down` on the integer and on the FP4 engine; 4096 routed rows (the last size of a prompt without the fix-up) and one token
+    more."""
+    H, E, k, I = shape
+    cfg = W.small_config(TYPE_NVFP4, n_embd=H, n_expert=E, top_k=k, n_ff=I, seed=290 + T)
+    layer = W.make_layer(cfg)
+    print("T=%d" % T, run_and_compare(gpu_ctx, checker, layer, W.make_tokens(cfg, T, bf16=True), bf16=True, path=0))
 
 
 @pytest.mark.parametrize("T", [64, 300])
