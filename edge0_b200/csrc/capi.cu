@@ -57,7 +57,7 @@ struct Plan {  // carved out of the scratch arena for one (layer shape, max_toke
     float * outb = nullptr; // [T][n_embd] staging for the host entry point
     int * one_group_ids = nullptr;  // [T] group of every token when a dense matvec runs on the indexed-matmul kernel
     __half * afp16 = nullptr;       // [T*k][max(n_in, n_ff)] expert-sorted fp16 activations of the tensor-core path (or the FP4 digit planes)
-    uint8_t * asf = nullptr;        // scale tiles of the FP4 digit planes: [token tiles][K / 256][2048]
+    uint8_t * asf = nullptr;        // scale tiles of the FP4 digit planes: [token tiles][K / 256][fp4_sfb_bytes(rows per tile)]
     size_t asf_bytes = 0;
     int * tile_expert = nullptr;    // expert of every token tile of the FP4 kernels
     float * arow_scale = nullptr;   // [T*k] power of two per expert-sorted routed row (FP4 digit planes)
@@ -82,7 +82,7 @@ struct b200moe_ctx {
     b200moe_counters counters{};
     int64_t launches = 0;
     bool timing = false;
-    int expert_path = 0;  // 0 auto, 1 integer GEMV always, 2 tensor-core GEMM whenever the shape allows
+    int expert_path = 0;  // b200moe_set_expert_path
     bool overlap = false; // launch the layer's kernels as programmatic dependents of one another (opt-in)
     bool overlap_now = false;  // set per call: only the small-batch regime uses it (see layer_overlap)
     bool dense_now = false;    // the expert kernels are running a dense product (kernel-timing kind 2)
@@ -218,11 +218,6 @@ constexpr float FIX_STEP_MARGIN = 0.015f;  // quantisation steps; largest GEMM e
 constexpr float FIX_REL_MARGIN = 1.2e-4f;  // of the block maximum; largest error measured: 3.0e-5 of it
 // after the block-scaled FP4 GEMM (exact digit planes; only fp32 accumulation differs):
 constexpr float FIX_STEP_MARGIN_FP4 = 2.5e-3f;  // largest error measured: 2.3e-4 steps (p99.99: 1.0e-4)
-// Routed rows per expert (on average) from which the FP4 kernels take the large token tile: from there an expert's rows spill over into a
-// second small tile and its weights are repacked again.  128 experts, 2048 -> 768, gate/up and down in us, small tile against large: 8 rows
-// 64 + 37 and 74 + 39, 12 rows 70 + 43 and 74 + 41, 16 rows 84 + 52 and 76 + 41, 32 rows 127 + 78 and 104 + 57.
-constexpr int FP4_LARGE_TILE_ROWS = 14;
-
 constexpr float FIX_REL_MARGIN_FP4 = 2.0e-5f;   // largest error measured: 1.8e-6 of the block maximum
 
 // need_router / need_experts: which weight pointers the entry point is going to read
@@ -633,7 +628,7 @@ Fp4Params fp4_params(b200moe_ctx * ctx, const float * s0, const float * s1, floa
     Plan & p = ctx->plan;
     Fp4Params f{};
     f.scale0 = s0; f.scale1 = s1; f.sf = p.asf; f.row_scale = p.arow_scale; f.offsets = p.groups.offsets; f.perm = p.groups.perm;
-    f.active = p.groups.active; f.meta = p.groups.meta; f.tile_of_expert = p.groups.cost + 3 * (n_as + 1); f.tile_expert = p.tile_expert; f.out = out; f.n_out = n_out;
+    f.tile_of_expert = p.groups.cost + 3 * (n_as + 1); f.tile_expert = p.tile_expert; f.out = out; f.n_out = n_out;
     f.n_as = n_as; f.err = ctx->d_err; f.prof = nullptr;
     return f;
 }
@@ -733,13 +728,18 @@ int launch_logits(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int 
 template <typename XT>
 int launch_front(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T, cudaStream_t st) {
     Plan & p = ctx->plan;
-    // beyond a few waves of logit tiles the quantising blocks only hold shared memory back from them (4096 tokens: 156 us in one
-    // launch, 99 + 39 in two before the quantiser took eight values a lane)
+    // beyond a few waves of logit tiles the quantising blocks only hold shared memory back from them
     const bool fused = T <= 256;
     const int rc = launch_logits_any<XT>(ctx, l->router_w, l->router_bias, x, p.logits, l->n_embd, l->n_expert, T, p.groups.counts, l->n_expert, st,
                                          fused ? p.xq : ActQuant{}, l->wtype == TYPE_Q3_K ? 1 : 0);
     return rc || fused ? rc : launch_quantize<XT>(ctx, x, l->n_embd, p.xq, T, l->n_embd, l->wtype, st);
 }
+
+// Routed rows per expert (on average) from which the FP4 kernels take the large token tile: from there an expert's rows spill over into a
+// second small tile and its weights are repacked again.  2048 -> 768, gate/up and down together in us, small tile against large.  128 experts:
+// 8 rows 100 and 113, 12 rows 113 and 115, 16 rows 133 and 119, 32 rows 205 and 164.  32 experts: 8 rows 49 and 53, 16 rows 59 and 53, 32
+// rows 74 and 68.  8 experts, whose units do not fill the GPU either way: 8 rows 33 and 35, 14 to 24 rows 35 and 35, 40 rows 45 and 37.
+constexpr int FP4_LARGE_TILE_ROWS = 14;
 
 // Routed rows per token tile of the FP4 kernels for `rows` rows in up to n_groups groups; kept in the plan from the grouping to the
 // kernels that walk the tiles.
@@ -1054,7 +1054,9 @@ int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const 
     // After `down` nothing is re-quantised, so a tensor-core `down` only adds its own ~1e-5 to the output.  A tensor-core gate/up
     // moves a few values of `hidden` across int8 rounding boundaries of the reference's re-quantisation; the exact fix-up
     // (requant_fixup.cuh) removes those flips where the bar needs it: beyond 4096 routed rows of a prompt, and on latent layers,
-    // which re-quantise once more after `down` (and keep `down` on the integer kernels at prompt sizes).
+    // which re-quantise once more after `down`.  At prompt sizes those keep `down` on the integer kernels: what U then quantises are the
+    // reference's values.  That is what the line at 24 rows buys, and it is dear: 256 tokens, 64 experts, top-10, 4096 -> 1024: 753 us and
+    // an output within 1e-6 of RMS; with the FP4 `down`, as below the line and behind path 8, 282 us and within 3.5e-3.
     const bool can_mma = mma_supported(l->wtype, n_in, l->n_ff) && mma_supported(l->wtype, l->n_ff, n_in);
     const bool can_fp4 = fp4_supported(l->wtype, n_in, l->n_ff);
     const int path = ctx->expert_path;

@@ -37,6 +37,7 @@
 // between rows and lanes and the waits of tcgen05.st have warps of their own because the repack warps' chain is the longest of a stage: with
 // both in the repack warps gate/up of 64 tokens over 512 experts (1024 -> 1024) took 107 us, like this 98; sixteen repack warps
 // that take the stages in turn gained nothing more and cost the prefill tile its registers (4096 tokens: 481 -> 685 us).
+// 24 warps leave a thread 80 registers, and every instantiation spills (72 bytes of stack at 14 rows, 32 at 27).
 #pragma once
 #include <cuda.h>
 
@@ -106,11 +107,11 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 // Expert-sorted routed row i -> seven plane rows 7i .. 7i+6 of `planes` (K/2 bytes each, ggml nibble order inside every
 // 16-block), its scale bytes in the scale tiles of its token tile, and the power of two the epilogue multiplies with.
 //   tile_of_expert[e]: index of expert e's first token tile (prefix of ceil(rows_e / rpt)); tile_expert[tile]: the inverse
-//   sf tiles: [tile][K / 256][4 steps][1 or 2 blocks of 128 plane rows][512 bytes], byte for (plane row n of the block, 16-block g of
+//   sf tiles: [tile][K / 256][4 steps][1 or 2 blocks (14 or 27 routed rows) of 128 plane rows][512 bytes], byte for (plane row n of the block, 16-block g of
 //   the step) at sf_tile_offset(n) + g
 struct PlaneOut {
     uint8_t * planes;       // [rows * 7][K / 2]
-    uint8_t * sf;           // [tiles][K / 256][2048]
+    uint8_t * sf;           // [tiles][K / 256][fp4_sfb_bytes(rpt)]
     float *   row_scale;    // [rows] by sorted position
     int *     tile_expert;  // [tiles] expert of every token tile
     int       rpt;          // routed rows per token tile
@@ -294,8 +295,6 @@ struct Fp4Params {
     const float * row_scale;
     const int * offsets;    // [n_as + 1]
     const int * perm;       // [rows]
-    const int * active;     // [n_as]
-    const int * meta;
     const int * tile_of_expert;   // [n_as + 1]: first token tile of every expert, total number of tiles at the end
     const int * tile_expert;      // [tiles]
     float * out;            // [rows][n_out] indexed by routed row

@@ -170,11 +170,8 @@ __device__ __forceinline__ void quantize_q8_0_block(const XT * __restrict__ src,
     if (lane == 0) *d = __half2float(__float2half_rn(dd));
 }
 
-// Q8_K as quantize_row_q8_K_ref (ggml-quants.c:2768-2805): the FIRST element with the largest |x| sets
-// iscale = -127/x; q = min(127, nearest_int(iscale*x)); d = 1/iscale; bsums over 16.
-// One warp per 256-element block, 8 elements per lane (lane owns elements 8*lane .. 8*lane+7).
-// The same for eight blocks at a time: a lane holds eight neighbouring values, four lanes one block.  src 16-byte aligned.  (A lane
-// per value moved 16 MB of a 4096-token prompt in 39 us.)
+// Q8_0 for eight blocks at a time: a lane holds eight neighbouring values, four lanes one block.  src 16-byte aligned.  (A lane per value
+// moved 16 MB of a 4096-token prompt in 39 us.)
 __device__ __forceinline__ void load8(const float * __restrict__ src, float (&v)[8]) {
     const float4 a = *reinterpret_cast<const float4 *>(src), b = *reinterpret_cast<const float4 *>(src + 4);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
@@ -203,6 +200,9 @@ __device__ __forceinline__ void quantize_q8_0_span(const XT * __restrict__ src, 
     if ((lane & 3) == 0) d[lane >> 2] = __half2float(__float2half_rn(dd));
 }
 
+// Q8_K as quantize_row_q8_K_ref (ggml-quants.c:2768-2805): the FIRST element with the largest |x| sets
+// iscale = -127/x; q = min(127, nearest_int(iscale*x)); d = 1/iscale; bsums over 16.
+// One warp per 256-element block, 8 elements per lane (lane owns elements 8*lane .. 8*lane+7).
 // src: the lane's eight values; q: its eight bytes; d: the block's scale, the same in every lane
 template <typename XT>
 __device__ __forceinline__ void q8_K_words(const XT * __restrict__ src, int lane, uint32_t (&q)[2], float & d) {

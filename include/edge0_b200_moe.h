@@ -122,8 +122,8 @@ B200MOE_API int  b200moe_synchronize(b200moe_ctx * ctx, void * stream); /* ggml_
 
 /* Which kernels run the expert matmuls (reference: model option switches such as `routing` / `experts`,
  * edge0-infer/docs/configuration.md:62-72; plain struct-style option, no environment variables).  Three engines exist:
- *   integer   kernels that follow the reference's fp32 summation order: bit-identical to the CPU path (dp4a; Q3_K from 8 routed rows
- *             per expert on the int8 matrix instruction)
+ *   integer   kernels that follow the reference's fp32 summation order: bit-identical to the CPU path (dp4a; Q3_K from 12 routed rows
+ *             per expert on average on the int8 matrix instruction)
  *   FP4       tcgen05 kind::mxf4nvf4 (block-scaled FP4 MMA, UE4M3 scale per 16): NVFP4 rows exactly as they lie in memory,
  *             activations as exact digit planes of the reference's int8 grid; differs from the integer engine only by fp32
  *             accumulation (~5e-6 of RMS on `hidden`); one pass over an expert's weights per 14 routed rows (batched decode) or
