@@ -505,6 +505,10 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
         const int e = p.active[ck.a];
         const int row_beg = p.offsets[e], n_e = p.offsets[e + 1] - row_beg;
         const uint8_t * st = ring + (size_t) stage * STAGE_BYTES;
+        // A warp without rows leaves a pass out: with two CTAs on the SM its idle chains would hold up the other's (8 experts, 256 -> 512, 400
+        // rows each: 1020 us with them, 547 without; one CTA per SM 906 and 547).  The chunks of the few-row kernel are whole.
+        const int first_row = warp * C::RPP, pass_rows = C::NWARPS * C::RPP;
+        const int my_passes = NW != 8 ? C::PASSES : ck.n > first_row ? (ck.n - first_row + pass_rows - 1) / pass_rows : 0;
         const int se = p.w_stride ? e : 0;      // every group of a dense product has the one matrix and its scale
         const float sc0 = p.scale0 ? p.scale0[se] : 1.0f;
         const float sc1 = (DUAL && p.scale1) ? p.scale1[se] : 1.0f;
@@ -579,10 +583,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
                 landed = true;
             }
 #pragma unroll 1
-            for (int ps = 0; ps < C::PASSES; ++ps) {
-                // A warp without rows leaves the pass out: with two CTAs on the SM its idle chains would hold up the other's (8 experts,
-                // 256 -> 512, 400 rows each: 1020 us with them, 547 without; one CTA per SM 906 and 547).
-                if ((ps * C::NWARPS + warp) * C::RPP >= ck.n) break;
+            for (int ps = 0; ps < my_passes; ++ps) {
                 const int lr = (ps * C::NWARPS + warp) * C::RPP + rgrp;  // row within the stage
                 const bool row_ok = lr < ck.n;
                 const uint8_t * wrow = st + (size_t) (row_ok ? lr : 0) * C::ROW_BYTES;
