@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
         const int row_beg = p.offsets[e], n_e = p.offsets[e + 1] - row_beg;
         const uint8_t * st = ring + (size_t) stage * STAGE_BYTES;
         // A warp without rows leaves a pass out: with two CTAs on the SM its idle chains would hold up the other's (8 experts, 256 -> 512, 400
-        // rows each: 1020 us with them, 547 without; one CTA per SM 906 and 547).  The chunks of the few-row kernel are whole.
+        // rows each: 1020 us with them, 547 without; one CTA per SM 906 and 547).  The chunks of the few-row kernel are whole at the widths of a layer.
         const int first_row = warp * C::RPP, pass_rows = C::NWARPS * C::RPP;
         const int my_passes = NW != 8 ? C::PASSES : ck.n > first_row ? (ck.n - first_row + pass_rows - 1) / pass_rows : 0;
         const int se = p.w_stride ? e : 0;      // every group of a dense product has the one matrix and its scale
@@ -583,7 +583,8 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
                 landed = true;
             }
 #pragma unroll 1
-            for (int ps = 0; ps < my_passes; ++ps) {
+            for (int ps = 0; ps < C::PASSES; ++ps) {
+                if (ps >= my_passes) break;
                 const int lr = (ps * C::NWARPS + warp) * C::RPP + rgrp;  // row within the stage
                 const bool row_ok = lr < ck.n;
                 const uint8_t * wrow = st + (size_t) (row_ok ? lr : 0) * C::ROW_BYTES;
