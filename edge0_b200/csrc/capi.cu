@@ -981,7 +981,7 @@ int route_impl(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T, 
 
 template <int K>
 int launch_fix_t(b200moe_ctx * ctx, const FixParams & fp, cudaStream_t st) {
-    constexpr size_t smem = requant_fix_smem_bytes<K>();
+    constexpr size_t smem = FixCfg<K>::SMEM;
     static bool configured[MAX_DEVICE_ORDINALS] = {};
     if (int rc = raise_smem_limit(ctx, requant_fix_kernel<K>, smem, configured)) return rc;
     launch_k(ctx, requant_fix_kernel<K>, dim3(ctx->sm_count * 8), dim3(256), smem, st, fp);

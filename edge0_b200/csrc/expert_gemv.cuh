@@ -38,7 +38,7 @@ struct GemvParams {
     const int * perm;     // [rows]
     const int * active;   // [n_as]
     const int * meta;     // meta[0] = number of active experts
-    const int * cost;     // [3][n_as+1] work prefixes (see Groups::cost)
+    const int * cost;     // work prefixes (see Groups::cost)
     float * out;          // [rows][n_out]
     int n_out;
     int n_ids;
@@ -240,77 +240,156 @@ __device__ __forceinline__ void lane_chain_pair(const uint8_t * __restrict__ row
     }
 }
 
-// The same pair for ONE activation row whose int8 values (q, K bytes) and block scales (d, K/32 floats) lie in separate arrays,
-// in any address space (the layout lane_chain_split reads).
-template <int K>
-__device__ __forceinline__ void lane_chain_split_pair(const uint8_t * __restrict__ row0, const uint8_t * __restrict__ row1, int L,
-                                                      const uint8_t * __restrict__ q, const float * __restrict__ d,
-                                                      const float * __restrict__ ue_tab, float & out0, float & out1) {
-    const int sub_in_half = L >> 2, mp = L & 3;
-    const int word_off = 4 + 8 * sub_in_half + 4 * (mp & 1);
-    const int nib_shift = 4 * (mp >> 1);
-    float a0 = 0.0f, a1 = 0.0f;
-#pragma unroll 4
-    for (int b = 0; b < K / 64; ++b) {
-        const uint8_t * blk0 = row0 + b * NVFP4_BLOCK_BYTES, * blk1 = row1 + b * NVFP4_BLOCK_BYTES;
-        const uint32_t dw0 = *reinterpret_cast<const uint32_t *>(blk0), dw1 = *reinterpret_cast<const uint32_t *>(blk1);
+// ---- two SIMD lanes per thread ---------------------------------------------------------------------------------------------
+// The low nibbles of a qs word belong to one lane of the reference and its high nibbles to another (lanes 4 sub + w and 4 sub + w + 2 of
+// sub-block `sub`, word w), so four threads can play the eight lanes of a row: a thread takes word m = 2 sub + w of every half-block, looks
+// all eight codes up at once and shares the block scale between its two chains.  That is 13 instructions of decode for eight codes where a
+// lane by itself spends 10 on four and throws the other nibbles away, and half the loads of words, scales and table entries.
+// `lo` and `hi`: four signed bytes each (twice the E2M1 values), in the order of the lane's activation word.
+__device__ __forceinline__ void nvfp4_word_to_s8(uint32_t w, uint32_t & lo, uint32_t & hi) {
+    const uint32_t wn = w ^ 0x88888888u;
+    const uint32_t pa = byte_perm(FP4_MAG_LO, FP4_MAG_HI, w), pb = byte_perm(FP4_MAG_LO, FP4_MAG_HI, w >> 16);
+    const uint32_t na = byte_perm(FP4_MAG_LO, FP4_MAG_HI, wn), nb = byte_perm(FP4_MAG_LO, FP4_MAG_HI, wn >> 16);
+    // signed bytes: a byte of `n` is a magnitude 0..12, 0x80 - it never borrows, the xor drops the guard bit
+    const uint32_t a = pa | ((0x80808080u - na) ^ 0x80808080u);   // low, high nibble of byte 0, low, high nibble of byte 1
+    const uint32_t b = pb | ((0x80808080u - nb) ^ 0x80808080u);   // the same of bytes 2 and 3
+    lo = byte_perm(a, b, 0x6420);
+    hi = byte_perm(a, b, 0x7531);
+}
+// Two fp32 values in one register pair: sm_100's packed instructions round each half as the scalar ones do.
+__device__ __forceinline__ uint64_t f32x2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 f32x2_halves(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// two integer dots as floats: the constant 1.5 * 2^23 rides in the accumulator of dp4a (see small_int_to_float)
+__device__ __forceinline__ uint64_t dots_to_f32x2(uint32_t code0, uint32_t act0, uint32_t code1, uint32_t act1) {
+    return add_f32x2(f32x2(__int_as_float(dot4((int) code0, (int) act0, 0x4B400000)), __int_as_float(dot4((int) code1, (int) act1, 0x4B400000))),
+                     f32x2(-12582912.0f, -12582912.0f));
+}
+// hsum_float_8 of a row whose lanes L0 = 4 (m >> 1) + (m & 1) and L0 + 2 thread m holds: (a0+a4), (a2+a6) / (a1+a5), (a3+a7) across the
+// threads of a word, (r0+r2) / (r1+r3) inside the thread, then the two words.  The result is valid in all four threads.
+__device__ __forceinline__ float hsum_two_lanes(float lo, float hi) {
+    lo = __fadd_rn(lo, __shfl_xor_sync(0xffffffffu, lo, 2));
+    hi = __fadd_rn(hi, __shfl_xor_sync(0xffffffffu, hi, 2));
+    lo = __fadd_rn(lo, hi);
+    return __fadd_rn(lo, __shfl_xor_sync(0xffffffffu, lo, 1));
+}
+// where the word of SIMD lane L of a 32-unit lies in activations staged for these chains: the two lanes of thread m are neighbours
+__host__ __device__ __forceinline__ constexpr int act_slot(int L) { return (L & 4) | ((L & 1) << 1) | ((L >> 1) & 1); }
+
+// The chains of NROW weight rows against NT activation rows (1, 2 or 4) as pairs of accumulators: of two tokens' same lane, or, for one
+// token, of its two lanes.
+template <int NROW, int NT>
+struct TwoLaneAcc {
+    static constexpr int N = NT == 1 ? 1 : NT;
+    uint64_t v[NROW][N];                                       // [row][lane lo: token pairs, lane hi: token pairs]
+    __device__ __forceinline__ void clear() {
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-            const uint32_t code0 = nvfp4_codes_to_s8(*reinterpret_cast<const uint32_t *>(blk0 + 16 * hf + word_off), nib_shift);
-            const uint32_t code1 = nvfp4_codes_to_s8(*reinterpret_cast<const uint32_t *>(blk1 + 16 * hf + word_off), nib_shift);
-            const float sw0 = ue_tab[(dw0 >> (8 * (2 * hf + sub_in_half))) & 0xff], sw1 = ue_tab[(dw1 >> (8 * (2 * hf + sub_in_half))) & 0xff];
-            const int unit = 2 * b + hf;
-            const uint32_t aw = reinterpret_cast<const uint32_t *>(q)[unit * 8 + L];
-            const float dy = d[unit];
-            a0 = __fmaf_rn(__fmul_rn(sw0, dy), small_int_to_float(dot4((int) code0, (int) aw, 0)), a0);
-            a1 = __fmaf_rn(__fmul_rn(sw1, dy), small_int_to_float(dot4((int) code1, (int) aw, 0)), a1);
+        for (int r = 0; r < NROW; ++r)
+#pragma unroll
+            for (int i = 0; i < N; ++i) v[r][i] = f32x2(0.0f, 0.0f);
+    }
+    __device__ __forceinline__ void lanes(int r, int t, float & lo, float & hi) const {
+        if (NT == 1) {
+            const float2 a = f32x2_halves(v[r][0]);
+            lo = a.x; hi = a.y;
+        } else {
+            const float2 a = f32x2_halves(v[r][t / 2]), b = f32x2_halves(v[r][(N / 2 + t / 2) % N]);
+            lo = t & 1 ? a.y : a.x; hi = t & 1 ? b.y : b.x;
         }
     }
-    a0 = __fadd_rn(a0, __shfl_xor_sync(0xffffffffu, a0, 4));
-    a1 = __fadd_rn(a1, __shfl_xor_sync(0xffffffffu, a1, 4));
-    a0 = __fadd_rn(a0, __shfl_xor_sync(0xffffffffu, a0, 2));
-    a1 = __fadd_rn(a1, __shfl_xor_sync(0xffffffffu, a1, 2));
-    a0 = __fadd_rn(a0, __shfl_xor_sync(0xffffffffu, a0, 1));
-    a1 = __fadd_rn(a1, __shfl_xor_sync(0xffffffffu, a1, 1));
-    out0 = a0;
-    out1 = a1;
+};
+
+// 256 elements (four blocks) of the weight rows: the chains go on in acc.
+//   blk[r]: first byte of the four blocks of row r; acts: the words of these eight units, [unit][act_slot][NTS]; dy: [unit][NTS]
+template <int NROW, int NT, int NTS>
+__device__ __forceinline__ void two_lane_chains(const uint8_t * const (&blk)[NROW], int m, const uint32_t * __restrict__ acts, const float * __restrict__ dy,
+                                                const float * __restrict__ ue_tab, TwoLaneAcc<NROW, NT> & acc) {
+    const int sub = m >> 1;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        uint32_t dw[NROW];
+#pragma unroll
+        for (int r = 0; r < NROW; ++r) dw[r] = *reinterpret_cast<const uint32_t *>(blk[r] + b * NVFP4_BLOCK_BYTES) >> (8 * sub);
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            const int unit = 2 * b + hf;
+            uint32_t alo[NT], ahi[NT];
+            float d[NT];
+            const uint32_t * aw = acts + (unit * 8 + 2 * m) * NTS;
+            load_vec<NT>(alo, aw);
+            load_vec<NT>(ahi, aw + NTS);
+            load_vec<NT>(d, dy + unit * NTS);
+#pragma unroll
+            for (int r = 0; r < NROW; ++r) {
+                uint32_t lo, hi;
+                nvfp4_word_to_s8(*reinterpret_cast<const uint32_t *>(blk[r] + b * NVFP4_BLOCK_BYTES + 4 + 16 * hf + 4 * m), lo, hi);
+                const float sw = ue_tab[(dw[r] >> (16 * hf)) & 0xff];
+                if constexpr (NT == 1) {
+                    const float s = __fmul_rn(sw, d[0]);
+                    acc.v[r][0] = fma_f32x2(f32x2(s, s), dots_to_f32x2(lo, alo[0], hi, ahi[0]), acc.v[r][0]);
+                } else {
+                    const uint64_t sw2 = f32x2(sw, sw);
+#pragma unroll
+                    for (int t = 0; t < NT; t += 2) {
+                        const uint64_t s = mul_f32x2(sw2, f32x2(d[t], d[t + 1]));
+                        acc.v[r][t / 2] = fma_f32x2(s, dots_to_f32x2(lo, alo[t], lo, alo[t + 1]), acc.v[r][t / 2]);
+                        acc.v[r][NT / 2 + t / 2] = fma_f32x2(s, dots_to_f32x2(hi, ahi[t], hi, ahi[t + 1]), acc.v[r][NT / 2 + t / 2]);
+                    }
+                }
+            }
+        }
+    }
 }
 
-// The NVFP4 chain of lane_chain for ONE activation row whose int8 values (q, K bytes) and block scales (d, K/32 floats)
-// lie in separate arrays, in any address space.  Same operations in the same order as lane_chain<TYPE_NVFP4, K, 1, 1>.
+// The chains of one weight row in shared memory against ONE activation row whose int8 values (q, K bytes) and block scales (d, K/32
+// floats, 8-byte aligned) lie in separate arrays in global memory.  The result is valid in the row's four threads.
 template <int K>
-__device__ __forceinline__ void lane_chain_split(const uint8_t * __restrict__ row, int L, const uint8_t * __restrict__ q,
-                                                 const float * __restrict__ d, const float * __restrict__ ue_tab, float (&acc)[1]) {
-    const int sub_in_half = L >> 2, mp = L & 3;
-    const int word_off = 4 + 8 * sub_in_half + 4 * (mp & 1);
-    const int nib_shift = 4 * (mp >> 1);
-    float a = 0.0f;
-#pragma unroll 4
+__device__ __forceinline__ float two_lane_chain_split(const uint8_t * __restrict__ row, int m, const uint8_t * __restrict__ q, const float * __restrict__ d,
+                                                      const float * __restrict__ ue_tab) {
+    const int sub = m >> 1;
+    const uint32_t * qw = reinterpret_cast<const uint32_t *>(q) + 4 * sub + (m & 1);
+    uint64_t acc = f32x2(0.0f, 0.0f);
+#pragma unroll 8
     for (int b = 0; b < K / 64; ++b) {
-        const uint8_t * blk = row + b * NVFP4_BLOCK_BYTES;
-        const uint32_t dw = *reinterpret_cast<const uint32_t *>(blk);
+        const float2 dy = __ldg(reinterpret_cast<const float2 *>(d) + b);
+        const uint8_t * const blk = row + b * NVFP4_BLOCK_BYTES;
+        const uint32_t dw = *reinterpret_cast<const uint32_t *>(blk) >> (8 * sub);
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
-            const uint32_t w = *reinterpret_cast<const uint32_t *>(blk + 16 * hf + word_off);
-            const uint32_t t4 = (w >> nib_shift) & 0x0f0f0f0fu;
-            const uint32_t u = t4 | (t4 >> 4);
-            const uint32_t sel = byte_perm(u, 0u, 0x4420u);
-            const uint32_t pos = byte_perm(FP4_MAG_LO, FP4_MAG_HI, sel);
-            const uint32_t neg = byte_perm(FP4_MAG_LO, FP4_MAG_HI, sel ^ 0x8888u);
-            const uint32_t code = pos | ((0x80808080u - neg) ^ 0x80808080u);
-            const float sw = ue_tab[(dw >> (8 * (2 * hf + sub_in_half))) & 0xff];
-            const int unit = 2 * b + hf;
-            const uint32_t aw = reinterpret_cast<const uint32_t *>(q)[unit * 8 + L];
-            const float dy = d[unit];
-            const int p = dot4((int) code, (int) aw, 0);
-            a = __fmaf_rn(__fmul_rn(sw, dy), small_int_to_float(p), a);
+            uint32_t lo, hi;
+            nvfp4_word_to_s8(*reinterpret_cast<const uint32_t *>(blk + 4 + 16 * hf + 4 * m), lo, hi);
+            const float s = __fmul_rn(ue_tab[(dw >> (16 * hf)) & 0xff], hf ? dy.y : dy.x);
+            acc = fma_f32x2(f32x2(s, s), dots_to_f32x2(lo, __ldg(qw + (2 * b + hf) * 8), hi, __ldg(qw + (2 * b + hf) * 8 + 2)), acc);
         }
     }
-    a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 4));
-    a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 2));
-    a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 1));
-    acc[0] = a;
+    const float2 a = f32x2_halves(acc);
+    return hsum_two_lanes(a.x, a.y);
 }
+
+// Distance of staged weight rows that the two-lane chains read: eight rows of a warp, four words of each, then fall on different banks.
+__host__ __device__ constexpr int two_lane_pitch(int row_bytes) { return row_bytes % 32 ? row_bytes : row_bytes + 16; }
 
 // The same chain run by a whole warp for ONE row: the four 8-lane groups split the half-blocks between them (group rg takes
 // units rg, rg + 4, ...), every lane fetches and decodes its share with all loads in flight at once, and the fp32 chain - which
@@ -449,7 +528,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>(
             s_span[tid] = (int) (u < total ? u : total);
         }
     } else if (tid < 2) {
-        const int * cw = p.cost + (NT == 1 ? 0 : NT == 2 ? 1 : 2) * (p.n_as + 1);
+        const int * cw = p.cost + (NT == 1 ? 0 : 2) * (p.n_as + 1);
         const long long total_work = (long long) cw[n_active] * upe;
         const long long c = total_work * (blockIdx.x + tid) / gridDim.x;
         int lo = 0, hi = n_active;  // largest a with cw[a]*upe <= c

@@ -134,30 +134,35 @@ struct FixParams {
     float rel_margin;          // the mark kernel's: relative uncertainty of a block maximum the GEMM left
 };
 
-// 8 lanes per listed value (the reference's 8 SIMD lanes), 4 values per warp at a time.  Each group runs the same chains as
-// the integer GEMV, so the patched value is the reference's, bit for bit.  The listed values are scattered - nothing streams - so
+// 8 threads per listed value, 4 values per warp at a time: four threads run the gate chains and four the up chains (two SIMD lanes of the
+// reference each), so the patched value is the reference's, bit for bit.  The listed values are scattered - nothing streams - so
 // every warp fetches the two weight rows of its four values with bulk copies into its own piece of shared memory (whole rows in
 // one request each instead of a few words per dependent load) and waits once; the activations are L2-resident and read directly.
-// Latency is hidden by the other warps of the SM.
+// Latency is hidden by the other warps of the SM; what bounds the kernel is the issue of the chains and the activations' way from L2.
+// 4096 tokens, 2048 -> 768, 1.3 % of the values: 399 us with a lane to a thread and rows that met on four banks, 240 so (both passes).
 template <int K>
-constexpr size_t requant_fix_smem_bytes() { return (size_t) 8 * 4 * 2 * (K / 64 * NVFP4_BLOCK_BYTES); }
+struct FixCfg {
+    static constexpr int ROW_BYTES = K / 64 * NVFP4_BLOCK_BYTES, PITCH = two_lane_pitch(ROW_BYTES);
+    static constexpr size_t SMEM = (size_t) 8 * 8 * PITCH;      // [8 warps][4 values][gate row, up row]
+    static_assert(ROW_BYTES % 16 == 0, "bulk copies move multiples of 16 bytes");
+};
 
 template <int K>
 __global__ void __launch_bounds__(256) requant_fix_kernel(const FixParams p) {
-    constexpr int ROW_BYTES = K / 64 * NVFP4_BLOCK_BYTES;
-    static_assert(ROW_BYTES % 16 == 0, "bulk copies move multiples of 16 bytes");
-    extern __shared__ __align__(128) uint8_t fix_rows[];   // [8 warps][4 values][gate row, up row]
+    constexpr int ROW_BYTES = FixCfg<K>::ROW_BYTES, PITCH = FixCfg<K>::PITCH;
+    extern __shared__ __align__(128) uint8_t fix_rows[];
     __shared__ float ue_tab[256];
     __shared__ uint64_t bars[8];
     pdl_wait();
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int L = lane & 7, rgrp = lane >> 3;
+    const int L = lane & 7, rgrp = lane >> 3, up = (lane >> 2) & 1, m = lane & 3;
     ue_tab[tid] = ue4m3_half_to_f32(tid);
     if (tid < 8) mbar_init(&bars[tid], 1);
     mbar_fence_init();
     __syncthreads();
-    uint8_t * const rows_smem = fix_rows + (size_t) (warp * 4 + rgrp) * 2 * ROW_BYTES;
+    uint8_t * const row_smem = fix_rows + (size_t) (warp * 8 + (lane >> 2)) * PITCH;
+    const uint8_t * const w = up ? p.w1 : p.w0;
     const int n = min(*p.list.count, p.list.capacity);
     const int groups_per_grid = gridDim.x * 32;
     uint32_t parity = 0;
@@ -171,10 +176,8 @@ __global__ void __launch_bounds__(256) requant_fix_kernel(const FixParams p) {
         if (e < 0 || e >= p.n_as) { report_error(p.err, DEV_ERR_BAD_EXPERT_ID); e = 0; }
         const int tok = r / p.n_ids;
         if (lane == 0) mbar_arrive_expect_tx(&bars[warp], 4 * 2 * ROW_BYTES);
-        if (L == 0) {
-            bulk_g2s(rows_smem, p.w0 + ((size_t) e * p.n_ff + f) * ROW_BYTES, ROW_BYTES, &bars[warp]);
-            bulk_g2s(rows_smem + ROW_BYTES, p.w1 + ((size_t) e * p.n_ff + f) * ROW_BYTES, ROW_BYTES, &bars[warp]);
-        }
+        __syncwarp();
+        if (m == 0) bulk_g2s(row_smem, w + ((size_t) e * p.n_ff + f) * ROW_BYTES, ROW_BYTES, &bars[warp]);
         const bool landed = mbar_wait_bounded(&bars[warp], parity);
         if (!__all_sync(0xffffffffu, landed)) {                     // warp-uniform: the chains below shuffle with the full mask
             report_error(p.err, DEV_ERR_BARRIER_TIMEOUT);
@@ -182,13 +185,10 @@ __global__ void __launch_bounds__(256) requant_fix_kernel(const FixParams p) {
             break;
         }
         parity ^= 1u;
-        const uint8_t * g_row = rows_smem;
-        const uint8_t * u_row = rows_smem + ROW_BYTES;
-        float g[1], u[1];
-        lane_chain_split_pair<K>(g_row, u_row, L, reinterpret_cast<const uint8_t *>(p.act.q + (size_t) tok * K), p.act.d + (size_t) tok * (K / 32), ue_tab,
-                                 g[0], u[0]);
+        const float dot = two_lane_chain_split<K>(row_smem, m, reinterpret_cast<const uint8_t *>(p.act.q + (size_t) tok * K), p.act.d + (size_t) tok * (K / 32), ue_tab);
+        const float g0 = __shfl_sync(0xffffffffu, dot, lane & ~4), u0 = __shfl_sync(0xffffffffu, dot, lane | 4);
         const float sc0 = p.scale0 ? p.scale0[e] : 1.0f, sc1 = p.scale1 ? p.scale1[e] : 1.0f;
-        const float hv = __fmul_rn(ggml_silu(__fmul_rn(g[0], sc0)), __fmul_rn(u[0], sc1));   // the same in all 8 lanes of the group
+        const float hv = __fmul_rn(ggml_silu(__fmul_rn(g0, sc0)), __fmul_rn(u0, sc1));   // the same in all 8 lanes of the group
         float * hrow = p.hid + (size_t) r * p.n_ff;
         if (valid && L == 0) hrow[f] = hv;
         // Is the rounding of the exact value decided whatever the last bits of the block maximum are?  The group's 8 lanes read
