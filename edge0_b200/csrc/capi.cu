@@ -21,6 +21,7 @@
 #include "expert_exchange.cuh"
 #include "expert_gemm_tm.cuh"
 #include "expert_gemv.cuh"
+#include "expert_gemv_nvfp4.cuh"
 #include "expert_mma.cuh"
 #include "expert_mma_q3k.cuh"
 #include "fp4_probe.cuh"
@@ -303,6 +304,42 @@ int check_launch(b200moe_ctx * ctx, const char * what) {
     return B200MOE_OK;
 }
 
+// ---- tensor maps of the kernels that fetch tiles (the encoder is a host-side driver entry point; looked up
+// once through the runtime so the library does not link against the driver library)
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiledFn encode_tiled_fn() {
+    static EncodeTiledFn fn = nullptr;
+    static bool tried = false;
+    if (!tried) {
+        tried = true;
+        void * ptr = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<EncodeTiledFn>(ptr);
+        else
+            cudaGetLastError();
+    }
+    return fn;
+}
+
+// 2-D map over a row-major [outer][inner] array whose rows are pitch_bytes apart
+int make_map_2d(b200moe_ctx * ctx, CUtensorMap * m, CUtensorMapDataType dt, const void * base, uint64_t inner, uint64_t outer,
+                uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle sw) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return fail(ctx, B200MOE_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+    const cuuint64_t dims[2] = { inner, outer };
+    const cuuint64_t strides[1] = { pitch_bytes };
+    const cuuint32_t box[2] = { box_inner, box_outer };
+    const cuuint32_t estr[2] = { 1, 1 };
+    const CUresult r = fn(m, dt, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(ctx, B200MOE_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int) r);
+    return B200MOE_OK;
+}
+
 // ---- kernel dispatch -----------------------------------------------------------------------------------
 template <int WT, int K, bool DUAL, int NT>
 int launch_gemv_t(b200moe_ctx * ctx, const GemvParams & p, cudaStream_t st) {
@@ -354,14 +391,46 @@ int launch_gemv_tiny(b200moe_ctx * ctx, const GemvParams & p, int rows, cudaStre
     return check_launch(ctx, "expert_gemv");
 }
 
+// NVFP4, more than a few rows: n_mats matrices behind one another (one when every group shares it)
+template <int K, bool DUAL>
+int launch_gemv_nvfp4(b200moe_ctx * ctx, const GemvParams & p, cudaStream_t st) {
+    using C = Nvfp4GemvCfg<K, DUAL>;
+    auto kern = nvfp4_gemv_kernel<K, DUAL>;
+    static bool configured[MAX_DEVICE_ORDINALS] = {};  // per instantiation and device
+    if (int rc = raise_smem_limit(ctx, kern, C::SMEM, configured)) return rc;
+    constexpr uint64_t ROW_BYTES = K / 64 * NVFP4_BLOCK_BYTES;
+    const uint64_t wrows = (uint64_t) (p.w_stride ? p.n_as : 1) * p.n_out;
+    CUtensorMap m0, m1;
+    if (int rc = make_map_2d(ctx, &m0, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.w0, ROW_BYTES, wrows, ROW_BYTES, GEMM_RAW_ROW, 8, CU_TENSOR_MAP_SWIZZLE_NONE)) return rc;
+    if (!DUAL) m1 = m0;
+    else if (int rc = make_map_2d(ctx, &m1, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.w1, ROW_BYTES, wrows, ROW_BYTES, GEMM_RAW_ROW, 8, CU_TENSOR_MAP_SWIZZLE_NONE)) return rc;
+    b200moe_ctx::Timed tm{};
+    if (ctx->timing) {
+        CUDA_TRY(ctx, cudaEventCreate(&tm.beg));
+        CUDA_TRY(ctx, cudaEventCreate(&tm.end));
+        tm.kind = DUAL ? 0 : ctx->dense_now ? 2 : 1;
+        CUDA_TRY(ctx, cudaEventRecord(tm.beg, st));
+    }
+    launch_k(ctx, kern, dim3(C::CTAS * ctx->sm_count), dim3(C::THREADS), C::SMEM, st, p, m0, m1);
+    if (ctx->timing) {
+        CUDA_TRY(ctx, cudaEventRecord(tm.end, st));
+        ctx->timed.push_back(tm);
+    }
+    return check_launch(ctx, "nvfp4_gemv");
+}
+
 template <int WT, int K, bool DUAL>
 int launch_gemv_k(b200moe_ctx * ctx, const GemvParams & p, int nt, cudaStream_t st) {
     if constexpr (DUAL && K > 2048) {
         return fail(ctx, B200MOE_ERR_UNSUPPORTED, "fused gate/up kernel is not built for K=%d", K);
     } else {
         if (nt <= 0) return launch_gemv_tiny<WT, K, DUAL>(ctx, p, -nt, st);   // nt = -(routed rows): the one-or-two-token kernel
-        if (nt <= 1) return launch_gemv_t<WT, K, DUAL, 1>(ctx, p, st);
-        return launch_gemv_t<WT, K, DUAL, 4>(ctx, p, st);
+        if constexpr (WT == TYPE_NVFP4) {
+            return launch_gemv_nvfp4<K, DUAL>(ctx, p, st);
+        } else {
+            if (nt <= 1) return launch_gemv_t<WT, K, DUAL, 1>(ctx, p, st);
+            return launch_gemv_t<WT, K, DUAL, 4>(ctx, p, st);
+        }
     }
 }
 
@@ -412,42 +481,6 @@ int launch_integer(b200moe_ctx * ctx, int wtype, int k, const GemvParams & p, in
         }
     }
     return launch_gemv<DUAL>(ctx, wtype, k, p, nt, st);
-}
-
-// ---- tensor maps for the warp-specialised grouped GEMM (the encoder is a host-side driver entry point; looked up
-// once through the runtime so the library does not link against the driver library)
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void * ptr = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(ptr);
-        else
-            cudaGetLastError();
-    }
-    return fn;
-}
-
-// 2-D map over a row-major [outer][inner] array whose rows are pitch_bytes apart
-int make_map_2d(b200moe_ctx * ctx, CUtensorMap * m, CUtensorMapDataType dt, const void * base, uint64_t inner, uint64_t outer,
-                uint64_t pitch_bytes, uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle sw) {
-    EncodeTiledFn fn = encode_tiled_fn();
-    if (!fn) return fail(ctx, B200MOE_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-    const cuuint64_t dims[2] = { inner, outer };
-    const cuuint64_t strides[1] = { pitch_bytes };
-    const cuuint32_t box[2] = { box_inner, box_outer };
-    const cuuint32_t estr[2] = { 1, 1 };
-    const CUresult r = fn(m, dt, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-                          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(ctx, B200MOE_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d", (int) r);
-    return B200MOE_OK;
 }
 
 template <int K, bool DUAL, int NT>

@@ -2,12 +2,14 @@
 // indexed matmul as an operator, `down` of latent prompts, dense products of a few tokens.
 //
 // Four threads play the eight SIMD lanes of a weight row (two_lane_chains), eight rows to a warp, up to four routed rows to a pass.  A CTA
-// of eight consumer warps walks chunks of up to 64 weight rows; their bytes arrive in K = 256 pieces as tiled copies of [8 rows][144 bytes],
-// one per warp and tensor, through a ring that a producer warp keeps ahead of them.  Pieces of that shape because their rows lie 36 words
-// apart - the 8 x 4 words a warp reads together fall on 32 different banks, where whole rows (K = 2048: 288 words apart) met on four - and
-// because a ring of them leaves room for two CTAs on an SM at every width.  A further pass over an expert's rows brings them from L2 again.
-// What bounds it is the issue of the chains: 18 instructions per eight codes and row for the decode, 8 for each routed row.
-// 320 routed rows over 128 experts, 2048 -> 768: 104 us with a lane to a thread and whole rows in the ring, TODO now.
+// of eight consumer warps takes items of 64 weight rows and one pass; their bytes arrive in K = 256 pieces as tiled copies of [8 rows][144
+// bytes], one per warp and tensor, through a ring that a producer warp keeps ahead of them.  Pieces of that shape because their rows lie 36
+// words apart - the 8 x 4 words a warp reads together fall on 32 different banks, where whole rows (K = 2048: 288 words apart) met on four -
+// and because a ring of them leaves room for two or three CTAs on an SM at every width.  A further pass over an expert's rows brings them
+// from L2 again; cutting the passes, too, over the CTAs is what fills the GPU when an expert has few weight rows and many routed ones.
+// What bounds it is the arithmetic unit of integers and permutes (half rate: 15 of them per eight codes and row) and the issue of the rest.
+// A lane to a thread, whole rows in the ring, spans of weight rows with all passes, us: 320 routed rows over 128 experts, 2048 -> 768, 104,
+// now 57 (two CTAs on an SM instead of three 61); whole calls: 1024 rows 264, now 143; 3200 over 8 experts, 256 -> 512, 604, now 53.
 #pragma once
 #include "expert_gemm.cuh"
 #include "expert_gemv.cuh"
@@ -22,19 +24,60 @@ struct Nvfp4GemvCfg {
     static constexpr int KC = K / 256;
     static constexpr int BOX = 8 * GEMM_RAW_ROW;              // a warp's rows of a piece
     static constexpr int STAGE = WARPS * BOX * NTENS;
-    static constexpr int STAGES = DUAL ? 4 : 8;
+    static constexpr int CTAS = DUAL || K > 2048 ? 2 : 3;
+    static constexpr int STAGES = DUAL ? 4 : CTAS == 3 ? 6 : 8;
     static constexpr int ACT_D = K / 32;
     static constexpr int ACTS = NT * (K + 4 * ACT_D);
     static constexpr size_t SMEM = (size_t) STAGES * STAGE + ACTS + 256 * 4;
     static constexpr int THREADS = WARPS * 32 + 32;
-    static_assert(K % 256 == 0 && BOX % 128 == 0 && 2 * (SMEM + 2048) <= 228 * 1024, "two CTAs fit an SM, boxes keep their alignment");
+    static_assert(K % 256 == 0 && BOX % 128 == 0 && CTAS * (SMEM + 2048) <= 228 * 1024, "the CTAs fit an SM, boxes keep their alignment");
 };
 
-// routed rows of the next pass when `left` are to be done: a remainder of 1 or 2 runs narrower chains instead of padding
-__device__ __forceinline__ int nvfp4_pass_rows(int left) { return left >= 3 ? 4 : left; }
+// A CTA's part of the work: items (active expert a, pass ps over four of its routed rows, chunk ch of its weight rows), chunks fastest.
+struct Nvfp4Span {
+    int a, ps, ch;          // next item
+    int a1, ps1, ch1;       // the next CTA's first
+    int chunks;             // of an expert
+    __device__ __forceinline__ bool more() const { return a < a1 || (a == a1 && (ps < ps1 || (ps == ps1 && ch < ch1))); }
+    __device__ __forceinline__ void next(int n_e) {          // n_e: routed rows of expert a
+        if (++ch < chunks) return;
+        ch = 0;
+        if (4 * ++ps < n_e) return;
+        ps = 0;
+        ++a;
+    }
+};
+// Boundary i sits at work i / grid of the total (cw: prefix of nvfp4_work over the active experts); both neighbours compute it the same
+// way, so the spans tile exactly.  The whole block looks for its two experts at once.
+template <int THREADS>
+__device__ __forceinline__ Nvfp4Span nvfp4_span(const int * __restrict__ cw, int n_active, int chunks) {
+    __shared__ int s_at[2];
+    const long long work = n_active ? (long long) cw[n_active] * chunks : 0;
+    const long long c[2] = { work * blockIdx.x / gridDim.x, work * (blockIdx.x + 1) / gridDim.x };
+    if (threadIdx.x < 2) s_at[threadIdx.x] = n_active;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n_active; i += THREADS) {
+        const long long here = (long long) cw[i] * chunks, next = (long long) cw[i + 1] * chunks;
+        if (here <= c[0] && c[0] < next) s_at[0] = i;
+        if (here <= c[1] && c[1] < next) s_at[1] = i;
+    }
+    __syncthreads();
+    int at[2][3] = { { n_active, 0, 0 }, { n_active, 0, 0 } };
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int a = s_at[k];
+        if (a == n_active) continue;                         // the end of the list
+        const int w = cw[a + 1] - cw[a];
+        const long long left = c[k] - (long long) cw[a] * chunks;
+        at[k][0] = a;
+        at[k][1] = (int) (left / (16 * chunks));
+        at[k][2] = (int) (left - (long long) at[k][1] * 16 * chunks) / min(16, w - 16 * at[k][1]);
+    }
+    return Nvfp4Span{ at[0][0], at[0][1], at[0][2], at[1][0], at[1][1], at[1][2], chunks };
+}
 
 template <int K, bool DUAL>
-__global__ void __launch_bounds__(Nvfp4GemvCfg<K, DUAL>::THREADS, 2)
+__global__ void __launch_bounds__(Nvfp4GemvCfg<K, DUAL>::THREADS, Nvfp4GemvCfg<K, DUAL>::CTAS)
 nvfp4_gemv_kernel(const GemvParams p, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1) {
     using C = Nvfp4GemvCfg<K, DUAL>;
     constexpr int NT = C::NT, NTENS = C::NTENS, CONSUMERS = C::WARPS * 32;
@@ -45,7 +88,6 @@ nvfp4_gemv_kernel(const GemvParams p, const __grid_constant__ CUtensorMap map_w0
     float * const ue_tab = dys + C::ACT_D * NT;
     __shared__ uint64_t full[C::STAGES], empty[C::STAGES];
     __shared__ volatile int s_abort;
-    __shared__ int s_span[2];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
@@ -59,162 +101,147 @@ nvfp4_gemv_kernel(const GemvParams p, const __grid_constant__ CUtensorMap map_w0
     pdl_launch_dependents();
 
     const int n_active = p.meta[0];
-    const int upe = p.n_out / 8;                             // span units (eight weight rows) per expert
-    // Span boundaries balance work, as in expert_gemv_kernel: boundary i sits at work i / grid of the total
-    if (tid < 2) {
-        const long long total = (long long) n_active * upe;
-        const int * cw = p.cost + 2 * (p.n_as + 1);
-        const long long c = (long long) cw[n_active] * upe * (blockIdx.x + tid) / gridDim.x;
-        int lo = 0, hi = n_active;                           // largest a with cw[a] * upe <= c
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if ((long long) cw[mid] * upe <= c) lo = mid; else hi = mid;
-        }
-        int u;
-        if (n_active == 0) u = 0;
-        else if (blockIdx.x + tid == gridDim.x) u = (int) total;
-        else {
-            const long long uu = (c - (long long) cw[lo] * upe) / max(cw[lo + 1] - cw[lo], 1);
-            u = lo * upe + (int) (uu < (long long) upe ? uu : (long long) upe);
-        }
-        s_span[tid] = u;
-    }
-    __syncthreads();
-    ChunkWalker walk;
-    walk.u = s_span[0];
-    walk.u_end = s_span[1];
-    walk.units_per_expert = upe;
-    walk.gran = 8;
-    walk.max_rows = C::ROWS;
-    Chunk ck;
+    const int * const cw = p.cost + (p.n_as + 1);
+    // Chunks of 64 weight rows; while there are items for less than every CTA, of as few rows as leaves one to a CTA.  (Passes: what is left of
+    // the work of the nt = 4 kernels, 3 to a pass and 2 to a row, without the rows.)
+    const long long passes = (p.cost[2 * (p.n_as + 1) + n_active] - 2 * p.meta[1]) / 3;
+    int boxes = 1;                                           // eight rows each
+    while (boxes < C::WARPS && passes * ((p.n_out + 8 * boxes - 1) / (8 * boxes)) > gridDim.x) boxes <<= 1;
+    const int chunk_rows = 8 * boxes;
+    Nvfp4Span span = nvfp4_span<C::THREADS>(cw, n_active, (p.n_out + chunk_rows - 1) / chunk_rows);
 
     if (warp == C::WARPS) {
         // ---------------------------------------------------------------- weight producer
         Ring st;
-        while (!s_abort && walk.next(ck)) {
-            const int e = p.active[ck.a], n_e = p.offsets[e + 1] - p.offsets[e];
-            const int row0 = e * p.w_stride + ck.r0, boxes = ck.n / 8;
-            for (int t0 = 0; t0 < n_e && !s_abort; t0 += nvfp4_pass_rows(n_e - t0))
-                for (int kc = 0; kc < C::KC; ++kc) {
-                    if (!__all_sync(0xffffffffu, wait_or_abort<40>(&empty[st.stage], st.phase ^ 1u, &s_abort, p.err))) break;
-                    uint8_t * dst = ring + (size_t) st.stage * C::STAGE;
-                    if (lane == 0) mbar_arrive_expect_tx(&full[st.stage], (uint32_t) (boxes * C::BOX * NTENS));
-                    __syncwarp();
-                    const int b = lane & 15;
-                    if (b < boxes && lane < 16) tma_load_2d(dst + b * C::BOX, &map_w0, kc * GEMM_RAW_ROW, row0 + 8 * b, &full[st.stage]);
-                    if (DUAL && b < boxes && lane >= 16)
-                        tma_load_2d(dst + (C::WARPS + b) * C::BOX, &map_w1, kc * GEMM_RAW_ROW, row0 + 8 * b, &full[st.stage]);
-                    st.template advance<C::STAGES>();
-                }
+        int at = -1, e = 0, n_e = 0;
+        for (; !s_abort && span.more(); span.next(n_e)) {
+            if (span.a != at) {
+                at = span.a;
+                e = p.active[at];
+                n_e = p.offsets[e + 1] - p.offsets[e];
+            }
+            const int r0 = span.ch * chunk_rows, row0 = e * p.w_stride + r0, live = min(boxes, (p.n_out - r0) / 8);
+            for (int kc = 0; kc < C::KC; ++kc) {
+                if (!__all_sync(0xffffffffu, wait_or_abort<40>(&empty[st.stage], st.phase ^ 1u, &s_abort, p.err))) break;
+                uint8_t * dst = ring + (size_t) st.stage * C::STAGE;
+                if (lane == 0) mbar_arrive_expect_tx(&full[st.stage], (uint32_t) (live * C::BOX * NTENS));
+                __syncwarp();
+                const int b = lane & 15;
+                if (b < live && lane < 16) tma_load_2d(dst + b * C::BOX, &map_w0, kc * GEMM_RAW_ROW, row0 + 8 * b, &full[st.stage]);
+                if (DUAL && b < live && lane >= 16) tma_load_2d(dst + (C::WARPS + b) * C::BOX, &map_w1, kc * GEMM_RAW_ROW, row0 + 8 * b, &full[st.stage]);
+                st.template advance<C::STAGES>();
+            }
         }
     } else {
         // ---------------------------------------------------------------- chains
-        // Every consumer warp walks every chunk and pass and meets the others at the same barriers; after an abort they walk on without work.
+        // Every consumer warp walks every item and meets the others at the same barriers; after an abort they walk on without work.
         auto meet = [] { asm volatile("bar.sync 1, %0;" ::"n"(CONSUMERS) : "memory"); };
         const int m = lane & 3, g = lane >> 2;
-        int loaded_e = -1, loaded_t0 = -1;
+        int at = -1, row_beg = 0, n_e = 0, loaded = -1, my_row = 0;      // of the expert; the pass whose activations are in place
+        float sc0 = 1.0f, sc1 = 1.0f;
         Ring st;
-        while (walk.next(ck)) {
-            const int e = p.active[ck.a], row_beg = p.offsets[e], n_e = p.offsets[e + 1] - row_beg;
-            const bool mine = 8 * warp < ck.n;
-            const int se = p.w_stride ? e : 0;               // every group of a dense product has the one matrix and its scale
-            const float sc0 = p.scale0 ? p.scale0[se] : 1.0f;
-            const float sc1 = (DUAL && p.scale1) ? p.scale1[se] : 1.0f;
-            for (int t0 = 0; t0 < n_e;) {
-                const int ntc = nvfp4_pass_rows(n_e - t0), n = min(ntc, n_e - t0);
-                if (loaded_e != e || loaded_t0 != t0) {
-                    // the activation rows of this pass into shared memory; the loads of all four are in flight together
-                    size_t arow[NT];
+        for (; span.more(); span.next(n_e)) {
+            if (span.a != at) {
+                at = span.a;
+                const int e = p.active[at], se = p.w_stride ? e : 0;     // every group of a dense product has the one matrix and its scale
+                row_beg = p.offsets[e];
+                n_e = p.offsets[e + 1] - row_beg;
+                if (p.scale0) sc0 = p.scale0[se];
+                if (DUAL && p.scale1) sc1 = p.scale1[se];
+                loaded = -1;
+            }
+            const int r0 = span.ch * chunk_rows, t0 = 4 * span.ps;
+            const int n = min(NT, n_e - t0);                             // routed rows of the pass: one or two run narrower chains
+            const bool mine = warp < min(boxes, (p.n_out - r0) / 8);
+            if (loaded != span.ps) {
+                // the activation rows of this pass into shared memory; the loads of all four are in flight together
+                size_t arow[NT];
 #pragma unroll
-                    for (int t = 0; t < NT; ++t) {
-                        const int r = p.perm[row_beg + t0 + (t < n ? t : 0)];
-                        arow[t] = (size_t) ((r / p.n_ids) * p.ne11 + (r % p.n_ids) % p.ne11);
-                    }
-                    meet();
-                    if (p.act_f32) {
-                        // Q8_0 on the fly, the arithmetic of quantize_q8_0_block: 8 lanes hold one block of 32 (4 values each)
-                        for (int i0 = 0; i0 < K / 4; i0 += CONSUMERS) {
-                            const int i = i0 + tid;
-                            const bool in = i < K / 4;
-                            float4 v[NT];
+                for (int t = 0; t < NT; ++t) {
+                    const int r = p.perm[row_beg + t0 + (t < n ? t : 0)];
+                    arow[t] = (size_t) ((r / p.n_ids) * p.ne11 + (r % p.n_ids) % p.ne11);
+                    if (t == m) my_row = r;
+                }
+                meet();
+                if (p.act_f32) {
+                    // Q8_0 on the fly, the arithmetic of quantize_q8_0_block: 8 lanes hold one block of 32 (4 values each)
+                    for (int i0 = 0; i0 < K / 4; i0 += CONSUMERS) {
+                        const int i = i0 + tid;
+                        const bool in = i < K / 4;
+                        float4 v[NT];
 #pragma unroll
-                            for (int t = 0; t < NT; ++t)
-                                v[t] = in && t < n ? __ldg(reinterpret_cast<const float4 *>(p.act_f32 + arow[t] * K) + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                            uint32_t q[NT];
-                            float d[NT];
+                        for (int t = 0; t < NT; ++t)
+                            v[t] = in && t < n ? __ldg(reinterpret_cast<const float4 *>(p.act_f32 + arow[t] * K) + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        uint32_t q[NT];
+                        float d[NT];
 #pragma unroll
-                            for (int t = 0; t < NT; ++t) {
-                                float amax = fmaxf(fmaxf(fabsf(v[t].x), fabsf(v[t].y)), fmaxf(fabsf(v[t].z), fabsf(v[t].w)));
-                                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-                                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-                                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-                                const float id = amax != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-                                q[t] = ((uint32_t) __float2int_rn(__fmul_rn(v[t].x, id)) & 0xffu) | (((uint32_t) __float2int_rn(__fmul_rn(v[t].y, id)) & 0xffu) << 8) |
-                                       (((uint32_t) __float2int_rn(__fmul_rn(v[t].z, id)) & 0xffu) << 16) | (((uint32_t) __float2int_rn(__fmul_rn(v[t].w, id)) & 0xffu) << 24);
-                                d[t] = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
-                            }
-                            if (in) {
-                                *reinterpret_cast<uint4 *>(acts + (size_t) ((i & ~7) | act_slot(i & 7)) * NT) = make_uint4(q[0], q[1], q[2], q[3]);
-                                if ((i & 7) == 0) *reinterpret_cast<float4 *>(dys + (i >> 3) * NT) = make_float4(d[0], d[1], d[2], d[3]);
-                            }
+                        for (int t = 0; t < NT; ++t) {
+                            float amax = fmaxf(fmaxf(fabsf(v[t].x), fabsf(v[t].y)), fmaxf(fabsf(v[t].z), fabsf(v[t].w)));
+                            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+                            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+                            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+                            const float id = amax != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+                            q[t] = ((uint32_t) __float2int_rn(__fmul_rn(v[t].x, id)) & 0xffu) | (((uint32_t) __float2int_rn(__fmul_rn(v[t].y, id)) & 0xffu) << 8) |
+                                   (((uint32_t) __float2int_rn(__fmul_rn(v[t].z, id)) & 0xffu) << 16) | (((uint32_t) __float2int_rn(__fmul_rn(v[t].w, id)) & 0xffu) << 24);
+                            d[t] = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
                         }
-                    } else {
-                        for (int i = tid; i < K / 4; i += CONSUMERS) {
-                            uint32_t q[NT];
-#pragma unroll
-                            for (int t = 0; t < NT; ++t) q[t] = t < n ? __ldg(reinterpret_cast<const uint32_t *>(p.act.q + arow[t] * K) + i) : 0u;
+                        if (in) {
                             *reinterpret_cast<uint4 *>(acts + (size_t) ((i & ~7) | act_slot(i & 7)) * NT) = make_uint4(q[0], q[1], q[2], q[3]);
-                        }
-                        if (tid < C::ACT_D) {
-                            float d[NT];
-#pragma unroll
-                            for (int t = 0; t < NT; ++t) d[t] = t < n ? __ldg(p.act.d + arow[t] * C::ACT_D + tid) : 0.0f;
-                            *reinterpret_cast<float4 *>(dys + tid * NT) = make_float4(d[0], d[1], d[2], d[3]);
+                            if ((i & 7) == 0) *reinterpret_cast<float4 *>(dys + (i >> 3) * NT) = make_float4(d[0], d[1], d[2], d[3]);
                         }
                     }
-                    meet();
-                    loaded_e = e;
-                    loaded_t0 = t0;
+                } else {
+                    for (int i = tid; i < K / 4; i += CONSUMERS) {
+                        uint32_t q[NT];
+#pragma unroll
+                        for (int t = 0; t < NT; ++t) q[t] = t < n ? __ldg(reinterpret_cast<const uint32_t *>(p.act.q + arow[t] * K) + i) : 0u;
+                        *reinterpret_cast<uint4 *>(acts + (size_t) ((i & ~7) | act_slot(i & 7)) * NT) = make_uint4(q[0], q[1], q[2], q[3]);
+                    }
+                    if (tid < C::ACT_D) {
+                        float d[NT];
+#pragma unroll
+                        for (int t = 0; t < NT; ++t) d[t] = t < n ? __ldg(p.act.d + arow[t] * C::ACT_D + tid) : 0.0f;
+                        *reinterpret_cast<float4 *>(dys + tid * NT) = make_float4(d[0], d[1], d[2], d[3]);
+                    }
                 }
-                float val[NTENS] = {};                       // thread m of a row ends up with the sums of routed row t0 + m
-                auto run = [&](auto ntag) {
-                    constexpr int NTC = decltype(ntag)::value;
-                    float acc[NTENS][2][NTC];
-#pragma unroll
-                    for (int r = 0; r < NTENS; ++r)
-#pragma unroll
-                        for (int t = 0; t < NTC; ++t) acc[r][0][t] = acc[r][1][t] = 0.0f;
+                meet();
+                loaded = span.ps;
+            }
+            float val[NTENS] = {};                       // thread m of a row ends up with the sums of routed row t0 + m
+            auto run = [&](auto ntag) {
+                constexpr int NTC = decltype(ntag)::value;
+                TwoLaneAcc<NTENS, NTC> acc;
+                acc.clear();
 #pragma unroll 1
-                    for (int kc = 0; kc < C::KC; ++kc) {
-                        const bool ok = __all_sync(0xffffffffu, wait_or_abort(&full[st.stage], st.phase, &s_abort, p.err));
-                        if (ok && mine) {
-                            const uint8_t * blk[NTENS];
+                for (int kc = 0; kc < C::KC; ++kc) {
+                    const bool ok = __all_sync(0xffffffffu, wait_or_abort(&full[st.stage], st.phase, &s_abort, p.err));
+                    if (ok && mine) {
+                        const uint8_t * blk[NTENS];
 #pragma unroll
-                            for (int r = 0; r < NTENS; ++r) blk[r] = ring + (size_t) st.stage * C::STAGE + (r * C::WARPS + warp) * C::BOX + g * GEMM_RAW_ROW;
-                            two_lane_chains<NTENS, NTC, NT>(blk, m, acts + kc * 64 * NT, dys + kc * 8 * NT, ue_tab, acc);
-                        }
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&empty[st.stage]);
-                        st.template advance<C::STAGES>();
+                        for (int r = 0; r < NTENS; ++r) blk[r] = ring + (size_t) st.stage * C::STAGE + (r * C::WARPS + warp) * C::BOX + g * GEMM_RAW_ROW;
+                        two_lane_chains<NTENS, NTC, NT>(blk, m, acts + kc * 64 * NT, dys + kc * 8 * NT, ue_tab, acc);
                     }
-#pragma unroll
-                    for (int r = 0; r < NTENS; ++r)
-#pragma unroll
-                        for (int t = 0; t < NTC; ++t) {
-                            const float v = hsum_two_lanes(acc[r][0][t], acc[r][1][t]);
-                            if (m == t) val[r] = v;
-                        }
-                };
-                if (ntc == 4) run(std::integral_constant<int, 4>{});
-                else if (ntc == 2) run(std::integral_constant<int, 2>{});
-                else run(std::integral_constant<int, 1>{});
-                if (mine && m < n) {
-                    const int r = p.perm[row_beg + t0 + m];
-                    float v = __fmul_rn(val[0], sc0);
-                    if (DUAL) v = __fmul_rn(ggml_silu(v), __fmul_rn(val[NTENS - 1], sc1));
-                    p.out[(size_t) r * p.n_out + ck.r0 + 8 * warp + g] = v;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&empty[st.stage]);
+                    st.template advance<C::STAGES>();
                 }
-                t0 += ntc;
+#pragma unroll
+                for (int r = 0; r < NTENS; ++r)
+#pragma unroll
+                    for (int t = 0; t < NTC; ++t) {
+                        float lo, hi;
+                        acc.lanes(r, t, lo, hi);
+                        const float v = hsum_two_lanes(lo, hi);
+                        if (m == t) val[r] = v;
+                    }
+            };
+            if (n >= 3) run(std::integral_constant<int, 4>{});
+            else if (n == 2) run(std::integral_constant<int, 2>{});
+            else run(std::integral_constant<int, 1>{});
+            if (mine && m < n) {
+                float v = __fmul_rn(val[0], sc0);
+                if (DUAL) v = __fmul_rn(ggml_silu(v), __fmul_rn(val[NTENS - 1], sc1));
+                p.out[(size_t) my_row * p.n_out + r0 + 8 * warp + g] = v;
             }
         }
     }

@@ -517,6 +517,10 @@ __global__ void __launch_bounds__(256) route_select_kernel(const float * __restr
 // routed rows per token tile of the FP4 tensor-core kernels (7 digit planes each): few and many rows per expert
 constexpr int TOKEN_TILE_SMALL = 14, TOKEN_TILE_LARGE = 27;
 
+// Work per weight row of the NVFP4 integer kernel for n routed rows: passes of four, or of two or one for what is left.  A pass of one
+// or two costs nearly what one of four does, the decode being most of it.
+__host__ __device__ __forceinline__ constexpr int nvfp4_work(int n) { return n / 4 * 16 + (n % 4 == 0 ? 0 : n % 4 == 1 ? 10 : n % 4 == 2 ? 12 : 16); }
+
 struct Groups {
     int * counts;   // [E]
     int * offsets;  // [E+1]
@@ -524,7 +528,8 @@ struct Groups {
     int * perm;     // [rows]
     int * active;   // [E]
     int * meta;     // [4]: number of active experts, rows in a group, two counters of the re-quantisation fix-up (cleared by the grouping)
-    int * cost;     // [4][E+1]: rows 0-2: prefix over active experts of the work per weight row for the nt = 1, 2, 4 kernels;
+    int * cost;     // [4][E+1]: rows 0-2: prefix over active experts of the work per weight row for the integer kernels: Q3_K with one
+                    // routed row to a pass, NVFP4 (nvfp4_work), Q3_K with up to four (3 for a pass, which decodes the weights, 2 for each row);
                     // row 3, indexed by EXPERT id: index of the expert's first token tile (prefix of ceil(rows / tile_rows))
     int tile_rows;  // TOKEN_TILE_SMALL or TOKEN_TILE_LARGE
     int * done;     // [n_done] arrival counters of the one-or-two-token down kernel (GemvParams::comb_cnt), cleared by the grouping
@@ -543,9 +548,9 @@ __device__ __forceinline__ void group_scan_body(Groups g, const int32_t * __rest
     __shared__ int s_tot[6][32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = tid < E ? g.counts[tid] : 0;
-    // rows; active experts; work per weight row: nt=1 kernels: one pass per routed row; nt=2; nt=4 kernels: 3 per pass (decode) + 2 per
-    // routed row; token tiles
-    const int own[5] = { n, n > 0 ? 1 : 0, (n + 1) / 2, 3 * ((n + 3) / 4) + 2 * n, (n + g.tile_rows - 1) / g.tile_rows };
+    // rows (also the work per weight row of the nt = 1 kernels: one pass per routed row); active experts; work per weight row of the NVFP4
+    // and of the nt = 4 kernels; token tiles
+    const int own[5] = { n, n > 0 ? 1 : 0, nvfp4_work(n), 3 * ((n + 3) / 4) + 2 * n, (n + g.tile_rows - 1) / g.tile_rows };
     int v[5];
 #pragma unroll
     for (int i = 0; i < 5; ++i) v[i] = own[i];
@@ -618,7 +623,7 @@ __global__ void __launch_bounds__(256) dense_groups_kernel(Groups g, int32_t * _
         const int last = T - (G - 1) * gsize, full = min(t, G - 1), tail = t == G ? 1 : 0;
         g.offsets[t] = full * gsize + tail * last;
         g.cost[t] = full * gsize + tail * last;
-        g.cost[(G + 1) + t] = full * ((gsize + 1) / 2) + tail * ((last + 1) / 2);
+        g.cost[(G + 1) + t] = full * nvfp4_work(gsize) + tail * nvfp4_work(last);
         g.cost[2 * (G + 1) + t] = full * (3 * ((gsize + 3) / 4) + 2 * gsize) + tail * (3 * ((last + 3) / 4) + 2 * last);
         g.cost[3 * (G + 1) + t] = full * ((gsize + g.tile_rows - 1) / g.tile_rows) + tail * ((last + g.tile_rows - 1) / g.tile_rows);
         if (t < G) g.active[t] = t;
