@@ -341,14 +341,14 @@ int make_map_2d(b200moe_ctx * ctx, CUtensorMap * m, CUtensorMapDataType dt, cons
 }
 
 // ---- kernel dispatch -----------------------------------------------------------------------------------
-template <int WT, int K, bool DUAL, int NT>
-int launch_gemv_t(b200moe_ctx * ctx, const GemvParams & p, cudaStream_t st) {
-    constexpr int GEMV_STAGES = gemv_stages<WT, K, DUAL, NT>();
-    constexpr size_t smem = gemv_smem_bytes<WT, K, DUAL, NT, GEMV_STAGES>();
-    static_assert(smem <= 227 * 1024, "ring does not fit shared memory");
-    auto kern = expert_gemv_kernel<WT, K, DUAL, NT, GEMV_STAGES>;
+// Q3_K on the int8 matrix instruction (expert_mma_q3k.cuh), 16 or 32 routed rows to a pass
+template <int K, bool DUAL, bool MANY>
+int launch_q3k_mma(b200moe_ctx * ctx, const GemvParams & p, cudaStream_t st) {
+    using C = Q3kCfg<K, DUAL, MANY ? 4 : 2>;
+    void (*kern)(const GemvParams) = q3k_expert_gemv_kernel<K, DUAL>;
+    if constexpr (MANY) kern = expert_mma_q3k_kernel<K, DUAL>;
     static bool configured[MAX_DEVICE_ORDINALS] = {};  // per instantiation and device
-    if (int rc = raise_smem_limit(ctx, kern, smem, configured)) return rc;
+    if (int rc = raise_smem_limit(ctx, kern, C::SMEM, configured)) return rc;
     b200moe_ctx::Timed tm{};
     if (ctx->timing) {
         CUDA_TRY(ctx, cudaEventCreate(&tm.beg));
@@ -356,12 +356,12 @@ int launch_gemv_t(b200moe_ctx * ctx, const GemvParams & p, cudaStream_t st) {
         tm.kind = DUAL ? 0 : ctx->dense_now ? 2 : 1;
         CUDA_TRY(ctx, cudaEventRecord(tm.beg, st));
     }
-    launch_k(ctx, kern, dim3(ctx->sm_count * gemv_ctas<WT, K, DUAL, NT>()), dim3(GemvCfg<WT, K>::NWARPS * 32), smem, st, p);
+    launch_k(ctx, kern, dim3(ctx->sm_count), dim3(C::THREADS), C::SMEM, st, p);
     if (ctx->timing) {
         CUDA_TRY(ctx, cudaEventRecord(tm.end, st));
         ctx->timed.push_back(tm);
     }
-    return check_launch(ctx, "expert_gemv");
+    return check_launch(ctx, "expert_mma_q3k");
 }
 
 // One or two tokens: the whole call is a few thousand weight rows.  Four-warp CTAs with a single 16-row stage, several per SM,
@@ -428,8 +428,7 @@ int launch_gemv_k(b200moe_ctx * ctx, const GemvParams & p, int nt, cudaStream_t 
         if constexpr (WT == TYPE_NVFP4) {
             return launch_gemv_nvfp4<K, DUAL>(ctx, p, st);
         } else {
-            if (nt <= 1) return launch_gemv_t<WT, K, DUAL, 1>(ctx, p, st);
-            return launch_gemv_t<WT, K, DUAL, 4>(ctx, p, st);
+            return launch_q3k_mma<K, DUAL, false>(ctx, p, st);
         }
     }
 }
@@ -444,29 +443,6 @@ int launch_gemv(b200moe_ctx * ctx, int wtype, int k, const GemvParams & p, int n
     return fail(ctx, B200MOE_ERR_UNSUPPORTED, "no expert kernel for type %d width %d", wtype, k);
 }
 
-// Q3_K on the int8 matrix instruction (expert_mma_q3k.cuh): the same bits as the integer GEMV.
-template <int K, bool DUAL>
-int launch_q3k_mma_t(b200moe_ctx * ctx, const GemvParams & p, cudaStream_t st) {
-    using C = Q3kMmaCfg<K, DUAL>;
-    static_assert(C::SMEM <= 220 * 1024, "operand buffers do not fit shared memory");
-    auto kern = expert_mma_q3k_kernel<K, DUAL>;
-    static bool configured[MAX_DEVICE_ORDINALS] = {};  // per instantiation and device
-    if (int rc = raise_smem_limit(ctx, kern, C::SMEM, configured)) return rc;
-    b200moe_ctx::Timed tm{};
-    if (ctx->timing) {
-        CUDA_TRY(ctx, cudaEventCreate(&tm.beg));
-        CUDA_TRY(ctx, cudaEventCreate(&tm.end));
-        tm.kind = DUAL ? 0 : ctx->dense_now ? 2 : 1;
-        CUDA_TRY(ctx, cudaEventRecord(tm.beg, st));
-    }
-    kern<<<ctx->sm_count, 256, C::SMEM, st>>>(p);
-    if (ctx->timing) {
-        CUDA_TRY(ctx, cudaEventRecord(tm.end, st));
-        ctx->timed.push_back(tm);
-    }
-    return check_launch(ctx, "expert_mma_q3k");
-}
-
 bool q3k_on_mma(int wtype, int64_t rows, int n_groups) { return wtype == TYPE_Q3_K && rows >= (int64_t) Q3K_MMA_MIN_ROWS * n_groups; }
 
 // the integer product of grouped rows: `rows` routed rows in up to n_groups groups
@@ -474,10 +450,10 @@ template <bool DUAL>
 int launch_integer(b200moe_ctx * ctx, int wtype, int k, const GemvParams & p, int64_t rows, int n_groups, int nt, cudaStream_t st) {
     if (q3k_on_mma(wtype, rows, n_groups)) {
         switch (k) {
-            case 256: return launch_q3k_mma_t<256, DUAL>(ctx, p, st);
-            case 512: return launch_q3k_mma_t<512, DUAL>(ctx, p, st);
-            case 768: return launch_q3k_mma_t<768, DUAL>(ctx, p, st);
-            case 2048: return launch_q3k_mma_t<2048, DUAL>(ctx, p, st);
+            case 256: return launch_q3k_mma<256, DUAL, true>(ctx, p, st);
+            case 512: return launch_q3k_mma<512, DUAL, true>(ctx, p, st);
+            case 768: return launch_q3k_mma<768, DUAL, true>(ctx, p, st);
+            case 2048: return launch_q3k_mma<2048, DUAL, true>(ctx, p, st);
         }
     }
     return launch_gemv<DUAL>(ctx, wtype, k, p, nt, st);

@@ -468,6 +468,51 @@ struct ChunkWalker {
     }
 };
 
+// A CTA's part of the work: items (active expert a, pass ps over PT of its routed rows, chunk ch of its weight rows), chunks fastest.
+template <int PT>
+struct PassSpan {
+    int a, ps, ch;          // next item
+    int a1, ps1, ch1;       // the next CTA's first
+    int chunks;             // of an expert
+    __device__ __forceinline__ bool more() const { return a < a1 || (a == a1 && (ps < ps1 || (ps == ps1 && ch < ch1))); }
+    __device__ __forceinline__ void next(int n_e) {          // n_e: routed rows of expert a
+        if (++ch < chunks) return;
+        ch = 0;
+        if (PT * ++ps < n_e) return;
+        ps = 0;
+        ++a;
+    }
+};
+// Boundary i sits at work i / grid of the total; both neighbours compute it the same way, so the spans tile exactly.  cw: prefix over the
+// active experts of the work per chunk: FULL for each pass, what is left of it for the last one.  The whole block looks for its two experts
+// at once.
+template <int THREADS, int PT, int FULL>
+__device__ __forceinline__ PassSpan<PT> pass_span(const int * __restrict__ cw, int n_active, int chunks) {
+    __shared__ int s_at[2];
+    const long long work = n_active ? (long long) cw[n_active] * chunks : 0;
+    const long long c[2] = { work * blockIdx.x / gridDim.x, work * (blockIdx.x + 1) / gridDim.x };
+    if (threadIdx.x < 2) s_at[threadIdx.x] = n_active;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n_active; i += THREADS) {
+        const long long here = (long long) cw[i] * chunks, next = (long long) cw[i + 1] * chunks;
+        if (here <= c[0] && c[0] < next) s_at[0] = i;
+        if (here <= c[1] && c[1] < next) s_at[1] = i;
+    }
+    __syncthreads();
+    int at[2][3] = { { n_active, 0, 0 }, { n_active, 0, 0 } };
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const int a = s_at[k];
+        if (a == n_active) continue;                         // the end of the list
+        const int w = cw[a + 1] - cw[a];
+        const long long left = c[k] - (long long) cw[a] * chunks;
+        at[k][0] = a;
+        at[k][1] = (int) (left / (FULL * chunks));
+        at[k][2] = (int) (left - (long long) at[k][1] * FULL * chunks) / min(FULL, w - FULL * at[k][1]);
+    }
+    return PassSpan<PT>{ at[0][0], at[0][1], at[0][2], at[1][0], at[1][1], at[1][2], chunks };
+}
+
 template <int WT, int K, bool DUAL, int NT, int STAGES, int NW = 8>
 constexpr size_t gemv_smem_bytes() {
     return (size_t) STAGES * GemvCfg<WT, K, NW>::TENSOR_STAGE_BYTES * (DUAL ? 2 : 1) + NT * GemvCfg<WT, K, NW>::ACT_TOKEN_BYTES + STAGES * 8 +

@@ -33,49 +33,6 @@ struct Nvfp4GemvCfg {
     static_assert(K % 256 == 0 && BOX % 128 == 0 && CTAS * (SMEM + 2048) <= 228 * 1024, "the CTAs fit an SM, boxes keep their alignment");
 };
 
-// A CTA's part of the work: items (active expert a, pass ps over four of its routed rows, chunk ch of its weight rows), chunks fastest.
-struct Nvfp4Span {
-    int a, ps, ch;          // next item
-    int a1, ps1, ch1;       // the next CTA's first
-    int chunks;             // of an expert
-    __device__ __forceinline__ bool more() const { return a < a1 || (a == a1 && (ps < ps1 || (ps == ps1 && ch < ch1))); }
-    __device__ __forceinline__ void next(int n_e) {          // n_e: routed rows of expert a
-        if (++ch < chunks) return;
-        ch = 0;
-        if (4 * ++ps < n_e) return;
-        ps = 0;
-        ++a;
-    }
-};
-// Boundary i sits at work i / grid of the total (cw: prefix of nvfp4_work over the active experts); both neighbours compute it the same
-// way, so the spans tile exactly.  The whole block looks for its two experts at once.
-template <int THREADS>
-__device__ __forceinline__ Nvfp4Span nvfp4_span(const int * __restrict__ cw, int n_active, int chunks) {
-    __shared__ int s_at[2];
-    const long long work = n_active ? (long long) cw[n_active] * chunks : 0;
-    const long long c[2] = { work * blockIdx.x / gridDim.x, work * (blockIdx.x + 1) / gridDim.x };
-    if (threadIdx.x < 2) s_at[threadIdx.x] = n_active;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n_active; i += THREADS) {
-        const long long here = (long long) cw[i] * chunks, next = (long long) cw[i + 1] * chunks;
-        if (here <= c[0] && c[0] < next) s_at[0] = i;
-        if (here <= c[1] && c[1] < next) s_at[1] = i;
-    }
-    __syncthreads();
-    int at[2][3] = { { n_active, 0, 0 }, { n_active, 0, 0 } };
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const int a = s_at[k];
-        if (a == n_active) continue;                         // the end of the list
-        const int w = cw[a + 1] - cw[a];
-        const long long left = c[k] - (long long) cw[a] * chunks;
-        at[k][0] = a;
-        at[k][1] = (int) (left / (16 * chunks));
-        at[k][2] = (int) (left - (long long) at[k][1] * 16 * chunks) / min(16, w - 16 * at[k][1]);
-    }
-    return Nvfp4Span{ at[0][0], at[0][1], at[0][2], at[1][0], at[1][1], at[1][2], chunks };
-}
-
 template <int K, bool DUAL>
 __global__ void __launch_bounds__(Nvfp4GemvCfg<K, DUAL>::THREADS, Nvfp4GemvCfg<K, DUAL>::CTAS)
 nvfp4_gemv_kernel(const GemvParams p, const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1) {
@@ -102,13 +59,13 @@ nvfp4_gemv_kernel(const GemvParams p, const __grid_constant__ CUtensorMap map_w0
 
     const int n_active = p.meta[0];
     const int * const cw = p.cost + (p.n_as + 1);
-    // Chunks of 64 weight rows; while there are items for less than every CTA, of as few rows as leaves one to a CTA.  (Passes: what is left of
-    // the work of the nt = 4 kernels, 3 to a pass and 2 to a row, without the rows.)
-    const long long passes = (p.cost[2 * (p.n_as + 1) + n_active] - 2 * p.meta[1]) / 3;
+    // Chunks of 64 weight rows; while there are items for less than every CTA, of as few rows as leaves one to a CTA.  (A pass is 10 to 16 of
+    // the work.)
+    const long long passes = (cw[n_active] + 9) / 10;
     int boxes = 1;                                           // eight rows each
     while (boxes < C::WARPS && passes * ((p.n_out + 8 * boxes - 1) / (8 * boxes)) > gridDim.x) boxes <<= 1;
     const int chunk_rows = 8 * boxes;
-    Nvfp4Span span = nvfp4_span<C::THREADS>(cw, n_active, (p.n_out + chunk_rows - 1) / chunk_rows);
+    auto span = pass_span<C::THREADS, NT, 16>(cw, n_active, (p.n_out + chunk_rows - 1) / chunk_rows);
 
     if (warp == C::WARPS) {
         // ---------------------------------------------------------------- weight producer

@@ -1,49 +1,56 @@
-// Grouped Q3_K expert matmul for prefill on the int8 matrix instruction, bit-identical to the reference.
+// Grouped Q3_K expert matmul on the int8 matrix instruction, bit-identical to the reference: every call but one or two tokens' (those take
+// expert_gemv_kernel's four-warp form).
 //
 // Why a matrix instruction can keep the reference's bits: ggml_vec_dot_q3_K_q8_K (ggml-cpu/arch/x86/quants.c:1766-1880) sums
 // INTEGERS over a whole super-block in every one of its eight SIMD lanes - lane L collects scale * code * activation over byte
 // columns 4L..4L+3 of the eight 32-groups - and only then runs one fma(d_w * d_x, (float) sum_L, acc_L).  Those 32 products are
 // one K = 32 step of mma.m16n8k32 (s8 x s8 -> s32, exact): one instruction per lane and super-block for 16 weight rows x 8 routed
 // rows, whose accumulators come out as the lane sums, followed by the reference's fp32 chain in registers.  The folded weight
-// scale * code lies in -128..128; its negative (-128..124) fits int8, so the tiles hold -scale * code and the sum is negated,
+// scale * code lies in -128..128; its negative (-128..124) fits int8, so the operand holds -scale * code and the sum is negated,
 // exactly, on its way to fp32 (|sum| <= 32 * 128 * 128 < 2^22).
 //
 // Why mma.sync and not tcgen05 (kind::i8): every accumulator is read after ONE K = 32 step.  With accumulators in tensor memory
-// each of those reads is a tcgen05.ld and a conversion more; here they are already in the registers of the thread that runs the chain, and
-// what bounds the kernel is that chain (per lane sum one add that converts and one fma) and the decode, not the matrix pipe.
+// each of those reads is a tcgen05.ld and a conversion more; here they are already in the registers of the thread that runs the chain.
 //
-// A CTA (8 warps) takes units of 64 weight rows (32 features of gate and up each, or 64 rows of one tensor) x up to 64 routed rows of
-// one expert.  A warp owns 32 weight rows x 16 routed rows: 128 fp32 chains per thread.  A weight is decoded once per unit:
-// one table look-up per (row, sub-block) gives the eight possible products as 8 bytes and one byte permute picks four of
-// them.  Decode of step s + 1 and the copies of its activations run beside the matrix work of step s (two operand buffers, one
-// barrier per super-block); the raw rows of the next unit arrive by bulk copy meanwhile.
-// What it waits for is its own decode and shared memory at two warps per scheduler (0.32 instructions per cycle); sixteen warps of half
-// the tile were no faster (581 against 537 us), the A fragments then being read twice as often.  1001 tokens, 128 experts: gate/up
-// 2823 -> 537 us, down 1986 -> 305 us.
-// Operand rows are 272 bytes apart (256 + 16), which makes the 16-byte fragment loads conflict-free.
+// A warp owns 16 weight rows (8 features of gate and up, or 16 rows of one tensor) and up to 32 routed rows.  It decodes the weights
+// straight into the instruction's operand: thread (row g, quarter q) holds 32-groups q and q + 4 of rows g and g + 8, so one funnel shift
+// brings the two low code bits of its group in place, one the high bits of both groups, and a byte permute picks four of the eight products
+// of a (row, sub-block) by the codes packed to a selector.  No operand tile in shared memory, no barrier between super-blocks: a warp fetches
+// its own raw rows and meets the others only when the routed rows change.  The code is separate for each number of token groups: with a test
+// between them nothing was scheduled across (1001 tokens, gate/up: 430 us, so 308).
+// What bounds it is the half-rate integer unit and, with 32 routed rows to a pass, its own dependences at two warps per scheduler (255
+// registers; IPC 0.58 per scheduler).  Decoding 64 x 64 tiles through shared memory, a barrier to a super-block (IPC 0.32), and a thread per
+// reference lane with dp4a took, 2048 -> 768 of 128 experts, us: gate/up of 32 tokens 130 and of 1001 tokens 537, down 71 and 311; so 73 and
+// 308, 45 and 196.
+// Activation rows are K + 16 bytes apart, which makes the 16-byte fragment loads conflict-free.
 #pragma once
 #include "common.cuh"
+#include "expert_gemm.cuh"
 #include "expert_gemv.cuh"
 #include "formats.cuh"
 #include "router.cuh"
 
 namespace b200moe {
 
-// Routed rows per expert (on average) from which this kernel replaces the GEMV, whose time grows with them while this one's does not up
-// to 64.  Gate/up (2048 -> 768), 128 experts: 4 rows GEMV 217 us, this 357; 8 rows 369 and 366; 16 rows 741 and 362; 63 rows 2825 and 537.
-// 16 experts: 8 rows 76 and 110 us, 16 rows 135 and 110.
+// Routed rows per expert (on average) from which a pass is 32 routed rows instead of 16.  Whole calls, us, 16 and 32: 128 experts, 2048 -> 768,
+// 5 rows 64 and 65, 9 rows 69 and 70, 12 rows 75 and 74, 16 rows 89 and 80, 48 rows 168 and 146; 256 -> 512: 5 rows 27 and 27, 24 rows 37 and 34.
 constexpr int Q3K_MMA_MIN_ROWS = 12;
 
-template <int K, bool DUAL>
-struct Q3kMmaCfg {
-    static constexpr int ROWS = 64, TOK = 64, PITCH = 272;
-    static constexpr int FEAT = DUAL ? 32 : 64;               // features of a unit
+template <int K, bool DUAL, int NTG>
+struct Q3kCfg {
+    static constexpr int TOK = 8 * NTG;                       // routed rows of a pass: NTG token groups
     static constexpr int ROW_BYTES = K / 256 * Q3K_BLOCK_BYTES;
-    static constexpr int RAW = ROWS * ROW_BYTES + 128;        // the last decode of a row may look past it by a word
-    static constexpr int TILE = ROWS * PITCH;
-    static constexpr size_t SMEM = 2 * (size_t) RAW + 4 * (size_t) TILE;
-    static_assert(RAW % 128 == 0 && TILE % 16 == 0 && ROWS == TOK, "buffers stay aligned for bulk copies");
-    static_assert((8 * ROW_BYTES) % 16 == 0, "a multiple of eight rows is a multiple of 16 bytes");
+    static constexpr int FEAT = DUAL ? 8 : 16;                // features of a warp's tile
+    static constexpr int TILE = 16 * ROW_BYTES;
+    static constexpr int WARPS = 8;
+    static constexpr int STAGES = K == 2048 ? 1 : 2;          // raw tiles of a warp
+    static constexpr int THREADS = WARPS * 32;
+    static constexpr int PITCH = K + 16;                      // of an activation row
+    static constexpr int SB = K / 256;
+    static constexpr int FULL = 4 + NTG;       // work of a full pass (q3k_work)
+    static constexpr size_t SMEM = (size_t) WARPS * STAGES * TILE + (size_t) TOK * PITCH;
+    static_assert(TILE % 32 == 0 && PITCH % 128 == 16, "halves of a tile are multiples of 16 bytes; fragment loads fall on different banks");
+    static_assert(SMEM + 4096 <= 227 * 1024, "one CTA fits an SM");
 };
 
 __device__ __forceinline__ void mma_s8_16832(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, int c) {
@@ -51,28 +58,24 @@ __device__ __forceinline__ void mma_s8_16832(int (&d)[4], const uint32_t (&a)[4]
         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c));
 }
-__device__ __forceinline__ void cp_async4(void * smem, const void * gmem) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
-}
-
-template <int K, bool DUAL>
-__global__ void __launch_bounds__(256, 1) expert_mma_q3k_kernel(const GemvParams p) {
-    using C = Q3kMmaCfg<K, DUAL>;
-    constexpr int SB = K / 256, PITCH = C::PITCH;
+template <int K, bool DUAL, int NTG>
+__device__ __forceinline__ void q3k_mma_body(const GemvParams & p) {
+    using C = Q3kCfg<K, DUAL, NTG>;
+    constexpr int SB = C::SB, RB = C::ROW_BYTES;
+    constexpr int MAGIC = 0x4B400000;                         // bits of 1.5 * 2^23: see small_int_to_float
     extern __shared__ __align__(128) uint8_t q3k_smem[];
-    uint8_t * const raws = q3k_smem;                          // [2] raw rows of a unit
-    uint8_t * const a_tiles = raws + 2 * C::RAW;              // [2] weights of one super-block as int8
-    uint8_t * const b_tiles = a_tiles + 2 * C::TILE;          // [2] activations of the same super-block
+    uint8_t * const acts = q3k_smem;                          // [TOK][PITCH]
+    uint8_t * const tiles = acts + (size_t) C::TOK * C::PITCH;   // [WARPS][STAGES][16 rows]
     __shared__ uint2 s_prod[64];                              // six-bit scale v -> bytes (32 - v) * (c - 4), c = 0..7
-    __shared__ float s_dw[2][C::ROWS], s_dx[2][C::TOK];
-    __shared__ int s_pref[1025];                              // 64-row token tiles before expert e
-    __shared__ uint64_t raw_full[2];
-    __shared__ int s_abort;
+    __shared__ float s_dx[C::TOK][SB];
+    __shared__ uint64_t full[C::WARPS][C::STAGES], act_full;
+    __shared__ volatile int s_abort;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
-        mbar_init(&raw_full[0], 1);
-        mbar_init(&raw_full[1], 1);
+        for (int w = 0; w < C::WARPS; ++w)
+            for (int s = 0; s < C::STAGES; ++s) mbar_init(&full[w][s], 1);
+        mbar_init(&act_full, 1);
         mbar_fence_init();
         s_abort = 0;
     }
@@ -81,250 +84,218 @@ __global__ void __launch_bounds__(256, 1) expert_mma_q3k_kernel(const GemvParams
         auto b = [&](int c) { return (uint32_t) ((s * (4 - c)) & 0xff); };
         s_prod[tid] = make_uint2(b(0) | b(1) << 8 | b(2) << 16 | b(3) << 24, b(4) | b(5) << 8 | b(6) << 16 | b(7) << 24);
     }
-    if (warp == 0) {
-        int run = 0;
-        for (int base = 0; base < p.n_as; base += 32) {
-            const int e = base + lane;
-            const int t = e < p.n_as ? (p.offsets[e + 1] - p.offsets[e] + C::TOK - 1) / C::TOK : 0;
-            int incl = t;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int up = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += up;
-            }
-            if (e < p.n_as) s_pref[e] = run + incl - t;
-            run += __shfl_sync(0xffffffffu, incl, 31);
-        }
-        if (lane == 0) s_pref[p.n_as] = run;
-    }
     __syncthreads();
+    pdl_wait();
+    pdl_launch_dependents();
 
-    const int f_tiles = (p.n_out + C::FEAT - 1) / C::FEAT;
-    const int n_units = s_pref[p.n_as] * f_tiles;
-    struct Unit { int e, f0, row0, nt; };
-    auto unit_at = [&](int u) {
-        Unit w;
-        const int tile = u / f_tiles;
-        w.f0 = (u - tile * f_tiles) * C::FEAT;
-        int lo = 0, hi = p.n_as;                              // largest e with s_pref[e] <= tile
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (s_pref[mid] <= tile) lo = mid; else hi = mid;
-        }
-        w.e = lo;
-        w.row0 = p.offsets[lo] + (tile - s_pref[lo]) * C::TOK;
-        w.nt = min(C::TOK, p.offsets[lo + 1] - w.row0);
-        return w;
-    };
-    auto load_raw = [&](int u, int buf) {                     // one thread
-        const Unit w = unit_at(u);
-        const uint32_t bytes = (uint32_t) min(C::FEAT, p.n_out - w.f0) * C::ROW_BYTES;
-        const size_t off = ((size_t) w.e * p.w_stride + w.f0) * C::ROW_BYTES;
-        uint8_t * dst = raws + (size_t) buf * C::RAW;
-        mbar_arrive_expect_tx(&raw_full[buf], bytes * (DUAL ? 2 : 1));
-        bulk_g2s(dst, p.w0 + off, bytes, &raw_full[buf]);
-        if (DUAL) bulk_g2s(dst + C::FEAT * C::ROW_BYTES, p.w1 + off, bytes, &raw_full[buf]);
-    };
-    // activation row that this thread copies (token tid / 4, a quarter of its 256 bytes); rows beyond the tile repeat its first
-    auto act_row = [&](const Unit & w) {
-        const int t = tid >> 2;
-        const int r = p.perm[w.row0 + (t < w.nt ? t : 0)];
-        return (r / p.n_ids) * p.ne11 + (r % p.n_ids) % p.ne11;
-    };
-    auto load_act = [&](int arow, int sb, int buf) {
-        const int8_t * src = p.act.q + (size_t) arow * K + sb * 256 + (tid & 3) * 64;
-        uint8_t * dst = b_tiles + (size_t) buf * C::TILE + (tid >> 2) * PITCH + (tid & 3) * 64;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) cp_async16(dst + 16 * i, src + 16 * i);
-        if ((tid & 3) == 0) cp_async4(&s_dx[buf][tid >> 2], p.act.d + (size_t) arow * SB + sb);
-    };
-    // thread = weight row tid / 4, lanes L = 2h and 2h + 1 (h = tid % 4) of its super-block
-    auto decode = [&](int raw_buf, int sb, int buf) {
-        const int row = tid >> 2, h = tid & 3;
-        const uint32_t at = (uint32_t) (row * C::ROW_BYTES + sb * Q3K_BLOCK_BYTES);
-        const uint32_t * blk = reinterpret_cast<const uint32_t *>(raws + (size_t) raw_buf * C::RAW + (at & ~3u));
-        const int sh = (int) (at & 2u) * 8;                   // a block starts on a 2-byte boundary
-        uint32_t hm[2], q[2][2], sc[4];
-        {
-            const uint32_t * s = blk + 2 * h;
-            hm[0] = __funnelshift_r(s[0], s[1], sh);  hm[1] = __funnelshift_r(s[1], s[2], sh);
-            q[0][0] = __funnelshift_r(s[8], s[9], sh);  q[0][1] = __funnelshift_r(s[9], s[10], sh);
-            q[1][0] = __funnelshift_r(s[16], s[17], sh);  q[1][1] = __funnelshift_r(s[17], s[18], sh);
-            const uint32_t w0 = blk[24], w1 = blk[25], w2 = blk[26], w3 = blk[27];
-            const uint32_t s0 = __funnelshift_r(w0, w1, sh), s1 = __funnelshift_r(w1, w2, sh), s2 = __funnelshift_r(w2, w3, sh);
-            const uint32_t m2 = 0x03030303u, m4 = 0x0f0f0f0fu;
-            const int hi = h >= 2 ? 8 : 0;                    // lanes 4..7 use the odd sub-blocks' scales
-            sc[0] = ((s0 & m4) | ((s2 & m2) << 4)) >> hi;
-            sc[1] = ((s1 & m4) | (((s2 >> 2) & m2) << 4)) >> hi;
-            sc[2] = (((s0 >> 4) & m4) | (((s2 >> 4) & m2) << 4)) >> hi;
-            sc[3] = (((s1 >> 4) & m4) | (((s2 >> 6) & m2) << 4)) >> hi;
-            if (h == 0) s_dw[buf][row] = __half2float(__ushort_as_half((unsigned short) (w3 >> sh)));
-        }
-        uint8_t * dst = a_tiles + (size_t) buf * C::TILE + row * PITCH + 8 * h;
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                const int bit = 4 * j + s;
-                const uint2 prod = s_prod[(sc[2 * j + (s >> 1)] >> (16 * (s & 1))) & 0x3fu];
-                uint32_t out[2];
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const uint32_t hb = bit >= 2 ? (hm[e] >> (bit - 2)) : (hm[e] << (2 - bit));
-                    const uint32_t t = ((q[j][e] >> (2 * s)) & 0x03030303u) | (hb & 0x04040404u);   // codes 0..7, one per byte
-                    out[e] = __byte_perm(prod.x, prod.y, __byte_perm(t | (t >> 4), 0u, 0x4420));    // packed to nibbles, looked up
-                }
-                *reinterpret_cast<uint2 *>(dst + bit * 32) = make_uint2(out[0], out[1]);
+    const int n_active = p.meta[0];
+    const int * const cw = p.cost + (NTG < 4 ? 0 : 2) * (p.n_as + 1);
+    // a tile for each warp to a chunk; while there are items for less than every CTA, as few as leaves one to a CTA
+    const int n_tiles = (p.n_out + C::FEAT - 1) / C::FEAT;
+    const long long passes = (cw[n_active] + 4) / 5;
+    int per = 1;
+    while (per < C::WARPS && passes * ((n_tiles + per - 1) / per) > gridDim.x) per = min(C::WARPS, 2 * per);
+    auto span = pass_span<C::THREADS, C::TOK, C::FULL>(cw, n_active, (n_tiles + per - 1) / per);
+
+    // raw rows of the warp's tile of an item, if it has one
+    auto has_tile = [&](int ch) { return warp < per && ch * per + warp < n_tiles; };
+    uint8_t * const my_tiles = tiles + (size_t) warp * C::STAGES * C::TILE;
+    auto pre = span;
+    int pre_at = -1, pre_e = 0, pre_n = 0, pre_stage = 0;
+    auto fetch = [&] {                                        // of the next item that has one
+        while (pre.more()) {
+            if (pre.a != pre_at) {
+                pre_at = pre.a;
+                pre_e = p.active[pre_at];
+                pre_n = p.offsets[pre_e + 1] - p.offsets[pre_e];
             }
-    };
-
-    const int wm = warp & 1, wn = warp >> 1;                  // a warp's half of the weight rows; its token groups are wn and wn + 4
-    const int gq = lane >> 2, tq = lane & 3;
-    const int m_row[2] = { DUAL ? wm * 16 : wm * 32, DUAL ? 32 + wm * 16 : wm * 32 + 16 };
-    constexpr int MAGIC = 0x4B400000;                         // bits of 1.5 * 2^23: see small_int_to_float
-
-    int issued = 0, waited = 0;
-    const int first = blockIdx.x, step_u = gridDim.x;
-    Unit cur{}, nxt{};
-    int arow = 0;
-    if (first < n_units) {
-        if (tid == 0) {
-            load_raw(first, 0);
-            ++issued;
-            if (first + step_u < n_units) { load_raw(first + step_u, 1); ++issued; }
+            const int ch = pre.ch;
+            pre.next(pre_n);
+            if (!has_tile(ch)) continue;
+            const int f0 = (ch * per + warp) * C::FEAT;
+            if (lane == 0) {
+                uint8_t * dst = my_tiles + (size_t) pre_stage * C::TILE;
+                uint64_t * bar = &full[warp][pre_stage];
+                const size_t off = ((size_t) pre_e * p.w_stride + f0) * RB;
+                const uint32_t bytes = DUAL ? C::TILE : (uint32_t) min(16, p.n_out - f0) * RB;
+                mbar_arrive_expect_tx(bar, bytes);
+                if (DUAL) {
+                    bulk_g2s(dst, p.w0 + off, C::TILE / 2, bar);
+                    bulk_g2s(dst + C::TILE / 2, p.w1 + off, C::TILE / 2, bar);
+                } else {
+                    bulk_g2s(dst, p.w0 + off, bytes, bar);
+                }
+            }
+            pre_stage = pre_stage + 1 == C::STAGES ? 0 : pre_stage + 1;
+            return;
         }
-        cur = unit_at(first);
-        arow = act_row(cur);
-        load_act(arow, 0, 0);
-        cp_async_commit();
-        if (!mbar_wait_bounded(&raw_full[0], 0)) { report_error(p.err, DEV_ERR_BARRIER_TIMEOUT); s_abort = 1; }
-        ++waited;
-        decode(0, 0, 0);
-        cp_async_wait<0>();
-    }
-    bool failed = __syncthreads_or(s_abort) != 0;
-    float acc[2][2][8][4];
-    int buf = 0;
-    for (int u = first, ui = 0; u < n_units && !failed; u += step_u, ++ui) {
+    };
+    for (int s = 0; s < C::STAGES; ++s) fetch();
+
+    const int g = lane >> 2, q = lane & 3;
+    const uint64_t minus_one = f32x2(-1.0f, -1.0f), magic2 = f32x2(12582912.0f, 12582912.0f);
+    int at = -1, row_beg = 0, n_e = 0, loaded = -1;           // of the expert; the pass whose activations are in place
+    float sc0 = 1.0f, sc1 = 1.0f;
+    uint32_t act_parity = 0;
+    Ring st;
+    for (; span.more(); span.next(n_e)) {
+        if (span.a != at) {
+            at = span.a;
+            const int e = p.active[at], se = p.w_stride ? e : 0;         // every group of a dense product has the one matrix and its scale
+            row_beg = p.offsets[e];
+            n_e = p.offsets[e + 1] - row_beg;
+            if (p.scale0) sc0 = p.scale0[se];
+            if (DUAL && p.scale1) sc1 = p.scale1[se];
+            loaded = -1;
+        }
+        const int t0 = C::TOK * span.ps, n = min(C::TOK, n_e - t0);
+        if (loaded != span.ps) {
+            __syncthreads();                                  // everybody is done with the rows that give way
+            if (warp == 0) {
+                if (lane == 0) mbar_arrive_expect_tx(&act_full, (uint32_t) (n * K));
+                __syncwarp();
+                if (lane < n) {
+                    const int r = p.perm[row_beg + t0 + lane];
+                    const int arow = (r / p.n_ids) * p.ne11 + (r % p.n_ids) % p.ne11;
+                    bulk_g2s(acts + (size_t) lane * C::PITCH, p.act.q + (size_t) arow * K, K, &act_full);
+                }
+            }
+            for (int i = tid; i < n * SB; i += C::THREADS) {
+                const int r = p.perm[row_beg + t0 + i / SB];
+                const int arow = (r / p.n_ids) * p.ne11 + (r % p.n_ids) % p.ne11;
+                s_dx[i / SB][i % SB] = p.act.d[(size_t) arow * SB + i % SB];
+            }
+            wait_or_abort(&act_full, act_parity, &s_abort, p.err);
+            act_parity ^= 1u;
+            __syncthreads();
+            loaded = span.ps;
+        }
+        if (!has_tile(span.ch)) continue;
+        const bool ok = __all_sync(0xffffffffu, wait_or_abort(&full[warp][st.stage], st.phase, &s_abort, p.err));
+        if (!ok) continue;                                    // the barriers above still see this warp
+        const uint8_t * const tile = my_tiles + (size_t) st.stage * C::TILE;
+
+        auto run = [&](auto gtag) {                           // token groups that exist: no branch between them
+            constexpr int G = decltype(gtag)::value;
+            uint64_t acc[G][8][2];                              // [token group][SIMD lane][row g, g + 8]: routed rows 2q and 2q + 1 of the group
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
+            for (int i = 0; i < G; ++i)
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int L = 0; L < 8; ++L)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[m][i][L][c] = 0.0f;
-        const bool more = u + step_u < n_units;
-        if (more) nxt = unit_at(u + step_u);
+                for (int L = 0; L < 8; ++L) acc[i][L][0] = acc[i][L][1] = f32x2(0.0f, 0.0f);
 #pragma unroll 1
-        for (int sb = 0; sb < SB; ++sb, buf ^= 1) {
-            // operands of the next step (the next super-block, or the first one of the next unit)
-            if (sb + 1 < SB) {
-                load_act(arow, sb + 1, buf ^ 1);
-                cp_async_commit();
-                decode(ui & 1, sb + 1, buf ^ 1);
-            } else {
-                // every thread has decoded the last super-block of this unit: its raw rows give way to those of the next but one
-                if (tid == 0 && u + 2 * step_u < n_units) { load_raw(u + 2 * step_u, ui & 1); ++issued; }
-                if (more) {
-                    arow = act_row(nxt);
-                    load_act(arow, 0, buf ^ 1);
-                    cp_async_commit();
-                    if (!mbar_wait_bounded(&raw_full[(ui + 1) & 1], (uint32_t) ((ui + 1) >> 1) & 1u)) { report_error(p.err, DEV_ERR_BARRIER_TIMEOUT); s_abort = 1; }
-                    ++waited;
-                    decode((ui + 1) & 1, 0, buf ^ 1);
+            for (int sb = 0; sb < SB; ++sb) {
+                const uint32_t * hw[2];                           // aligned words of the block of rows g and g + 8
+                int sh[2];                                        // a block starts on a 2-byte boundary
+                uint32_t sc[2];
+                uint64_t s2[G][2];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const uint32_t off = (uint32_t) ((r * 8 + g) * RB + sb * Q3K_BLOCK_BYTES);
+                    const uint8_t * blk = tile + off;
+                    hw[r] = reinterpret_cast<const uint32_t *>(tile + (off & ~3u));
+                    sh[r] = (int) (off & 2u) * 8;
+                    // scales of sub-blocks 8j + 2q and 8j + 2q + 1: nibble j of bytes 2q, 2q + 1, two more bits from the last four bytes
+                    const uint32_t lo4 = *reinterpret_cast<const uint16_t *>(blk + 96 + 2 * q);
+                    const uint32_t hi2 = (uint32_t) *reinterpret_cast<const uint16_t *>(blk + 104 + (2 * q & 2)) >> (q & 2);
+                    sc[r] = (lo4 & 0x0f0fu) + (lo4 & 0xf0f0u) * 4096u + (hi2 & 0x0303u) * 16u + (hi2 & 0x3030u) * 65536u;   // byte 2j + hf
+                    const float dw = __half2float(*reinterpret_cast<const __half *>(blk + 108));
+#pragma unroll
+                    for (int i = 0; i < G; ++i) s2[i][r] = mul_f32x2(f32x2(s_dx[8 * i + 2 * q][sb], s_dx[8 * i + 2 * q + 1][sb]), f32x2(dw, dw));
                 }
-            }
-            if (8 * wn < cur.nt) {
-                const uint8_t * at = a_tiles + (size_t) buf * C::TILE;
-                const uint8_t * bt = b_tiles + (size_t) buf * C::TILE;
-                const bool two = 8 * (wn + 4) < cur.nt;       // warp-uniform: the second token group exists
-                float dw[2][2], dx[2][2];
 #pragma unroll
-                for (int m = 0; m < 2; ++m) { dw[m][0] = s_dw[buf][m_row[m] + gq]; dw[m][1] = s_dw[buf][m_row[m] + gq + 8]; }
+                for (int hf = 0; hf < 2; ++hf) {                  // lanes 4 hf .. 4 hf + 3, which have their sub-blocks' scales in common
+                    uint2 prod[2][2];                             // [row][j]
 #pragma unroll
-                for (int i = 0; i < 2; ++i) { dx[i][0] = s_dx[buf][8 * (wn + 4 * i) + 2 * tq]; dx[i][1] = s_dx[buf][8 * (wn + 4 * i) + 2 * tq + 1]; }
+                    for (int r = 0; r < 2; ++r)
 #pragma unroll
-                for (int hf = 0; hf < 2; ++hf) {              // lanes 4 hf .. 4 hf + 3
-                    uint4 b[2][2];
+                        for (int j = 0; j < 2; ++j) prod[r][j] = s_prod[(sc[r] >> (16 * j + 8 * hf)) & 0xffu];
+                    uint4 b[G][2];
 #pragma unroll
-                    for (int i = 0; i < 2; ++i)
+                    for (int i = 0; i < G; ++i)
 #pragma unroll
-                        for (int g = 0; g < 2; ++g)
-                            if (i == 0 || two)
-                                b[i][g] = *reinterpret_cast<const uint4 *>(bt + (8 * (wn + 4 * i) + gq) * PITCH + (tq + 4 * g) * 32 + 16 * hf);
+                        for (int j = 0; j < 2; ++j)
+                            b[i][j] = *reinterpret_cast<const uint4 *>(acts + (size_t) (8 * i + g) * C::PITCH + sb * 256 + j * 128 + q * 32 + 16 * hf);
+                    auto word = [](const uint4 & v, int l) { return l == 0 ? v.x : l == 1 ? v.y : l == 2 ? v.z : v.w; };
 #pragma unroll
-                    for (int m = 0; m < 2; ++m) {
-                        uint4 a[2][2];                        // [row gq, gq + 8][group tq, tq + 4]
+                    for (int l = 0; l < 4; ++l) {
+                        const int L = 4 * hf + l;
+                        uint32_t a[4];                            // [row g, g + 8] of group q, then of group q + 4
 #pragma unroll
-                        for (int r = 0; r < 2; ++r)
+                        for (int r = 0; r < 2; ++r) {
+                            const uint32_t hb = __funnelshift_r(hw[r][L], hw[r][L + 1], sh[r] + q);          // bit 0: group q, bit 4: group q + 4
+                            const uint32_t q0 = __funnelshift_r(hw[r][8 + L], hw[r][9 + L], sh[r] + 2 * q) & 0x03030303u;
+                            const uint32_t q1 = __funnelshift_r(hw[r][16 + L], hw[r][17 + L], sh[r] + 2 * q) & 0x03030303u;
+                            // Codes c = 4 hb + q, 0..7, one per byte; c * 272 is c in the high nibble of its byte and in the low nibble of
+                            // the next, so bytes 1 and 3 hold the selector of the four products.  (Multiplications: the integer unit is the busy one.)
+                            const uint32_t u0 = (hb & 0x01010101u) * 1088u + q0 * 272u, u1 = (hb & 0x10101010u) * 68u + q1 * 272u;
+                            a[r] = __byte_perm(prod[r][0].x, prod[r][0].y, __byte_perm(u0, 0u, 0x4431));
+                            a[2 + r] = __byte_perm(prod[r][1].x, prod[r][1].y, __byte_perm(u1, 0u, 0x4431));
+                        }
 #pragma unroll
-                            for (int g = 0; g < 2; ++g)
-                                a[r][g] = *reinterpret_cast<const uint4 *>(at + (m_row[m] + gq + 8 * r) * PITCH + (tq + 4 * g) * 32 + 16 * hf);
-                        auto word = [](const uint4 & v, int l) { return l == 0 ? v.x : l == 1 ? v.y : l == 2 ? v.z : v.w; };
+                        for (int i = 0; i < G; ++i) {
+                                int d[4];
+                                mma_s8_16832(d, a, word(b[i][0], l), word(b[i][1], l), MAGIC);
 #pragma unroll
-                        for (int i = 0; i < 2; ++i)
-                            if (i == 0 || two) {
-                                const float s[4] = { __fmul_rn(dx[i][0], dw[m][0]), __fmul_rn(dx[i][1], dw[m][0]), __fmul_rn(dx[i][0], dw[m][1]),
-                                                     __fmul_rn(dx[i][1], dw[m][1]) };
-#pragma unroll
-                                for (int l = 0; l < 4; ++l) {
-                                    const uint32_t af[4] = { word(a[0][0], l), word(a[1][0], l), word(a[0][1], l), word(a[1][1], l) };
-                                    int d[4];
-                                    mma_s8_16832(d, af, word(b[i][0], l), word(b[i][1], l), MAGIC);
-#pragma unroll
-                                    for (int c = 0; c < 4; ++c)
-                                        acc[m][i][4 * hf + l][c] = __fmaf_rn(s[c], __fsub_rn(12582912.0f, __int_as_float(d[c])), acc[m][i][4 * hf + l][c]);
+                                for (int r = 0; r < 2; ++r) {
+                                    const uint64_t sum = fma_f32x2(f32x2(__int_as_float(d[2 * r]), __int_as_float(d[2 * r + 1])), minus_one, magic2);
+                                    acc[i][L][r] = fma_f32x2(s2[i][r], sum, acc[i][L][r]);
                                 }
                             }
                     }
                 }
             }
-            cp_async_wait<0>();
-            if (__syncthreads_or(s_abort)) { failed = true; break; }
-        }
-        if (failed) break;
-        // hsum_float_8 of every value, scales, SwiGLU, scatter
-        const int se = p.w_stride ? cur.e : 0;   // every group of a dense product has the one matrix and its scale
-        const float sc0 = p.scale0 ? p.scale0[se] : 1.0f;
-        const float sc1 = (DUAL && p.scale1) ? p.scale1[se] : 1.0f;
+            __syncwarp();                                         // all lanes are done with the raw rows
+            fetch();
+            st.template advance<C::STAGES>();
+
+            // hsum_float_8 of every value, scales, SwiGLU, scatter
+            const int f0 = (span.ch * per + warp) * C::FEAT;
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+            for (int i = 0; i < G; ++i) {
+                float v[2][2];                                    // [row][routed row]
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const int t = 8 * (wn + 4 * i) + 2 * tq + c;
-                if (t < cur.nt) {
-                    float * orow = p.out + (size_t) p.perm[cur.row0 + t] * p.n_out;
+                for (int r = 0; r < 2; ++r) {
+                    uint64_t s4[4];
 #pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        float v[2];
+                    for (int l = 0; l < 4; ++l) s4[l] = add_f32x2(acc[i][l][r], acc[i][l + 4][r]);
+                    const float2 s = f32x2_halves(add_f32x2(add_f32x2(s4[0], s4[2]), add_f32x2(s4[1], s4[3])));
+                    v[r][0] = s.x;
+                    v[r][1] = s.y;
+                }
 #pragma unroll
-                        for (int m = 0; m < 2; ++m) {
-                            float s4[4];
-#pragma unroll
-                            for (int l = 0; l < 4; ++l) s4[l] = __fadd_rn(acc[m][i][l][2 * r + c], acc[m][i][l + 4][2 * r + c]);
-                            v[m] = __fadd_rn(__fadd_rn(s4[0], s4[2]), __fadd_rn(s4[1], s4[3]));
-                        }
-                        if (DUAL) {
-                            const int f = cur.f0 + wm * 16 + gq + 8 * r;
-                            if (f < p.n_out) orow[f] = __fmul_rn(ggml_silu(__fmul_rn(v[0], sc0)), __fmul_rn(v[1], sc1));
-                        } else {
-#pragma unroll
-                            for (int m = 0; m < 2; ++m) {
-                                const int f = cur.f0 + m_row[m] + gq + 8 * r;
-                                if (f < p.n_out) orow[f] = __fmul_rn(v[m], sc0);
-                            }
-                        }
+                for (int c = 0; c < 2; ++c) {
+                    const int t = 8 * i + 2 * q + c;
+                    if (t >= n) continue;
+                    float * orow = p.out + (size_t) p.perm[row_beg + t0 + t] * p.n_out + f0;
+                    if (DUAL) {
+                        orow[g] = __fmul_rn(ggml_silu(__fmul_rn(v[0][c], sc0)), __fmul_rn(v[1][c], sc1));
+                    } else {
+                        orow[g] = __fmul_rn(v[0][c], sc0);
+                        if (f0 + 8 < p.n_out) orow[g + 8] = __fmul_rn(v[1][c], sc0);
                     }
                 }
             }
-        cur = nxt;
+        };
+        const int groups = (n + 7) / 8;
+        if (groups == 1) run(std::integral_constant<int, 1>{});
+        else if (NTG == 2 || groups == 2) run(std::integral_constant<int, 2>{});
+        else if (groups == 3) run(std::integral_constant<int, NTG == 2 ? 1 : 3>{});
+        else run(std::integral_constant<int, NTG>{});
     }
-    if (failed && tid == 0) {
-        // bounded drain of copies still in flight before the block (and its shared memory) goes away
-        cp_async_wait<0>();
-        for (int k = waited; k < issued; ++k) mbar_wait_bounded(&raw_full[k & 1], (uint32_t) (k >> 1) & 1u, 200000000ull);
+    if (s_abort) {   // copies still in flight land before the block (and its shared memory) goes away
+        const uint64_t t = global_timer_ns();
+        while (global_timer_ns() - t < 1000000ull) { }
     }
+    __syncthreads();
+}
+
+template <int K, bool DUAL>
+__global__ void __launch_bounds__(Q3kCfg<K, DUAL, 2>::THREADS, 1) q3k_expert_gemv_kernel(const GemvParams p) {
+    q3k_mma_body<K, DUAL, 2>(p);
+}
+template <int K, bool DUAL>
+__global__ void __launch_bounds__(Q3kCfg<K, DUAL, 4>::THREADS, 1) expert_mma_q3k_kernel(const GemvParams p) {
+    q3k_mma_body<K, DUAL, 4>(p);
 }
 
 }  // namespace b200moe

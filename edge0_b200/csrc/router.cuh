@@ -521,6 +521,10 @@ constexpr int TOKEN_TILE_SMALL = 14, TOKEN_TILE_LARGE = 27;
 // or two costs nearly what one of four does, the decode being most of it.
 __host__ __device__ __forceinline__ constexpr int nvfp4_work(int n) { return n / 4 * 16 + (n % 4 == 0 ? 0 : n % 4 == 1 ? 10 : n % 4 == 2 ? 12 : 16); }
 
+// The same for Q3_K in passes of TOK (16 or 32) routed rows, eight at a time: the decode is worth four times eight rows.
+template <int TOK>
+__host__ __device__ __forceinline__ constexpr int q3k_work(int n) { return n / TOK * (4 + TOK / 8) + (n % TOK ? 4 + (n % TOK + 7) / 8 : 0); }
+
 struct Groups {
     int * counts;   // [E]
     int * offsets;  // [E+1]
@@ -528,8 +532,8 @@ struct Groups {
     int * perm;     // [rows]
     int * active;   // [E]
     int * meta;     // [4]: number of active experts, rows in a group, two counters of the re-quantisation fix-up (cleared by the grouping)
-    int * cost;     // [4][E+1]: rows 0-2: prefix over active experts of the work per weight row for the integer kernels: Q3_K with one
-                    // routed row to a pass, NVFP4 (nvfp4_work), Q3_K with up to four (3 for a pass, which decodes the weights, 2 for each row);
+    int * cost;     // [4][E+1]: rows 0-2: prefix over active experts of the work per weight row for the integer kernels: Q3_K with 16
+                    // routed rows to a pass (q3k_work), NVFP4 (nvfp4_work), Q3_K with 32;
                     // row 3, indexed by EXPERT id: index of the expert's first token tile (prefix of ceil(rows / tile_rows))
     int tile_rows;  // TOKEN_TILE_SMALL or TOKEN_TILE_LARGE
     int * done;     // [n_done] arrival counters of the one-or-two-token down kernel (GemvParams::comb_cnt), cleared by the grouping
@@ -545,27 +549,27 @@ __device__ __forceinline__ void group_scan_body(Groups g, const int32_t * __rest
         for (int i = threadIdx.x; i < g.n_done; i += blockDim.x) g.done[i] = 0;
     // thread = expert (the launchers use 1024 threads, the largest expert count): a scan per warp, then one over the warps' totals
     int * off = sh;                      // [E]
-    __shared__ int s_tot[6][32];
+    __shared__ int s_tot[7][32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int n = tid < E ? g.counts[tid] : 0;
-    // rows (also the work per weight row of the nt = 1 kernels: one pass per routed row); active experts; work per weight row of the NVFP4
-    // and of the nt = 4 kernels; token tiles
-    const int own[5] = { n, n > 0 ? 1 : 0, nvfp4_work(n), 3 * ((n + 3) / 4) + 2 * n, (n + g.tile_rows - 1) / g.tile_rows };
-    int v[5];
+    // rows; active experts; work per weight row of the Q3_K kernel of few rows, of NVFP4's and of the Q3_K kernel of many; token tiles
+    constexpr int N = 6;
+    const int own[N] = { n, n > 0 ? 1 : 0, q3k_work<16>(n), nvfp4_work(n), q3k_work<32>(n), (n + g.tile_rows - 1) / g.tile_rows };
+    int v[N];
 #pragma unroll
-    for (int i = 0; i < 5; ++i) v[i] = own[i];
+    for (int i = 0; i < N; ++i) v[i] = own[i];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1)
 #pragma unroll
-        for (int i = 0; i < 5; ++i) {
+        for (int i = 0; i < N; ++i) {
             const int up = __shfl_up_sync(0xffffffffu, v[i], o);
             if (lane >= o) v[i] += up;
         }
     if (lane == 31)
 #pragma unroll
-        for (int i = 0; i < 5; ++i) s_tot[i][warp] = v[i];
+        for (int i = 0; i < N; ++i) s_tot[i][warp] = v[i];
     __syncthreads();
-    if (warp < 5) {
+    if (warp < N) {
         const int own_t = lane < (int) (blockDim.x >> 5) ? s_tot[warp][lane] : 0;
         int t = own_t;
 #pragma unroll
@@ -574,28 +578,29 @@ __device__ __forceinline__ void group_scan_body(Groups g, const int32_t * __rest
             if (lane >= o) t += up;
         }
         s_tot[warp][lane] = t - own_t;
-        if (lane == 31) s_tot[5][warp] = t;
+        if (lane == 31) s_tot[N][warp] = t;
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 5; ++i) v[i] += s_tot[i][warp] - own[i];     // exclusive prefixes
+    for (int i = 0; i < N; ++i) v[i] += s_tot[i][warp] - own[i];     // exclusive prefixes
     if (tid < E) {
         off[tid] = v[0];
         if (block == 0) {
             g.offsets[tid] = v[0];
-            g.cost[3 * (E + 1) + tid] = v[4];
+            g.cost[3 * (E + 1) + tid] = v[5];
             if (n > 0) {
                 g.active[v[1]] = tid;
-                g.cost[v[1]] = v[0];
-                g.cost[(E + 1) + v[1]] = v[2];
-                g.cost[2 * (E + 1) + v[1]] = v[3];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) g.cost[i * (E + 1) + v[1]] = v[2 + i];
             }
         }
     }
     if (tid == 0 && block == 0) {
-        const int run = s_tot[5][0], na = s_tot[5][1];
+        const int run = s_tot[N][0], na = s_tot[N][1];
         g.offsets[E] = run;
-        g.cost[na] = run; g.cost[(E + 1) + na] = s_tot[5][2]; g.cost[2 * (E + 1) + na] = s_tot[5][3]; g.cost[3 * (E + 1) + E] = s_tot[5][4];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) g.cost[i * (E + 1) + na] = s_tot[N][2 + i];
+        g.cost[3 * (E + 1) + E] = s_tot[N][5];
         g.meta[0] = na;
         g.meta[1] = run;
         g.meta[2] = g.meta[3] = 0;       // the counters of the re-quantisation fix-up
@@ -622,9 +627,9 @@ __global__ void __launch_bounds__(256) dense_groups_kernel(Groups g, int32_t * _
         // prefixes over t groups: all of gsize rows but for the last group
         const int last = T - (G - 1) * gsize, full = min(t, G - 1), tail = t == G ? 1 : 0;
         g.offsets[t] = full * gsize + tail * last;
-        g.cost[t] = full * gsize + tail * last;
+        g.cost[t] = full * q3k_work<16>(gsize) + tail * q3k_work<16>(last);
         g.cost[(G + 1) + t] = full * nvfp4_work(gsize) + tail * nvfp4_work(last);
-        g.cost[2 * (G + 1) + t] = full * (3 * ((gsize + 3) / 4) + 2 * gsize) + tail * (3 * ((last + 3) / 4) + 2 * last);
+        g.cost[2 * (G + 1) + t] = full * q3k_work<32>(gsize) + tail * q3k_work<32>(last);
         g.cost[3 * (G + 1) + t] = full * ((gsize + g.tile_rows - 1) / g.tile_rows) + tail * ((last + g.tile_rows - 1) / g.tile_rows);
         if (t < G) g.active[t] = t;
     }
