@@ -58,9 +58,8 @@ struct Plan {  // carved out of the scratch arena for one (layer shape, max_toke
     float * outb = nullptr; // [T][n_embd] staging for the host entry point
     int * one_group_ids = nullptr;  // [T] group of every token when a dense matvec runs on the indexed-matmul kernel
     __half * afp16 = nullptr;       // [T*k][max(n_in, n_ff)] expert-sorted fp16 activations of the tensor-core path (or the FP4 digit planes)
-    uint8_t * asf = nullptr;        // scale tiles of the FP4 digit planes: [token tiles][K / 256][fp4_sfb_bytes(rows per tile)]
-    size_t asf_bytes = 0;
-    int * tile_expert = nullptr;    // expert of every token tile of the FP4 kernels
+    uint8_t * asf = nullptr;        // scales of the FP4 digit planes: [K / 256][rows][16]
+    int4 * tiles = nullptr;         // the token tiles of the FP4 kernels (PlaneOut::tiles)
     float * arow_scale = nullptr;   // [T*k] power of two per expert-sorted routed row (FP4 digit planes)
     float * sh_a = nullptr;         // [T][n_ff_sh] shared expert: gate product, then silu(gate) * up
     float * sh_b = nullptr;         // [T][n_ff_sh] shared expert: up product
@@ -161,13 +160,9 @@ void carve(Plan & p, uint8_t * base) {
     p.outb = c.take<float>(T * H);
     p.one_group_ids = c.take<int>(T);
     p.afp16 = c.take<__half>(2 * std::max<size_t>(std::max(R, T), 64) * std::max({kin, I, H, Ish}));   // hi plane, then lo plane
-    // scale tiles: at most one partial token tile per expert, whatever the tile size
-    const size_t sf_stage = std::max((std::min(E, std::max(R, T)) + std::max(R, T) / FP4_RPT_SMALL + 1) * fp4_sfb_bytes(FP4_RPT_SMALL),
-                                     (std::min(E, std::max(R, T)) + std::max(R, T) / FP4_RPT_LARGE + 1) * fp4_sfb_bytes(FP4_RPT_LARGE));
-    p.asf_bytes = sf_stage * ((std::max({kin, I, H, Ish}) + 255) / 256);
-    p.asf = c.take<uint8_t>(p.asf_bytes);
+    p.asf = c.take<uint8_t>(std::max(R, T) * ((std::max({kin, I, H, Ish}) + 255) / 256) * 16);
     p.arow_scale = c.take<float>(std::max(R, T));
-    p.tile_expert = c.take<int>(std::min(E, std::max(R, T)) + std::max(R, T) / FP4_RPT_SMALL + 1);
+    p.tiles = c.take<int4>(std::min(E, std::max(R, T)) + std::max(R, T) / FP4_RPT_SMALL + 1);
     if (Ish) {
         p.sh_a = c.take<float>(T * Ish);
         p.sh_b = c.take<float>(T * Ish);
@@ -544,12 +539,13 @@ int launch_gemm(b200moe_ctx * ctx, int k, const MmaParams & p, int rows, bool sm
 
 // block-scaled FP4 grouped GEMM (expert_gemm_fp4.cuh): digit planes of the routed rows, then the GEMM
 template <int K, bool DUAL, int RPT>
-int launch_gemm_fp4_t(b200moe_ctx * ctx, const Fp4Params & fp, const void * w0, const void * w1, const uint8_t * planes, int rows, cudaStream_t st) {
+int launch_gemm_fp4_t(b200moe_ctx * ctx, Fp4Params fp, const void * w0, const void * w1, const uint8_t * planes, int rows, cudaStream_t st) {
     using C = Fp4Cfg<K, RPT>;
     static_assert(C::SMEM <= 226 * 1024, "rings do not fit shared memory");
     auto kern = expert_gemm_fp4_kernel<K, DUAL, RPT>;
     static bool configured[MAX_DEVICE_ORDINALS] = {};  // per instantiation and device
     if (int rc = raise_smem_limit(ctx, kern, C::SMEM, configured)) return rc;
+    fp.sf_rows = rows;
     constexpr uint64_t ROW_BYTES = K / 64 * 36;
     CUtensorMap mw0, mw1, mpl;
     int rc;
@@ -560,8 +556,8 @@ int launch_gemm_fp4_t(b200moe_ctx * ctx, const Fp4Params & fp, const void * w0, 
     } else {
         mw1 = mw0;
     }
-    const uint64_t prows = std::max<uint64_t>((uint64_t) rows * FP4_PLANES, C::NROW);
-    if ((rc = make_map_2d(ctx, &mpl, CU_TENSOR_MAP_DATA_TYPE_UINT8, planes, K / 2, prows, K / 2, 128, C::NROW, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
+    const uint64_t prows = std::max<uint64_t>((uint64_t) rows * FP4_PLANES, C::BOX_ROWS * FP4_PLANES);
+    if ((rc = make_map_2d(ctx, &mpl, CU_TENSOR_MAP_DATA_TYPE_UINT8, planes, K / 2, prows, K / 2, 128, C::BOX_ROWS * FP4_PLANES, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
     b200moe_ctx::Timed tm{};
     if (ctx->timing) {
         CUDA_TRY(ctx, cudaEventCreate(&tm.beg));
@@ -619,11 +615,11 @@ bool fp4_supported(int wtype, int n_in, int n_ff) { return wtype == TYPE_NVFP4 &
 int launch_act_planes(b200moe_ctx * ctx, ActQuant act, const float * src, const int32_t * ids, int rows, int k, int n_ids, int ne11, int n_as,
                       cudaStream_t st, ActQuant emit = ActQuant{}, int64_t src_stride = 0) {
     Plan & p = ctx->plan;
-    PlaneOut po{ reinterpret_cast<uint8_t *>(p.afp16), p.asf, p.arow_scale, p.tile_expert, p.groups.tile_rows };
+    PlaneOut po{ reinterpret_cast<uint8_t *>(p.afp16), p.asf, p.arow_scale, p.tiles, p.groups.tile_rows, rows };
     const int * tiles = p.groups.cost + 3 * (n_as + 1);
     if (src_stride == 0) src_stride = k;
     if (src && (((uintptr_t) src & 15) || src_stride % 4)) return fail(ctx, B200MOE_ERR_INVALID_ARG, "fp32 activation rows must be 16-byte aligned");
-    const int rows_per_block = 256 / std::min(256, k / 8);
+    const int rows_per_block = 256 / (k / 16);
     const int act_rows = rows / n_ids * ne11;
     // few rows (8 tokens: 8 blocks): the routed rows of a token are shared out over further blocks, which work the digits out again
     const int bx = (act_rows + rows_per_block - 1) / rows_per_block;
@@ -636,8 +632,8 @@ int launch_act_planes(b200moe_ctx * ctx, ActQuant act, const float * src, const 
 Fp4Params fp4_params(b200moe_ctx * ctx, const float * s0, const float * s1, float * out, int n_out, int n_as) {
     Plan & p = ctx->plan;
     Fp4Params f{};
-    f.scale0 = s0; f.scale1 = s1; f.sf = p.asf; f.row_scale = p.arow_scale; f.offsets = p.groups.offsets; f.perm = p.groups.perm;
-    f.tile_of_expert = p.groups.cost + 3 * (n_as + 1); f.tile_expert = p.tile_expert; f.out = out; f.n_out = n_out;
+    f.scale0 = s0; f.scale1 = s1; f.sf = p.asf; f.row_scale = p.arow_scale; f.perm = p.groups.perm;
+    f.tile_of_expert = p.groups.cost + 3 * (n_as + 1); f.tiles = p.tiles; f.out = out; f.n_out = n_out;
     f.n_as = n_as; f.err = ctx->d_err; f.prof = nullptr;
     return f;
 }

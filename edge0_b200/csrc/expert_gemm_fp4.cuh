@@ -9,24 +9,24 @@
 // activations are simply stored in ggml's nibble order (byte j = elements j and j+8 of the block).
 //
 // Activations stay on the reference's int8 grid (q * d with d an fp16 number per 32 elements, the Q8_0 rows the CPU path
-// multiplies with).  With d = M * 2^e (M an 11-bit integer) the product q * M is an 18-bit integer; its seven balanced
-// radix-8 digits (each in [-4, 4], all E2M1 values) are seven "planes" of one routed row, and 2^e - relative to the row's
+// multiplies with).  With d = M * 2^e (M an 11-bit integer) the product q * M is an integer of at most 127 * 2047 = 259969; its six balanced
+// radix-9 digits (each in [-4, 4], all E2M1 values; six reach 265720) are six "planes" of one routed row, and 2^e - relative to the row's
 // largest block exponent - is a power of two that UE4M3 holds exactly.  So
-//     x_hat[k] = 2^(E_row - 8) * sum_p 8^p * digit_p[k] * sf[k / 16]
+//     x_hat[k] = 2^(E_row - 8) * sum_p 9^p * digit_p[k] * sf[k / 16]
 // is exact (blocks more than 17 binades below the row's largest flush to zero: a relative 2^-17 of the row's unit), every
 // product inside the tensor core is exact, and the result differs from the integer path only by fp32 accumulation.
 //
-// Operand roles: D[feature, plane] = W[feature, k] * P[plane, k].  M = 128 weight rows, N = 7 planes x up to 14 routed rows
-// (N = 8 .. 104; prefill: up to 27 rows, N = 192), K = 64 per instruction.  The seven plane columns of a routed row sit next to each other in one lane of tensor
-// memory, so the epilogue recombines them with a Horner chain in registers and stores 32 consecutive features per warp.
+// Operand roles: D[feature, plane] = W[feature, k] * P[plane, k].  M = 128 weight rows, N = 6 planes x up to 14 routed rows
+// (N = 8 .. 88; prefill: up to 27 rows, N = 168), K = 64 per instruction.  The six plane columns of a routed row sit next to each other in
+// one lane of tensor memory, so the epilogue recombines them with a Horner chain in registers and stores 32 consecutive features per warp.
 // Two weight tiles are in flight per stage with an accumulator each (gate and up rows of the same 128 features, or two
 // consecutive 128-row tiles of `down`): dependent MMAs on one accumulator issue every ~190-230 cycles, MMAs that alternate
 // between two accumulators every ~116 (measured with the probe kernel in fp4_probe.cuh).
 //
 // Roles (every wait bounded, as in expert_gemm.cuh):
 //   warp 0       raw-weight producer: tiled TMA of [128 rows][144 bytes] boxes (K = 256 per row) of both tiles
-//   warp 1       activation producer: one tiled TMA box of the token tile's plane rows (128 bytes each) + one bulk copy of its scale
-//                tile, into a ring of its own that runs three stages ahead (the planes come from L2 with about a microsecond of latency)
+//   warp 1       activation producer: tiled TMA boxes of the plane rows (128 bytes each) of four routed rows + one bulk copy of the rows'
+//                scales, into a ring of its own that runs three stages ahead (the planes come from L2 with about a microsecond of latency)
 //   warp 2       MMA issuer: two tcgen05.mma per K = 64 step
 //   warp 3       owns tensor memory
 //   warps 4-7, 20-23  epilogue
@@ -37,7 +37,10 @@
 // between rows and lanes and the waits of tcgen05.st have warps of their own because the repack warps' chain is the longest of a stage: with
 // both in the repack warps gate/up of 64 tokens over 512 experts (1024 -> 1024) took 107 us, like this 98; sixteen repack warps
 // that take the stages in turn gained nothing more and cost the prefill tile its registers (4096 tokens: 481 -> 685 us).
-// 24 warps leave a thread 80 registers, and every instantiation spills (72 bytes of stack at 14 rows, 32 at 27).
+// 24 warps leave a thread 80 registers (see the register split in the kernel).  What a stage takes is the hand-over between the roles: repack,
+// scale factors and MMAs each keep busy for some 1,150 cycles of its 1,500 to 2,200.  One weight tile against two token tiles in a stage
+// (half the weight bytes through shared memory) took as long to a stage and twice as many of them below 27 rows an expert; scale words
+// through a buffer of their own or warps of their own for either operand's scales gained nothing or lost.
 #pragma once
 #include <cuda.h>
 
@@ -48,13 +51,10 @@
 
 namespace b200moe {
 
-constexpr int FP4_PLANES = 7;
+constexpr int FP4_PLANES = 6;
 // Routed rows per token tile: 14 for few rows per expert (two accumulator buffers, so the epilogue runs beside the next unit), 27 for
-// more (N = 192 fills tensor memory with one buffer; a weight tile is repacked and fetched half as often per routed row).
+// more (N = 168, one buffer; a weight tile is repacked and fetched half as often per routed row).
 constexpr int FP4_RPT_SMALL = TOKEN_TILE_SMALL, FP4_RPT_LARGE = TOKEN_TILE_LARGE;
-constexpr int FP4_SF_TILE = 4 * 512;              // scale factors of 128 rows for the four K = 64 steps of a stage
-// bytes of one token tile's scale factors per K = 256 stage: one block of 128 plane rows, or two
-__host__ __device__ constexpr int fp4_sfb_bytes(int rpt) { return (FP4_PLANES * rpt + 127) / 128 * FP4_SF_TILE; }
 constexpr int FP4_THREADS = 768;
 
 __device__ __forceinline__ void umma_fp4(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc, uint32_t sfa, uint32_t sfb,
@@ -104,175 +104,157 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 }
 
 // ---- activation planes ---------------------------------------------------------------------------------------------------
-// Expert-sorted routed row i -> seven plane rows 7i .. 7i+6 of `planes` (K/2 bytes each, ggml nibble order inside every
-// 16-block), its scale bytes in the scale tiles of its token tile, and the power of two the epilogue multiplies with.
-//   tile_of_expert[e]: index of expert e's first token tile (prefix of ceil(rows_e / rpt)); tile_expert[tile]: the inverse
-//   sf tiles: [tile][K / 256][4 steps][1 or 2 blocks (14 or 27 routed rows) of 128 plane rows][512 bytes], byte for (plane row n of the block, 16-block g of
-//   the step) at sf_tile_offset(n) + g
+// Expert-sorted routed row i -> six plane rows 6i .. 6i+5 of `planes` (K/2 bytes each, ggml nibble order inside every
+// 16-block), its scale bytes, which its planes have in common, and the power of two the epilogue multiplies with.
 struct PlaneOut {
-    uint8_t * planes;       // [rows * 7][K / 2]
-    uint8_t * sf;           // [tiles][K / 256][fp4_sfb_bytes(rpt)]
+    uint8_t * planes;       // [rows * 6][K / 2]
+    uint8_t * sf;           // [K / 256][rows][16]: scale of every 16-block
     float *   row_scale;    // [rows] by sorted position
-    int *     tile_expert;  // [tiles] expert of every token tile
+    int4 *    tiles;        // [tiles] of every token tile: expert, first sorted row, routed rows
     int       rpt;          // routed rows per token tile
+    int       rows;
 };
 
-// digits and codes of one quad: 16-block g, bytes j0 .. j0+3 (elements 16g + j and 16g + j + 8) with int8 values lo[], hi[] and the
-// fp32 bits of the block scale d (an fp16 number: d = M * 2^(exp8 - 137) with M the top 11 bits of the significand).  words[p]: the
-// four code bytes of plane p; returned: the UE4M3 byte of the block's scale.
-__device__ __forceinline__ uint8_t plane_quad(const int (&lo)[4], const int (&hi)[4], uint32_t dbits, int E_row, uint32_t (&words)[FP4_PLANES]) {
-    const bool nz = (dbits & 0x7fffffffu) != 0;
-    const int M = nz ? (int) (((dbits & 0x7fffffu) | 0x800000u) >> 13) : 0;
-    const int s = nz ? (int) ((dbits >> 23) & 0xff) - 137 - E_row + 8 : -100;           // scale exponent, at most 8
-    const int Ms = s >= -9 ? M : 0;                                                     // flushed blocks contribute nothing
-    int p0[4], p1[4];
+// E2M1 codes of the balanced radix-9 digits of 0 .. 728, less four each: lowest digit in byte 0, highest in byte 2
+__device__ __forceinline__ uint32_t digit_codes(int v) {
+    uint32_t w = 0;
 #pragma unroll
-    for (int m = 0; m < 4; ++m) { p0[m] = lo[m] * Ms; p1[m] = hi[m] * Ms; }
-    // Balanced radix-8 digits, lowest first: digit = ((p + 4) & 7) - 4 and carry (p + 4) >> 3.  The digit's E2M1 code comes from
-    // a table indexed by p & 7 (residues 0..3 are the digits 0..3, residues 4..7 the digits -4..-1): codes 0,2,4,5 and, with the
-    // sign bit, E,D,C,A.  The top plane takes what is left (|p| <= 4) through the magnitude table 0,2,4,5,6.
-#pragma unroll
-    for (int p = 0; p < FP4_PLANES; ++p) {
-        uint32_t word = 0;
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            uint32_t c0, c1;
-            if (p < FP4_PLANES - 1) {
-                c0 = (0xACDE5420u >> (4 * (p0[m] & 7))) & 0xfu;
-                c1 = (0xACDE5420u >> (4 * (p1[m] & 7))) & 0xfu;
-                p0[m] = (p0[m] + 4) >> 3;
-                p1[m] = (p1[m] + 4) >> 3;
-            } else {
-                c0 = ((0x65420u >> (4 * abs(p0[m]))) & 0xfu) | (p0[m] < 0 ? 8u : 0u);
-                c1 = ((0x65420u >> (4 * abs(p1[m]))) & 0xfu) | (p1[m] < 0 ? 8u : 0u);
-            }
-            word |= (c0 | (c1 << 4)) << (8 * m);
-        }
-        words[p] = word;
+    for (int p = 0; p < 3; ++p) {
+        const int d = v % 9 - 4;
+        v /= 9;
+        w |= (((0x65420u >> (4 * abs(d))) & 0xfu) | (d < 0 ? 8u : 0u)) << (8 * p);
     }
-    // normal for s >= -6, the three power-of-two subnormals below, zero when flushed
-    return (uint8_t) (s >= -6 ? (uint32_t) (s + 7) << 3 : s == -7 ? 4u : s == -8 ? 2u : s == -9 ? 1u : 0u);
+    return w;
 }
 
-// K / 8 threads per ACTIVATION row (at most 256: a block holds 256 * 8 / K rows, and a thread two quads when K = 4096).  The digits of
-// a row are worked out once and stored for each of the n_ids / ne11 routed rows that read it (gate/up: the k experts of a token).
+// K / 16 threads per ACTIVATION row, a thread for a 16-block (a block of threads holds 256 * 16 / K rows).  The digits of a row are worked
+// out once and stored for each of the n_ids / ne11 routed rows that read it (gate/up: the k experts of a token).
 // SRC_F32 = false: the row's activations are already quantised (ActQuant planes, Q8_0).
 // SRC_F32 = true: they are fp32 (`src`, rows `src_stride` floats apart) and are quantised here exactly as quantize_q8_0_block
 // does it (d = half(amax / 127), q = rint(v * (127 / amax))), which saves the separate quantisation pass; `emit`, when it has
 // planes, receives that quantised form as well (row index as in `src`).
-// Bound by the stores: 3.5 bytes per routed value.
+// Three digits at a time come from a table, a byte each, so eight of them merge into a word of one plane by byte permutes: some 10 instructions
+// a value where dividing out digit by digit took 40.  Bound by the stores: 3 bytes per routed value, 8 of them at a time.
+// 4096 tokens top-8, K = 2048: 94 us with seven planes, scales per plane and digits one by one, so 39; fp32 rows of K = 768: 104 us, so 48.
 template <bool SRC_F32>
 __global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const float * __restrict__ src, int64_t src_stride,
                                                         const int * __restrict__ pos, const int32_t * __restrict__ ids,
                                                         const int * __restrict__ offsets, const int * __restrict__ tile_of_expert,
                                                         int act_rows, int K, int n_ids, int ne11, int n_as, PlaneOut out, ActQuant emit) {
-    constexpr int MAX_QUADS = 2;
-    __shared__ int s_E[8];
-    __shared__ int s_at[8][32], s_tile[8][32], s_in[8][32];   // sorted position, token tile and row in it of every routed row of a block row
+    constexpr int MAX_ROWS = 16;             // K = 256
+    __shared__ uint32_t s_digits[729];
+    __shared__ int s_E[MAX_ROWS];
+    __shared__ int s_at[MAX_ROWS][32];       // sorted position of every routed row of a block row
     const int tid = threadIdx.x, lane = tid & 31;
-    const int tpr = min(256, K / 8), rpb = 256 / tpr, qpt = (K / 8) / tpr;
-    const int lrow = tid / tpr, t_in = tid % tpr;
+    const int tpr = K / 16, rpb = 256 / tpr;
+    const int lrow = tid / tpr, g = tid % tpr;
     const int arow = blockIdx.x * rpb + lrow;
     const int n_dst = n_ids / ne11;
     const int dst_step = gridDim.y, dst0 = blockIdx.y;    // few rows: the blocks of a column store every dst_step-th routed row each
-    if (tid < 8) s_E[tid] = -1000;
+    for (int i = tid; i < 729; i += 256) s_digits[i] = digit_codes(i);
+    if (tid < MAX_ROWS) s_E[tid] = -1000;
     const bool live = lrow < rpb && arow < act_rows;   // threads beyond the block's last whole row idle (K = 768)
-    if (live && t_in < n_dst) {
-        const int r = (arow / ne11) * n_ids + arow % ne11 + ne11 * t_in;
+    for (int j = g; live && j < n_dst; j += tpr) {
+        const int r = (arow / ne11) * n_ids + arow % ne11 + ne11 * j;
         const int e = ids[r];
-        int at = -1, tile = 0, in_tile = 0;            // an id of -1 is an empty slot; other bad ids were reported by the grouping kernels
+        int at = -1;                                   // an id of -1 is an empty slot; other bad ids were reported by the grouping kernels
         if (e >= 0 && e < n_as) {
             const int in_e = pos[r];
             at = offsets[e] + in_e;
-            tile = tile_of_expert[e] + in_e / out.rpt;
-            in_tile = in_e % out.rpt;
-            if (in_tile == 0) out.tile_expert[tile] = e;
+            if (in_e % out.rpt == 0) out.tiles[tile_of_expert[e] + in_e / out.rpt] = make_int4(e, at, min(out.rpt, offsets[e + 1] - at), 0);
         }
-        s_at[lrow][t_in] = at; s_tile[lrow][t_in] = tile; s_in[lrow][t_in] = in_tile;
+        s_at[lrow][j] = at;
     }
+    // the block's values in order and its scale's bits
+    int v[16];
+    uint32_t dbits = 0;
+    if (SRC_F32) {
+        float x[16];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const float4 f = live ? __ldg(reinterpret_cast<const float4 *>(src + (size_t) arow * src_stride + 16 * g) + m) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            x[4 * m] = f.x; x[4 * m + 1] = f.y; x[4 * m + 2] = f.z; x[4 * m + 3] = f.w;
+        }
+        float amax = fabsf(x[0]);                      // NaN only for a block of nothing else
+#pragma unroll
+        for (int m = 1; m < 16; ++m) amax = fmaxf(amax, fabsf(x[m]));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));   // the 32-block's other half: the neighbour (an even number of threads to a row)
+        const float d = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
+        const float id = amax != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+#pragma unroll
+        for (int m = 0; m < 16; ++m) v[m] = __float2int_rn(__fmul_rn(x[m], id));
+        dbits = __float_as_uint(d);
+        if (emit.q && blockIdx.y == 0 && live) {
+            uint32_t w[4];
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+                w[m] = (uint32_t) (v[4 * m] & 0xff) | ((uint32_t) (v[4 * m + 1] & 0xff) << 8) | ((uint32_t) (v[4 * m + 2] & 0xff) << 16) |
+                       ((uint32_t) (v[4 * m + 3] & 0xff) << 24);
+            *reinterpret_cast<uint4 *>(emit.q + (size_t) arow * K + 16 * g) = make_uint4(w[0], w[1], w[2], w[3]);
+            if ((g & 1) == 0) emit.d[(size_t) arow * (K / 32) + (g >> 1)] = d;
+        }
+    } else {
+        const uint4 f = live ? *reinterpret_cast<const uint4 *>(act.q + (size_t) arow * K + 16 * g) : make_uint4(0u, 0u, 0u, 0u);
+        const uint32_t w[4] = { f.x, f.y, f.z, f.w };
+#pragma unroll
+        for (int m = 0; m < 16; ++m) v[m] = (int) (int8_t) (w[m >> 2] >> (8 * (m & 3)));
+        if (live) dbits = __float_as_uint(act.d[(size_t) arow * (K / 32) + (g >> 1)]);
+    }
+    // d is an fp16 number: d = M * 2^(exp8 - 137) with M the top 11 bits of the significand
+    const bool nz = (dbits & 0x7fffffffu) != 0;
+    const int e8 = nz && live ? (int) ((dbits >> 23) & 0xff) - 137 : -1000;
     __syncthreads();
-    const int nb32 = K / 32;
-    int lo[MAX_QUADS][4], hi[MAX_QUADS][4];
-    uint32_t db[MAX_QUADS];
-    int emax = -1000;
-#pragma unroll
-    for (int u = 0; u < MAX_QUADS; ++u) {
-        db[u] = 0u;
-        if (u < qpt && live) {
-            const int qd = t_in + tpr * u, g = qd >> 1, j0 = (qd & 1) * 4;
-            if (SRC_F32) {
-                const float * xrow = src + (size_t) arow * src_stride + 16 * g + j0;
-                const float4 a = *reinterpret_cast<const float4 *>(xrow), b = *reinterpret_cast<const float4 *>(xrow + 8);
-                const float va[4] = { a.x, a.y, a.z, a.w }, vb[4] = { b.x, b.y, b.z, b.w };
-                float amax = fmaxf(fabsf(va[0]), fabsf(vb[0]));   // NaN only for a block of nothing else
-#pragma unroll
-                for (int m = 1; m < 4; ++m) amax = fmaxf(amax, fmaxf(fabsf(va[m]), fabsf(vb[m])));
-                // the four quads of a 32-block sit in four consecutive lanes (all live or none: a row never splits a warp)
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-                const float d = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
-                const float id = amax != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    lo[u][m] = __float2int_rn(__fmul_rn(va[m], id));
-                    hi[u][m] = __float2int_rn(__fmul_rn(vb[m], id));
-                }
-                db[u] = __float_as_uint(d);
-                if (emit.q && blockIdx.y == 0) {
-                    int8_t * qo = emit.q + (size_t) arow * K + 16 * g + j0;
-                    *reinterpret_cast<uint32_t *>(qo) = (uint32_t) (lo[u][0] & 0xff) | ((uint32_t) (lo[u][1] & 0xff) << 8) |
-                                                        ((uint32_t) (lo[u][2] & 0xff) << 16) | ((uint32_t) (lo[u][3] & 0xff) << 24);
-                    *reinterpret_cast<uint32_t *>(qo + 8) = (uint32_t) (hi[u][0] & 0xff) | ((uint32_t) (hi[u][1] & 0xff) << 8) |
-                                                            ((uint32_t) (hi[u][2] & 0xff) << 16) | ((uint32_t) (hi[u][3] & 0xff) << 24);
-                    if ((qd & 3) == 0) emit.d[(size_t) arow * nb32 + (g >> 1)] = d;
-                }
-            } else {
-                const int8_t * qrow = act.q + (size_t) arow * K + 16 * g + j0;
-                const uint32_t wa = *reinterpret_cast<const uint32_t *>(qrow), wb = *reinterpret_cast<const uint32_t *>(qrow + 8);
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    lo[u][m] = (int) (int8_t) (wa >> (8 * m));
-                    hi[u][m] = (int) (int8_t) (wb >> (8 * m));
-                }
-                db[u] = __float_as_uint(act.d[(size_t) arow * nb32 + (g >> 1)]);
-            }
-            if (db[u] & 0x7fffffffu) emax = max(emax, (int) ((db[u] >> 23) & 0xff) - 137);
-        } else if (SRC_F32 && u < qpt) {   // keep the warp's shuffles uniform
-            __shfl_xor_sync(0xffffffffu, 0.0f, 1);
-            __shfl_xor_sync(0xffffffffu, 0.0f, 2);
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
-    if (lane == 0 && live) atomicMax(&s_E[lrow], emax);
+    // the row's largest exponent; sixteen threads never belong to two rows
+    const int emax = __reduce_max_sync(0xffffu << (lane & 16), e8);
+    if ((lane & 15) == 0 && live) atomicMax(&s_E[lrow], emax);
     __syncthreads();
     if (!live) return;
     const int E_row = s_E[lrow];
-    if (t_in < n_dst && s_at[lrow][t_in] >= 0)
-        // 2^(E_row - 8): far from the fp32 limits.  A block scale that is infinite or NaN has no digits: the row's results are NaN, which is
-        // what 0 * inf makes of them on the other engines (and in the reference).
-        out.row_scale[s_at[lrow][t_in]] = E_row == 255 - 137 ? __uint_as_float(0x7fc00000u) : E_row > -1000 ? __uint_as_float((uint32_t) (E_row - 8 + 127) << 23) : 0.0f;
-    const int sfb_bytes = fp4_sfb_bytes(out.rpt);
+    for (int j = g; j < n_dst; j += tpr)
+        if (s_at[lrow][j] >= 0)
+            // 2^(E_row - 8): far from the fp32 limits.  A block scale that is infinite or NaN has no digits: the row's results are NaN, which is
+            // what 0 * inf makes of them on the other engines (and in the reference).
+            out.row_scale[s_at[lrow][j]] = E_row == 255 - 137 ? __uint_as_float(0x7fc00000u) : E_row > -1000 ? __uint_as_float((uint32_t) (E_row - 8 + 127) << 23) : 0.0f;
+    const int s = nz ? e8 - E_row + 8 : -100;                                           // scale exponent, at most 8
+    const int M = s >= -9 ? (int) (((dbits & 0x7fffffu) | 0x800000u) >> 13) : 0;        // flushed blocks contribute nothing
+    // the scale's UE4M3 byte: normal for s >= -6, the three power-of-two subnormals below, zero when flushed
+    const uint8_t sb = (uint8_t) (s >= -6 ? (uint32_t) (s + 7) << 3 : s == -7 ? 4u : s == -8 ? 2u : s == -9 ? 1u : 0u);
+    // digits: elements m and m + 8 of the block share byte m, low and high nibble.  An out-of-range v (a block of infinities) must not leave
+    // the table: its row is NaN whatever its digits are.
+    uint32_t words[FP4_PLANES][2];
 #pragma unroll
-    for (int u = 0; u < MAX_QUADS; ++u)
-        if (u < qpt) {
-            const int qd = t_in + tpr * u, g = qd >> 1;
-            uint32_t words[FP4_PLANES];
-            const uint8_t sb = plane_quad(lo[u], hi[u], db[u], E_row, words);
-            for (int j = dst0; j < n_dst; j += dst_step) {
-                const int at = s_at[lrow][j];
-                if (at < 0) continue;
-                uint32_t * pw = reinterpret_cast<uint32_t *>(out.planes + (size_t) at * FP4_PLANES * (K / 2)) + qd;
+    for (int h = 0; h < 2; ++h) {
+        uint32_t lo3[4], hi3[4];                       // bytes: planes 0 .. 2 and 3 .. 5 of byte 4h + m
 #pragma unroll
-                for (int p = 0; p < FP4_PLANES; ++p) pw[(size_t) p * (K / 8)] = words[p];
-                if ((qd & 1) == 0) {
-                    uint8_t * dst = out.sf + ((size_t) s_tile[lrow][j] * (K / 256) + (g >> 4)) * sfb_bytes + ((g >> 2) & 3) * (sfb_bytes / 4) + (g & 3);
-                    const int n0 = s_in[lrow][j] * FP4_PLANES;
+        for (int m = 0; m < 4; ++m) {
+            uint32_t c[2][2];
 #pragma unroll
-                    for (int p = 0; p < FP4_PLANES; ++p) dst[((n0 + p) >> 7) * 512 + sf_tile_offset((n0 + p) & 127)] = sb;
-                }
+            for (int n = 0; n < 2; ++n) {
+                const uint32_t u = min((uint32_t) (v[4 * h + m + 8 * n] * M + 265720), 531440u);
+                const uint32_t up = u / 729u;
+                c[n][0] = s_digits[u - up * 729u];
+                c[n][1] = s_digits[up];
             }
+            lo3[m] = c[0][0] | (c[1][0] << 4);
+            hi3[m] = c[0][1] | (c[1][1] << 4);
         }
+        auto planes3 = [&](const uint32_t (&t)[4], int p) {
+            const uint32_t a = __byte_perm(t[0], t[1], 0x5140), b = __byte_perm(t[2], t[3], 0x5140);
+            words[p][h] = __byte_perm(a, b, 0x5410);
+            words[p + 1][h] = __byte_perm(a, b, 0x7632);
+            words[p + 2][h] = __byte_perm(__byte_perm(t[0], t[1], 0x0062), __byte_perm(t[2], t[3], 0x0062), 0x5410);
+        };
+        planes3(lo3, 0);
+        planes3(hi3, 3);
+    }
+    for (int j = dst0; j < n_dst; j += dst_step) {
+        const int at = s_at[lrow][j];
+        if (at < 0) continue;
+        uint2 * pw = reinterpret_cast<uint2 *>(out.planes + (size_t) at * FP4_PLANES * (K / 2)) + g;
+#pragma unroll
+        for (int p = 0; p < FP4_PLANES; ++p) pw[(size_t) p * (K / 16)] = make_uint2(words[p][0], words[p][1]);
+        out.sf[((size_t) (g >> 4) * out.rows + at) * 16 + (g & 15)] = sb;
+    }
 }
 
 // Development builds (-DB200MOE_FP4_PROF) record, per CTA, the cycles each role spends waiting on each of its barriers.
@@ -291,45 +273,48 @@ __global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const flo
 struct Fp4Params {
     const float * scale0;   // per-expert fp32 scale of tile 0's tensor (or null)
     const float * scale1;
-    const uint8_t * sf;     // activation scale tiles
+    const uint8_t * sf;     // activation scales [K / 256][sf_rows][16]
     const float * row_scale;
-    const int * offsets;    // [n_as + 1]
     const int * perm;       // [rows]
     const int * tile_of_expert;   // [n_as + 1]: first token tile of every expert, total number of tiles at the end
-    const int * tile_expert;      // [tiles]
+    const int4 * tiles;           // [tiles]: see PlaneOut
     float * out;            // [rows][n_out] indexed by routed row
     int n_out;
     int n_as;
+    int sf_rows;
     int * err;
     long long * prof;       // development builds only
 };
 
 template <int K, int RPT>
 struct Fp4Cfg {
-    static constexpr int NROW = FP4_PLANES * RPT;                    // plane rows of a token tile (98, 189)
+    static constexpr bool LARGE = RPT == FP4_RPT_LARGE;
+    static constexpr int NROW = FP4_PLANES * RPT;                    // plane rows of a token tile (84, 162)
     static constexpr int NCOL = (NROW + 7) / 8 * 8;                  // accumulator columns per weight tile: N of the instruction is a multiple of 8
-    static constexpr int NACC = RPT == FP4_RPT_SMALL ? 2 : 1;        // accumulator buffers
-    static constexpr int NBLK = (NROW + 127) / 128;                  // blocks of 128 plane rows in the scale tile
+    static constexpr int NACC = LARGE ? 1 : 2;                        // accumulator buffers
+    static constexpr int NBLK = (NROW + 127) / 128;                  // blocks of 128 plane rows in the scale factors
     static constexpr int A_TILE = 128 * 128;                         // 128 weight rows x 256 K as fp4
-    static constexpr int B_BYTES = NROW * 128;                       // plane rows that arrive per stage
-    static constexpr int B_TILE = (NCOL * 128 + 1023) / 1024 * 1024; // their room (rows beyond NROW are read by the instruction: columns nobody uses)
-    static constexpr int SFB = fp4_sfb_bytes(RPT);
+    // Routed rows whose planes one tiled copy brings: four (24 x 128 bytes, whole swizzle atoms) where a tile holds few of its rows, all of
+    // them where it is mostly full (seven boxes to a stage instead of one: gate/up of 4096 tokens 433 us and 511).
+    static constexpr int BOX_ROWS = LARGE ? RPT : 4;
+    static constexpr int BOX_BYTES = BOX_ROWS * FP4_PLANES * 128;
+    static constexpr int B_TILE = ((RPT + BOX_ROWS - 1) / BOX_ROWS * BOX_BYTES + 1023) / 1024 * 1024;   // (rows beyond the tile's are read by the instruction: columns nobody uses)
+    static constexpr int SFB = 1024;                                 // room for the rows' scales, 16 bytes each
     static constexpr int STAGE = 2 * A_TILE;                         // repacked weights of both tiles
-    static constexpr int ACT_STAGE = B_TILE + SFB;                   // digit planes, then their scale tile
+    static constexpr int ACT_STAGE = B_TILE + SFB;                   // digit planes, then their scales
     static constexpr int RAW_STAGE = 256 * GEMM_RAW_ROW;
-    static constexpr int RS = RPT == FP4_RPT_SMALL ? 3 : 2;
-    static constexpr int TS = 2;
+    static constexpr int RS = LARGE ? 2 : 3, TS = 2;
     static constexpr int AS = 3;                                      // plane tiles come from L2 with ~1 us latency: fetched three stages ahead
     static constexpr uint32_t TMEM_COLS = 512;                        // NACC buffers x 2 accumulators, then two sets of scale factors
     static constexpr uint32_t SF_COL = NACC * 2 * NCOL;
     static constexpr uint32_t SF_SET = 32 + 16 * NBLK;                // [tile 0][tile 1][planes]: 4 columns per K = 64 step and 128 rows
     static_assert(SF_COL + TS * SF_SET <= TMEM_COLS, "accumulators and one scale-factor set per operand stage fit tensor memory");
-    static_assert(NROW <= 256 && B_TILE >= B_BYTES, "plane rows fit one box and their room");
+    static_assert(NCOL * 128 <= B_TILE && RPT * 16 <= SFB, "operand rows and scales fit their room");
+    static_assert(BOX_ROWS == RPT || BOX_BYTES % 1024 == 0, "boxes start on a swizzle atom");
     static_assert(STAGE % 1024 == 0 && ACT_STAGE % 1024 == 0, "stages keep the 1024-byte alignment of swizzled tiles");
     static_assert(K % GEMM_RAW_K == 0, "K must be a multiple of 256");
     static constexpr size_t SMEM = (size_t) TS * STAGE + (size_t) AS * ACT_STAGE + (size_t) RS * RAW_STAGE + 1024;
 };
-
 // DUAL: tile 0 = gate rows f .. f+127, tile 1 = up rows of the same features; epilogue = SwiGLU; 128 features per item.
 // single: tiles 0 and 1 = 256 consecutive rows of the one tensor; 256 features per item.
 template <int K, bool DUAL, int RPT>
@@ -377,24 +362,22 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
     // expert follow each other, so a second pass over an expert's weights comes from L2 as well.
     const int f_tiles = p.n_out / FEAT;
     const int n_units = p.tile_of_expert[p.n_as] * f_tiles;
-    struct Unit { int e, ft, row0, nt, tile; };
+    struct Unit { int e, ft, row0, nt; };
     auto unit_at = [&](int u) {
-        Unit w;
-        w.tile = u / f_tiles;
-        w.ft = u - w.tile * f_tiles;
-        w.e = p.tile_expert[w.tile];
-        const int row_beg = p.offsets[w.e], t0 = (w.tile - p.tile_of_expert[w.e]) * RPT;
-        w.row0 = row_beg + t0;                                   // first expert-sorted row of the token tile
-        w.nt = min(RPT, p.offsets[w.e + 1] - w.row0);
-        return w;
+        const int tile = u / f_tiles;
+        const int4 t = __ldg(p.tiles + tile);
+        return Unit{ t.x, u - tile * f_tiles, t.y, t.z };
     };
     const int my_stages = n_units > (int) blockIdx.x ? (n_units - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x * KC : 0;
     // weight stage: [A0][A1]; activation stage: [B][SFB]
     constexpr uint32_t OFF_A1 = C::A_TILE, OFF_SFB = C::B_TILE;
-
-    if (warp == 0) {
-        // ---------------------------------------------------------------- raw weight producer
-        if (lane == 0) {
+    // 768 threads leave 80 registers to a thread.  With the small tile producers and issuer give theirs to the epilogue, which spilled without
+    // (40 + 2 x 104 + 3 x 72 = 464 of the launch's 480 per 128 threads; 64 tokens over 128 experts: gate/up 51.7 us, so 49.9, down 29.4 and 27.0).
+    // The large one has no spills without it and loses with it (4096 tokens, down: 244 us, 283 so).
+    if (warp < 4) {
+        if constexpr (!C::LARGE) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+        if (warp == 0 && lane == 0) {
+            // ------------------------------------------------------------ raw weight producer
             Ring raw;
             FP4_PROF_DECL();
             for (int u = blockIdx.x; u < n_units && !s_abort; u += gridDim.x) {
@@ -413,94 +396,92 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                 }
             }
             FP4_PROF_STORE(0, 1);
-        }
-    } else if (warp == 1) {
-        // ---------------------------------------------------------------- activation producer
-        if (lane == 0) {
+        } else if (warp == 1 && lane == 0) {
+            // ------------------------------------------------------------ activation producer
             Ring act;
             FP4_PROF_DECL();
             for (int u = blockIdx.x; u < n_units && !s_abort; u += gridDim.x) {
                 const Unit w = unit_at(u);
-                const uint8_t * sft = p.sf + (size_t) w.tile * KC * C::SFB;
+                const uint8_t * sfr = p.sf + (size_t) w.row0 * 16;
+                const int boxes = (w.nt + C::BOX_ROWS - 1) / C::BOX_ROWS;
                 for (int kc = 0; kc < KC; ++kc) {
                     FP4_PROF_T0();
                     if (!wait_or_abort<40>(&act_empty[act.stage], act.phase ^ 1u, &s_abort, p.err)) break;
                     FP4_PROF_ADD(0);
                     uint8_t * st = acts + (size_t) act.stage * C::ACT_STAGE;
-                    mbar_arrive_expect_tx(&act_full[act.stage], C::B_BYTES + C::SFB);
-                    tma_load_2d(st, &map_planes, kc * 128, FP4_PLANES * w.row0, &act_full[act.stage]);
-                    bulk_g2s(st + OFF_SFB, sft + (size_t) kc * C::SFB, C::SFB, &act_full[act.stage]);
+                    mbar_arrive_expect_tx(&act_full[act.stage], (uint32_t) (boxes * C::BOX_BYTES + w.nt * 16));
+                    for (int b = 0; b < boxes; ++b)
+                        tma_load_2d(st + b * C::BOX_BYTES, &map_planes, kc * 128, FP4_PLANES * (w.row0 + C::BOX_ROWS * b), &act_full[act.stage]);
+                    bulk_g2s(st + OFF_SFB, sfr + (size_t) kc * p.sf_rows * 16, (uint32_t) w.nt * 16, &act_full[act.stage]);
                     act.template advance<AS>();
                 }
             }
             FP4_PROF_STORE(2, 1);
-        }
-    } else if (warp == 2) {
-        // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
+        } else if (warp == 2 && lane == 0) {
+            // ------------------------------------------------------------ MMA issuer
             Ring tile, act, acc;
             FP4_PROF_DECL();
             for (int u = blockIdx.x; u < n_units && !s_abort; u += gridDim.x) {
+                const uint32_t idesc = umma_idesc_fp4((FP4_PLANES * unit_at(u).nt + 7) & ~7);
                 {
-                    const int nt = unit_at(u).nt;
-                    const uint32_t idesc = umma_idesc_fp4((FP4_PLANES * nt + 7) & ~7);
+                    FP4_PROF_T0();
+                    if (!wait_or_abort<40>(&acc_empty[acc.stage], acc.phase ^ 1u, &s_abort, p.err)) break;
+                    FP4_PROF_ADD(0);
+                }
+                tc_fence_after();
+                const uint32_t d0 = tmem + (uint32_t) acc.stage * (2 * C::NCOL), d1 = d0 + C::NCOL;
+                bool ok = true;
+                for (int kc = 0; kc < KC; ++kc) {
                     {
                         FP4_PROF_T0();
-                        if (!wait_or_abort<40>(&acc_empty[acc.stage], acc.phase ^ 1u, &s_abort, p.err)) break;
-                        FP4_PROF_ADD(0);
+                        if (!(ok = wait_or_abort<20>(&act_full[act.stage], act.phase, &s_abort, p.err))) break;
+                        FP4_PROF_ADD(1);
+                    }
+                    {
+                        FP4_PROF_T0();
+                        if (!(ok = wait_or_abort<20>(&tile_full[tile.stage], tile.phase, &s_abort, p.err))) break;
+                        FP4_PROF_ADD(2);
                     }
                     tc_fence_after();
-                    const uint32_t d0 = tmem + (uint32_t) acc.stage * (2 * C::NCOL), d1 = d0 + C::NCOL;
-                    for (int kc = 0; kc < KC; ++kc) {
-                        {
-                            FP4_PROF_T0();
-                            if (!wait_or_abort<20>(&act_full[act.stage], act.phase, &s_abort, p.err)) break;
-                            FP4_PROF_ADD(1);
-                        }
-                        {
-                            FP4_PROF_T0();
-                            if (!wait_or_abort<20>(&tile_full[tile.stage], tile.phase, &s_abort, p.err)) break;
-                            FP4_PROF_ADD(2);
-                        }
-                        tc_fence_after();
-                        const uint32_t sbase = smem_u32(tiles + (size_t) tile.stage * C::STAGE);
-                        const uint32_t abase = smem_u32(acts + (size_t) act.stage * C::ACT_STAGE);
-                        const uint32_t da = DESC_LO | (sbase >> 4), db = DESC_LO | (abase >> 4);
-                        const uint32_t sf_set = tmem + C::SF_COL + C::SF_SET * (uint32_t) tile.stage;   // [tile 0][tile 1][planes]
+                    const uint32_t sbase = smem_u32(tiles + (size_t) tile.stage * C::STAGE);
+                    const uint32_t abase = smem_u32(acts + (size_t) act.stage * C::ACT_STAGE);
+                    const uint32_t da = DESC_LO | (sbase >> 4), db = DESC_LO | (abase >> 4);
+                    const uint32_t sf_set = tmem + C::SF_COL + C::SF_SET * (uint32_t) tile.stage;   // [tile 0][tile 1][planes]
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {   // 4 x K64 = 256; 32 bytes (2 units) further along the 128-byte row each
-                            const uint32_t t_sfa0 = sf_set + 4 * kk, t_sfa1 = t_sfa0 + 16, t_sfb = sf_set + 32 + 4 * C::NBLK * kk;
-                            const bool accum = kc != 0 || kk != 0;
-                            umma_fp4(d0, da + 2 * kk, db + 2 * kk, DESC_HI, idesc, t_sfa0, t_sfb, accum);
-                            umma_fp4(d1, da + (OFF_A1 >> 4) + 2 * kk, db + 2 * kk, DESC_HI, idesc, t_sfa1, t_sfb, accum);
-                        }
-                        umma_commit(&tile_empty[tile.stage]);   // frees both operand stages when these MMAs have read them
-                        umma_commit(&act_empty[act.stage]);
-                        tile.template advance<TS>();
-                        act.template advance<AS>();
+                    for (int kk = 0; kk < 4; ++kk) {   // 4 x K64 = 256; 32 bytes (2 units) further along the 128-byte row each
+                        const uint32_t t_sfa0 = sf_set + 4 * kk, t_sfa1 = t_sfa0 + 16, t_sfb = sf_set + 32 + 4 * C::NBLK * kk;
+                        const bool accum = kc != 0 || kk != 0;
+                        umma_fp4(d0, da + 2 * kk, db + 2 * kk, DESC_HI, idesc, t_sfa0, t_sfb, accum);
+                        umma_fp4(d1, da + (OFF_A1 >> 4) + 2 * kk, db + 2 * kk, DESC_HI, idesc, t_sfa1, t_sfb, accum);
                     }
-                    umma_commit(&acc_full[acc.stage]);
-                    acc.template advance<NACC>();
+                    umma_commit(&tile_empty[tile.stage]);   // frees both operand stages when these MMAs have read them
+                    umma_commit(&act_empty[act.stage]);
+                    tile.template advance<TS>();
+                    act.template advance<AS>();
                 }
+                if (!ok) break;
+                umma_commit(&acc_full[acc.stage]);
+                acc.template advance<NACC>();
             }
             FP4_PROF_STORE(4, 3);
         }
-    } else if ((warp >= 4 && warp < 8) || warp >= 20) {
+    } else if (warp < 8 || warp >= 20) {
         // ---------------------------------------------------------------- epilogue
+        if constexpr (!C::LARGE) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
         Ring acc;
         FP4_PROF_DECL();
         const int q = warp & 3;                 // TMEM lane quarter this warp may read
-        // two warps per quarter: the first takes the tile's first rows, the second the rest
-        constexpr int HALF = (RPT + 7) / 8 * 4;
+        // two warps per quarter: the first takes the tile's first rows, the second the rest.  Routed rows to a tensor memory load of 32 columns: five
+        // fill it, four cost a tile of few rows less.
+        constexpr int FOLD = C::LARGE ? 5 : 4, HALF = (RPT + 2 * FOLD - 1) / (2 * FOLD) * FOLD;
         const int first = warp >= 20 ? HALF : 0;
         for (int u = blockIdx.x; u < n_units && !s_abort; u += gridDim.x) {
             const Unit w = unit_at(u);
-            const float sc0 = p.scale0 ? p.scale0[w.e] : 1.0f;
-            const float sc1 = DUAL ? (p.scale1 ? p.scale1[w.e] : 1.0f) : sc0;
-            const int feature = w.ft * FEAT + q * 32 + lane;
+            const float sc0 = p.scale0 ? __ldg(p.scale0 + w.e) : 1.0f;
+            const float sc1 = DUAL ? (p.scale1 ? __ldg(p.scale1 + w.e) : 1.0f) : sc0;
             // lane i holds the routed row and the power of two of the tile's row i (a tile has at most 27)
-            const int my_row = lane < w.nt ? p.perm[w.row0 + lane] : 0;
-            const float my_rs = lane < w.nt ? p.row_scale[w.row0 + lane] : 0.0f;
+            const int my_row = lane < w.nt ? __ldg(p.perm + w.row0 + lane) : 0;
+            const float my_rs = lane < w.nt ? __ldg(p.row_scale + w.row0 + lane) : 0.0f;
             // lanes leave the polling loop one by one: the vote reconverges the warp (tcgen05.ld below needs all of it)
             {
                 FP4_PROF_T0();
@@ -513,26 +494,27 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
             // sums: with a single accumulator buffer the next unit's instructions wait for this loop.
             float x0[HALF], x1[HALF];
 #pragma unroll
-            for (int j = 0; j < HALF; j += 4)             // four routed rows = 28 plane columns per load (the last load may read past the tile's columns)
+            for (int j = 0; j < HALF; j += FOLD)          // (the last load may read past the tile's columns)
                 if (first + j < w.nt) {
-                    auto fold = [&](uint32_t col, float (&x)[HALF]) {
+                    auto fold = [&](uint32_t col, float * x) {
                         float v[32];
                         tmem_ld32(col, v);
 #pragma unroll
-                        for (int rr = 0; rr < 4; ++rr) {
-                            float a = v[7 * rr + 6];     // sum_p 8^p * plane_p, highest plane first
+                        for (int rr = 0; rr < FOLD; ++rr) {
+                            float a = v[FP4_PLANES * rr + FP4_PLANES - 1];     // sum_p 9^p * plane_p, highest plane first
 #pragma unroll
-                            for (int pl = 5; pl >= 0; --pl) a = __fmaf_rn(a, 8.0f, v[7 * rr + pl]);
-                            x[j + rr] = a;
+                            for (int pl = FP4_PLANES - 2; pl >= 0; --pl) a = __fmaf_rn(a, 9.0f, v[FP4_PLANES * rr + pl]);
+                            x[rr] = a;
                         }
                     };
-                    fold(d0 + FP4_PLANES * (first + j), x0);
-                    fold(d0 + C::NCOL + FP4_PLANES * (first + j), x1);
+                    fold(d0 + FP4_PLANES * (first + j), x0 + j);
+                    fold(d0 + C::NCOL + FP4_PLANES * (first + j), x1 + j);
                 }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[acc.stage]);
             acc.template advance<NACC>();
+            const int feature = w.ft * FEAT + q * 32 + lane;
 #pragma unroll
             for (int i = 0; i < HALF; ++i)
                 if (first + i < w.nt) {
@@ -544,8 +526,9 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                 }
         }
         if (warp == 4 && lane == 0) FP4_PROF_STORE(8, 1);
-    } else if (warp >= 8 && warp < 16) {
+    } else if (warp < 16) {
         // ---------------------------------------------------------------- repack: strip the scale bytes, keep everything else
+        if constexpr (!C::LARGE) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
         const int dq = tid - 256;
         const int trow = dq & 127, tsel = dq >> 7;
         const uint32_t a_off = tsel * C::A_TILE + sw128_offset(trow, 0);   // 16-byte chunk c of the row lies at a_off ^ (16 c)
@@ -597,10 +580,11 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
             tile.template advance<TS>();
         }
         if (tid == 256) FP4_PROF_STORE(10, 2);
-    } else if (warp >= 16 && warp < 20) {
+    } else {
         // ---------------------------------------------------------------- scale factors: registers -> tensor memory
         // One warp per lane quarter of tensor memory; each writes all of a stage's scales to its quarter.  Lane l holds those of rows l,
-        // l + 32, l + 64 and l + 96 of either weight tile (what tcgen05.cp 32x128b.warpx4 would put there) and of the planes.
+        // l + 32, l + 64 and l + 96 of a weight tile (what tcgen05.cp 32x128b.warpx4 would put there) and of a block of planes.
+        if constexpr (!C::LARGE) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
         const uint32_t quarter = (uint32_t) ((warp & 3) * 32) << 16;
         Ring raw, tile, act;
         FP4_PROF_DECL();
@@ -628,16 +612,6 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
             raw.template advance<RS>();
             {
                 FP4_PROF_T0();
-                if (!__all_sync(0xffffffffu, wait_or_abort<20>(&act_full[act.stage], act.phase, &s_abort, p.err))) break;
-                FP4_PROF_ADD(1);
-            }
-            const uint8_t * sfb = acts + (size_t) act.stage * C::ACT_STAGE + OFF_SFB + lane * 16;
-            uint4 b[C::NBLK][4];
-#pragma unroll
-            for (int j = 0; j < 4 * C::NBLK; ++j) b[j >> 2][j & 3] = *reinterpret_cast<const uint4 *>(sfb + 512 * j);
-            act.template advance<AS>();
-            {
-                FP4_PROF_T0();
                 if (!__all_sync(0xffffffffu, wait_or_abort<20>(&tile_empty[tile.stage], tile.phase ^ 1u, &s_abort, p.err))) break;
                 FP4_PROF_ADD(2);
             }
@@ -645,8 +619,29 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
             const uint32_t sf_set = tmem + C::SF_COL + C::SF_SET * (uint32_t) tile.stage + quarter;
             tmem_st16(sf_set, a[0]);
             tmem_st16(sf_set + 16, a[1]);
+            {
+                FP4_PROF_T0();
+                if (!__all_sync(0xffffffffu, wait_or_abort<20>(&act_full[act.stage], act.phase, &s_abort, p.err))) break;
+                FP4_PROF_ADD(1);
+            }
+            // plane rows l + 32 j of a block of 128 read the scales of their routed row (behind the stores of the weights' scales: there is no
+            // room for both in the registers)
+            const uint8_t * sfb = acts + (size_t) act.stage * C::ACT_STAGE + OFF_SFB;
+            uint4 b[C::NBLK][4];           // in memory order: [K = 64 step][block]
+            auto put = [&](int step, int n, const uint4 & v) { b[(step * C::NBLK + n) >> 2][(step * C::NBLK + n) & 3] = v; };
+#pragma unroll
+            for (int n = 0; n < C::NBLK; ++n) {
+                uint4 r[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) r[j] = *reinterpret_cast<const uint4 *>(sfb + min((128 * n + 32 * j + lane) / FP4_PLANES, RPT - 1) * 16);
+                put(0, n, make_uint4(r[0].x, r[1].x, r[2].x, r[3].x));
+                put(1, n, make_uint4(r[0].y, r[1].y, r[2].y, r[3].y));
+                put(2, n, make_uint4(r[0].z, r[1].z, r[2].z, r[3].z));
+                put(3, n, make_uint4(r[0].w, r[1].w, r[2].w, r[3].w));
+            }
 #pragma unroll
             for (int n = 0; n < C::NBLK; ++n) tmem_st16(sf_set + 32 + 16 * n, b[n]);
+            act.template advance<AS>();
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();

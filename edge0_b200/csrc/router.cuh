@@ -514,7 +514,7 @@ __global__ void __launch_bounds__(256) route_select_kernel(const float * __restr
 //   offsets[e]   first slot of expert e in perm, offsets[E] = total rows
 //   perm[i]      routed row index (token*K + slot) placed i-th
 //   active[a]    a-th expert that has at least one row; n_active in meta[0], total rows in meta[1]
-// routed rows per token tile of the FP4 tensor-core kernels (7 digit planes each): few and many rows per expert
+// routed rows per token tile of the FP4 tensor-core kernels (6 digit planes each): few and many rows per expert
 constexpr int TOKEN_TILE_SMALL = 14, TOKEN_TILE_LARGE = 27;
 
 // Work per weight row of the NVFP4 integer kernel for n routed rows: passes of four, or of two or one for what is left.  A pass of one
