@@ -359,15 +359,13 @@ int launch_q3k_mma(b200moe_ctx * ctx, const GemvParams & p, cudaStream_t st) {
     return check_launch(ctx, "expert_mma_q3k");
 }
 
-// One or two tokens: the whole call is a few thousand weight rows.  Four-warp CTAs with a single 16-row stage, several per SM,
-// give every CTA one pass over one chunk instead of two or three passes of a half-empty eight-warp CTA.
+// one or two tokens (expert_gemv.cuh): `rows` routed rows, their experts read from p.ids
 template <int WT, int K, bool DUAL>
-int launch_gemv_tiny(b200moe_ctx * ctx, const GemvParams & p, int rows, cudaStream_t st) {
-    constexpr int NW = 4;
-    constexpr size_t smem = gemv_smem_bytes<WT, K, DUAL, 1, 1, NW>();
-    auto kern = expert_gemv_kernel<WT, K, DUAL, 1, 1, NW>;
+int launch_few_rows(b200moe_ctx * ctx, const GemvParams & p, int rows, cudaStream_t st) {
+    using C = FewCfg<WT, K, DUAL>;
+    auto kern = expert_few_rows_kernel<WT, K, DUAL>;
     static bool configured[MAX_DEVICE_ORDINALS] = {};  // per instantiation and device
-    if (int rc = raise_smem_limit(ctx, kern, smem, configured)) return rc;
+    if (int rc = raise_smem_limit(ctx, kern, C::SMEM, configured)) return rc;
     b200moe_ctx::Timed tm{};
     if (ctx->timing) {
         CUDA_TRY(ctx, cudaEventCreate(&tm.beg));
@@ -375,15 +373,12 @@ int launch_gemv_tiny(b200moe_ctx * ctx, const GemvParams & p, int rows, cudaStre
         tm.kind = DUAL ? 0 : ctx->dense_now ? 2 : 1;
         CUDA_TRY(ctx, cudaEventRecord(tm.beg, st));
     }
-    // one CTA per stage-sized chunk; at most `rows` experts are active, CTAs past the end of the row list leave at once
-    const int64_t chunks = ((int64_t) rows * p.n_out + GemvCfg<WT, K, NW>::ROWS_PER_STAGE - 1) / GemvCfg<WT, K, NW>::ROWS_PER_STAGE;
-    const int grid = (int) std::max<int64_t>(1, chunks);
-    launch_k(ctx, kern, dim3(grid), dim3(NW * 32), smem, st, p);
+    launch_k(ctx, kern, dim3((p.n_out + C::FEAT - 1) / C::FEAT, rows), dim3(C::THREADS), C::SMEM, st, p);
     if (ctx->timing) {
         CUDA_TRY(ctx, cudaEventRecord(tm.end, st));
         ctx->timed.push_back(tm);
     }
-    return check_launch(ctx, "expert_gemv");
+    return check_launch(ctx, "expert_few_rows");
 }
 
 // NVFP4, more than a few rows: n_mats matrices behind one another (one when every group shares it)
@@ -419,7 +414,7 @@ int launch_gemv_k(b200moe_ctx * ctx, const GemvParams & p, int nt, cudaStream_t 
     if constexpr (DUAL && K > 2048) {
         return fail(ctx, B200MOE_ERR_UNSUPPORTED, "fused gate/up kernel is not built for K=%d", K);
     } else {
-        if (nt <= 0) return launch_gemv_tiny<WT, K, DUAL>(ctx, p, -nt, st);   // nt = -(routed rows): the one-or-two-token kernel
+        if (nt <= 0) return launch_few_rows<WT, K, DUAL>(ctx, p, -nt, st);    // nt = -(routed rows)
         if constexpr (WT == TYPE_NVFP4) {
             return launch_gemv_nvfp4<K, DUAL>(ctx, p, st);
         } else {
@@ -439,6 +434,9 @@ int launch_gemv(b200moe_ctx * ctx, int wtype, int k, const GemvParams & p, int n
 }
 
 bool q3k_on_mma(int wtype, int64_t rows, int n_groups) { return wtype == TYPE_Q3_K && rows >= (int64_t) Q3K_MMA_MIN_ROWS * n_groups; }
+
+// Rows of one or two tokens: the integer kernel that takes them one by one, unless there are so few groups that Q3_K is on passes of 32.
+bool few_rows(int wtype, int64_t rows, int n_groups) { return rows <= 16 && !q3k_on_mma(wtype, rows, n_groups); }
 
 // the integer product of grouped rows: `rows` routed rows in up to n_groups groups
 template <bool DUAL>
@@ -756,7 +754,9 @@ int launch_select_group(b200moe_ctx * ctx, const b200moe_layer * l, int T, float
     p.groups.tile_rows = token_tile_rows((int64_t) T * K, E);
     p.groups.n_done = T * K <= 16 ? T * (p.n_in / 16) : 0;
     const size_t sh = (size_t) E * sizeof(int);
-#define SELG(EPL) launch_k(ctx, route_select_group_kernel<EPL>, dim3(1), dim3(1024), sh, st, p.logits, E, K, T, p.ids, p.wts, probs, p.groups, ctx->d_err)
+    // the kernels of one or two tokens need no groups
+    const bool grouped = !(ctx->expert_path <= 1 && few_rows(l->wtype, (int64_t) T * K, E));
+#define SELG(EPL) launch_k(ctx, route_select_group_kernel<EPL>, dim3(1), dim3(grouped ? 1024 : 256), sh, st, p.logits, E, K, T, p.ids, p.wts, probs, p.groups, ctx->d_err, grouped ? 1 : 0)
     if (E <= 32) SELG(1);
     else if (E <= 64) SELG(2);
     else if (E <= 128) SELG(4);
@@ -808,6 +808,8 @@ GemvParams gemv_params(b200moe_ctx * ctx, const void * w0, const void * w1, cons
     g.active = p.groups.active;
     g.meta = p.groups.meta;
     g.cost = p.groups.cost;
+    g.ids = p.ids;
+    g.ids_stride = n_ids;
     g.out = out;
     g.w_stride = n_out;
     g.n_out = n_out;
@@ -869,6 +871,9 @@ bool dense_on_fp4(const b200moe_ctx * ctx, int wtype, int k, int n_out, int T) {
     return wtype == TYPE_NVFP4 && fp4_width(k) && n_out % 256 == 0 && T >= 4 && path != 1 && path != 5 && path != 7;
 }
 
+// tokens of a dense product that the kernel of few rows takes one by one
+constexpr int DENSE_FEW_ROWS = 4;
+
 // exact_requant: see dense_matmul_fp4; `hidden` scratch holds the list (free before the experts run)
 // w1 != null: y = silu(w . x) * (w1 . x), the gate/up pair of a dense expert in one pass over x (no tensor scales, no exact_requant);
 // y1_tmp [T][n_out] is used when the pair cannot be fused (integer kernel beyond 2048 columns)
@@ -886,9 +891,17 @@ int dense_matvec(b200moe_ctx * ctx, int wtype, const void * w, const float * sca
         silu_mul_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(y, y1_tmp, n);
         return check_launch(ctx, "silu_mul");
     }
-    // few tokens of an NVFP4 product: the kernel quantises the rows while it stages them
-    const bool fused_quant = wtype == TYPE_NVFP4 && T < 4 && !((uintptr_t) x & 15);
-    if (!fused_quant && (rc = launch_quantize<float>(ctx, x, k, xq, T, k, wtype, st))) return rc;
+    // few tokens: the kernel of few rows, which quantises them while it stages them.  NVFP4, 3 tokens, us, as passes
+    // of the grouped kernel (with its groups' launch, 1.7) and so: 4096 -> 1024 17.5 and 8.5, 1024 -> 4096 9.9 and 6.4.
+    if (T <= DENSE_FEW_ROWS && !((uintptr_t) x & 15)) {
+        GemvParams g = gemv_params(ctx, w, w1, scale, nullptr, xq, y, n_out, 1, 1, 1);
+        g.w_stride = 0;
+        g.ids = nullptr;
+        g.act_f32 = x;
+        if (w1) return launch_gemv<true>(ctx, wtype, k, g, -T, st);
+        return launch_gemv<false>(ctx, wtype, k, g, -T, st);
+    }
+    if ((rc = launch_quantize<float>(ctx, x, k, xq, T, k, wtype, st))) return rc;
     const int G = std::max(1, std::min({32, T / 8, p.n_expert}));
     const int gsize = (T + G - 1) / G;
     const int groups = (T + gsize - 1) / gsize;
@@ -897,7 +910,6 @@ int dense_matvec(b200moe_ctx * ctx, int wtype, const void * w, const float * sca
     if ((rc = check_launch(ctx, "dense_groups"))) return rc;
     GemvParams g = gemv_params(ctx, w, w1, scale, nullptr, xq, y, n_out, 1, 1, groups);
     g.w_stride = 0;
-    if (fused_quant) g.act_f32 = x;
     if (w1) return launch_integer<true>(ctx, wtype, k, g, T, groups, 4, st);
     return launch_integer<false>(ctx, wtype, k, g, T, groups, 4, st);
 }
@@ -1109,6 +1121,7 @@ int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const 
         if ((rc = tm_gu ? launch_gemm_tm<true>(ctx, n_in, m, rows, st) : launch_gemm<true>(ctx, n_in, m, rows, small_tiles, st))) return rc;
     } else {
         GemvParams gu = gemv_params(ctx, l->gate, l->up, l->gate_scale, l->up_scale, xq, p.hid, l->n_ff, k, 1, l->n_expert);
+        gu.allow_empty = y_direct ? 1 : 0;
         if ((rc = launch_integer<true>(ctx, l->wtype, n_in, gu, likely_rows, l->n_expert, nt, st))) return rc;
     }
     if (fixup && (rc = launch_requant_fixup(ctx, l, xq, rows, n_in, k, fp4_gu, st))) return rc;
@@ -1127,6 +1140,7 @@ int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const 
         if ((rc = tm_down ? launch_gemm_tm<false>(ctx, l->n_ff, m, rows, st) : launch_gemm<false>(ctx, l->n_ff, m, rows, small_tiles, st))) return rc;
     } else {
         GemvParams dn = gemv_params(ctx, l->down, nullptr, l->down_scale, nullptr, p.hq, y, n_in, k, k, l->n_expert);
+        dn.allow_empty = y_direct ? 1 : 0;
         if (fused_quant) dn.act_f32 = p.hid;
         if (fused_combine) { dn.comb_out = out; dn.comb_w = wts; dn.comb_cnt = p.groups.done; }
         if ((rc = launch_integer<false>(ctx, l->wtype, l->n_ff, dn, likely_rows, l->n_expert, nt, st))) return rc;
@@ -1545,11 +1559,16 @@ int b200moe_mul_mat_id(b200moe_ctx * ctx, int wtype, const void * as, int64_t ne
     const int rows = (int) (T * n_ids);
     // activations: T*ne11 rows of ne00; plan.hq holds T*k rows of width n_ff (= ne00 here), ne11 <= k
     if ((rc = launch_quantize<float>(ctx, b, ne00, p.hq, (int) (T * ne11), (int) ne00, wtype, st))) return rc;
-    CUDA_TRY(ctx, cudaMemsetAsync(p.groups.counts, 0, sizeof(int) * n_as, st));
-    count_ids_kernel<<<(rows + 255) / 256, 256, 0, st>>>(ids, ids_nb1 / 4, (int) n_ids, (int) T, (int) n_as, p.ids, p.groups.counts, p.groups.pos, ctx->d_err);
-    if ((rc = check_launch(ctx, "count_ids"))) return rc;
-    if ((rc = launch_group(ctx, p.ids, (int) n_as, rows, st))) return rc;
     GemvParams g = gemv_params(ctx, as, nullptr, nullptr, nullptr, p.hq, dst, (int) ne01, (int) n_ids, (int) ne11, (int) n_as);
+    if (few_rows(wtype, rows, (int) n_as)) {   // read the ids as they are and need no groups
+        g.ids = ids;
+        g.ids_stride = ids_nb1 / 4;
+    } else {
+        CUDA_TRY(ctx, cudaMemsetAsync(p.groups.counts, 0, sizeof(int) * n_as, st));
+        count_ids_kernel<<<(rows + 255) / 256, 256, 0, st>>>(ids, ids_nb1 / 4, (int) n_ids, (int) T, (int) n_as, p.ids, p.groups.counts, p.groups.pos, ctx->d_err);
+        if ((rc = check_launch(ctx, "count_ids"))) return rc;
+        if ((rc = launch_group(ctx, p.ids, (int) n_as, rows, st))) return rc;
+    }
     return launch_integer<false>(ctx, wtype, (int) ne00, g, rows, (int) n_as, tokens_per_pass(rows, (int) n_as), st);
 }
 

@@ -1,23 +1,16 @@
-// Grouped expert GEMV for decode / batched decode: streams only the routed experts' quantised rows from HBM through
-// a shared-memory ring filled by 1-D bulk async copies (TMA), integer dot products against the reference's int8
-// activation grid, and fp32 accumulation in EXACTLY the order of the reference's AVX2 kernels, so every dot product
-// is bit-identical to the CPU path (and with it every later re-quantisation of activations).
+// The integer chains of the reference's dot products and the kernel of one or two tokens built on them.
 //
 // How the reference sums (ggml-cpu/arch/x86/quants.c, AVX2 branches): eight fp32 lanes; lane L collects, block after
 // block, fma(scale, (float) p_L, acc_L) where p_L is the integer dot of a fixed group of 4 elements per 32
 // (NVFP4: group L of each Q8_0 block; Q3_K: elements 4L..4L+3 of every 32-group of the super-block, scale-weighted and
 // summed over the super-block first); the eight lanes are folded at the end as ((a0+a4)+(a2+a6))+((a1+a5)+(a3+a7)).
-// Here 8 GPU lanes play the 8 AVX lanes of one weight row (4 rows per warp), each running its chain over K in
-// order; three xor-shuffles reproduce the fold.
+// Integer partial sums are exact in any order and the fp32 chains run in the reference's, so every dot product is bit-identical to
+// the CPU path (and with it every later re-quantisation of activations).
 //
-// One kernel template serves
+// Shared by the integer kernels (this file, expert_gemv_nvfp4.cuh, expert_mma_q3k.cuh, requant_fixup.cuh):
 //   DUAL = true : gate and up projections of the same rows + SwiGLU epilogue  -> hidden[row][n_out]
 //   DUAL = false: one indexed matmul (ggml MUL_MAT_ID semantics)               -> dst[row][n_out]
 // "row" is a routed row: token*n_ids + slot.
-//
-// Work distribution: the rows of all active experts form one flat list (active expert a, output row r); every CTA of
-// the persistent grid takes a contiguous span of equal WORK (rows x passes over the expert's routed rows).  A span is
-// walked in chunks of at most ROWS_PER_STAGE rows of one expert; chunk c lives in ring stage c % STAGES.
 #pragma once
 #include <type_traits>
 
@@ -39,6 +32,9 @@ struct GemvParams {
     const int * active;   // [n_as]
     const int * meta;     // meta[0] = number of active experts
     const int * cost;     // work prefixes (see Groups::cost)
+    const int32_t * ids;  // expert of routed row r at [r / n_ids * ids_stride + r % n_ids] (the kernel of one or two tokens, which needs no groups)
+    int64_t ids_stride;
+    int allow_empty;      // ids of -1 mark rows that do not exist
     float * out;          // [rows][n_out]
     int n_out;
     int n_ids;
@@ -46,26 +42,9 @@ struct GemvParams {
     int n_as;
     float * comb_out;     // one-or-two-token kernel only, or null: the weighted sum over a token's rows goes here ([tokens][n_out])
     const float * comb_w; // [rows] combine weights
-    int * comb_cnt;       // [tokens][n_out / 16] rows of `out` finished so far, cleared by the grouping
+    int * comb_cnt;       // [tokens][n_out / 16] rows of `out` finished so far, cleared by the routing
     int w_stride;         // rows between consecutive experts' matrices: n_out, or 0 when every group uses the same matrix
     int * err;
-};
-
-template <int WT, int K, int NW = 8>
-struct GemvCfg {
-    static constexpr int LPR = 8;            // lanes per row = the reference's 8 SIMD lanes
-    static constexpr int RPP = 4;            // rows per warp pass
-    static constexpr int ROW_BYTES = WT == TYPE_NVFP4 ? K / 64 * 36 : K / 256 * 110;
-    static constexpr int GRAN = (ROW_BYTES % 16 == 0) ? 1 : 8;  // span granularity in rows (16-byte rule of bulk copies)
-    static constexpr int NWARPS = NW;        // 8; 4 for the one-or-two-token kernel (several small CTAs per SM)
-    // passes per warp per stage chosen so a (single-tensor) stage is roughly 12-40 KB
-    static constexpr int PASSES = (ROW_BYTES * RPP * NWARPS >= 12288) ? 1 : (ROW_BYTES * RPP * NWARPS >= 6144) ? 2 : 4;
-    static constexpr int ROWS_PER_STAGE = NWARPS * RPP * PASSES;
-    static constexpr int TENSOR_STAGE_BYTES = ROWS_PER_STAGE * ROW_BYTES;
-    static_assert(TENSOR_STAGE_BYTES % 16 == 0, "stage must keep 16-byte alignment");
-    // activations of one token in shared memory: K int8, then the block scales as floats (padded to 16 bytes)
-    static constexpr int ACT_D = WT == TYPE_NVFP4 ? K / 32 : K / 256;
-    static constexpr int ACT_TOKEN_BYTES = K + ((ACT_D * 4 + 15) / 16) * 16;
 };
 
 __device__ __forceinline__ uint32_t lds_u32_a2(const uint8_t * p) {  // 2-byte aligned 32-bit load from shared memory
@@ -73,10 +52,6 @@ __device__ __forceinline__ uint32_t lds_u32_a2(const uint8_t * p) {  // 2-byte a
     return (uint32_t) h[0] | ((uint32_t) h[1] << 16);
 }
 
-// One SIMD lane (L = 0..7) of the reference's dot product of one weight row with NT activation rows.
-//   row   : the quantised weight row in shared memory
-//   acts  : the activations of NTS rows, token-interleaved: words [K/4][NTS] of int8x4, then block scales [ACT_D][NTS];
-//           the first NT of the NTS rows are used
 template <int N, typename T>
 __device__ __forceinline__ void load_vec(T (&dst)[N], const T * src) {
     static_assert(sizeof(T) == 4, "32-bit elements");
@@ -92,152 +67,28 @@ __device__ __forceinline__ void load_vec(T (&dst)[N], const T * src) {
     }
 }
 
-template <int WT, int K, int NT, int NTS>
-__device__ __forceinline__ void lane_chain(const uint8_t * __restrict__ row, int L, const uint8_t * __restrict__ acts,
-                                           const float * __restrict__ ue_tab, float (&acc)[NT]) {
-    using C = GemvCfg<WT, K>;
+// Integer part of SIMD lane L (0..7) of a super-block: the signed 6-bit sub-block scales times the dots of byte columns 4L..4L+3
+// (ggml_vec_dot_q3_K_q8_K, ggml-cpu/arch/x86/quants.c:1766-1880).  blk: 2-byte aligned; acts: the 256 activations of the super-block.
+__device__ __forceinline__ int q3k_lane_sum(const uint8_t * __restrict__ blk, int L, const uint32_t * __restrict__ acts) {
+    const int hi = L >= 4 ? 1 : 0;
+    const uint32_t hm = lds_u32_a2(blk + 4 * L);
+    const uint32_t qs0 = lds_u32_a2(blk + 32 + 4 * L);
+    const uint32_t qs1 = lds_u32_a2(blk + 64 + 4 * L);
+    uint32_t sc[4];
+    q3k_unpack_scales(lds_u32_a2(blk + 96), lds_u32_a2(blk + 100), lds_u32_a2(blk + 104), sc);
+    int sum = 0;
 #pragma unroll
-    for (int t = 0; t < NT; ++t) acc[t] = 0.0f;
-    if (WT == TYPE_NVFP4) {
-        // lane L: sub-block (L>>2) of each half block, elements 4*(L&3) .. +3 of it = the low (L&3 < 2) or high nibbles of
-        // one qs word; they meet word L of the Q8_0 block.  ggml_vec_dot_nvfp4_q8_0, ggml-cpu/arch/x86/quants.c:1004-1062.
-        const int sub_in_half = L >> 2, mp = L & 3;
-        const int word_off = 4 + 8 * sub_in_half + 4 * (mp & 1);
-        const int nib_shift = 4 * (mp >> 1);
-#pragma unroll 2
-        for (int b = 0; b < K / 64; ++b) {
-            const uint8_t * blk = row + b * NVFP4_BLOCK_BYTES;
-            const uint32_t dw = *reinterpret_cast<const uint32_t *>(blk);
+    for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-                const uint32_t w = *reinterpret_cast<const uint32_t *>(blk + 16 * hf + word_off);
-                const uint32_t t4 = (w >> nib_shift) & 0x0f0f0f0fu;          // four codes, one per byte
-                const uint32_t u = t4 | (t4 >> 4);
-                const uint32_t sel = byte_perm(u, 0u, 0x4420u);              // the four codes packed into 16 bits (bytes 0 and 2 of u)
-                const uint32_t pos = byte_perm(FP4_MAG_LO, FP4_MAG_HI, sel);
-                const uint32_t neg = byte_perm(FP4_MAG_LO, FP4_MAG_HI, sel ^ 0x8888u);
-                // signed bytes: a byte of `neg` is a magnitude 0..12, 0x80 - it never borrows, the xor drops the guard bit
-                const uint32_t code = pos | ((0x80808080u - neg) ^ 0x80808080u);
-                const float sw = ue_tab[(dw >> (8 * (2 * hf + sub_in_half))) & 0xff];
-                const int unit = 2 * b + hf;
-                // activations are stored [unit][lane word][token] and [unit][token]: one vector load serves all NT rows
-                uint32_t aw[NT];
-                float dy[NT];
-                load_vec<NT>(aw, reinterpret_cast<const uint32_t *>(acts) + (size_t) (unit * 8 + L) * NTS);
-                load_vec<NT>(dy, reinterpret_cast<const float *>(acts + (size_t) K * NTS) + (size_t) unit * NTS);
-#pragma unroll
-                for (int t = 0; t < NT; ++t) {
-                    const int p = dot4((int) code, (int) aw[t], 0);
-                    acc[t] = __fmaf_rn(__fmul_rn(sw, dy[t]), small_int_to_float(p), acc[t]);
-                }
-            }
+        for (int s = 0; s < 4; ++s) {
+            const int bit = 4 * j + s;
+            const uint32_t lo2 = ((j ? qs1 : qs0) >> (2 * s)) & 0x03030303u;
+            const uint32_t hb4 = bit >= 2 ? ((hm >> (bit - 2)) & 0x04040404u) : ((hm << (2 - bit)) & 0x04040404u);
+            // codes 0..7 -> signed -4..3 in every byte without borrows between bytes
+            const uint32_t code = (((lo2 | hb4) | 0x80808080u) - 0x04040404u) ^ 0x80808080u;
+            sum += q3k_scale_at(sc, 8 * j + 2 * s + hi) * dot4((int) code, (int) acts[8 * bit + L], 0);
         }
-    } else {
-        // lane L: byte columns 4L..4L+3 of every super-block; integer sum over the super-block with the signed 6-bit
-        // sub-block scales, then one fma with d_w*d_x.  ggml_vec_dot_q3_K_q8_K, ggml-cpu/arch/x86/quants.c:1766-1880.
-        const int hi = L >= 4 ? 1 : 0;
-#pragma unroll 1
-        for (int sb = 0; sb < K / 256; ++sb) {
-            const uint8_t * blk = row + sb * Q3K_BLOCK_BYTES;  // 2-byte aligned
-            const uint32_t hm = lds_u32_a2(blk + 4 * L);
-            const uint32_t qs0 = lds_u32_a2(blk + 32 + 4 * L);
-            const uint32_t qs1 = lds_u32_a2(blk + 64 + 4 * L);
-            uint32_t sc[4];
-            q3k_unpack_scales(lds_u32_a2(blk + 96), lds_u32_a2(blk + 100), lds_u32_a2(blk + 104), sc);
-            const float dw = __half2float(*reinterpret_cast<const __half *>(blk + 108));
-            int sumi[NT];
-#pragma unroll
-            for (int t = 0; t < NT; ++t) sumi[t] = 0;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const uint32_t w = j ? qs1 : qs0;
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    const int bit = 4 * j + s;
-                    const uint32_t lo2 = (w >> (2 * s)) & 0x03030303u;
-                    const uint32_t hb4 = bit >= 2 ? ((hm >> (bit - 2)) & 0x04040404u) : ((hm << (2 - bit)) & 0x04040404u);
-                    // codes 0..7 -> signed -4..3 in every byte without borrows between bytes
-                    const uint32_t code = (((lo2 | hb4) | 0x80808080u) - 0x04040404u) ^ 0x80808080u;
-                    const int scale = q3k_scale_at(sc, 8 * j + 2 * s + hi);
-                    uint32_t aw[NT];
-                    load_vec<NT>(aw, reinterpret_cast<const uint32_t *>(acts) + (size_t) (sb * 64 + 8 * (4 * j + s) + L) * NTS);
-#pragma unroll
-                    for (int t = 0; t < NT; ++t) sumi[t] += scale * dot4((int) code, (int) aw[t], 0);
-                }
-            }
-            float dx[NT];
-            load_vec<NT>(dx, reinterpret_cast<const float *>(acts + (size_t) K * NTS) + (size_t) sb * NTS);
-#pragma unroll
-            for (int t = 0; t < NT; ++t) acc[t] = __fmaf_rn(__fmul_rn(dx[t], dw), small_int_to_float(sumi[t]), acc[t]);
-        }
-    }
-    // hsum_float_8: (a4+a0, a5+a1, a6+a2, a7+a3) -> (r0+r2, r1+r3) -> s0+s1
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-        float v = acc[t];
-        v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 4));
-        v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 2));
-        v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
-        acc[t] = v;
-    }
-}
-
-// decode of four NVFP4 codes (one per byte of t4's nibbles) to signed int8 (twice the E2M1 value)
-__device__ __forceinline__ uint32_t nvfp4_codes_to_s8(uint32_t w, int nib_shift) {
-    const uint32_t t4 = (w >> nib_shift) & 0x0f0f0f0fu;          // four codes, one per byte
-    const uint32_t u = t4 | (t4 >> 4);
-    const uint32_t sel = byte_perm(u, 0u, 0x4420u);              // the four codes packed into 16 bits (bytes 0 and 2 of u)
-    const uint32_t pos = byte_perm(FP4_MAG_LO, FP4_MAG_HI, sel);
-    const uint32_t neg = byte_perm(FP4_MAG_LO, FP4_MAG_HI, sel ^ 0x8888u);
-    // signed bytes: a byte of `neg` is a magnitude 0..12, 0x80 - it never borrows, the xor drops the guard bit
-    return pos | ((0x80808080u - neg) ^ 0x80808080u);
-}
-
-// lane_chain<TYPE_NVFP4> for TWO weight rows against the same activations (the gate row and the up row of a feature): the two
-// chains are independent, so running them in one loop doubles the work in flight per lane - and each activation word and block
-// scale is fetched once for both.  Every chain keeps its own order of operations: the results are those of two lane_chain calls.
-template <int K, int NT, int NTS>
-__device__ __forceinline__ void lane_chain_pair(const uint8_t * __restrict__ row0, const uint8_t * __restrict__ row1, int L,
-                                                const uint8_t * __restrict__ acts, const float * __restrict__ ue_tab, float (&acc0)[NT],
-                                                float (&acc1)[NT]) {
-#pragma unroll
-    for (int t = 0; t < NT; ++t) acc0[t] = acc1[t] = 0.0f;
-    const int sub_in_half = L >> 2, mp = L & 3;
-    const int word_off = 4 + 8 * sub_in_half + 4 * (mp & 1);
-    const int nib_shift = 4 * (mp >> 1);
-#pragma unroll 2
-    for (int b = 0; b < K / 64; ++b) {
-        const uint8_t * blk0 = row0 + b * NVFP4_BLOCK_BYTES, * blk1 = row1 + b * NVFP4_BLOCK_BYTES;
-        const uint32_t dw0 = *reinterpret_cast<const uint32_t *>(blk0), dw1 = *reinterpret_cast<const uint32_t *>(blk1);
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
-            const uint32_t code0 = nvfp4_codes_to_s8(*reinterpret_cast<const uint32_t *>(blk0 + 16 * hf + word_off), nib_shift);
-            const uint32_t code1 = nvfp4_codes_to_s8(*reinterpret_cast<const uint32_t *>(blk1 + 16 * hf + word_off), nib_shift);
-            const float sw0 = ue_tab[(dw0 >> (8 * (2 * hf + sub_in_half))) & 0xff], sw1 = ue_tab[(dw1 >> (8 * (2 * hf + sub_in_half))) & 0xff];
-            const int unit = 2 * b + hf;
-            uint32_t aw[NT];
-            float dy[NT];
-            load_vec<NT>(aw, reinterpret_cast<const uint32_t *>(acts) + (size_t) (unit * 8 + L) * NTS);
-            load_vec<NT>(dy, reinterpret_cast<const float *>(acts + (size_t) K * NTS) + (size_t) unit * NTS);
-#pragma unroll
-            for (int t = 0; t < NT; ++t) {
-                acc0[t] = __fmaf_rn(__fmul_rn(sw0, dy[t]), small_int_to_float(dot4((int) code0, (int) aw[t], 0)), acc0[t]);
-                acc1[t] = __fmaf_rn(__fmul_rn(sw1, dy[t]), small_int_to_float(dot4((int) code1, (int) aw[t], 0)), acc1[t]);
-            }
-        }
-    }
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-        float v = acc0[t], w = acc1[t];
-        v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 4));
-        w = __fadd_rn(w, __shfl_xor_sync(0xffffffffu, w, 4));
-        v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 2));
-        w = __fadd_rn(w, __shfl_xor_sync(0xffffffffu, w, 2));
-        v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
-        w = __fadd_rn(w, __shfl_xor_sync(0xffffffffu, w, 1));
-        acc0[t] = v;
-        acc1[t] = w;
-    }
+    return sum;
 }
 
 // ---- two SIMD lanes per thread ---------------------------------------------------------------------------------------------
@@ -446,28 +297,6 @@ __device__ __forceinline__ float lane_chain_warp(const uint8_t * __restrict__ ro
     return a;
 }
 
-// chunk walker shared by the producer thread and the consumers
-struct Chunk {
-    int a;      // index into active[]
-    int r0;     // first output row
-    int n;      // rows
-};
-struct ChunkWalker {
-    int u, u_end, units_per_expert, gran, max_rows;
-    __device__ __forceinline__ bool next(Chunk & c) {
-        if (u >= u_end) return false;
-        const int a = u / units_per_expert;
-        const int uu = u - a * units_per_expert;
-        int n_units = min(u_end - u, units_per_expert - uu);
-        n_units = min(n_units, max_rows / gran);
-        c.a = a;
-        c.r0 = uu * gran;
-        c.n = n_units * gran;
-        u += n_units;
-        return true;
-    }
-};
-
 // A CTA's part of the work: items (active expert a, pass ps over PT of its routed rows, chunk ch of its weight rows), chunks fastest.
 template <int PT>
 struct PassSpan {
@@ -513,280 +342,253 @@ __device__ __forceinline__ PassSpan<PT> pass_span(const int * __restrict__ cw, i
     return PassSpan<PT>{ at[0][0], at[0][1], at[0][2], at[1][0], at[1][1], at[1][2], chunks };
 }
 
-template <int WT, int K, bool DUAL, int NT, int STAGES, int NW = 8>
-constexpr size_t gemv_smem_bytes() {
-    return (size_t) STAGES * GemvCfg<WT, K, NW>::TENSOR_STAGE_BYTES * (DUAL ? 2 : 1) + NT * GemvCfg<WT, K, NW>::ACT_TOKEN_BYTES + STAGES * 8 +
-           256 * 4 + 64;
-}
+// ---- one or two tokens -------------------------------------------------------------------------------------------------
+// The whole call is a few thousand weight rows, so its time is what one row takes: a CTA has 8 features of gate and up (or 32 rows of one
+// tensor) for one routed row, reads their expert straight from the ids, and cuts every row's K into SEG segments of a warp each.  All the
+// integer work and the products of the scales run at once; only the fp32 chains, a few steps to a segment, go from segment to segment.
+//   NVFP4: four threads to a weight row, two SIMD lanes each; Q3_K: a thread per SIMD lane; either way two rows to a thread (gate and up of a
+//   feature), which share the activations and the thread's fixed work.
+// A chain per thread over the whole K, 16 rows to a four-warp CTA, chunks looked up in the group tables: one token, 2048 -> 768, top-8
+// of 128, gate/up and down 12.1 and 9.8 us (Q3_K 9.9 and 8.6), so 10.4 and 8.3 (8.8 and 8.3).  16 features of gate and up to a CTA 11.1, eight
+// segments 12.1; a segment's bytes behind a barrier of their own gained nothing.
+template <int WT, int K, bool DUAL>
+struct FewCfg {
+    static constexpr int PAIRS = DUAL ? 8 : 16;               // row pairs of a CTA
+    static constexpr int FEAT = DUAL ? PAIRS : 2 * PAIRS;     // its features
+    static constexpr int ROW_BYTES = WT == TYPE_NVFP4 ? K / 64 * NVFP4_BLOCK_BYTES : K / 256 * Q3K_BLOCK_BYTES;
+    static constexpr int PITCH = WT == TYPE_NVFP4 ? two_lane_pitch(ROW_BYTES) : ROW_BYTES;
+    static constexpr int TPR = WT == TYPE_NVFP4 ? 4 : 8;      // threads of a row pair
+    static constexpr int GROUPS = PAIRS * TPR / 32;           // warps of a segment
+    static constexpr int STEPS = WT == TYPE_NVFP4 ? K / 32 : K / 256;   // of a chain
+    static constexpr int SEG = WT == TYPE_NVFP4 ? (K == 4096 ? 8 : 4) : STEPS == 8 ? 4 : STEPS;
+    static constexpr int U = STEPS / SEG;                     // steps of a segment
+    static constexpr int THREADS = GROUPS * SEG * 32;
+    static constexpr int ACT_D = WT == TYPE_NVFP4 ? K / 32 : K / 256;
+    static constexpr size_t WBYTES = (size_t) 2 * PAIRS * PITCH;
+    static constexpr size_t SMEM = WBYTES + K + (ACT_D * 4 + 15) / 16 * 16;
+    static_assert(U * SEG == STEPS && (WT != TYPE_NVFP4 || U % 2 == 0), "segments hold whole blocks");
+    static_assert(8 * ROW_BYTES % 16 == 0 && WBYTES % 16 == 0, "bulk copies move multiples of 16 bytes");
+};
 
-// CTAs per SM: the kernel waits on the latency of its own lane chains, so two CTAs (16 warps) beat one with a deeper ring; two
-// whenever two stages and the activations fit twice.  Ring depth: what fits then, up to four stages.
-template <int WT, int K, bool DUAL, int NT>
-constexpr int gemv_ctas() { return 2 * (gemv_smem_bytes<WT, K, DUAL, NT, 2>() + 1024 + 128) <= 228 * 1024 ? 2 : 1; }
-template <int WT, int K, bool DUAL, int NT>
-constexpr int gemv_stages() {
-    if (gemv_ctas<WT, K, DUAL, NT>() == 2)
-        return 2 * (gemv_smem_bytes<WT, K, DUAL, NT, 4>() + 1024 + 128) <= 228 * 1024 ? 4 : 2 * (gemv_smem_bytes<WT, K, DUAL, NT, 3>() + 1024 + 128) <= 228 * 1024 ? 3 : 2;
-    constexpr int stage = GemvCfg<WT, K>::TENSOR_STAGE_BYTES * (DUAL ? 2 : 1);
-    return (4 * stage <= 190 * 1024) ? 4 : (3 * stage <= 190 * 1024) ? 3 : 2;
-}
+// ue4m3_half_to_f32 of every byte
+struct UeTable {
+    float v[256];
+    constexpr UeTable() : v() {
+        for (int x = 0; x < 256; ++x) {
+            const int exp = (x >> 3) & 0xf, man = x & 7;
+            float f = exp ? 1.0f + man * 0.125f : man * 0.125f;
+            for (int e = exp ? exp : 1; e < 8; ++e) f *= 0.5f;          // 2^(exp - 7) / 2
+            for (int e = 8; e < exp; ++e) f *= 2.0f;
+            v[x] = x == 0 || x == 0x7f ? 0.0f : f;
+        }
+    }
+};
+__device__ __align__(16) const UeTable g_ue_table = UeTable();
 
-template <int WT, int K, bool DUAL, int NT, int STAGES, int NW = 8>
-__global__ void __launch_bounds__(NW * 32, NW == 8 ? gemv_ctas<WT, K, DUAL, NT>() : 4) expert_gemv_kernel(const GemvParams p) {
-    using C = GemvCfg<WT, K, NW>;
-    constexpr int NTENS = DUAL ? 2 : 1;
-    constexpr int STAGE_BYTES = C::TENSOR_STAGE_BYTES * NTENS;
-    constexpr int NTHREADS = C::NWARPS * 32;
-
-    extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t * ring = smem;                                                        // STAGES * STAGE_BYTES
-    uint8_t * acts = smem + STAGES * STAGE_BYTES;                                 // NT * ACT_TOKEN_BYTES (16-byte aligned)
-    uint64_t * full = reinterpret_cast<uint64_t *>(acts + NT * C::ACT_TOKEN_BYTES);  // STAGES barriers
-    float * ue_tab = reinterpret_cast<float *>(full + STAGES);                    // 256 floats (NVFP4 only)
-    __shared__ int s_abort, s_last;
-    __shared__ int s_span[2];
+template <int WT, int K, bool DUAL>
+__global__ void __launch_bounds__(FewCfg<WT, K, DUAL>::THREADS) expert_few_rows_kernel(const GemvParams p) {
+    using C = FewCfg<WT, K, DUAL>;
+    extern __shared__ __align__(128) uint8_t few_smem[];
+    uint8_t * const wrows = few_smem;                         // [2 * PAIRS][PITCH]; DUAL: gate rows, then up rows
+    uint32_t * const acts = reinterpret_cast<uint32_t *>(few_smem + C::WBYTES);
+    float * const act_d = reinterpret_cast<float *>(acts + K / 4);
+    __shared__ uint64_t full;
+    __shared__ float ue_tab[WT == TYPE_NVFP4 ? 256 : 4];
+    __shared__ float s_val[2 * C::PAIRS];
+    __shared__ float s_acc[2][2][C::PAIRS][C::TPR];                 // [row of the pair][SIMD lane of the thread][pair][thread]
+    __shared__ int s_last;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int L = lane & 7;       // SIMD lane of the reference this thread plays
-    const int rgrp = lane >> 3;   // which of the 4 rows of a warp pass
-
-    if (tid == 0) {
-        for (int s = 0; s < STAGES; ++s) mbar_init(&full[s], 1);
-        mbar_fence_init();
-        s_abort = 0;
-    }
+    if (tid == 0) { mbar_init(&full, 1); mbar_fence_init(); }
     if (WT == TYPE_NVFP4)
-        for (int i = tid; i < 256; i += NTHREADS) ue_tab[i] = ue4m3_half_to_f32(i);
+        for (int i = tid; i < 256; i += C::THREADS) ue_tab[i] = g_ue_table.v[i];
     __syncthreads();
     pdl_wait();                 // programmatic dependent launch: everything before this ran alongside the previous kernel's tail
     pdl_launch_dependents();
 
-    const int n_active = p.meta[0];
-    const int upe = p.n_out / C::GRAN;                       // span units per expert
-    const long long total = (long long) n_active * upe;
-    // Span boundaries balance WORK, not rows: a weight row of an expert with n routed rows costs 3 per pass (decode) + 2 per routed row.
-    // Boundary i sits at work i/grid of the total; both neighbours compute it the same way, so spans tile exactly.
-    if (NW != 8) {
-        // one-or-two-token kernel: CTA b owns stage-sized chunk b of the flat row list - no search, no dependent loads
-        if (tid < 2) {
-            const long long u = (long long) (blockIdx.x + tid) * (C::ROWS_PER_STAGE / C::GRAN);
-            s_span[tid] = (int) (u < total ? u : total);
-        }
-    } else if (tid < 2) {
-        const int * cw = p.cost + (NT == 1 ? 0 : 2) * (p.n_as + 1);
-        const long long total_work = (long long) cw[n_active] * upe;
-        const long long c = total_work * (blockIdx.x + tid) / gridDim.x;
-        int lo = 0, hi = n_active;  // largest a with cw[a]*upe <= c
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if ((long long) cw[mid] * upe <= c) lo = mid; else hi = mid;
-        }
-        int u;
-        if (n_active == 0) u = 0;
-        else if (blockIdx.x + tid == gridDim.x) u = (int) total;
-        else {
-            const int per = max(cw[lo + 1] - cw[lo], 1);
-            const long long uu = (c - (long long) cw[lo] * upe) / per;
-            u = lo * upe + (int) (uu < (long long) upe ? uu : (long long) upe);
-        }
-        s_span[tid] = u;
+    const int r = blockIdx.y, f0 = blockIdx.x * C::FEAT, n = min(C::FEAT, p.n_out - f0);
+    const int tok = r / p.n_ids, slot = r - tok * p.n_ids;
+    const int e = p.ids ? p.ids[(size_t) tok * p.ids_stride + slot] : 0;   // (a dense product has one matrix)
+    if (e < 0 || e >= p.n_as) {                               // the whole block; nothing is addressed with it
+        if (tid == 0 && !(p.allow_empty && e == -1)) report_error(p.err, DEV_ERR_BAD_EXPERT_ID);
+        return;
     }
-    __syncthreads();
-    ChunkWalker cons, prod;
-    cons.u = s_span[0];
-    cons.u_end = s_span[1];
-    cons.units_per_expert = upe;
-    cons.gran = C::GRAN;
-    cons.max_rows = C::ROWS_PER_STAGE;
-    prod = cons;
-
-    auto issue = [&](const Chunk & c, int stage) {
-        const int e = p.active[c.a];
-        const uint32_t bytes = (uint32_t) c.n * C::ROW_BYTES;
-        uint8_t * dst = ring + (size_t) stage * STAGE_BYTES;
-        mbar_arrive_expect_tx(&full[stage], bytes * NTENS);
-        const size_t off = ((size_t) e * p.w_stride + c.r0) * C::ROW_BYTES;
-        bulk_g2s(dst, p.w0 + off, bytes, &full[stage]);
-        if (DUAL) bulk_g2s(dst + C::TENSOR_STAGE_BYTES, p.w1 + off, bytes, &full[stage]);
-    };
-
-    int issued = 0;
-    if (tid == 0) {
-        Chunk c;
-        for (int s = 0; s < STAGES; ++s)
-            if (prod.next(c)) { issue(c, s); ++issued; }
+    const size_t off = ((size_t) e * p.w_stride + f0) * C::ROW_BYTES;
+    if (warp == 0) {
+        if (lane == 0) mbar_arrive_expect_tx(&full, (uint32_t) (n * C::ROW_BYTES * (DUAL ? 2 : 1)));
+        __syncwarp();
+        if (C::PITCH == C::ROW_BYTES) {                       // rows stay as they lie
+            if (lane == 0) bulk_g2s(wrows, p.w0 + off, n * C::ROW_BYTES, &full);
+            if (DUAL && lane == 1) bulk_g2s(wrows + C::PAIRS * C::PITCH, p.w1 + off, n * C::ROW_BYTES, &full);
+        } else if (DUAL) {
+            const int i = lane % C::PAIRS;
+            if (i < n && lane < 2 * C::PAIRS) bulk_g2s(wrows + lane * C::PITCH, (lane < C::PAIRS ? p.w0 : p.w1) + off + (size_t) i * C::ROW_BYTES, C::ROW_BYTES, &full);
+        } else if (lane < n) {
+            bulk_g2s(wrows + lane * C::PITCH, p.w0 + off + (size_t) lane * C::ROW_BYTES, C::ROW_BYTES, &full);
+        }
+    }
+    // the routed row's activations meanwhile
+    const size_t arow = (size_t) tok * p.ne11 + slot % p.ne11;
+    if (WT == TYPE_NVFP4 && p.act_f32) {
+        // Q8_0 on the fly, the arithmetic of quantize_q8_0_block: 8 lanes hold one block of 32 (4 values each)
+        const float4 * src = reinterpret_cast<const float4 *>(p.act_f32 + arow * K);
+        for (int i0 = 0; i0 < K / 4; i0 += C::THREADS) {
+            const int i = i0 + tid;
+            const bool in = i < K / 4;
+            const float4 v = in ? __ldg(src + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
+            const float id = amax != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
+            if (in) {
+                acts[i] = ((uint32_t) __float2int_rn(__fmul_rn(v.x, id)) & 0xffu) | (((uint32_t) __float2int_rn(__fmul_rn(v.y, id)) & 0xffu) << 8) |
+                          (((uint32_t) __float2int_rn(__fmul_rn(v.z, id)) & 0xffu) << 16) | (((uint32_t) __float2int_rn(__fmul_rn(v.w, id)) & 0xffu) << 24);
+                if ((i & 7) == 0) act_d[i >> 3] = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
+            }
+        }
+    } else if (WT == TYPE_Q3_K && p.act_f32) {
+        for (int b = warp; b < K / 256; b += C::THREADS / 32) {               // a warp quantises one 256-block
+            uint32_t q[2] = { 0u, 0u };
+            float d = 0.0f;
+            q8_K_words(p.act_f32 + arow * K + b * 256 + lane * 8, lane, q, d);
+            acts[b * 64 + lane * 2] = q[0];
+            acts[b * 64 + lane * 2 + 1] = q[1];
+            if (lane == 0) act_d[b] = d;
+        }
+    } else {
+        const uint4 * src = reinterpret_cast<const uint4 *>(p.act.q + arow * K);
+        for (int i = tid; i < K / 16; i += C::THREADS) reinterpret_cast<uint4 *>(acts)[i] = __ldg(src + i);
+        for (int i = tid; i < C::ACT_D; i += C::THREADS) act_d[i] = __ldg(p.act.d + arow * C::ACT_D + i);
+    }
+    const float sc0 = p.scale0 ? p.scale0[p.w_stride ? e : 0] : 1.0f, sc1 = DUAL && p.scale1 ? p.scale1[p.w_stride ? e : 0] : 1.0f;
+    const bool landed = mbar_wait_bounded(&full, 0);
+    if (!landed) report_error(p.err, DEV_ERR_BARRIER_TIMEOUT);
+    if (__syncthreads_or(!landed)) {                          // bounded drain before the block (and its shared memory) goes away
+        if (tid == 0) mbar_wait_bounded(&full, 0, 200000000ull);
+        __syncthreads();
+        return;
     }
 
-    int loaded_e = -1, loaded_tc = -1;
-    Chunk ck;
-    int ci = 0;
-    bool failed = false;
-    while (cons.next(ck)) {
-        const int stage = ci % STAGES;
-        const uint32_t parity = (uint32_t) (ci / STAGES) & 1u;
-        bool landed = false;    // the weights are waited for behind the loads of the first pass's activations
-
-        const int e = p.active[ck.a];
-        const int row_beg = p.offsets[e], n_e = p.offsets[e + 1] - row_beg;
-        const uint8_t * st = ring + (size_t) stage * STAGE_BYTES;
-        // A warp without rows leaves a pass out: with two CTAs on the SM its idle chains would hold up the other's (8 experts, 256 -> 512, 400
-        // rows each: 1020 us with them, 547 without; one CTA per SM 906 and 547).  The chunks of the few-row kernel are whole at the widths of a layer.
-        const int first_row = warp * C::RPP, pass_rows = C::NWARPS * C::RPP;
-        const int my_passes = NW != 8 ? C::PASSES : ck.n > first_row ? (ck.n - first_row + pass_rows - 1) / pass_rows : 0;
-        const int se = p.w_stride ? e : 0;      // every group of a dense product has the one matrix and its scale
-        const float sc0 = p.scale0 ? p.scale0[se] : 1.0f;
-        const float sc1 = (DUAL && p.scale1) ? p.scale1[se] : 1.0f;
-
-        // Routed rows of this expert are taken NT at a time; a remainder of 1 or 2 runs the narrower chains instead of
-        // padding to NT (the weight decode is shared by the rows of a pass, the per-row work is not).
-        for (int t0 = 0, tc = 0; t0 < n_e; ++tc) {
-            const int left = n_e - t0;
-            const int ntc = (NT >= 4 && left >= 3) ? 4 : (NT >= 2 && left >= 2) ? 2 : 1;
-            int rows[NT];
+    const int seg = warp / C::GROUPS, pair = (warp % C::GROUPS) * (32 / C::TPR) + lane / C::TPR, m = lane % C::TPR;
+    const uint8_t * wrow[2];                                  // where the segment's bytes of the pair lie
 #pragma unroll
-            for (int t = 0; t < NT; ++t) {
-                const int i = t0 + t;
-                rows[t] = (t < ntc && i < n_e) ? p.perm[row_beg + i] : -1;
-            }
-            if (loaded_e != e || loaded_tc != tc) {
-                // the activation rows of this pass into shared memory (all warps use the same ones)
-                __syncthreads();
+    for (int r = 0; r < 2; ++r)
+        wrow[r] = wrows + (pair + r * C::PAIRS) * C::PITCH + (WT == TYPE_NVFP4 ? C::U / 2 * NVFP4_BLOCK_BYTES : C::U * Q3K_BLOCK_BYTES) * seg;
+    if constexpr (WT == TYPE_NVFP4) {
+        float s[2][C::U];
+        uint64_t dots[2][C::U];
+        const uint32_t * aw = acts + seg * C::U * 8 + 4 * (m >> 1) + (m & 1);
 #pragma unroll
-                for (int t = 0; t < NT; ++t) {
-                    if (t >= ntc) break;
-                    const int r = rows[t];
-                    const int arow = r >= 0 ? (r / p.n_ids) * p.ne11 + (r % p.n_ids) % p.ne11 : 0;
-                    uint32_t * dq = reinterpret_cast<uint32_t *>(acts);
-                    float * dd = reinterpret_cast<float *>(acts + (size_t) K * NT);
-                    if (WT == TYPE_NVFP4 && p.act_f32) {
-                        // Q8_0 on the fly, the arithmetic of quantize_q8_0_block: 8 lanes hold one block of 32 (4 values each)
-                        const float4 * src = reinterpret_cast<const float4 *>(p.act_f32 + (size_t) arow * K);
-                        for (int i0 = 0; i0 < K / 4; i0 += NTHREADS) {
-                            const int i = i0 + tid;
-                            const bool in = i < K / 4;
-                            const float4 v = (in && r >= 0) ? __ldg(src + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                            float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-                            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-                            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-                            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 4));
-                            const float id = amax != 0.0f ? __fdiv_rn(127.0f, amax) : 0.0f;
-                            const uint32_t q = ((uint32_t) __float2int_rn(__fmul_rn(v.x, id)) & 0xffu) |
-                                               (((uint32_t) __float2int_rn(__fmul_rn(v.y, id)) & 0xffu) << 8) |
-                                               (((uint32_t) __float2int_rn(__fmul_rn(v.z, id)) & 0xffu) << 16) |
-                                               (((uint32_t) __float2int_rn(__fmul_rn(v.w, id)) & 0xffu) << 24);
-                            if (in) {
-                                dq[(size_t) i * NT + t] = q;
-                                if ((i & 7) == 0) dd[(size_t) (i >> 3) * NT + t] = __half2float(__float2half_rn(__fdiv_rn(amax, 127.0f)));
-                            }
-                        }
-                    } else if (WT == TYPE_Q3_K && p.act_f32) {
-                        for (int b = warp; b < K / 256; b += C::NWARPS) {      // a warp quantises one 256-block
-                            uint32_t q[2] = { 0u, 0u };
-                            float d = 0.0f;
-                            if (r >= 0) q8_K_words(p.act_f32 + (size_t) arow * K + b * 256 + lane * 8, lane, q, d);
-                            dq[(size_t) (b * 64 + lane * 2) * NT + t] = q[0];
-                            dq[(size_t) (b * 64 + lane * 2 + 1) * NT + t] = q[1];
-                            if (lane == 0) dd[(size_t) b * NT + t] = d;
-                        }
-                    } else {
-                        const uint32_t * srcq = reinterpret_cast<const uint32_t *>(p.act.q + (size_t) arow * K);
-                        for (int i = tid; i < K / 4; i += NTHREADS) dq[(size_t) i * NT + t] = r >= 0 ? __ldg(srcq + i) : 0u;
-                        for (int i = tid; i < C::ACT_D; i += NTHREADS) dd[(size_t) i * NT + t] = r >= 0 ? __ldg(p.act.d + (size_t) arow * C::ACT_D + i) : 0.0f;
-                    }
+        for (int b = 0; b < C::U / 2; ++b) {
+            const int at = b * NVFP4_BLOCK_BYTES;
+            const float2 d = *reinterpret_cast<const float2 *>(act_d + seg * C::U + 2 * b);
+            uint32_t dw[2];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) dw[r] = *reinterpret_cast<const uint32_t *>(wrow[r] + at) >> (8 * (m >> 1));
+#pragma unroll
+            for (int hf = 0; hf < 2; ++hf) {
+                const int u = 2 * b + hf;
+                const uint32_t alo = aw[u * 8], ahi = aw[u * 8 + 2];
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    uint32_t lo, hi;
+                    nvfp4_word_to_s8(*reinterpret_cast<const uint32_t *>(wrow[r] + at + 4 + 16 * hf + 4 * m), lo, hi);
+                    s[r][u] = __fmul_rn(ue_tab[(dw[r] >> (16 * hf)) & 0xff], hf ? d.y : d.x);
+                    dots[r][u] = dots_to_f32x2(lo, alo, hi, ahi);
                 }
-                __syncthreads();
-                loaded_e = e;
-                loaded_tc = tc;
             }
-            if (!landed) {
-                if (!mbar_wait_bounded(&full[stage], parity)) {
-                    report_error(p.err, DEV_ERR_BARRIER_TIMEOUT);
-                    s_abort = 1;
-                }
-                if (__syncthreads_or(s_abort)) { failed = true; break; }
-                landed = true;
-            }
+        }
 #pragma unroll 1
-            for (int ps = 0; ps < C::PASSES; ++ps) {
-                if (ps >= my_passes) break;
-                const int lr = (ps * C::NWARPS + warp) * C::RPP + rgrp;  // row within the stage
-                const bool row_ok = lr < ck.n;
-                const uint8_t * wrow = st + (size_t) (row_ok ? lr : 0) * C::ROW_BYTES;
-                float g[NT], uacc[NT];
-                auto run = [&](auto ntag) {
-                    constexpr int NTC = decltype(ntag)::value;
-                    float gg[NTC], uu[NTC];
-                    if constexpr (DUAL && WT == TYPE_NVFP4) {
-                        lane_chain_pair<K, NTC, NT>(wrow, wrow + C::TENSOR_STAGE_BYTES, L, acts, ue_tab, gg, uu);
+        for (int g = 0; g < C::SEG; ++g) {
+            if (seg == g) {
+                uint64_t acc[2] = { f32x2(0.0f, 0.0f), f32x2(0.0f, 0.0f) };
+                if (g > 0) {
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) acc[r] = f32x2(s_acc[r][0][pair][m], s_acc[r][1][pair][m]);
+                }
+#pragma unroll
+                for (int u = 0; u < C::U; ++u)
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) acc[r] = fma_f32x2(f32x2(s[r][u], s[r][u]), dots[r][u], acc[r]);
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const float2 a = f32x2_halves(acc[r]);
+                    if (g < C::SEG - 1) {
+                        s_acc[r][0][pair][m] = a.x;
+                        s_acc[r][1][pair][m] = a.y;
                     } else {
-                        lane_chain<WT, K, NTC, NT>(wrow, L, acts, ue_tab, gg);
-                        if (DUAL) lane_chain<WT, K, NTC, NT>(wrow + C::TENSOR_STAGE_BYTES, L, acts, ue_tab, uu);
-                    }
-#pragma unroll
-                    for (int t = 0; t < NTC; ++t) { g[t] = gg[t]; uacc[t] = DUAL ? uu[t] : 0.0f; }
-                };
-                if (NT >= 4 && ntc == 4) run(std::integral_constant<int, (NT >= 4 ? 4 : 1)>{});
-                else if (NT >= 2 && ntc == 2) run(std::integral_constant<int, (NT >= 2 ? 2 : 1)>{});
-                else run(std::integral_constant<int, 1>{});
-                if (row_ok && L == 0) {
-#pragma unroll
-                    for (int t = 0; t < NT; ++t) {
-                        const int r = rows[t];
-                        if (t < ntc && r >= 0) {
-                            float v = __fmul_rn(g[t], sc0);
-                            if (DUAL) v = __fmul_rn(ggml_silu(v), __fmul_rn(uacc[t], sc1));
-                            p.out[(size_t) r * p.n_out + ck.r0 + lr] = v;
-                        }
+                        const float v = hsum_two_lanes(a.x, a.y);
+                        if (m == 0) s_val[pair + C::PAIRS * r] = v;
                     }
                 }
             }
-            t0 += ntc;
-        }
-        if (failed) break;
-        if (NW != 8 && !DUAL && p.comb_out) {
-            // The rows of this chunk are finished for every routed row of this expert.  The CTA that finishes the last of a token's
-            // rows sums them - in slot order, so which CTA that is does not show - and saves the combine its launch.
-            __threadfence();
             __syncthreads();
-            for (int i = 0; i < n_e; ++i) {
-                const int tok = p.perm[row_beg + i] / p.n_ids;
-                if (tid == 0) s_last = atomicAdd(&p.comb_cnt[tok * (p.n_out / 16) + ck.r0 / 16], 1) == p.n_ids - 1;
-                __syncthreads();
-                if (s_last) {
-                    __threadfence();
-                    const float * wr = p.comb_w + (size_t) tok * p.n_ids;
-                    for (int j = tid; j < ck.n; j += NTHREADS) {
-                        const float * y = p.out + (size_t) tok * p.n_ids * p.n_out + ck.r0 + j;
-                        float a = 0.0f;
-                        for (int s0 = 0; s0 < p.n_ids; s0 += 8) {          // eight rows' loads in flight, added in slot order
-                            float v[8], w[8];
+        }
+    } else {
+        float s[2][C::U], sums[2][C::U];
 #pragma unroll
-                            for (int s = 0; s < 8; ++s) {
-                                const bool in = s0 + s < p.n_ids;
-                                v[s] = in ? __ldcg(y + (size_t) (s0 + s) * p.n_out) : 0.0f;
-                                w[s] = in ? wr[s0 + s] : 0.0f;
-                            }
+        for (int u = 0; u < C::U; ++u) {
+            const int sb = seg * C::U + u;
 #pragma unroll
-                            for (int s = 0; s < 8; ++s)
-                                if (s0 + s < p.n_ids) a = s0 + s == 0 ? __fmul_rn(v[s], w[s]) : __fadd_rn(a, __fmul_rn(v[s], w[s]));
-                        }
-                        p.comb_out[(size_t) tok * p.n_out + ck.r0 + j] = a;
-                    }
-                }
-                __syncthreads();
+            for (int r = 0; r < 2; ++r) {
+                const uint8_t * blk = wrow[r] + u * Q3K_BLOCK_BYTES;
+                sums[r][u] = small_int_to_float(q3k_lane_sum(blk, m, acts + sb * 64));
+                s[r][u] = __fmul_rn(act_d[sb], __half2float(*reinterpret_cast<const __half *>(blk + 108)));
             }
         }
-        __syncthreads();  // everyone is done reading this stage
-        if (tid == 0) {
-            Chunk c;
-            if (prod.next(c)) { issue(c, stage); ++issued; }
+#pragma unroll 1
+        for (int g = 0; g < C::SEG; ++g) {
+            if (seg == g) {
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    float acc = g > 0 ? s_acc[r][0][pair][m] : 0.0f;
+#pragma unroll
+                    for (int u = 0; u < C::U; ++u) acc = __fmaf_rn(s[r][u], sums[r][u], acc);
+                    if (g < C::SEG - 1) {
+                        s_acc[r][0][pair][m] = acc;
+                    } else {                                  // hsum_float_8: (a4+a0, a5+a1, a6+a2, a7+a3) -> (r0+r2, r1+r3) -> s0+s1
+                        acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 4));
+                        acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 2));
+                        acc = __fadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 1));
+                        if (m == 0) s_val[pair + C::PAIRS * r] = acc;
+                    }
+                }
+            }
+            __syncthreads();
         }
-        ++ci;
     }
-
-    if (failed && tid == 0) {
-        // bounded drain of copies still in flight before the block (and its shared memory) goes away
-        for (int k = ci; k < issued; ++k) mbar_wait_bounded(&full[k % STAGES], (uint32_t) (k / STAGES) & 1u, 200000000ull);
+    if (tid < n) {
+        float v = __fmul_rn(s_val[tid], sc0);
+        if (DUAL) v = __fmul_rn(ggml_silu(v), __fmul_rn(s_val[C::PAIRS + tid], sc1));
+        p.out[(size_t) r * p.n_out + f0 + tid] = v;
+    }
+    if (!DUAL && p.comb_out) {
+        // The CTA that finishes the last of a token's rows sums them - in slot order, so which CTA that is does not show - and saves the
+        // combine its launch.
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) s_last = atomicAdd(&p.comb_cnt[tok * (p.n_out / 16) + blockIdx.x], 1) == p.n_ids - 1;
+        __syncthreads();
+        if (s_last && tid < n) {
+            __threadfence();
+            const float * wr = p.comb_w + (size_t) tok * p.n_ids;
+            const float * y = p.out + (size_t) tok * p.n_ids * p.n_out + f0 + tid;
+            float a = 0.0f;
+            for (int s0 = 0; s0 < p.n_ids; s0 += 8) {          // eight rows' loads in flight, added in slot order
+                float v[8], w[8];
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    const bool in = s0 + s < p.n_ids;
+                    v[s] = in ? __ldcg(y + (size_t) (s0 + s) * p.n_out) : 0.0f;
+                    w[s] = in ? wr[s0 + s] : 0.0f;
+                }
+#pragma unroll
+                for (int s = 0; s < 8; ++s)
+                    if (s0 + s < p.n_ids) a = s0 + s == 0 ? __fmul_rn(v[s], w[s]) : __fadd_rn(a, __fmul_rn(v[s], w[s]));
+            }
+            p.comb_out[(size_t) tok * p.n_out + f0 + tid] = a;
+        }
     }
 }
 

@@ -19,6 +19,18 @@ struct ActQuant {
     int16_t * bsum;
 };
 
+// eight neighbouring values; src 16-byte aligned
+__device__ __forceinline__ void load8(const float * __restrict__ src, float (&v)[8]) {
+    const float4 a = *reinterpret_cast<const float4 *>(src), b = *reinterpret_cast<const float4 *>(src + 4);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void load8(const __nv_bfloat16 * __restrict__ src, float (&v)[8]) {
+    const uint4 a = *reinterpret_cast<const uint4 *>(src);
+    const uint32_t w[4] = { a.x, a.y, a.z, a.w };
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+}
+
 // ---- K0: router logits (+ optional bias) --------------------------------------------------------
 // One warp per (expert, tile of TT tokens).  Lane l owns the reference's SIMD chain l: AVX2
 // ggml_vec_dot_f32 keeps 4 accumulators x 8 lanes, element i feeding accumulator (i/8)%4 lane i%8,
@@ -33,29 +45,44 @@ template <int TT, typename XT, int CH = TT == 1 ? 32 : 8>
 __device__ __forceinline__ void router_warp(const float * __restrict__ W, const float * __restrict__ bias, const XT * __restrict__ x,
                                             float * __restrict__ logits, int H, int E, int T, int warp, int lane) {
     constexpr bool STAGE = TT == 1 && sizeof(XT) == 2;
-    __shared__ float s_x[STAGE ? ROUTER_ROW : 1];
+    __shared__ __align__(16) float s_x[STAGE ? ROUTER_ROW : 4];
     const int n_tt = (T + TT - 1) / TT;
     const bool row_staged = STAGE && E % 8 == 0 && H <= ROUTER_ROW;
+    const int e = warp % E;
+    const float * w = W + (size_t) e * H;
+    float wv[CH];                              // the first steps' weights are on their way while the row is staged
+#pragma unroll
+    for (int c = 0; c < CH; ++c) wv[c] = STAGE && lane + 32 * c < H ? __ldg(w + lane + 32 * c) : 0.0f;
     if (row_staged) {
         const XT * xr = x + (size_t) min((warp & ~7) / E, T - 1) * H;
-        for (int i = threadIdx.x; i < H; i += blockDim.x) s_x[i] = (float) xr[i];
+        if (H % 8 == 0 && ((uintptr_t) xr & 15) == 0) {
+            for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
+                float v[8];
+                load8(xr + i, v);
+                *reinterpret_cast<float4 *>(s_x + i) = make_float4(v[0], v[1], v[2], v[3]);
+                *reinterpret_cast<float4 *>(s_x + i + 4) = make_float4(v[4], v[5], v[6], v[7]);
+            }
+        } else {
+            for (int i = threadIdx.x; i < H; i += blockDim.x) s_x[i] = (float) xr[i];
+        }
         __syncthreads();
     }
     if (warp >= E * n_tt) return;
-    const int e = warp % E;
     const int t0 = (warp / E) * TT;
     float acc[TT];
 #pragma unroll
     for (int i = 0; i < TT; ++i) acc[i] = 0.0f;
-    const float * w = W + (size_t) e * H;
     // The FMA chain of a lane is sequential by definition of the reference's order, but its loads are not:
     // fetch CH steps of weights and activations at once, then run the chain over them.
     for (int j0 = lane; j0 < H; j0 += 32 * CH) {
-        float wv[CH], xv[TT][CH];
+        float xv[TT][CH];
+        if (!STAGE || j0 != lane) {
+#pragma unroll
+            for (int c = 0; c < CH; ++c) wv[c] = j0 + 32 * c < H ? __ldg(w + j0 + 32 * c) : 0.0f;
+        }
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
             const int j = j0 + 32 * c;
-            wv[c] = j < H ? __ldg(w + j) : 0.0f;
 #pragma unroll
             for (int i = 0; i < TT; ++i) {
                 const int t = min(t0 + i, T - 1);
@@ -172,16 +199,6 @@ __device__ __forceinline__ void quantize_q8_0_block(const XT * __restrict__ src,
 
 // Q8_0 for eight blocks at a time: a lane holds eight neighbouring values, four lanes one block.  src 16-byte aligned.  (A lane per value
 // moved 16 MB of a 4096-token prompt in 39 us.)
-__device__ __forceinline__ void load8(const float * __restrict__ src, float (&v)[8]) {
-    const float4 a = *reinterpret_cast<const float4 *>(src), b = *reinterpret_cast<const float4 *>(src + 4);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
-__device__ __forceinline__ void load8(const __nv_bfloat16 * __restrict__ src, float (&v)[8]) {
-    const uint4 a = *reinterpret_cast<const uint4 *>(src);
-    const uint32_t w[4] = { a.x, a.y, a.z, a.w };
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { v[2 * i] = __uint_as_float(w[i] << 16); v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
-}
 template <typename XT>
 __device__ __forceinline__ void quantize_q8_0_span(const XT * __restrict__ src, int8_t * __restrict__ q, float * __restrict__ d, int lane) {
     float v[8];
@@ -646,16 +663,21 @@ __global__ void __launch_bounds__(1024) group_scan_kernel(Groups g, const int32_
 }
 
 // Small batches: selection for every token and the grouping in ONE single-block launch (one warp per token, looping).
+// grouped = 0: one or two tokens, whose kernels read the ids; only their arrival counters are cleared.
 template <int EPL>
 __global__ void __launch_bounds__(1024) route_select_group_kernel(const float * __restrict__ logits, int E, int K, int T,
                                                                  int32_t * __restrict__ ids, float * __restrict__ weights,
-                                                                 float * __restrict__ probs_out, Groups g, int * err) {
+                                                                 float * __restrict__ probs_out, Groups g, int * err, int grouped) {
     pdl_wait();
     pdl_launch_dependents();
 
     extern __shared__ int sh[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int t = warp; t < T; t += nw) route_select_token<EPL>(logits, E, K, t, lane, ids, weights, probs_out, g.counts, g.pos);
+    for (int t = warp; t < T; t += nw) route_select_token<EPL>(logits, E, K, t, lane, ids, weights, probs_out, grouped ? g.counts : nullptr, g.pos);
+    if (!grouped) {
+        for (int i = threadIdx.x; i < g.n_done; i += blockDim.x) g.done[i] = 0;
+        return;
+    }
     __syncthreads();  // global writes of this block (counts, pos, ids) are visible to the whole block afterwards
     group_scan_body(g, ids, E, T * K, err, sh);
 }
