@@ -83,8 +83,9 @@ struct b200moe_ctx {
     int64_t launches = 0;
     bool timing = false;
     int expert_path = 0;  // b200moe_set_expert_path
-    bool overlap = false; // launch the layer's kernels as programmatic dependents of one another (opt-in)
-    bool overlap_now = false;  // set per call: only the small-batch regime uses it (see layer_overlap)
+    int overlap = -1;     // b200moe_set_launch_overlap: 0 off, 1 on; -1 as it was created (see layer_overlap)
+    bool overlap_now = false;  // set per call: only the small-batch regime uses it
+    bool chained = false;      // the call has launched a kernel, or its first may overlap what is before it
     bool dense_now = false;    // the expert kernels are running a dense product (kernel-timing kind 2)
     struct Timed { cudaEvent_t beg, end; int kind; };
     std::vector<Timed> timed;
@@ -179,20 +180,32 @@ bool gemv_supported(int wtype, int64_t k) {
     return false;
 }
 
-// Programmatic dependent launch (opt-in, b200moe_set_launch_overlap) is applied in the batched-decode regime only (few routed
-// rows per expert), where launch latency and kernel prologues are a visible share of an eagerly launched step.  Measured:
-// +7 % end to end through the host entry point, nothing under CUDA-graph replay (and slower at 8 tokens), which is why it is
-// off by default.  With prefill-sized grids it gains nothing, and the gate/up grouped GEMM with 128-token tiles was measured
+// Programmatic dependent launch of the small kernels and the integer expert kernels, in the batched-decode regime only (few routed rows per
+// expert), where launch latency and kernel prologues are a visible share of a step.  A whole layer call overlaps its launches unless
+// b200moe_set_launch_overlap switched that off; other calls (an expert-parallel step's, which run beside one another) when it was switched
+// on.  With prefill-sized grids it gains nothing, and an early gate/up grouped GEMM with 128-token tiles was measured
 // to return wrong values when a large dependent grid was resident beside it (cause not found by reading; serial launches are
 // correct), so large calls always launch serially, and the tensor-core kernels are never launched with the attribute nor
 // release their dependents early: nothing becomes resident beside a kernel that holds tensor memory.
-void layer_overlap(b200moe_ctx * ctx, int64_t rows, int n_expert) { ctx->overlap_now = rows < (int64_t) 24 * n_expert; }
+// Layers called one by one, us: one token, four layers 123 and 91 (Q3_K; replayed from a graph, NVFP4, 112 and 104), 3 tokens of a latent layer
+// 125 and 105, 8 tokens from host buffers 104 and 100, 17 with a shared expert 153 and 147, 32 (Q3_K) 155 and 141, 64 tokens 120 and 118.
+void layer_overlap(b200moe_ctx * ctx, int64_t rows, int n_expert) {
+    ctx->overlap_now = ctx->overlap > 0 && rows < (int64_t) 24 * n_expert;
+    ctx->chained = true;
+}
+// the same for a call that is one layer: inside a stream capture its first kernel, which may have dependencies on other streams, is launched
+// as usual
+void whole_layer_overlap(b200moe_ctx * ctx, int64_t rows, int n_expert, cudaStream_t st) {
+    ctx->overlap_now = ctx->overlap != 0 && rows < (int64_t) 24 * n_expert;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    ctx->chained = ctx->overlap_now && cudaStreamIsCapturing(st, &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
+}
 
 // Launch with programmatic stream serialisation: the kernel may start while its predecessor in the stream is still running;
-// every kernel of this library calls griddepcontrol.wait before it touches global memory, so only prologues (barrier and
-// table set-up, tensor-memory allocation) and launch latency overlap.  Falls back to an ordinary launch when switched off.
+// every kernel of this library calls griddepcontrol.wait before it touches global memory that another kernel writes, so only prologues
+// (barrier and table set-up) and launch latency overlap.  Falls back to an ordinary launch when switched off.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_k(const b200moe_ctx * ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&... args) {
+cudaError_t launch_k(b200moe_ctx * ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -202,7 +215,8 @@ cudaError_t launch_k(const b200moe_ctx * ctx, void (*kern)(KArgs...), dim3 grid,
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = (ctx->overlap && ctx->overlap_now) ? 1 : 0;
+    cfg.numAttrs = ctx->overlap_now && ctx->chained ? 1 : 0;
+    ctx->chained = true;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
@@ -1318,7 +1332,7 @@ int b200moe_set_expert_path(b200moe_ctx * ctx, int path) {
 
 int b200moe_set_launch_overlap(b200moe_ctx * ctx, int enable) {
     if (!ctx) return B200MOE_ERR_INVALID_ARG;
-    ctx->overlap = enable != 0;
+    ctx->overlap = enable != 0 ? 1 : 0;
     return B200MOE_OK;
 }
 
@@ -1684,9 +1698,9 @@ int b200moe_layer_forward(b200moe_ctx * ctx, const b200moe_layer * l, const void
     if (x_type != TYPE_F32 && x_type != TYPE_BF16) return fail(ctx, B200MOE_ERR_UNSUPPORTED, "activations must be F32 or BF16");
     if (T == 0) return B200MOE_OK;
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert);
     if ((rc = b200moe_reserve(ctx, l, T))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    whole_layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert, st);
     if (x_type == TYPE_F32) return layer_impl<float>(ctx, l, static_cast<const float *>(x), T, out, ob, st);
     return layer_impl<__nv_bfloat16>(ctx, l, static_cast<const __nv_bfloat16 *>(x), T, out, ob, st);
 }
@@ -1700,9 +1714,9 @@ int b200moe_layer_forward_host(b200moe_ctx * ctx, const b200moe_layer * l, const
     if (x_type != TYPE_F32 && x_type != TYPE_BF16) return fail(ctx, B200MOE_ERR_UNSUPPORTED, "activations must be F32 or BF16");
     if (T == 0) return B200MOE_OK;
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert);
     if ((rc = b200moe_reserve(ctx, l, T))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    whole_layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert, st);
     Plan & p = ctx->plan;
     const size_t xbytes = (size_t) T * l->n_embd * (x_type == TYPE_F32 ? 4 : 2);
     CUDA_TRY(ctx, cudaMemcpyAsync(p.xin, x_host, xbytes, cudaMemcpyHostToDevice, st));

@@ -151,13 +151,13 @@ B200MOE_API int  b200moe_synchronize(b200moe_ctx * ctx, void * stream); /* ggml_
  * Paths 6-8 fail with B200MOE_ERR_UNSUPPORTED when the layer is not NVFP4 with n_ff % 128 == 0 and n_in % 256 == 0. */
 B200MOE_API int  b200moe_set_expert_path(b200moe_ctx * ctx, int path);
 
-/* Launch overlap (no counterpart in the reference; comparable to a backend's own stream options).  OFF by default.  When on, calls
- * in the batched-decode regime (fewer than 24 routed rows per expert on average; larger calls always launch serially) launch the
- * small kernels and the integer expert kernels of one layer as programmatic dependents of one another, so a kernel's launch and
+/* Launch overlap (no counterpart in the reference; comparable to a backend's own stream options).  In the batched-decode regime (fewer
+ * than 24 routed rows per expert on average; larger calls always launch serially) the small kernels and the integer expert kernels of one
+ * layer can be launched as programmatic dependents of one another, so a kernel's launch and
  * set-up (barriers, tables) run alongside the tail of its predecessor; every kernel waits for its predecessor to finish before it
  * reads or writes global memory.  The tensor-core kernels are never launched this way and never release their dependents early:
- * nothing becomes resident beside a kernel that holds tensor memory.  Helps eagerly launched steps (+7 % through
- * b200moe_layer_forward_host when measured on the integer path), not CUDA-graph replay. */
+ * nothing becomes resident beside a kernel that holds tensor memory.  As a context is created b200moe_layer_forward and
+ * b200moe_layer_forward_host do so, b200moe_route and b200moe_ffn do not; enable = 1 switches it on for all four, 0 off. */
 B200MOE_API int  b200moe_set_launch_overlap(b200moe_ctx * ctx, int enable);
 /* Per-kernel device timing (reference: DecodeTiming with an injectable clock, include/edge0/timing.h:4-9).
  * When enabled, every expert-matmul launch is bracketed by CUDA events on its stream; b200moe_kernel_times
