@@ -83,7 +83,7 @@ struct b200moe_ctx {
     int64_t launches = 0;
     bool timing = false;
     int expert_path = 0;  // b200moe_set_expert_path
-    int overlap = -1;     // b200moe_set_launch_overlap: 0 off, 1 on; -1 as it was created (see layer_overlap)
+    bool overlap = true;       // b200moe_set_launch_overlap (see layer_overlap)
     bool overlap_now = false;  // set per call: only the small-batch regime uses it
     bool chained = false;      // the call has launched a kernel, or its first may overlap what is before it
     bool dense_now = false;    // the expert kernels are running a dense product (kernel-timing kind 2)
@@ -180,23 +180,23 @@ bool gemv_supported(int wtype, int64_t k) {
     return false;
 }
 
-// Programmatic dependent launch of the small kernels and the integer expert kernels, in the batched-decode regime only (few routed rows per
-// expert), where launch latency and kernel prologues are a visible share of a step.  A whole layer call overlaps its launches unless
-// b200moe_set_launch_overlap switched that off; other calls (an expert-parallel step's, which run beside one another) when it was switched
-// on.  With prefill-sized grids it gains nothing, and an early gate/up grouped GEMM with 128-token tiles was measured
+// Programmatic dependent launch of the kernels other than the tensor-core ones, in the batched-decode regime only (few routed rows per
+// expert), where launch latency and kernel prologues are a visible share of a step, unless b200moe_set_launch_overlap switched it off.
+// With prefill-sized grids it gains nothing, and an early gate/up grouped GEMM with 128-token tiles was measured
 // to return wrong values when a large dependent grid was resident beside it (cause not found by reading; serial launches are
 // correct), so large calls always launch serially, and the tensor-core kernels are never launched with the attribute nor
 // release their dependents early: nothing becomes resident beside a kernel that holds tensor memory.
-// Layers called one by one, us: one token, four layers 123 and 91 (Q3_K; replayed from a graph, NVFP4, 112 and 104), 3 tokens of a latent layer
-// 125 and 105, 8 tokens from host buffers 104 and 100, 17 with a shared expert 153 and 147, 32 (Q3_K) 155 and 141, 64 tokens 120 and 118.
+// Layers called one by one, us without and with: one token, four layers 123 and 90 (Q3_K; replayed from a graph, NVFP4, 112 and 96), 3 tokens
+// of a latent layer 125 and 83, 8 tokens from host buffers 104 and 94, 17 with a shared expert 153 and 127, 32 (Q3_K) 155 and 141, 64
+// tokens 120 and 112; 64 tokens of an expert-parallel latent layer 288 and 266, the indexed product of 40 tokens 72 and 65.
+// Here for calls that a layer is made of: their first kernel, which may have dependencies on other streams, is launched as usual.
 void layer_overlap(b200moe_ctx * ctx, int64_t rows, int n_expert) {
-    ctx->overlap_now = ctx->overlap > 0 && rows < (int64_t) 24 * n_expert;
-    ctx->chained = true;
+    ctx->overlap_now = ctx->overlap && rows < (int64_t) 24 * n_expert;
+    ctx->chained = false;
 }
-// the same for a call that is one layer: inside a stream capture its first kernel, which may have dependencies on other streams, is launched
-// as usual
+// The same for a call that is a whole layer; outside of a stream capture its first kernel overlaps what is before it, too.
 void whole_layer_overlap(b200moe_ctx * ctx, int64_t rows, int n_expert, cudaStream_t st) {
-    ctx->overlap_now = ctx->overlap != 0 && rows < (int64_t) 24 * n_expert;
+    layer_overlap(ctx, rows, n_expert);
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     ctx->chained = ctx->overlap_now && cudaStreamIsCapturing(st, &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
 }
@@ -218,6 +218,12 @@ cudaError_t launch_k(b200moe_ctx * ctx, void (*kern)(KArgs...), dim3 grid, dim3 
     cfg.numAttrs = ctx->overlap_now && ctx->chained ? 1 : 0;
     ctx->chained = true;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+// a copy between two kernels of a call: the one behind it depends on the copy, in a captured graph too
+cudaError_t copy_out(b200moe_ctx * ctx, void * dst, const void * src, size_t bytes, cudaStream_t st) {
+    ctx->chained = false;
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, st);
 }
 
 // Exact re-quantisation behind the tensor-core gate/up GEMM (requant_fixup.cuh): list the values of `hidden` whose int8
@@ -636,8 +642,8 @@ int launch_act_planes(b200moe_ctx * ctx, ActQuant act, const float * src, const 
     // few rows (8 tokens: 8 blocks): the routed rows of a token are shared out over further blocks, which work the digits out again
     const int bx = (act_rows + rows_per_block - 1) / rows_per_block;
     const dim3 blocks((unsigned) bx, (unsigned) std::max(1, std::min(n_ids / ne11, 2 * ctx->sm_count / std::max(1, bx))));
-    if (src) act_planes_kernel<true><<<blocks, 256, 0, st>>>(act, src, src_stride, p.groups.pos, ids, p.groups.offsets, tiles, act_rows, k, n_ids, ne11, n_as, po, emit);
-    else act_planes_kernel<false><<<blocks, 256, 0, st>>>(act, nullptr, 0, p.groups.pos, ids, p.groups.offsets, tiles, act_rows, k, n_ids, ne11, n_as, po, ActQuant{});
+    launch_k(ctx, src ? act_planes_kernel<true> : act_planes_kernel<false>, blocks, dim3(256), 0, st, act, src, src ? src_stride : 0, p.groups.pos, ids, p.groups.offsets,
+             tiles, act_rows, k, n_ids, ne11, n_as, po, src ? emit : ActQuant{});
     return check_launch(ctx, "act_planes");
 }
 
@@ -726,7 +732,7 @@ int launch_logits_any(b200moe_ctx * ctx, const float * w, const float * bias, co
     if (T >= 16 && E >= 8) {   // batches whose rows cannot be staged: 4 experts x 8 tokens per warp
         constexpr int TE = 4, TT = 8;
         const int64_t warps = (int64_t) ((E + TE - 1) / TE) * ((T + TT - 1) / TT);
-        router_logits_tiled_kernel<TE, TT, XT><<<(unsigned) ((warps * 32 + 255) / 256), 256, 0, st>>>(w, bias, x, logits, H, E, T, zero_buf, zero_n);
+        launch_k(ctx, router_logits_tiled_kernel<TE, TT, XT>, dim3((unsigned) ((warps * 32 + 255) / 256)), dim3(256), 0, st, w, bias, x, logits, H, E, T, zero_buf, zero_n);
         return check_launch(ctx, "router_logits");
     }
     if (tt == 1) launch_k(ctx, router_logits_kernel<1, XT>, dim3(lblocks), dim3(256), 0, st, w, bias, x, logits, H, E, T, zero_buf, zero_n);
@@ -902,7 +908,7 @@ int dense_matvec(b200moe_ctx * ctx, int wtype, const void * w, const float * sca
         if ((rc = dense_matvec(ctx, wtype, w, nullptr, x, xq, k, n_out, T, y, st))) return rc;
         if ((rc = dense_matvec(ctx, wtype, w1, nullptr, x, xq, k, n_out, T, y1_tmp, st))) return rc;
         const size_t n = (size_t) T * n_out;
-        silu_mul_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(y, y1_tmp, n);
+        launch_k(ctx, silu_mul_kernel, dim3((unsigned) ((n + 255) / 256)), dim3(256), 0, st, y, y1_tmp, n);
         return check_launch(ctx, "silu_mul");
     }
     // few tokens: the kernel of few rows, which quantises them while it stages them.  NVFP4, 3 tokens, us, as passes
@@ -920,7 +926,7 @@ int dense_matvec(b200moe_ctx * ctx, int wtype, const void * w, const float * sca
     const int gsize = (T + G - 1) / G;
     const int groups = (T + gsize - 1) / gsize;
     p.groups.tile_rows = FP4_RPT_SMALL;
-    dense_groups_kernel<<<(T + 256) / 256, 256, 0, st>>>(p.groups, p.one_group_ids, T, gsize);
+    launch_k(ctx, dense_groups_kernel, dim3((T + 256) / 256), dim3(256), 0, st, p.groups, p.one_group_ids, T, gsize);
     if ((rc = check_launch(ctx, "dense_groups"))) return rc;
     GemvParams g = gemv_params(ctx, w, w1, scale, nullptr, xq, y, n_out, 1, 1, groups);
     g.w_stride = 0;
@@ -932,7 +938,7 @@ int dense_matvec(b200moe_ctx * ctx, int wtype, const void * w, const float * sca
 // rows (digit planes made straight from the fp32 activations).  Not bit-identical to the integer kernel: fp32 accumulation order.
 template <int K>
 int launch_fix_single_t(b200moe_ctx * ctx, const FixSingleParams & fp, cudaStream_t st) {
-    requant_fix_single_kernel<K><<<ctx->sm_count * 8, 256, 0, st>>>(fp);
+    launch_k(ctx, requant_fix_single_kernel<K>, dim3(ctx->sm_count * 8), dim3(256), 0, st, fp);
     return check_launch(ctx, "requant_fix_single");
 }
 
@@ -945,7 +951,7 @@ int dense_matmul_fp4(b200moe_ctx * ctx, const void * w, const float * scale, con
     int rc;
     // a dense product has one group: the large tile once its units fill the GPU
     p.groups.tile_rows = (int64_t) ((T + FP4_RPT_LARGE - 1) / FP4_RPT_LARGE) * (n_out / (w1 ? 128 : 256)) >= ctx->sm_count ? FP4_RPT_LARGE : FP4_RPT_SMALL;
-    dense_groups_kernel<<<(T + 256) / 256, 256, 0, st>>>(p.groups, p.one_group_ids, T, T);
+    launch_k(ctx, dense_groups_kernel, dim3((T + 256) / 256), dim3(256), 0, st, p.groups, p.one_group_ids, T, T);
     if ((rc = check_launch(ctx, "dense_groups"))) return rc;
     // the fix-up recomputes with the quantised activations: have the plane kernel leave them in xq
     if ((rc = launch_act_planes(ctx, ActQuant{}, x, p.one_group_ids, T, k, 1, 1, 1, st, exact_requant ? xq : ActQuant{}))) return rc;
@@ -958,7 +964,7 @@ int dense_matmul_fp4(b200moe_ctx * ctx, const void * w, const float * scale, con
     list.capacity = (int) std::min<size_t>(list_room_bytes / sizeof(int2), (size_t) T * n_out / 4);
     list.overflow = reinterpret_cast<unsigned long long *>(ctx->d_err + 2);
     const int64_t warps = (int64_t) T * (n_out / 128);
-    requant_mark_kernel<<<(unsigned) ((warps * 32 + 255) / 256), 256, 0, st>>>(y, p.groups.perm, p.groups.meta, T, n_out, FIX_STEP_MARGIN_FP4, FIX_REL_MARGIN_FP4, list);
+    launch_k(ctx, requant_mark_kernel, dim3((unsigned) ((warps * 32 + 255) / 256)), dim3(256), 0, st, y, p.groups.perm, p.groups.meta, T, n_out, FIX_STEP_MARGIN_FP4, FIX_REL_MARGIN_FP4, list);
     if ((rc = check_launch(ctx, "requant_mark"))) return rc;
     FixSingleParams fs{ static_cast<const uint8_t *>(w), scale, xq, n_out, y, list, FIX_REL_MARGIN_FP4 };
     switch (k) {
@@ -1006,7 +1012,7 @@ int route_impl(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T, 
     float * probs = (ob && ob->ffn_moe_probs) ? ob->ffn_moe_probs : nullptr;
     if ((rc = launch_select(ctx, l, T, ids, wts, probs, count, st))) return rc;
     if (ob && ob->ffn_moe_logits)
-        CUDA_TRY(ctx, cudaMemcpyAsync(ob->ffn_moe_logits, p.logits, sizeof(float) * (size_t) T * l->n_expert, cudaMemcpyDeviceToDevice, st));
+        CUDA_TRY(ctx, copy_out(ctx, ob->ffn_moe_logits, p.logits, sizeof(float) * (size_t) T * l->n_expert, st));
     return B200MOE_OK;
 }
 
@@ -1165,9 +1171,9 @@ int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const 
         if ((rc = check_launch(ctx, "combine"))) return rc;
     }
     if (ob && ob->ffn_moe_hidden)
-        CUDA_TRY(ctx, cudaMemcpyAsync(ob->ffn_moe_hidden, p.hid, sizeof(float) * (size_t) rows * l->n_ff, cudaMemcpyDeviceToDevice, st));
+        CUDA_TRY(ctx, copy_out(ctx, ob->ffn_moe_hidden, p.hid, sizeof(float) * (size_t) rows * l->n_ff, st));
     if (ob && ob->ffn_moe_down)
-        CUDA_TRY(ctx, cudaMemcpyAsync(ob->ffn_moe_down, y, sizeof(float) * (size_t) rows * n_in, cudaMemcpyDeviceToDevice, st));
+        CUDA_TRY(ctx, copy_out(ctx, ob->ffn_moe_down, y, sizeof(float) * (size_t) rows * n_in, st));
     (void) ids;
     return B200MOE_OK;
 }
@@ -1189,7 +1195,7 @@ int shared_expert_impl(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x,
         xf32 = reinterpret_cast<const float *>(x);
     } else {
         const size_t n = (size_t) T * H;
-        bf16_to_f32_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16 *>(x), p.xf, n);
+        launch_k(ctx, bf16_to_f32_kernel, dim3((unsigned) ((n + 255) / 256)), dim3(256), 0, st, reinterpret_cast<const __nv_bfloat16 *>(x), p.xf, n);
         if ((rc = check_launch(ctx, "bf16_to_f32"))) return rc;
         xf32 = p.xf;
     }
@@ -1198,7 +1204,7 @@ int shared_expert_impl(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x,
     if ((rc = dense_matvec(ctx, l->wtype, l->gate_shexp, nullptr, xf32, p.xq, H, Is, T, p.sh_a, st, false, l->up_shexp, p.sh_b))) return rc;
     if ((rc = dense_matvec(ctx, l->wtype, l->down_shexp, nullptr, p.sh_a, p.shq, Is, H, T, p.sh_out, st))) return rc;
     dim3 grid((H + 255) / 256, T);
-    shexp_add_kernel<<<grid, 256, 0, st>>>(out, p.sh_out, p.sh_gate, H, T, ob ? ob->ffn_shexp_gated : nullptr);
+    launch_k(ctx, shexp_add_kernel, grid, dim3(256), 0, st, out, p.sh_out, p.sh_gate, H, T, ob ? ob->ffn_shexp_gated : nullptr);
     return check_launch(ctx, "shexp_add");
 }
 
@@ -1214,7 +1220,7 @@ int layer_impl(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T, 
             xf32 = reinterpret_cast<const float *>(x);
         } else {
             const size_t n = (size_t) T * l->n_embd;
-            bf16_to_f32_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16 *>(x), p.xf, n);
+            launch_k(ctx, bf16_to_f32_kernel, dim3((unsigned) ((n + 255) / 256)), dim3(256), 0, st, reinterpret_cast<const __nv_bfloat16 *>(x), p.xf, n);
             if ((rc = check_launch(ctx, "bf16_to_f32"))) return rc;
             xf32 = p.xf;
         }
@@ -1231,11 +1237,11 @@ int layer_impl(b200moe_ctx * ctx, const b200moe_layer * l, const XT * x, int T, 
             if ((rc = launch_group(ctx, p.ids, l->n_expert, T * k, st))) return rc;
         }
         if (ob && ob->ffn_moe_logits)
-            CUDA_TRY(ctx, cudaMemcpyAsync(ob->ffn_moe_logits, p.logits, sizeof(float) * (size_t) T * l->n_expert, cudaMemcpyDeviceToDevice, st));
+            CUDA_TRY(ctx, copy_out(ctx, ob->ffn_moe_logits, p.logits, sizeof(float) * (size_t) T * l->n_expert, st));
     }
-    if (ob && ob->ffn_moe_topk) CUDA_TRY(ctx, cudaMemcpyAsync(ob->ffn_moe_topk, p.ids, sizeof(int32_t) * (size_t) T * k, cudaMemcpyDeviceToDevice, st));
+    if (ob && ob->ffn_moe_topk) CUDA_TRY(ctx, copy_out(ctx, ob->ffn_moe_topk, p.ids, sizeof(int32_t) * (size_t) T * k, st));
     if (ob && ob->ffn_moe_weights_norm)
-        CUDA_TRY(ctx, cudaMemcpyAsync(ob->ffn_moe_weights_norm, p.wts, sizeof(float) * (size_t) T * k, cudaMemcpyDeviceToDevice, st));
+        CUDA_TRY(ctx, copy_out(ctx, ob->ffn_moe_weights_norm, p.wts, sizeof(float) * (size_t) T * k, st));
 
     if (!l->n_latent) {
         rc = experts_impl(ctx, l, p.xq, p.ids, p.wts, T, out, ob, st);
@@ -1332,7 +1338,7 @@ int b200moe_set_expert_path(b200moe_ctx * ctx, int path) {
 
 int b200moe_set_launch_overlap(b200moe_ctx * ctx, int enable) {
     if (!ctx) return B200MOE_ERR_INVALID_ARG;
-    ctx->overlap = enable != 0 ? 1 : 0;
+    ctx->overlap = enable != 0;
     return B200MOE_OK;
 }
 
@@ -1551,7 +1557,6 @@ int b200moe_route(b200moe_ctx * ctx, const b200moe_layer * l, const void * x, in
 
 int b200moe_mul_mat_id(b200moe_ctx * ctx, int wtype, const void * as, int64_t ne00, int64_t ne01, int64_t n_as, const float * b, int64_t ne11,
                        const int32_t * ids, int64_t n_ids, int64_t ids_nb1, int64_t T, float * dst, void * stream) {
-    if (ctx) ctx->overlap_now = false;
     if (!ctx) return B200MOE_ERR_INVALID_ARG;
     if (T == 0) return B200MOE_OK;
     if (!as || !b || !ids || !dst) return fail(ctx, B200MOE_ERR_INVALID_ARG, "null pointer");
@@ -1571,15 +1576,18 @@ int b200moe_mul_mat_id(b200moe_ctx * ctx, int wtype, const void * as, int64_t ne
     if (rc) return rc;
     Plan & p = ctx->plan;
     const int rows = (int) (T * n_ids);
+    const bool few = few_rows(wtype, rows, (int) n_as);
+    layer_overlap(ctx, rows, (int) n_as);
+    if (!few) CUDA_TRY(ctx, cudaMemsetAsync(p.groups.counts, 0, sizeof(int) * n_as, st));
     // activations: T*ne11 rows of ne00; plan.hq holds T*k rows of width n_ff (= ne00 here), ne11 <= k
     if ((rc = launch_quantize<float>(ctx, b, ne00, p.hq, (int) (T * ne11), (int) ne00, wtype, st))) return rc;
     GemvParams g = gemv_params(ctx, as, nullptr, nullptr, nullptr, p.hq, dst, (int) ne01, (int) n_ids, (int) ne11, (int) n_as);
-    if (few_rows(wtype, rows, (int) n_as)) {   // read the ids as they are and need no groups
+    if (few) {   // read the ids as they are and need no groups
         g.ids = ids;
         g.ids_stride = ids_nb1 / 4;
     } else {
-        CUDA_TRY(ctx, cudaMemsetAsync(p.groups.counts, 0, sizeof(int) * n_as, st));
-        count_ids_kernel<<<(rows + 255) / 256, 256, 0, st>>>(ids, ids_nb1 / 4, (int) n_ids, (int) T, (int) n_as, p.ids, p.groups.counts, p.groups.pos, ctx->d_err);
+        launch_k(ctx, count_ids_kernel, dim3((unsigned) ((rows + 255) / 256)), dim3(256), 0, st, ids, ids_nb1 / 4, (int) n_ids, (int) T, (int) n_as, p.ids, p.groups.counts,
+                 p.groups.pos, ctx->d_err, 0);
         if ((rc = check_launch(ctx, "count_ids"))) return rc;
         if ((rc = launch_group(ctx, p.ids, (int) n_as, rows, st))) return rc;
     }
@@ -1588,13 +1596,13 @@ int b200moe_mul_mat_id(b200moe_ctx * ctx, int wtype, const void * as, int64_t ne
 
 int b200moe_mul_mat(b200moe_ctx * ctx, int wtype, const void * w, int64_t ne00, int64_t ne01, const float * x, int64_t T, const float * scale,
                     float * dst, void * stream) {
-    if (ctx) ctx->overlap_now = false;
     if (!ctx) return B200MOE_ERR_INVALID_ARG;
     if (T == 0) return B200MOE_OK;
     if (!w || !x || !dst || ne00 <= 0 || ne01 <= 0 || T < 0) return fail(ctx, B200MOE_ERR_INVALID_ARG, "null pointer or non-positive size");
     if ((uintptr_t) w & 15) return fail(ctx, B200MOE_ERR_INVALID_ARG, "weight tensor must be 16-byte aligned");
     if (!gemv_supported(wtype, ne00) || ne01 % 8) return fail(ctx, B200MOE_ERR_UNSUPPORTED, "no kernel for type %d, K=%lld", wtype, (long long) ne00);
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
+    layer_overlap(ctx, T, 1);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int rc = ensure_plan(ctx, (int) ne00, (int) ne00, 8, 1, (int) ne00, wtype, (int) T);
     if (rc) return rc;
@@ -1611,14 +1619,14 @@ int b200moe_latent_down(b200moe_ctx * ctx, const b200moe_layer * l, const void *
     if (x_type != TYPE_F32 && x_type != TYPE_BF16) return fail(ctx, B200MOE_ERR_UNSUPPORTED, "activations must be F32 or BF16");
     if ((uintptr_t) l->lat_down & 15) return fail(ctx, B200MOE_ERR_INVALID_ARG, "quantised tensors must be 16-byte aligned");
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    ctx->overlap_now = false;
+    layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert);
     if ((rc = ensure_plan(ctx, l->n_embd, l->n_latent, l->n_expert, l->n_expert_used, l->n_ff, l->wtype, T))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     Plan & p = ctx->plan;
     const float * xf32 = static_cast<const float *>(x);
     if (x_type == TYPE_BF16) {
         const size_t n = (size_t) T * l->n_embd;
-        bf16_to_f32_kernel<<<(unsigned) ((n + 255) / 256), 256, 0, st>>>(static_cast<const __nv_bfloat16 *>(x), p.xf, n);
+        launch_k(ctx, bf16_to_f32_kernel, dim3((unsigned) ((n + 255) / 256)), dim3(256), 0, st, static_cast<const __nv_bfloat16 *>(x), p.xf, n);
         if ((rc = check_launch(ctx, "bf16_to_f32"))) return rc;
         xf32 = p.xf;
     }
@@ -1634,7 +1642,7 @@ int b200moe_latent_up(b200moe_ctx * ctx, const b200moe_layer * l, const float * 
     if (!m || !out || T < 0) return fail(ctx, B200MOE_ERR_INVALID_ARG, "null pointer or negative token count");
     if ((uintptr_t) l->lat_up & 15) return fail(ctx, B200MOE_ERR_INVALID_ARG, "quantised tensors must be 16-byte aligned");
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    ctx->overlap_now = false;
+    layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert);
     if ((rc = ensure_plan(ctx, l->n_embd, l->n_latent, l->n_expert, l->n_expert_used, l->n_ff, l->wtype, T))) return rc;
     return dense_matvec(ctx, l->wtype, l->lat_up, l->lat_up_scale, m, ctx->plan.moq, l->n_latent, l->n_embd, T, out, static_cast<cudaStream_t>(stream));
 }
@@ -1678,7 +1686,7 @@ int b200moe_ffn(b200moe_ctx * ctx, const b200moe_layer * l, const void * x, int 
     Plan & p = ctx->plan;
     const int n_in = l->n_latent ? l->n_latent : l->n_embd, k = l->n_expert_used;
     CUDA_TRY(ctx, cudaMemsetAsync(p.groups.counts, 0, sizeof(int) * l->n_expert, st));
-    count_ids_kernel<<<(T * k + 255) / 256, 256, 0, st>>>(ids, k, k, T, l->n_expert, p.ids, p.groups.counts, p.groups.pos, ctx->d_err);
+    launch_k(ctx, count_ids_kernel, dim3((T * k + 255) / 256), dim3(256), 0, st, ids, k, k, T, l->n_expert, p.ids, p.groups.counts, p.groups.pos, ctx->d_err, 0);
     if ((rc = check_launch(ctx, "count_ids"))) return rc;
     if ((rc = launch_group(ctx, p.ids, l->n_expert, T * k, st))) return rc;
     if (x_type == TYPE_F32) rc = launch_quantize<float>(ctx, static_cast<const float *>(x), n_in, p.xq, T, n_in, l->wtype, st);
@@ -1767,7 +1775,7 @@ int b200moe_ep_expert_rows_expected(b200moe_ctx * ctx, const b200moe_layer * l, 
     if (expected_rows < 0 || expected_rows > n_slots) return fail(ctx, B200MOE_ERR_INVALID_ARG, "expected rows outside 0 .. slots");
     if ((uintptr_t) slots & 15) return fail(ctx, B200MOE_ERR_INVALID_ARG, "slots must be 16-byte aligned");
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    ctx->overlap_now = false;
+    layer_overlap(ctx, n_slots, l->n_expert);
     const int n_in = l->n_embd, R = (int) n_slots, slot_words = n_in + EP_SLOT_EXTRA;
     // one slot = one routed row of a one-slot layer
     if ((rc = ensure_plan(ctx, l->n_embd, n_in, l->n_expert, 1, l->n_ff, l->wtype, R))) return rc;
@@ -1776,7 +1784,7 @@ int b200moe_ep_expert_rows_expected(b200moe_ctx * ctx, const b200moe_layer * l, 
     const float * rows = static_cast<const float *>(slots);
     const int32_t * ids = reinterpret_cast<const int32_t *>(rows + n_in);
     CUDA_TRY(ctx, cudaMemsetAsync(p.groups.counts, 0, sizeof(int) * l->n_expert, st));
-    count_ids_kernel<<<(R + 255) / 256, 256, 0, st>>>(ids, slot_words, 1, R, l->n_expert, p.ids, p.groups.counts, p.groups.pos, ctx->d_err, 1);
+    launch_k(ctx, count_ids_kernel, dim3((R + 255) / 256), dim3(256), 0, st, ids, slot_words, 1, R, l->n_expert, p.ids, p.groups.counts, p.groups.pos, ctx->d_err, 1);
     if ((rc = check_launch(ctx, "count_ids"))) return rc;
     if ((rc = launch_group(ctx, p.ids, l->n_expert, R, st, true, expected_rows))) return rc;
     // the slots' rows are quantised by whichever engine runs gate/up (empty slots hold garbage nobody reads)

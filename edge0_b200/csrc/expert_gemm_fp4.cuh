@@ -153,6 +153,8 @@ __global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const flo
     const int dst_step = gridDim.y, dst0 = blockIdx.y;    // few rows: the blocks of a column store every dst_step-th routed row each
     for (int i = tid; i < 729; i += 256) s_digits[i] = digit_codes(i);
     if (tid < MAX_ROWS) s_E[tid] = -1000;
+    pdl_wait();                              // the table is made while the previous kernel ends
+    pdl_launch_dependents();
     const bool live = lrow < rpb && arow < act_rows;   // threads beyond the block's last whole row idle (K = 768)
     for (int j = g; live && j < n_dst; j += tpr) {
         const int r = (arow / ne11) * n_ids + arow % ne11 + ne11 * j;

@@ -240,6 +240,8 @@ __global__ void __launch_bounds__(256) requant_fix_single_kernel(const FixSingle
     __shared__ float ue_tab[256];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     ue_tab[tid] = ue4m3_half_to_f32(tid);
+    pdl_wait();
+    pdl_launch_dependents();
     __syncthreads();
     const int n = min(*p.list.count, p.list.capacity);
     for (int i = blockIdx.x * 8 + warp; i < n; i += gridDim.x * 8) {

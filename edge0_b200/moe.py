@@ -199,7 +199,7 @@ class Context:
         self.check(self.lib.b200moe_set_expert_path(self.handle, path))
 
     def set_launch_overlap(self, enable: bool) -> None:
-        """Programmatic dependent launches between the kernels of a layer (default: in forward and forward_host); see b200moe_set_launch_overlap."""
+        """Programmatic dependent launches between the kernels of a layer (default on); see b200moe_set_launch_overlap."""
         self.check(self.lib.b200moe_set_launch_overlap(self.handle, int(bool(enable))))
 
     def enable_kernel_timing(self, on: bool = True):

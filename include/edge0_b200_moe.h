@@ -156,8 +156,8 @@ B200MOE_API int  b200moe_set_expert_path(b200moe_ctx * ctx, int path);
  * layer can be launched as programmatic dependents of one another, so a kernel's launch and
  * set-up (barriers, tables) run alongside the tail of its predecessor; every kernel waits for its predecessor to finish before it
  * reads or writes global memory.  The tensor-core kernels are never launched this way and never release their dependents early:
- * nothing becomes resident beside a kernel that holds tensor memory.  As a context is created b200moe_layer_forward and
- * b200moe_layer_forward_host do so, b200moe_route and b200moe_ffn do not; enable = 1 switches it on for all four, 0 off. */
+ * nothing becomes resident beside a kernel that holds tensor memory.  On as a context is created, in the layer calls and in those
+ * a layer is made of; enable = 0 switches it off, 1 on again. */
 B200MOE_API int  b200moe_set_launch_overlap(b200moe_ctx * ctx, int enable);
 /* Per-kernel device timing (reference: DecodeTiming with an injectable clock, include/edge0/timing.h:4-9).
  * When enabled, every expert-matmul launch is bracketed by CUDA events on its stream; b200moe_kernel_times
