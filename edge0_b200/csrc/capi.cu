@@ -840,9 +840,8 @@ GemvParams gemv_params(b200moe_ctx * ctx, const void * w0, const void * w1, cons
     return g;
 }
 
-// activation rows per pass of the integer kernel: 4, 1 when experts see about one row each, -(rows) selects the
-// one-or-two-token kernel
-int tokens_per_pass(int rows, int n_as) { return rows <= 16 ? -rows : rows <= n_as ? (rows <= 32 ? 1 : 4) : 4; }
+// up to 16 rows, negated: they go to the kernel of few rows, one by one; 0: to the kernels of grouped rows
+int few_or_grouped(int rows) { return rows <= 16 ? -rows : 0; }
 
 __global__ void bf16_to_f32_kernel(const __nv_bfloat16 * src, float * dst, size_t n) {
     pdl_wait();
@@ -930,8 +929,23 @@ int dense_matvec(b200moe_ctx * ctx, int wtype, const void * w, const float * sca
     if ((rc = check_launch(ctx, "dense_groups"))) return rc;
     GemvParams g = gemv_params(ctx, w, w1, scale, nullptr, xq, y, n_out, 1, 1, groups);
     g.w_stride = 0;
-    if (w1) return launch_integer<true>(ctx, wtype, k, g, T, groups, 4, st);
-    return launch_integer<false>(ctx, wtype, k, g, T, groups, 4, st);
+    if (w1) return launch_integer<true>(ctx, wtype, k, g, T, groups, 0, st);
+    return launch_integer<false>(ctx, wtype, k, g, T, groups, 0, st);
+}
+
+// The values of h [rows][n] whose rounding is in doubt, onto `list` (requant_mark_kernel).  MARK_ROWS rows to a warp where that still
+// leaves half of the warps the GPU can hold, else one: 4096 tokens (32768 x 768 values, 49152 warps of four rows) 69 us with one row
+// and 37 with four, 777 tokens (9324 warps) 15 and 10; below that the whole list is one wave of blocks, which several rows only make longer.
+constexpr int MARK_ROWS = 4;
+constexpr int64_t MARK_FULL_WARPS = 148 * 32;
+int launch_mark(b200moe_ctx * ctx, const float * h, int rows, int n, float step_margin, float rel_margin, const FixList & list, cudaStream_t st) {
+    const int * perm = ctx->plan.groups.perm, * meta = ctx->plan.groups.meta;
+    const int64_t chunks = n / 128, several = (rows + MARK_ROWS - 1) / MARK_ROWS * chunks;
+    if (several >= MARK_FULL_WARPS)
+        launch_k(ctx, requant_mark_kernel<MARK_ROWS>, dim3((unsigned) ((several + 7) / 8)), dim3(256), 0, st, h, perm, meta, rows, n, step_margin, rel_margin, list);
+    else
+        launch_k(ctx, requant_mark_kernel<1>, dim3((unsigned) ((rows * chunks + 7) / 8)), dim3(256), 0, st, h, perm, meta, rows, n, step_margin, rel_margin, list);
+    return check_launch(ctx, "requant_mark");
 }
 
 // The same product on the FP4 tensor-core kernel: the matrix is the single "expert" of a one-group routing, the tokens its routed
@@ -963,9 +977,7 @@ int dense_matmul_fp4(b200moe_ctx * ctx, const void * w, const float * scale, con
     list.count = p.groups.meta + 2;
     list.capacity = (int) std::min<size_t>(list_room_bytes / sizeof(int2), (size_t) T * n_out / 4);
     list.overflow = reinterpret_cast<unsigned long long *>(ctx->d_err + 2);
-    const int64_t warps = (int64_t) T * (n_out / 128);
-    launch_k(ctx, requant_mark_kernel, dim3((unsigned) ((warps * 32 + 255) / 256)), dim3(256), 0, st, y, p.groups.perm, p.groups.meta, T, n_out, FIX_STEP_MARGIN_FP4, FIX_REL_MARGIN_FP4, list);
-    if ((rc = check_launch(ctx, "requant_mark"))) return rc;
+    if ((rc = launch_mark(ctx, y, T, n_out, FIX_STEP_MARGIN_FP4, FIX_REL_MARGIN_FP4, list, st))) return rc;
     FixSingleParams fs{ static_cast<const uint8_t *>(w), scale, xq, n_out, y, list, FIX_REL_MARGIN_FP4 };
     switch (k) {
         case 256: return launch_fix_single_t<256>(ctx, fs, st);
@@ -1038,10 +1050,7 @@ int launch_requant_fixup(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq
     more.count = p.groups.meta + 3;
     more.capacity = (int) (room - room * 3 / 4);
     more.overflow = list.overflow;
-    const int64_t warps = (int64_t) rows * (l->n_ff / 128);
-    launch_k(ctx, requant_mark_kernel, dim3((unsigned) ((warps * 32 + 255) / 256)), dim3(256), 0, st, (const float *) p.hid,
-             (const int *) p.groups.perm, (const int *) p.groups.meta, rows, l->n_ff, after_fp4 ? FIX_STEP_MARGIN_FP4 : FIX_STEP_MARGIN, after_fp4 ? FIX_REL_MARGIN_FP4 : FIX_REL_MARGIN, list);
-    int rc = check_launch(ctx, "requant_mark");
+    int rc = launch_mark(ctx, p.hid, rows, l->n_ff, after_fp4 ? FIX_STEP_MARGIN_FP4 : FIX_STEP_MARGIN, after_fp4 ? FIX_REL_MARGIN_FP4 : FIX_REL_MARGIN, list, st);
     if (rc) return rc;
     FixParams fp{};
     fp.w0 = static_cast<const uint8_t *>(l->gate); fp.w1 = static_cast<const uint8_t *>(l->up);
@@ -1078,7 +1087,7 @@ int experts_impl(b200moe_ctx * ctx, const b200moe_layer * l, ActQuant xq, const 
     const int n_in = l->n_latent ? l->n_latent : l->n_embd;
     const int k = l->n_expert_used, rows = T * k;
     const int64_t likely_rows = expected_rows >= 0 ? expected_rows : rows;
-    const int nt = tokens_per_pass(rows, l->n_expert);
+    const int nt = few_or_grouped(rows);
     int rc;
     // Which engine runs which matmul (b200moe_set_expert_path documents the paths).
     //   integer kernels   reproduce the reference's fp32 summation order: bit-identical to the CPU path; cost grows with the rows an
@@ -1591,7 +1600,7 @@ int b200moe_mul_mat_id(b200moe_ctx * ctx, int wtype, const void * as, int64_t ne
         if ((rc = check_launch(ctx, "count_ids"))) return rc;
         if ((rc = launch_group(ctx, p.ids, (int) n_as, rows, st))) return rc;
     }
-    return launch_integer<false>(ctx, wtype, (int) ne00, g, rows, (int) n_as, tokens_per_pass(rows, (int) n_as), st);
+    return launch_integer<false>(ctx, wtype, (int) ne00, g, rows, (int) n_as, few_or_grouped(rows), st);
 }
 
 int b200moe_mul_mat(b200moe_ctx * ctx, int wtype, const void * w, int64_t ne00, int64_t ne01, const float * x, int64_t T, const float * scale,

@@ -1,5 +1,5 @@
 // Grouped Q3_K expert matmul on the int8 matrix instruction, bit-identical to the reference: every call but one or two tokens' (those take
-// expert_gemv_kernel's four-warp form).
+// expert_few_rows_kernel).
 //
 // Why a matrix instruction can keep the reference's bits: ggml_vec_dot_q3_K_q8_K (ggml-cpu/arch/x86/quants.c:1766-1880) sums
 // INTEGERS over a whole super-block in every one of its eight SIMD lanes - lane L collects scale * code * activation over byte

@@ -41,48 +41,54 @@ __device__ __forceinline__ bool near_half_rounding_boundary(float x, float rel) 
     return fabsf(x - 0.5f * (lo + hi)) <= rel * x;
 }
 
-// One warp per (routed row, 128 features): a lane holds four neighbouring values, eight lanes one block of 32.
+// One warp per (ROWS sorted routed rows, 128 features): a lane holds four neighbouring values of each, eight lanes one block of 32.
 //   step_margin : distance from a rounding boundary, in quantisation steps, below which a value is recomputed
 //   rel_margin  : relative distance from the block maximum below which a value counts as a candidate for it; the same
 //                 relative uncertainty of the scale widens the step margin of large values
-//   perm        : routed rows sorted by expert.  Warps walk (feature chunk, sorted row) with the row fastest, so values that need
+//   perm        : routed rows sorted by expert.  Warps walk (feature chunk, sorted rows) with the rows fastest, so values that need
 //                 the same weight rows (same expert, same features) are listed next to each other and the recomputation
 //                 finds those rows in cache instead of fetching 2 x row_bytes from HBM per value.
 //   meta[1]     : number of routed rows that are in a group (fewer than `rows` when an exchange left slots empty)
 // n_ff must be a multiple of 128 and the rows 16-byte aligned.
+// What bounds it is the chain of a block (row number, values, list counter, list), not its bytes: with several rows to a warp their
+// loads are in flight together and a block's counter is asked for once for all of them (launch_mark has the line).
+template <int ROWS>
 __global__ void __launch_bounds__(256) requant_mark_kernel(const float * __restrict__ hid, const int * __restrict__ perm, const int * __restrict__ meta,
                                                           int rows, int n_ff, float step_margin, float rel_margin, FixList list) {
     pdl_wait();
     pdl_launch_dependents();
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    const int chunks = n_ff / 128;
-    const bool live = warp < rows * chunks && warp % rows < meta[1];     // the whole block meets at the barriers below
-    const int c = live ? warp / rows : 0, r = live ? perm[warp % rows] : 0;
+    const int steps = (rows + ROWS - 1) / ROWS, c = warp / steps, row0 = (warp - c * steps) * ROWS;
+    const int n_live = c < n_ff / 128 ? min(ROWS, meta[1] - row0) : 0;   // <= 0: none; the whole block meets at the barriers below
     const int f0 = c * 128 + lane * 4;
-    const float4 v4 = live ? *reinterpret_cast<const float4 *>(hid + (size_t) r * n_ff + f0) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    const float a[4] = { fabsf(v4.x), fabsf(v4.y), fabsf(v4.z), fabsf(v4.w) };
-    float amax = fmaxf(fmaxf(a[0], a[1]), fmaxf(a[2], a[3]));
+    int r[ROWS];
+    float4 v4[ROWS];
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));   // the block's eight lanes
-    bool risky[4] = { false, false, false, false };
-    if (amax > 0.0f) {
-        const float id = 127.0f / amax;
+    for (int i = 0; i < ROWS; ++i) r[i] = i < n_live ? perm[row0 + i] : 0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float t = a[j] * id;                                // 0 .. 127
-            const float dist = fabsf((t - floorf(t)) - 0.5f);         // distance from the rounding boundary, in steps
-            risky[j] = dist < step_margin + t * rel_margin;
+    for (int i = 0; i < ROWS; ++i)
+        v4[i] = i < n_live ? *reinterpret_cast<const float4 *>(hid + (size_t) r[i] * n_ff + f0) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    uint32_t risky = 0;          // bit i * 4 + j: value j of row i
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        const float a[4] = { fabsf(v4[i].x), fabsf(v4[i].y), fabsf(v4[i].z), fabsf(v4[i].w) };
+        float amax = fmaxf(fmaxf(a[0], a[1]), fmaxf(a[2], a[3]));
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));   // the block's eight lanes
+        if (amax > 0.0f) {
+            const float id = 127.0f / amax;
+            // the maximum's candidates: when the block scale half(amax / 127) is in doubt (near an fp16 rounding boundary).  (A
+            // recomputed value whose rounding hangs on the maximum's last bits is dealt with by the fix kernel.)
+            const bool need_max = near_half_rounding_boundary(amax / 127.0f, 2.0f * rel_margin);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float t = a[j] * id;                                // 0 .. 127
+                const float dist = fabsf((t - floorf(t)) - 0.5f);         // distance from the rounding boundary, in steps
+                if (dist < step_margin + t * rel_margin || (need_max && a[j] >= amax * (1.0f - rel_margin))) risky |= 1u << (i * 4 + j);
+            }
         }
     }
-    // the maximum's candidates: when the block scale half(amax / 127) is in doubt (near an fp16 rounding boundary).  (A recomputed
-    // value whose rounding hangs on the maximum's last bits is dealt with by the fix kernel.)
-    const bool need_max = amax > 0.0f && near_half_rounding_boundary(amax / 127.0f, 2.0f * rel_margin);
-    int n_mine = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        risky[j] = risky[j] || (need_max && amax > 0.0f && a[j] >= amax * (1.0f - rel_margin));
-        n_mine += risky[j] ? 1 : 0;
-    }
+    const int n_mine = __popc(risky);
     int incl = n_mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -110,11 +116,14 @@ __global__ void __launch_bounds__(256) requant_mark_kernel(const float * __restr
     int slot = s_base + incl - n_mine;
     for (int w = 0; w < wib; ++w) slot += s_total[w];
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-        if (risky[j]) {
-            if (slot < list.capacity) list.items[slot] = make_int2(r, f0 + j);
-            ++slot;
-        }
+    for (int i = 0; i < ROWS; ++i) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (risky >> (i * 4 + j) & 1) {
+                if (slot < list.capacity) list.items[slot] = make_int2(r[i], f0 + j);
+                ++slot;
+            }
+    }
 }
 
 struct FixParams {
