@@ -434,7 +434,7 @@ int launch_gemv_k(b200moe_ctx * ctx, const GemvParams & p, int nt, cudaStream_t 
     if constexpr (DUAL && K > 2048) {
         return fail(ctx, B200MOE_ERR_UNSUPPORTED, "fused gate/up kernel is not built for K=%d", K);
     } else {
-        if (nt <= 0) return launch_few_rows<WT, K, DUAL>(ctx, p, -nt, st);    // nt = -(routed rows)
+        if (nt < 0) return launch_few_rows<WT, K, DUAL>(ctx, p, -nt, st);    // few_or_grouped
         if constexpr (WT == TYPE_NVFP4) {
             return launch_gemv_nvfp4<K, DUAL>(ctx, p, st);
         } else {
