@@ -122,8 +122,8 @@ B200MOE_API int  b200moe_synchronize(b200moe_ctx * ctx, void * stream); /* ggml_
 
 /* Which kernels run the expert matmuls (reference: model option switches such as `routing` / `experts`,
  * edge0-infer/docs/configuration.md:62-72; plain struct-style option, no environment variables).  Three engines exist:
- *   integer   kernels that follow the reference's fp32 summation order: bit-identical to the CPU path (dp4a; Q3_K from 12 routed rows
- *             per expert on average on the int8 matrix instruction)
+ *   integer   kernels that follow the reference's fp32 summation order: bit-identical to the CPU path (dp4a; Q3_K beyond 16 routed
+ *             rows on the int8 matrix instruction)
  *   FP4       tcgen05 kind::mxf4nvf4 (block-scaled FP4 MMA, UE4M3 scale per 16): NVFP4 rows exactly as they lie in memory,
  *             activations as exact digit planes of the reference's int8 grid; differs from the integer engine only by fp32
  *             accumulation (~5e-6 of RMS on `hidden`); one pass over an expert's weights per 14 routed rows (batched decode) or
@@ -152,8 +152,8 @@ B200MOE_API int  b200moe_synchronize(b200moe_ctx * ctx, void * stream); /* ggml_
 B200MOE_API int  b200moe_set_expert_path(b200moe_ctx * ctx, int path);
 
 /* Launch overlap (no counterpart in the reference; comparable to a backend's own stream options).  In the batched-decode regime (fewer
- * than 24 routed rows per expert on average; larger calls always launch serially) the small kernels and the integer expert kernels of one
- * layer can be launched as programmatic dependents of one another, so a kernel's launch and
+ * than 24 routed rows per expert on average; larger calls always launch serially) the kernels of one call other than the tensor-core ones
+ * are launched as programmatic dependents of one another, so a kernel's launch and
  * set-up (barriers, tables) run alongside the tail of its predecessor; every kernel waits for its predecessor to finish before it
  * reads or writes global memory.  The tensor-core kernels are never launched this way and never release their dependents early:
  * nothing becomes resident beside a kernel that holds tensor memory.  On as a context is created, in the layer calls and in those
