@@ -204,6 +204,9 @@ void whole_layer_overlap(b200moe_ctx * ctx, int64_t rows, int n_expert, cudaStre
 // Launch with programmatic stream serialisation: the kernel may start while its predecessor in the stream is still running;
 // every kernel of this library calls griddepcontrol.wait before it touches global memory that another kernel writes, so only prologues
 // (barrier and table set-up) and launch latency overlap.  Falls back to an ordinary launch when switched off.
+// Such a kernel reads global memory with plain loads only, weights too (a caller may just have written them): the non-coherent path
+// (__ldg, const __restrict__ parameters) is defined for data that is read-only for the kernel's whole life, and an invariant load may
+// be moved above the wait.
 template <typename... KArgs, typename... Args>
 cudaError_t launch_k(b200moe_ctx * ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&... args) {
     cudaLaunchConfig_t cfg = {};
@@ -858,7 +861,7 @@ int dense_matmul_fp4(b200moe_ctx * ctx, const void * w, const float * scale, con
                      bool exact_requant, ActQuant xq, void * list_room, size_t list_room_bytes, const void * w1 = nullptr);
 
 // a[i] = silu(a[i]) * b[i]: ggml_silu then ggml_mul, the same bits as the fused swiglu of the expert kernels
-__global__ void silu_mul_kernel(float * __restrict__ a, const float * __restrict__ b, size_t n) {
+__global__ void silu_mul_kernel(float * __restrict__ a, const float * b, size_t n) {
     pdl_wait();
     pdl_launch_dependents();
     const size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;
@@ -868,7 +871,7 @@ __global__ void silu_mul_kernel(float * __restrict__ a, const float * __restrict
 // Shared expert onto the routed sum (forward.cpp:313-314): gated = sh * sigmoid(logit), out += gated.  The reference's
 // sigmoid is 1 / (1 + expf(-x)) through the C library (ggml-cpu/vec.h:936); expf is evaluated here as the double-precision
 // exponential rounded to float, which is the correctly rounded value but for double-rounding cases rarer than 1 in 2^28.
-__global__ void shexp_add_kernel(float * __restrict__ out, const float * __restrict__ sh, const float * __restrict__ logit, int H, int T,
+__global__ void shexp_add_kernel(float * __restrict__ out, const float * sh, const float * logit, int H, int T,
                                  float * __restrict__ gated_out) {
     pdl_wait();
     pdl_launch_dependents();
@@ -991,7 +994,7 @@ int dense_matmul_fp4(b200moe_ctx * ctx, const void * w, const float * scale, con
     return fail(ctx, B200MOE_ERR_UNSUPPORTED, "no re-quantisation fix-up for width %d", k);
 }
 
-__global__ void gather_rows_kernel(const float4 * __restrict__ src, const int * __restrict__ idx, float4 * __restrict__ dst, int n_rows,
+__global__ void gather_rows_kernel(const float4 * src, const int * idx, float4 * __restrict__ dst, int n_rows,
                                    int w4, int src_rows) {
     pdl_wait();
     pdl_launch_dependents();

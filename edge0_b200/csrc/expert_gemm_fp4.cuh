@@ -137,9 +137,9 @@ __device__ __forceinline__ uint32_t digit_codes(int v) {
 // a value where dividing out digit by digit took 40.  Bound by the stores: 3 bytes per routed value, 8 of them at a time.
 // 4096 tokens top-8, K = 2048: 94 us with seven planes, scales per plane and digits one by one, so 39; fp32 rows of K = 768: 104 us, so 48.
 template <bool SRC_F32>
-__global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const float * __restrict__ src, int64_t src_stride,
-                                                        const int * __restrict__ pos, const int32_t * __restrict__ ids,
-                                                        const int * __restrict__ offsets, const int * __restrict__ tile_of_expert,
+__global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const float * src, int64_t src_stride,
+                                                        const int * pos, const int32_t * ids,
+                                                        const int * offsets, const int * tile_of_expert,
                                                         int act_rows, int K, int n_ids, int ne11, int n_as, PlaneOut out, ActQuant emit) {
     constexpr int MAX_ROWS = 16;             // K = 256
     __shared__ uint32_t s_digits[729];
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(256) act_planes_kernel(ActQuant act, const flo
         float x[16];
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
-            const float4 f = live ? __ldg(reinterpret_cast<const float4 *>(src + (size_t) arow * src_stride + 16 * g) + m) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 f = live ? reinterpret_cast<const float4 *>(src + (size_t) arow * src_stride + 16 * g)[m] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             x[4 * m] = f.x; x[4 * m + 1] = f.y; x[4 * m + 2] = f.z; x[4 * m + 3] = f.w;
         }
         float amax = fabsf(x[0]);                      // NaN only for a block of nothing else

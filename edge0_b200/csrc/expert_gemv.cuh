@@ -217,14 +217,14 @@ __device__ __forceinline__ void two_lane_chains(const uint8_t * const (&blk)[NRO
 // The chains of one weight row in shared memory against ONE activation row whose int8 values (q, K bytes) and block scales (d, K/32
 // floats, 8-byte aligned) lie in separate arrays in global memory.  The result is valid in the row's four threads.
 template <int K>
-__device__ __forceinline__ float two_lane_chain_split(const uint8_t * __restrict__ row, int m, const uint8_t * __restrict__ q, const float * __restrict__ d,
+__device__ __forceinline__ float two_lane_chain_split(const uint8_t * row, int m, const uint8_t * q, const float * d,
                                                       const float * __restrict__ ue_tab) {
     const int sub = m >> 1;
     const uint32_t * qw = reinterpret_cast<const uint32_t *>(q) + 4 * sub + (m & 1);
     uint64_t acc = f32x2(0.0f, 0.0f);
 #pragma unroll 8
     for (int b = 0; b < K / 64; ++b) {
-        const float2 dy = __ldg(reinterpret_cast<const float2 *>(d) + b);
+        const float2 dy = reinterpret_cast<const float2 *>(d)[b];
         const uint8_t * const blk = row + b * NVFP4_BLOCK_BYTES;
         const uint32_t dw = *reinterpret_cast<const uint32_t *>(blk) >> (8 * sub);
 #pragma unroll
@@ -232,7 +232,7 @@ __device__ __forceinline__ float two_lane_chain_split(const uint8_t * __restrict
             uint32_t lo, hi;
             nvfp4_word_to_s8(*reinterpret_cast<const uint32_t *>(blk + 4 + 16 * hf + 4 * m), lo, hi);
             const float s = __fmul_rn(ue_tab[(dw >> (16 * hf)) & 0xff], hf ? dy.y : dy.x);
-            acc = fma_f32x2(f32x2(s, s), dots_to_f32x2(lo, __ldg(qw + (2 * b + hf) * 8), hi, __ldg(qw + (2 * b + hf) * 8 + 2)), acc);
+            acc = fma_f32x2(f32x2(s, s), dots_to_f32x2(lo, qw[(2 * b + hf) * 8], hi, qw[(2 * b + hf) * 8 + 2]), acc);
         }
     }
     const float2 a = f32x2_halves(acc);
@@ -247,8 +247,8 @@ __host__ __device__ constexpr int two_lane_pitch(int row_bytes) { return row_byt
 // must stay sequential to keep the reference's bits - then collects scale and dot product of every unit in order through
 // shuffles.  All four groups end with the same eight partial sums; the result is valid in every lane.
 template <int K>
-__device__ __forceinline__ float lane_chain_warp(const uint8_t * __restrict__ row, int lane, const uint8_t * __restrict__ q,
-                                                 const float * __restrict__ d, const float * __restrict__ ue_tab) {
+__device__ __forceinline__ float lane_chain_warp(const uint8_t * row, int lane, const uint8_t * q,
+                                                 const float * d, const float * __restrict__ ue_tab) {
     constexpr int UNITS = K / 32, UPL = UNITS / 4;       // half-blocks in the row, and per lane
     constexpr int BATCH = UPL < 8 ? UPL : 8;             // fetched and decoded at a time (bounds the registers)
     static_assert(UNITS % 4 == 0 && UPL % BATCH == 0, "half-blocks must split over four lane groups in whole batches");
@@ -316,7 +316,7 @@ struct PassSpan {
 // active experts of the work per chunk: FULL for each pass, what is left of it for the last one.  The whole block looks for its two experts
 // at once.
 template <int THREADS, int PT, int FULL>
-__device__ __forceinline__ PassSpan<PT> pass_span(const int * __restrict__ cw, int n_active, int chunks) {
+__device__ __forceinline__ PassSpan<PT> pass_span(const int * cw, int n_active, int chunks) {
     __shared__ int s_at[2];
     const long long work = n_active ? (long long) cw[n_active] * chunks : 0;
     const long long c[2] = { work * blockIdx.x / gridDim.x, work * (blockIdx.x + 1) / gridDim.x };
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(FewCfg<WT, K, DUAL>::THREADS) expert_few_rows_
         for (int i0 = 0; i0 < K / 4; i0 += C::THREADS) {
             const int i = i0 + tid;
             const bool in = i < K / 4;
-            const float4 v = in ? __ldg(src + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 v = in ? src[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
             amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
             amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
@@ -458,8 +458,8 @@ __global__ void __launch_bounds__(FewCfg<WT, K, DUAL>::THREADS) expert_few_rows_
         }
     } else {
         const uint4 * src = reinterpret_cast<const uint4 *>(p.act.q + arow * K);
-        for (int i = tid; i < K / 16; i += C::THREADS) reinterpret_cast<uint4 *>(acts)[i] = __ldg(src + i);
-        for (int i = tid; i < C::ACT_D; i += C::THREADS) act_d[i] = __ldg(p.act.d + arow * C::ACT_D + i);
+        for (int i = tid; i < K / 16; i += C::THREADS) reinterpret_cast<uint4 *>(acts)[i] = src[i];
+        for (int i = tid; i < C::ACT_D; i += C::THREADS) act_d[i] = p.act.d[arow * C::ACT_D + i];
     }
     const float sc0 = p.scale0 ? p.scale0[p.w_stride ? e : 0] : 1.0f, sc1 = DUAL && p.scale1 ? p.scale1[p.w_stride ? e : 0] : 1.0f;
     const bool landed = mbar_wait_bounded(&full, 0);
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(FewCfg<WT, K, DUAL>::THREADS) expert_few_rows_
 }
 
 // ---- weighted combine: out[t][i] = sum over slots in slot order of y[t*k+s][i] * w[t][s] (forward.cpp:308-310)
-__global__ void __launch_bounds__(256) combine_kernel(const float * __restrict__ y, const float * __restrict__ w, float * __restrict__ out,
+__global__ void __launch_bounds__(256) combine_kernel(const float * y, const float * w, float * __restrict__ out,
                                                      int n, int k, int T) {
     pdl_wait();
     pdl_launch_dependents();

@@ -128,7 +128,7 @@ nvfp4_gemv_kernel(const GemvParams p, const __grid_constant__ CUtensorMap map_w0
                         float4 v[NT];
 #pragma unroll
                         for (int t = 0; t < NT; ++t)
-                            v[t] = in && t < n ? __ldg(reinterpret_cast<const float4 *>(p.act_f32 + arow[t] * K) + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                            v[t] = in && t < n ? reinterpret_cast<const float4 *>(p.act_f32 + arow[t] * K)[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                         uint32_t q[NT];
                         float d[NT];
 #pragma unroll
@@ -151,13 +151,13 @@ nvfp4_gemv_kernel(const GemvParams p, const __grid_constant__ CUtensorMap map_w0
                     for (int i = tid; i < K / 4; i += CONSUMERS) {
                         uint32_t q[NT];
 #pragma unroll
-                        for (int t = 0; t < NT; ++t) q[t] = t < n ? __ldg(reinterpret_cast<const uint32_t *>(p.act.q + arow[t] * K) + i) : 0u;
+                        for (int t = 0; t < NT; ++t) q[t] = t < n ? reinterpret_cast<const uint32_t *>(p.act.q + arow[t] * K)[i] : 0u;
                         *reinterpret_cast<uint4 *>(acts + (size_t) ((i & ~7) | act_slot(i & 7)) * NT) = make_uint4(q[0], q[1], q[2], q[3]);
                     }
                     if (tid < C::ACT_D) {
                         float d[NT];
 #pragma unroll
-                        for (int t = 0; t < NT; ++t) d[t] = t < n ? __ldg(p.act.d + arow[t] * C::ACT_D + tid) : 0.0f;
+                        for (int t = 0; t < NT; ++t) d[t] = t < n ? p.act.d[arow[t] * C::ACT_D + tid] : 0.0f;
                         *reinterpret_cast<float4 *>(dys + tid * NT) = make_float4(d[0], d[1], d[2], d[3]);
                     }
                 }

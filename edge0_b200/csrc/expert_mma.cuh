@@ -82,7 +82,7 @@ __device__ __forceinline__ uint32_t sw128_offset(int r, int c) { return (uint32_
 // [0,8,1,9,2,10,3,11,4,12,5,13,6,14,7,15], the order in which the NVFP4 nibbles of a sub-block unpack.
 // One warp per (sorted row, 32-element activation block).  Rows are row_stride halfs apart in both planes: K with the lo
 // plane stored after the hi plane, 2K with out_lo = out_hi + K when hi and lo rows alternate.
-__global__ void __launch_bounds__(256) sorted_act_fp16_kernel(ActQuant act, const int * __restrict__ perm, const int * __restrict__ meta, int rows,
+__global__ void __launch_bounds__(256) sorted_act_fp16_kernel(ActQuant act, const int * perm, const int * meta, int rows,
                                                              int K, int n_ids, int ne11, __half * __restrict__ out_hi,
                                                              __half * __restrict__ out_lo, int row_stride) {
     pdl_wait();

@@ -53,7 +53,7 @@ __device__ __forceinline__ bool near_half_rounding_boundary(float x, float rel) 
 // What bounds it is the chain of a block (row number, values, list counter, list), not its bytes: with several rows to a warp their
 // loads are in flight together and a block's counter is asked for once for all of them (launch_mark has the line).
 template <int ROWS>
-__global__ void __launch_bounds__(256) requant_mark_kernel(const float * __restrict__ hid, const int * __restrict__ perm, const int * __restrict__ meta,
+__global__ void __launch_bounds__(256) requant_mark_kernel(const float * hid, const int * perm, const int * meta,
                                                           int rows, int n_ff, float step_margin, float rel_margin, FixList list) {
     pdl_wait();
     pdl_launch_dependents();

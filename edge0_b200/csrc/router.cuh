@@ -20,11 +20,11 @@ struct ActQuant {
 };
 
 // eight neighbouring values; src 16-byte aligned
-__device__ __forceinline__ void load8(const float * __restrict__ src, float (&v)[8]) {
+__device__ __forceinline__ void load8(const float * src, float (&v)[8]) {
     const float4 a = *reinterpret_cast<const float4 *>(src), b = *reinterpret_cast<const float4 *>(src + 4);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
-__device__ __forceinline__ void load8(const __nv_bfloat16 * __restrict__ src, float (&v)[8]) {
+__device__ __forceinline__ void load8(const __nv_bfloat16 * src, float (&v)[8]) {
     const uint4 a = *reinterpret_cast<const uint4 *>(src);
     const uint32_t w[4] = { a.x, a.y, a.z, a.w };
 #pragma unroll
@@ -42,7 +42,7 @@ __device__ __forceinline__ void load8(const __nv_bfloat16 * __restrict__ src, fl
 constexpr int ROUTER_ROW = 4096;
 // CH: steps of a lane's chain whose loads are in flight together
 template <int TT, typename XT, int CH = TT == 1 ? 32 : 8>
-__device__ __forceinline__ void router_warp(const float * __restrict__ W, const float * __restrict__ bias, const XT * __restrict__ x,
+__device__ __forceinline__ void router_warp(const float * W, const float * bias, const XT * x,
                                             float * __restrict__ logits, int H, int E, int T, int warp, int lane) {
     constexpr bool STAGE = TT == 1 && sizeof(XT) == 2;
     __shared__ __align__(16) float s_x[STAGE ? ROUTER_ROW : 4];
@@ -52,7 +52,7 @@ __device__ __forceinline__ void router_warp(const float * __restrict__ W, const 
     const float * w = W + (size_t) e * H;
     float wv[CH];                              // the first steps' weights are on their way while the row is staged
 #pragma unroll
-    for (int c = 0; c < CH; ++c) wv[c] = STAGE && lane + 32 * c < H ? __ldg(w + lane + 32 * c) : 0.0f;
+    for (int c = 0; c < CH; ++c) wv[c] = STAGE && lane + 32 * c < H ? w[lane + 32 * c] : 0.0f;
     if (row_staged) {
         const XT * xr = x + (size_t) min((warp & ~7) / E, T - 1) * H;
         if (H % 8 == 0 && ((uintptr_t) xr & 15) == 0) {
@@ -78,7 +78,7 @@ __device__ __forceinline__ void router_warp(const float * __restrict__ W, const 
         float xv[TT][CH];
         if (!STAGE || j0 != lane) {
 #pragma unroll
-            for (int c = 0; c < CH; ++c) wv[c] = j0 + 32 * c < H ? __ldg(w + j0 + 32 * c) : 0.0f;
+            for (int c = 0; c < CH; ++c) wv[c] = j0 + 32 * c < H ? w[j0 + 32 * c] : 0.0f;
         }
 #pragma unroll
         for (int c = 0; c < CH; ++c) {
@@ -112,8 +112,8 @@ __device__ __forceinline__ void router_warp(const float * __restrict__ W, const 
 }
 
 template <int TT, typename XT, int CH = TT == 1 ? 32 : 8>
-__global__ void __launch_bounds__(256) router_logits_kernel(const float * __restrict__ W, const float * __restrict__ bias,
-                                                           const XT * __restrict__ x, float * __restrict__ logits, int H,
+__global__ void __launch_bounds__(256) router_logits_kernel(const float * W, const float * bias,
+                                                           const XT * x, float * __restrict__ logits, int H,
                                                            int E, int T, int * __restrict__ zero_buf, int zero_n) {
     pdl_wait();
     pdl_launch_dependents();
@@ -128,8 +128,8 @@ __global__ void __launch_bounds__(256) router_logits_kernel(const float * __rest
 // chains - lane l owns elements l, l + 32, ... in increasing order - but a weight value now meets TT tokens and an activation value
 // TE experts per load, so the kernel is bound by FMAs instead of by re-reading x once per expert from L2.
 template <int TE, int TT, typename XT>
-__global__ void __launch_bounds__(256) router_logits_tiled_kernel(const float * __restrict__ W, const float * __restrict__ bias,
-                                                                 const XT * __restrict__ x, float * __restrict__ logits, int H, int E, int T,
+__global__ void __launch_bounds__(256) router_logits_tiled_kernel(const float * W, const float * bias,
+                                                                 const XT * x, float * __restrict__ logits, int H, int E, int T,
                                                                  int * __restrict__ zero_buf, int zero_n) {
     pdl_wait();
     pdl_launch_dependents();
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(256) router_logits_tiled_kernel(const float * 
     for (int j = lane; j < H; j += 32) {
         float wv[TE], xv[TT];
 #pragma unroll
-        for (int a = 0; a < TE; ++a) wv[a] = __ldg(wrow[a] + j);
+        for (int a = 0; a < TE; ++a) wv[a] = wrow[a][j];
 #pragma unroll
         for (int b = 0; b < TT; ++b) xv[b] = (float) xrow[b][j];
 #pragma unroll
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) router_logits_tiled_kernel(const float * 
 // as half, multiplier 127/amax in fp32, round to nearest even.  One warp per 32-element block... here one
 // thread per element, a warp per block.
 template <typename XT>
-__device__ __forceinline__ void quantize_q8_0_block(const XT * __restrict__ src, int8_t * __restrict__ q, float * __restrict__ d,
+__device__ __forceinline__ void quantize_q8_0_block(const XT * src, int8_t * __restrict__ q, float * __restrict__ d,
                                                    int lane) {
     const float v = (float) src[lane];
     float amax = fabsf(v);
@@ -200,7 +200,7 @@ __device__ __forceinline__ void quantize_q8_0_block(const XT * __restrict__ src,
 // Q8_0 for eight blocks at a time: a lane holds eight neighbouring values, four lanes one block.  src 16-byte aligned.  (A lane per value
 // moved 16 MB of a 4096-token prompt in 39 us.)
 template <typename XT>
-__device__ __forceinline__ void quantize_q8_0_span(const XT * __restrict__ src, int8_t * __restrict__ q, float * __restrict__ d, int lane) {
+__device__ __forceinline__ void quantize_q8_0_span(const XT * src, int8_t * __restrict__ q, float * __restrict__ d, int lane) {
     float v[8];
     load8(src + lane * 8, v);
     float amax = fabsf(v[0]);    // not zero: a block of nothing but NaN must come out with a NaN scale, as it does a value a lane
@@ -222,7 +222,7 @@ __device__ __forceinline__ void quantize_q8_0_span(const XT * __restrict__ src, 
 // One warp per 256-element block, 8 elements per lane (lane owns elements 8*lane .. 8*lane+7).
 // src: the lane's eight values; q: its eight bytes; d: the block's scale, the same in every lane
 template <typename XT>
-__device__ __forceinline__ void q8_K_words(const XT * __restrict__ src, int lane, uint32_t (&q)[2], float & d) {
+__device__ __forceinline__ void q8_K_words(const XT * src, int lane, uint32_t (&q)[2], float & d) {
     float v[8];
     float amax = 0.0f, mx = 0.0f;
     int arg = 0;
@@ -248,7 +248,7 @@ __device__ __forceinline__ void q8_K_words(const XT * __restrict__ src, int lane
     d = __fdiv_rn(1.0f, iscale);
 }
 template <typename XT>
-__device__ __forceinline__ void quantize_q8_K_block(const XT * __restrict__ src, int8_t * __restrict__ q, float * __restrict__ d,
+__device__ __forceinline__ void quantize_q8_K_block(const XT * src, int8_t * __restrict__ q, float * __restrict__ d,
                                                    int16_t * __restrict__ bsum, int lane) {
     uint32_t w[2];
     float dd;
@@ -264,7 +264,7 @@ __device__ __forceinline__ void quantize_q8_K_block(const XT * __restrict__ src,
 // src row r starts at src + r*src_stride.
 // spans: K is a multiple of 256 and the rows are 16-byte aligned, so a warp takes 256 values of either kind at a time
 template <typename XT>
-__device__ __forceinline__ void quantize_warp(const XT * __restrict__ src, int64_t src_stride, const ActQuant & dst, int rows, int K, int kind, bool spans,
+__device__ __forceinline__ void quantize_warp(const XT * src, int64_t src_stride, const ActQuant & dst, int rows, int K, int kind, bool spans,
                                               int warp, int n_warps, int lane) {
     const int nb = K / (kind == 0 && !spans ? 32 : 256);
     for (int i = warp; i < rows * nb; i += n_warps) {
@@ -278,7 +278,7 @@ __device__ __forceinline__ void quantize_warp(const XT * __restrict__ src, int64
 }
 
 template <typename XT>
-__global__ void __launch_bounds__(256) quantize_act_kernel(const XT * __restrict__ src, int64_t src_stride, ActQuant dst, int rows,
+__global__ void __launch_bounds__(256) quantize_act_kernel(const XT * src, int64_t src_stride, ActQuant dst, int rows,
                                                           int K, int kind, int spans) {
     pdl_wait();
     pdl_launch_dependents();
@@ -289,8 +289,8 @@ __global__ void __launch_bounds__(256) quantize_act_kernel(const XT * __restrict
 // Router logits and activation quantisation in one launch (few tokens): blocks [0, n_logit_blocks) compute logits,
 // the rest quantise x for the expert matmuls.  Both only read x.
 template <int TT, typename XT>
-__global__ void __launch_bounds__(256) route_front_kernel(const float * __restrict__ W, const float * __restrict__ bias,
-                                                         const XT * __restrict__ x, float * __restrict__ logits, int H, int E, int T,
+__global__ void __launch_bounds__(256) route_front_kernel(const float * W, const float * bias,
+                                                         const XT * x, float * __restrict__ logits, int H, int E, int T,
                                                          int * __restrict__ zero_buf, int zero_n, int n_logit_blocks, ActQuant dst,
                                                          int kind, int spans) {
     pdl_wait();
@@ -324,8 +324,8 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 template <int WE, int WT, int RT, typename XT>
-__global__ void __launch_bounds__(WE * WT * 32) router_logits_smem_kernel(const float * __restrict__ W, const float * __restrict__ bias,
-                                                                         const XT * __restrict__ x, float * __restrict__ logits, int H, int E, int T,
+__global__ void __launch_bounds__(WE * WT * 32) router_logits_smem_kernel(const float * W, const float * bias,
+                                                                         const XT * x, float * __restrict__ logits, int H, int E, int T,
                                                                          int * __restrict__ zero_buf, int zero_n, int n_logit_blocks, ActQuant dst,
                                                                          int kind, int spans) {
     constexpr int EB = 8 * WE, TB = RT * WT, KC = ROUTER_KC, ST = ROUTER_ST, NTHR = WE * WT * 32;
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(WE * WT * 32) router_logits_smem_kernel(const 
 // weights = p[ids] / max((float)sum_double(p[ids]), 2^-14) (forward.cpp:268-269).
 // Also counts rows per expert and remembers each row's arrival position for the grouping kernel.
 template <int EPL>  // experts per lane; E <= 32*EPL, E % 8 == 0
-__device__ __forceinline__ void route_select_token(const float * __restrict__ logits, int E, int K, int t, int lane,
+__device__ __forceinline__ void route_select_token(const float * logits, int E, int K, int t, int lane,
                                                    int32_t * __restrict__ ids, float * __restrict__ weights,
                                                    float * __restrict__ probs_out, int * __restrict__ counts,
                                                    int * __restrict__ pos) {
@@ -513,7 +513,7 @@ __device__ __forceinline__ void route_select_token(const float * __restrict__ lo
 }
 
 template <int EPL>
-__global__ void __launch_bounds__(256) route_select_kernel(const float * __restrict__ logits, int E, int K, int T,
+__global__ void __launch_bounds__(256) route_select_kernel(const float * logits, int E, int K, int T,
                                                           int32_t * __restrict__ ids, float * __restrict__ weights,
                                                           float * __restrict__ probs_out, int * __restrict__ counts,
                                                           int * __restrict__ pos) {
@@ -560,7 +560,7 @@ struct Groups {
 // Block-wide: counts must be final and visible to this block.  With several blocks every one scans the counts for itself (a
 // microsecond) and fills its share of perm, which is what takes long with thousands of rows; block 0 writes the tables.
 // allow_empty: ids equal to -1 mark routed rows that do not exist (empty slots of an expert-parallel exchange): they are in no group.
-__device__ __forceinline__ void group_scan_body(Groups g, const int32_t * __restrict__ ids, int E, int rows, int * err, int * sh, bool allow_empty = false,
+__device__ __forceinline__ void group_scan_body(Groups g, const int32_t * ids, int E, int rows, int * err, int * sh, bool allow_empty = false,
                                                 int block = 0, int n_blocks = 1) {
     if (block == 0)
         for (int i = threadIdx.x; i < g.n_done; i += blockDim.x) g.done[i] = 0;
@@ -654,7 +654,7 @@ __global__ void __launch_bounds__(256) dense_groups_kernel(Groups g, int32_t * _
 }
 
 // counts must be final (selection kernel finished).
-__global__ void __launch_bounds__(1024) group_scan_kernel(Groups g, const int32_t * __restrict__ ids, int E, int rows, int * err, int allow_empty) {
+__global__ void __launch_bounds__(1024) group_scan_kernel(Groups g, const int32_t * ids, int E, int rows, int * err, int allow_empty) {
     pdl_wait();
     pdl_launch_dependents();
 
@@ -665,7 +665,7 @@ __global__ void __launch_bounds__(1024) group_scan_kernel(Groups g, const int32_
 // Small batches: selection for every token and the grouping in ONE single-block launch (one warp per token, looping).
 // grouped = 0: one or two tokens, whose kernels read the ids; only their arrival counters are cleared.
 template <int EPL>
-__global__ void __launch_bounds__(1024) route_select_group_kernel(const float * __restrict__ logits, int E, int K, int T,
+__global__ void __launch_bounds__(1024) route_select_group_kernel(const float * logits, int E, int K, int T,
                                                                  int32_t * __restrict__ ids, float * __restrict__ weights,
                                                                  float * __restrict__ probs_out, Groups g, int * err, int grouped) {
     pdl_wait();
@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(1024) route_select_group_kernel(const float * 
 
 // Counting pass for routing that was not produced by route_select_kernel (ids given by the caller,
 // possibly as a strided view: row t starts at ids + t*ids_stride).  Writes compact ids as well.
-__global__ void __launch_bounds__(256) count_ids_kernel(const int32_t * __restrict__ ids, int64_t ids_stride, int n_ids, int T, int E,
+__global__ void __launch_bounds__(256) count_ids_kernel(const int32_t * ids, int64_t ids_stride, int n_ids, int T, int E,
                                                        int32_t * __restrict__ ids_compact, int * __restrict__ counts,
                                                        int * __restrict__ pos, int * err, int allow_empty = 0) {
     pdl_wait();
