@@ -190,15 +190,22 @@ bool gemv_supported(int wtype, int64_t k) {
 // of a latent layer 125 and 83, 8 tokens from host buffers 104 and 94, 17 with a shared expert 153 and 127, 32 (Q3_K) 155 and 141, 64
 // tokens 120 and 112; 64 tokens of an expert-parallel latent layer 288 and 266, the indexed product of 40 tokens 72 and 65.
 // Here for calls that a layer is made of: their first kernel, which may have dependencies on other streams, is launched as usual.
-void layer_overlap(b200moe_ctx * ctx, int64_t rows, int n_expert) {
+// Holds until the returned scope ends, with the call: no call inherits the mode of the one before it.
+struct OverlapScope {
+    b200moe_ctx * ctx;
+    ~OverlapScope() { ctx->overlap_now = ctx->chained = false; }
+};
+[[nodiscard]] OverlapScope layer_overlap(b200moe_ctx * ctx, int64_t rows, int n_expert) {
     ctx->overlap_now = ctx->overlap && rows < (int64_t) 24 * n_expert;
     ctx->chained = false;
+    return OverlapScope{ ctx };
 }
 // The same for a call that is a whole layer; outside of a stream capture its first kernel overlaps what is before it, too.
-void whole_layer_overlap(b200moe_ctx * ctx, int64_t rows, int n_expert, cudaStream_t st) {
-    layer_overlap(ctx, rows, n_expert);
+[[nodiscard]] OverlapScope whole_layer_overlap(b200moe_ctx * ctx, int64_t rows, int n_expert, cudaStream_t st) {
+    ctx->overlap_now = ctx->overlap && rows < (int64_t) 24 * n_expert;
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     ctx->chained = ctx->overlap_now && cudaStreamIsCapturing(st, &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
+    return OverlapScope{ ctx };
 }
 
 // Launch with programmatic stream serialisation: the kernel may start while its predecessor in the stream is still running;
@@ -1561,7 +1568,7 @@ int b200moe_route(b200moe_ctx * ctx, const b200moe_layer * l, const void * x, in
     if (x_type != TYPE_F32 && x_type != TYPE_BF16) return fail(ctx, B200MOE_ERR_UNSUPPORTED, "activations must be F32 or BF16");
     if (T == 0) return B200MOE_OK;
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert);
+    const OverlapScope scope = layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert);
     if ((rc = ensure_plan(ctx, l->n_embd, l->n_latent ? l->n_latent : l->n_embd, l->n_expert, l->n_expert_used, l->n_ff, l->wtype, T))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (x_type == TYPE_F32) return route_impl<float>(ctx, l, static_cast<const float *>(x), T, ids, weights, ob, false, st);
@@ -1590,7 +1597,7 @@ int b200moe_mul_mat_id(b200moe_ctx * ctx, int wtype, const void * as, int64_t ne
     Plan & p = ctx->plan;
     const int rows = (int) (T * n_ids);
     const bool few = few_rows(wtype, rows, (int) n_as);
-    layer_overlap(ctx, rows, (int) n_as);
+    const OverlapScope scope = layer_overlap(ctx, rows, (int) n_as);
     if (!few) CUDA_TRY(ctx, cudaMemsetAsync(p.groups.counts, 0, sizeof(int) * n_as, st));
     // activations: T*ne11 rows of ne00; plan.hq holds T*k rows of width n_ff (= ne00 here), ne11 <= k
     if ((rc = launch_quantize<float>(ctx, b, ne00, p.hq, (int) (T * ne11), (int) ne00, wtype, st))) return rc;
@@ -1615,7 +1622,7 @@ int b200moe_mul_mat(b200moe_ctx * ctx, int wtype, const void * w, int64_t ne00, 
     if ((uintptr_t) w & 15) return fail(ctx, B200MOE_ERR_INVALID_ARG, "weight tensor must be 16-byte aligned");
     if (!gemv_supported(wtype, ne00) || ne01 % 8) return fail(ctx, B200MOE_ERR_UNSUPPORTED, "no kernel for type %d, K=%lld", wtype, (long long) ne00);
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    layer_overlap(ctx, T, 1);
+    const OverlapScope scope = layer_overlap(ctx, T, 1);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int rc = ensure_plan(ctx, (int) ne00, (int) ne00, 8, 1, (int) ne00, wtype, (int) T);
     if (rc) return rc;
@@ -1632,7 +1639,7 @@ int b200moe_latent_down(b200moe_ctx * ctx, const b200moe_layer * l, const void *
     if (x_type != TYPE_F32 && x_type != TYPE_BF16) return fail(ctx, B200MOE_ERR_UNSUPPORTED, "activations must be F32 or BF16");
     if ((uintptr_t) l->lat_down & 15) return fail(ctx, B200MOE_ERR_INVALID_ARG, "quantised tensors must be 16-byte aligned");
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert);
+    const OverlapScope scope = layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert);
     if ((rc = ensure_plan(ctx, l->n_embd, l->n_latent, l->n_expert, l->n_expert_used, l->n_ff, l->wtype, T))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     Plan & p = ctx->plan;
@@ -1655,13 +1662,12 @@ int b200moe_latent_up(b200moe_ctx * ctx, const b200moe_layer * l, const float * 
     if (!m || !out || T < 0) return fail(ctx, B200MOE_ERR_INVALID_ARG, "null pointer or negative token count");
     if ((uintptr_t) l->lat_up & 15) return fail(ctx, B200MOE_ERR_INVALID_ARG, "quantised tensors must be 16-byte aligned");
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert);
+    const OverlapScope scope = layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert);
     if ((rc = ensure_plan(ctx, l->n_embd, l->n_latent, l->n_expert, l->n_expert_used, l->n_ff, l->wtype, T))) return rc;
     return dense_matvec(ctx, l->wtype, l->lat_up, l->lat_up_scale, m, ctx->plan.moq, l->n_latent, l->n_embd, T, out, static_cast<cudaStream_t>(stream));
 }
 
 int b200moe_combine(b200moe_ctx * ctx, const float * y, const float * weights, float * out, int64_t n, int64_t k, int64_t T, void * stream) {
-    if (ctx) ctx->overlap_now = false;
     if (!ctx) return B200MOE_ERR_INVALID_ARG;
     if (T == 0) return B200MOE_OK;
     if (!y || !weights || !out || n <= 0 || k <= 0 || T < 0 || n % 4) return fail(ctx, B200MOE_ERR_INVALID_ARG, "null pointer, non-positive size or width not a multiple of 4");
@@ -1673,7 +1679,6 @@ int b200moe_combine(b200moe_ctx * ctx, const float * y, const float * weights, f
 
 int b200moe_gather_rows(b200moe_ctx * ctx, const float * src, int64_t src_rows, const int32_t * idx, float * dst, int64_t n_rows, int64_t width,
                         void * stream) {
-    if (ctx) ctx->overlap_now = false;
     if (!ctx) return B200MOE_ERR_INVALID_ARG;
     if (n_rows == 0) return B200MOE_OK;
     if (!src || !idx || !dst || n_rows < 0 || src_rows <= 0 || width <= 0 || width % 4) return fail(ctx, B200MOE_ERR_INVALID_ARG, "null pointer, bad size or width not a multiple of 4");
@@ -1693,7 +1698,7 @@ int b200moe_ffn(b200moe_ctx * ctx, const b200moe_layer * l, const void * x, int 
     if (x_type != TYPE_F32 && x_type != TYPE_BF16) return fail(ctx, B200MOE_ERR_UNSUPPORTED, "activations must be F32 or BF16");
     if (T == 0) return B200MOE_OK;
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert);
+    const OverlapScope scope = layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert);
     if ((rc = ensure_plan(ctx, l->n_embd, l->n_latent ? l->n_latent : l->n_embd, l->n_expert, l->n_expert_used, l->n_ff, l->wtype, T))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     Plan & p = ctx->plan;
@@ -1721,7 +1726,7 @@ int b200moe_layer_forward(b200moe_ctx * ctx, const b200moe_layer * l, const void
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     if ((rc = b200moe_reserve(ctx, l, T))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    whole_layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert, st);
+    const OverlapScope scope = whole_layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert, st);
     if (x_type == TYPE_F32) return layer_impl<float>(ctx, l, static_cast<const float *>(x), T, out, ob, st);
     return layer_impl<__nv_bfloat16>(ctx, l, static_cast<const __nv_bfloat16 *>(x), T, out, ob, st);
 }
@@ -1737,7 +1742,7 @@ int b200moe_layer_forward_host(b200moe_ctx * ctx, const b200moe_layer * l, const
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     if ((rc = b200moe_reserve(ctx, l, T))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    whole_layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert, st);
+    const OverlapScope scope = whole_layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert, st);
     Plan & p = ctx->plan;
     const size_t xbytes = (size_t) T * l->n_embd * (x_type == TYPE_F32 ? 4 : 2);
     CUDA_TRY(ctx, cudaMemcpyAsync(p.xin, x_host, xbytes, cudaMemcpyHostToDevice, st));
@@ -1788,7 +1793,7 @@ int b200moe_ep_expert_rows_expected(b200moe_ctx * ctx, const b200moe_layer * l, 
     if (expected_rows < 0 || expected_rows > n_slots) return fail(ctx, B200MOE_ERR_INVALID_ARG, "expected rows outside 0 .. slots");
     if ((uintptr_t) slots & 15) return fail(ctx, B200MOE_ERR_INVALID_ARG, "slots must be 16-byte aligned");
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    layer_overlap(ctx, n_slots, l->n_expert);
+    const OverlapScope scope = layer_overlap(ctx, n_slots, l->n_expert);
     const int n_in = l->n_embd, R = (int) n_slots, slot_words = n_in + EP_SLOT_EXTRA;
     // one slot = one routed row of a one-slot layer
     if ((rc = ensure_plan(ctx, l->n_embd, n_in, l->n_expert, 1, l->n_ff, l->wtype, R))) return rc;
