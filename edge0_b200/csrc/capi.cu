@@ -900,8 +900,17 @@ bool dense_on_fp4(const b200moe_ctx * ctx, int wtype, int k, int n_out, int T) {
     return wtype == TYPE_NVFP4 && fp4_width(k) && n_out % 256 == 0 && T >= 4 && path != 1 && path != 5 && path != 7;
 }
 
-// tokens of a dense product that the kernel of few rows takes one by one
+// Dense products that the kernel of few rows takes token by token: up to four of them while what they read and decode, the matrix once for
+// each, is no more than this; beyond it they share a pass of the grouped kernel, behind a launch for the groups and one that quantises.
+// Few rows and grouped, us: NVFP4, 4 tokens, 2048 -> 2048 (9 MB) 10 and 14, 6144 (28 MB) 21 and 19, 65536 162 and 56, 512 -> 12288 (14 MB) 15
+// and 14, 24576 (28 MB) 23 and 14; 2 tokens, 2048 -> 12288 (28 MB) 21 and 21, 32768 44 and 29.  Q3_K, 4 tokens, 2048 -> 4096 (14 MB) 13 and
+// 14, 6144 (22 MB) 17 and 14, 248320 457 and 152 (before one kernel per token was the rule).  One token shares nothing: NVFP4, 2048 -> 24576
+// (28 MB) 21 and 21, 4096 -> 16384 (38 MB) 33 and 24, 131072 207 and 106; Q3_K, 2048 -> 32768 (29 MB) 19 and 25, 131072 (115 MB) 66 and 60.
 constexpr int DENSE_FEW_ROWS = 4;
+constexpr int64_t DENSE_FEW_BYTES_ONE = 32 << 20, DENSE_FEW_BYTES = 20 << 20;
+bool dense_few(int wtype, int64_t k, int64_t n_rows, int T) {
+    return T <= DENSE_FEW_ROWS && T * n_rows * weight_row_bytes(wtype, k) <= (T == 1 ? DENSE_FEW_BYTES_ONE : DENSE_FEW_BYTES);
+}
 
 // exact_requant: see dense_matmul_fp4; `hidden` scratch holds the list (free before the experts run)
 // w1 != null: y = silu(w . x) * (w1 . x), the gate/up pair of a dense expert in one pass over x (no tensor scales, no exact_requant);
@@ -920,9 +929,8 @@ int dense_matvec(b200moe_ctx * ctx, int wtype, const void * w, const float * sca
         launch_k(ctx, silu_mul_kernel, dim3((unsigned) ((n + 255) / 256)), dim3(256), 0, st, y, y1_tmp, n);
         return check_launch(ctx, "silu_mul");
     }
-    // few tokens: the kernel of few rows, which quantises them while it stages them.  NVFP4, 3 tokens, us, as passes
-    // of the grouped kernel (with its groups' launch, 1.7) and so: 4096 -> 1024 17.5 and 8.5, 1024 -> 4096 9.9 and 6.4.
-    if (T <= DENSE_FEW_ROWS && !((uintptr_t) x & 15)) {
+    // few tokens: the kernel of few rows, which quantises them while it stages them
+    if (dense_few(wtype, k, (int64_t) n_out * (w1 ? 2 : 1), T) && !((uintptr_t) x & 15)) {
         GemvParams g = gemv_params(ctx, w, w1, scale, nullptr, xq, y, n_out, 1, 1, 1);
         g.w_stride = 0;
         g.ids = nullptr;

@@ -62,6 +62,27 @@ def test_dense_products_of_few_tokens(wtype, K, N, gpu_ctx, checker):
         assert float(whole[0, r]) == checker.vec_dot(wtype, K, w[r], aq)
 
 
+@pytest.mark.parametrize("wtype", [TYPE_NVFP4, TYPE_Q3_K])
+def test_tokens_share_a_large_matrix(wtype, gpu_ctx):
+    """A dense product of a few tokens reads a matrix for each of them only while that is less than a pass of the grouped kernel (by the
+    launches); the bits are the same on either side of the line."""
+    K, row = 256, 144 if wtype == TYPE_NVFP4 else 110
+    x = torch.randn((6, K), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
+    for T, line in ((1, 32 << 20), (3, 20 << 20)):
+        N = line // (T * row) // 8 * 8
+        w = torch.from_numpy(matrix(np.random.default_rng(T), wtype, 1, 512, K)[0]).cuda().repeat((N + 8 + 511) // 512, 1)
+        gpu_ctx.set_expert_path(1)
+        try:
+            whole = gpu_ctx.mul_mat(wtype, w[:N + 8], x, K)
+        finally:
+            gpu_ctx.set_expert_path(0)
+        for n, few in ((N, True), (N + 8, False)):
+            before = gpu_ctx.launches()
+            got = gpu_ctx.mul_mat(wtype, w[:n], x[:T].contiguous(), K)
+            assert gpu_ctx.launches() - before == (1 if few else 3), (T, n)      # or: quantiser, groups, product
+            assert torch.equal(got, whole[:T, :n]), (T, n)
+
+
 def test_an_expert_that_does_not_exist_is_reported(gpu_ctx):
     rng = np.random.default_rng(1)
     w = torch.from_numpy(matrix(rng, TYPE_NVFP4, 9, 8, 256)).cuda()
