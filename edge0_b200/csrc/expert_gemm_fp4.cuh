@@ -375,7 +375,8 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
     constexpr uint32_t OFF_A1 = C::A_TILE, OFF_SFB = C::B_TILE;
     // 768 threads leave 80 registers to a thread.  With the small tile producers and issuer give theirs to the epilogue, which spilled without
     // (40 + 2 x 104 + 3 x 72 = 464 of the launch's 480 per 128 threads; 64 tokens over 128 experts: gate/up 51.7 us, so 49.9, down 29.4 and 27.0).
-    // The large one has no spills without it and loses with it (4096 tokens, down: 244 us, 283 so).
+    // The large one loses with it (4096 tokens, down: 244 us, 283 so); what kept a short K from spilling there is that the loops over
+    // K = 256 pieces stay loops (K = 512, 1024 tokens x 32768 features: 111 us unrolled, so 98).
     if (warp < 4) {
         if constexpr (!C::LARGE) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
         if (warp == 0 && lane == 0) {
@@ -385,6 +386,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
             for (int u = blockIdx.x; u < n_units && !s_abort; u += gridDim.x) {
                 const Unit w = unit_at(u);
                 const int row0 = w.e * p.n_out + w.ft * FEAT;
+#pragma unroll 1
                 for (int kc = 0; kc < KC; ++kc) {
                     FP4_PROF_T0();
                     if (!wait_or_abort<40>(&raw_empty[raw.stage], raw.phase ^ 1u, &s_abort, p.err)) break;
@@ -406,6 +408,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                 const Unit w = unit_at(u);
                 const uint8_t * sfr = p.sf + (size_t) w.row0 * 16;
                 const int boxes = (w.nt + C::BOX_ROWS - 1) / C::BOX_ROWS;
+#pragma unroll 1
                 for (int kc = 0; kc < KC; ++kc) {
                     FP4_PROF_T0();
                     if (!wait_or_abort<40>(&act_empty[act.stage], act.phase ^ 1u, &s_abort, p.err)) break;
@@ -433,6 +436,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
                 tc_fence_after();
                 const uint32_t d0 = tmem + (uint32_t) acc.stage * (2 * C::NCOL), d1 = d0 + C::NCOL;
                 bool ok = true;
+#pragma unroll 1
                 for (int kc = 0; kc < KC; ++kc) {
                     {
                         FP4_PROF_T0();
@@ -474,8 +478,9 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
         FP4_PROF_DECL();
         const int q = warp & 3;                 // TMEM lane quarter this warp may read
         // two warps per quarter: the first takes the tile's first rows, the second the rest.  Routed rows to a tensor memory load of 32 columns: five
-        // fill it, four cost a tile of few rows less.
-        constexpr int FOLD = C::LARGE ? 5 : 4, HALF = (RPT + 2 * FOLD - 1) / (2 * FOLD) * FOLD;
+        // fill it, four cost a tile of few rows less, and the large tile where five spill (one tensor, K = 256: 33 tokens x 32768 features 8.8 us,
+        // so 8.4; elsewhere four spill and five do not: K = 512, 1024 x 32768 115 and 98; 768, 512 x 32768 67.4 and 65.7).
+        constexpr int FOLD = C::LARGE && (DUAL || K > 256) ? 5 : 4, HALF = (RPT + 2 * FOLD - 1) / (2 * FOLD) * FOLD;
         const int first = warp >= 20 ? HALF : 0;
         for (int u = blockIdx.x; u < n_units && !s_abort; u += gridDim.x) {
             const Unit w = unit_at(u);
