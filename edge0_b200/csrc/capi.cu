@@ -189,7 +189,7 @@ bool gemv_supported(int wtype, int64_t k) {
 // Layers called one by one, us without and with: one token, four layers 123 and 90 (Q3_K; replayed from a graph, NVFP4, 112 and 96), 3 tokens
 // of a latent layer 125 and 83, 8 tokens from host buffers 104 and 94, 17 with a shared expert 153 and 127, 32 (Q3_K) 155 and 141, 64
 // tokens 120 and 112; 64 tokens of an expert-parallel latent layer 288 and 266, the indexed product of 40 tokens 72 and 65.
-// Here for calls that a layer is made of: their first kernel, which may have dependencies on other streams, is launched as usual.
+// Here for calls that a layer is made of: their first kernel is launched as usual.
 // Holds until the returned scope ends, with the call: no call inherits the mode of the one before it.
 struct OverlapScope {
     b200moe_ctx * ctx;
@@ -200,7 +200,9 @@ struct OverlapScope {
     ctx->chained = false;
     return OverlapScope{ ctx };
 }
-// The same for a call that is a whole layer; outside of a stream capture its first kernel overlaps what is before it, too.
+// The same for a call that is a whole layer; outside of a stream capture its first kernel overlaps a kernel right before it in the stream,
+// too, if that one releases its dependents early.  Waits and copies before it order the launch itself.  (Behind the calls that a layer is
+// made of there is as a rule a kernel of the caller's, which releases nothing early: they would gain nothing.)
 [[nodiscard]] OverlapScope whole_layer_overlap(b200moe_ctx * ctx, int64_t rows, int n_expert, cudaStream_t st) {
     ctx->overlap_now = ctx->overlap && rows < (int64_t) 24 * n_expert;
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
@@ -1750,7 +1752,7 @@ int b200moe_layer_forward_host(b200moe_ctx * ctx, const b200moe_layer * l, const
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     if ((rc = b200moe_reserve(ctx, l, T))) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const OverlapScope scope = whole_layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert, st);
+    const OverlapScope scope = layer_overlap(ctx, (int64_t) T * l->n_expert_used, l->n_expert);   // the first kernel is behind the copy of x
     Plan & p = ctx->plan;
     const size_t xbytes = (size_t) T * l->n_embd * (x_type == TYPE_F32 ? 4 : 2);
     CUDA_TRY(ctx, cudaMemcpyAsync(p.xin, x_host, xbytes, cudaMemcpyHostToDevice, st));

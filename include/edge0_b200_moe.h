@@ -157,7 +157,8 @@ B200MOE_API int  b200moe_set_expert_path(b200moe_ctx * ctx, int path);
  * set-up (barriers, tables) run alongside the tail of its predecessor; every kernel waits for its predecessor to finish before it
  * reads or writes global memory.  The tensor-core kernels are never launched this way and never release their dependents early:
  * nothing becomes resident beside a kernel that holds tensor memory.  On as a context is created, in the layer calls and in those
- * a layer is made of; enable = 0 switches it off, 1 on again. */
+ * a layer is made of; enable = 0 switches it off, 1 on again.  Outside of a stream capture the first kernel of b200moe_layer_forward may
+ * in the same way be resident beside a kernel of the caller's right before it in the stream, if that one releases its dependents early. */
 B200MOE_API int  b200moe_set_launch_overlap(b200moe_ctx * ctx, int enable);
 /* Per-kernel device timing (reference: DecodeTiming with an injectable clock, include/edge0/timing.h:4-9).
  * When enabled, every expert-matmul launch is bracketed by CUDA events on its stream; b200moe_kernel_times

@@ -52,3 +52,18 @@ def test_dependents_read_through_the_coherent_path():
             if kernel or m.group(1) not in SHARED:
                 bad.append((name, "const __restrict__", m.group(1)))
     assert not bad, bad
+
+
+def test_no_dependent_right_behind_a_copy():
+    """A kernel behind a copy or a memset is an ordinary launch: a call copies before it sets its launch mode or launches anything, behind
+    its last launch, or with copy_out, which says so."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(ROOT, "edge0_b200", "csrc", "capi.cu")).read())
+    bad = []
+    for m in re.finditer(r"\n(?:\w[\w ]*)?\bint (\w+)\([^;{}]*\) \{\n(.*?)\n\}", text, re.S):
+        marks = [("raw" if "Async" in t.group(0) else "launch", t.group(0)) for t in
+                 re.finditer(r"cudaMem(?:cpy|set)Async\(|\blaunch_\w+[<(]|\w+_impl[<(]|\bdense_mat\w+\(|whole_layer_overlap\(", m.group(2))]
+        for i, (kind, _) in enumerate(marks):
+            before, after = (any(k == "launch" for k, _ in part) for part in (marks[:i], marks[i + 1:]))
+            if kind == "raw" and before and after:
+                bad.append(m.group(1))
+    assert not bad, bad

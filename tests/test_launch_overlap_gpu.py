@@ -73,3 +73,36 @@ def test_captured_layer_overlaps_inside_only(gpu_ctx):
     inside, edges = dependent_edges(alone)
     assert inside == edges > 0
     assert dependent_edges(behind) == (inside, edges + 1)
+
+
+@pytest.mark.parametrize("T", [1, 20])
+def test_layer_waits_for_what_its_stream_waits_for(T, gpu_ctx):
+    """x made on a second stream that the layer's stream has joined, right behind a copy, right behind a kernel, and on the host."""
+    layer = W.make_layer(CFG).to_device(gpu_ctx)
+    tokens = torch.from_numpy(W.make_tokens(CFG, T)).cuda()
+    xs = [tokens * (i + 1) for i in range(4)]
+    want = [layer.forward(x).clone() for x in xs]
+    gpu_ctx.synchronize()
+    x, out = torch.zeros_like(tokens), torch.empty((T, 512), device="cuda")
+    host = [v.cpu().pin_memory() for v in xs]
+    side, cur = torch.cuda.Stream(), torch.cuda.current_stream()
+    busy = torch.randn((2048, 2048), device="cuda")
+    for i in range(24):
+        src, how = xs[i % 4], (i // 4) % 3
+        if how == 0:
+            side.wait_stream(cur)
+            with torch.cuda.stream(side):
+                busy @ busy                      # x arrives long after the host has launched the layer
+                torch.mul(src, 1, out=x)
+            cur.wait_stream(side)
+        elif how == 1:
+            busy @ busy
+            x.copy_(host[i % 4], non_blocking=True)
+        else:
+            busy @ busy
+            torch.mul(src, 1, out=x)
+        layer.forward(x, out=out)
+        assert torch.equal(out, want[i % 4]), i
+        x.zero_()
+    for i in range(8):
+        assert torch.equal(layer.forward_host(host[i % 4]), want[i % 4].cpu()), i
