@@ -904,12 +904,12 @@ bool dense_on_fp4(const b200moe_ctx * ctx, int wtype, int k, int n_out, int T) {
 
 // Dense products that the kernel of few rows takes token by token: up to four of them while what they read and decode, the matrix once for
 // each, is no more than this; beyond it they share a pass of the grouped kernel, behind a launch for the groups and one that quantises.
-// Few rows and grouped, us: NVFP4, 4 tokens, 2048 -> 2048 (9 MB) 10 and 14, 6144 (28 MB) 21 and 19, 65536 162 and 56, 512 -> 12288 (14 MB) 15
-// and 14, 24576 (28 MB) 23 and 14; 2 tokens, 2048 -> 12288 (28 MB) 21 and 21, 32768 44 and 29.  Q3_K, 4 tokens, 2048 -> 4096 (14 MB) 13 and
-// 14, 6144 (22 MB) 17 and 14, 248320 457 and 152 (before one kernel per token was the rule).  One token shares nothing: NVFP4, 2048 -> 24576
-// (28 MB) 21 and 21, 4096 -> 16384 (38 MB) 33 and 24, 131072 207 and 106; Q3_K, 2048 -> 32768 (29 MB) 19 and 25, 131072 (115 MB) 66 and 60.
+// Few rows and grouped, us: NVFP4, 4 tokens, 2048 -> 2048 (9 MB) 11 and 15, 6144 (28 MB) 21 and 17, 65536 162 and 54, 512 -> 12288 (14 MB) 15
+// and 15, 24576 (28 MB) 23 and 15; 2 tokens, 2048 -> 12288 (28 MB) 21 and 17, 32768 44 and 29.  Q3_K, 4 tokens, 2048 -> 4096 (14 MB) 13 and
+// 15, 6144 (22 MB) 17 and 15, 248320 457 and 107.  One token shares nothing, so its line lies where the last of the shapes crosses: NVFP4,
+// 2048 -> 24576 (28 MB) 21 and 21, 65536 (76 MB) 44 and 40, 4096 -> 131072 207 and 106; Q3_K, 2048 -> 65536 (58 MB) 35 and 40, 131072 66 and 60.
 constexpr int DENSE_FEW_ROWS = 4;
-constexpr int64_t DENSE_FEW_BYTES_ONE = 32 << 20, DENSE_FEW_BYTES = 20 << 20;
+constexpr int64_t DENSE_FEW_BYTES_ONE = 64 << 20, DENSE_FEW_BYTES = 24 << 20;
 bool dense_few(int wtype, int64_t k, int64_t n_rows, int T) {
     return T <= DENSE_FEW_ROWS && T * n_rows * weight_row_bytes(wtype, k) <= (T == 1 ? DENSE_FEW_BYTES_ONE : DENSE_FEW_BYTES);
 }

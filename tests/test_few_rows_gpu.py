@@ -68,7 +68,7 @@ def test_tokens_share_a_large_matrix(wtype, gpu_ctx):
     launches); the bits are the same on either side of the line."""
     K, row = 256, 144 if wtype == TYPE_NVFP4 else 110
     x = torch.randn((6, K), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
-    for T, line in ((1, 32 << 20), (3, 20 << 20)):
+    for T, line in ((1, 64 << 20), (3, 24 << 20)):
         N = line // (T * row) // 8 * 8
         w = torch.from_numpy(matrix(np.random.default_rng(T), wtype, 1, 512, K)[0]).cuda().repeat((N + 8 + 511) // 512, 1)
         gpu_ctx.set_expert_path(1)
