@@ -470,6 +470,12 @@ bool q3k_on_mma(int wtype, int64_t rows, int n_groups) { return wtype == TYPE_Q3
 // Rows of one or two tokens: the integer kernel that takes them one by one, unless there are so few groups that Q3_K is on passes of 32.
 bool few_rows(int wtype, int64_t rows, int n_groups) { return rows <= 16 && !q3k_on_mma(wtype, rows, n_groups); }
 
+// Indexed products whose rows share experts, two to each or more, leave the kernel of few rows where it would read and decode more than this,
+// an expert's rows once for each of them; the line lies where the last of the shapes crosses.  Few rows and grouped, us: 2048 -> 2048, 16 rows
+// over 2 experts, Q3_K (28 MB) 19 and 19, NVFP4 (36 MB) 25 and 30; 2048 -> 4096 over 2, 12 rows, Q3_K (41 MB) 27 and 19, NVFP4 (54 MB) 35 and
+// 29; 256 -> 16384 over 4, 16 rows, NVFP4 (36 MB) 31 and 21; 768 -> 65536 over 2, 4 rows, Q3_K (82 MB) 58 and 35.
+constexpr int64_t INDEXED_FEW_BYTES = 40 << 20;
+
 // the integer product of grouped rows: `rows` routed rows in up to n_groups groups
 template <bool DUAL>
 int launch_integer(b200moe_ctx * ctx, int wtype, int k, const GemvParams & p, int64_t rows, int n_groups, int nt, cudaStream_t st) {
@@ -1606,7 +1612,7 @@ int b200moe_mul_mat_id(b200moe_ctx * ctx, int wtype, const void * as, int64_t ne
     if (rc) return rc;
     Plan & p = ctx->plan;
     const int rows = (int) (T * n_ids);
-    const bool few = few_rows(wtype, rows, (int) n_as);
+    const bool few = few_rows(wtype, rows, (int) n_as) && (rows < 2 * n_as || rows * ne01 * weight_row_bytes(wtype, ne00) <= INDEXED_FEW_BYTES);
     const OverlapScope scope = layer_overlap(ctx, rows, (int) n_as);
     if (!few) CUDA_TRY(ctx, cudaMemsetAsync(p.groups.counts, 0, sizeof(int) * n_as, st));
     // activations: T*ne11 rows of ne00; plan.hq holds T*k rows of width n_ff (= ne00 here), ne11 <= k
@@ -1621,7 +1627,7 @@ int b200moe_mul_mat_id(b200moe_ctx * ctx, int wtype, const void * as, int64_t ne
         if ((rc = check_launch(ctx, "count_ids"))) return rc;
         if ((rc = launch_group(ctx, p.ids, (int) n_as, rows, st))) return rc;
     }
-    return launch_integer<false>(ctx, wtype, (int) ne00, g, rows, (int) n_as, few_or_grouped(rows), st);
+    return launch_integer<false>(ctx, wtype, (int) ne00, g, rows, (int) n_as, few ? -rows : 0, st);
 }
 
 int b200moe_mul_mat(b200moe_ctx * ctx, int wtype, const void * w, int64_t ne00, int64_t ne01, const float * x, int64_t T, const float * scale,

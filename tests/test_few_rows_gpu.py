@@ -83,6 +83,23 @@ def test_tokens_share_a_large_matrix(wtype, gpu_ctx):
             assert torch.equal(got, whole[:T, :n]), (T, n)
 
 
+@pytest.mark.parametrize("wtype", [TYPE_NVFP4, TYPE_Q3_K])
+def test_rows_share_large_experts(wtype, gpu_ctx):
+    """The same of indexed products of which each expert has several rows."""
+    K, row, E = 256, 144 if wtype == TYPE_NVFP4 else 110, 4
+    b = torch.randn((8, 1, K), generator=torch.Generator(device="cuda").manual_seed(2), device="cuda")
+    N = (40 << 20) // (8 * row) // 8 * 8
+    w = torch.from_numpy(matrix(np.random.default_rng(5), wtype, E, 512, K)).cuda().repeat(1, (N + 8 + 511) // 512, 1)
+    for n, T, few in ((N, 8, True), (N + 8, 8, False), (N + 8, 7, True)):
+        ids = (torch.arange(T, device="cuda") % E).reshape(T, 1).to(torch.int32)
+        mats = w[:, :n].contiguous()
+        before = gpu_ctx.launches()
+        got = gpu_ctx.mul_mat_id(wtype, mats, b[:T].contiguous(), ids, K)
+        assert gpu_ctx.launches() - before == (2 if few else 4), (n, T)       # quantiser, product, or counts and groups in between
+        for t in range(T):
+            assert torch.equal(got[t], gpu_ctx.mul_mat_id(wtype, mats, b[t:t + 1], ids[t:t + 1], K)[0]), (n, T, t)
+
+
 def test_an_expert_that_does_not_exist_is_reported(gpu_ctx):
     rng = np.random.default_rng(1)
     w = torch.from_numpy(matrix(rng, TYPE_NVFP4, 9, 8, 256)).cuda()
