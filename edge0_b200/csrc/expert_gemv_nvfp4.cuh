@@ -63,10 +63,10 @@ nvfp4_gemv_kernel(const GemvParams p, const __grid_constant__ CUtensorMap map_w0
     // the work; of one group, a dense product of a few tokens, the passes are known, and twice as many would leave half of the CTAs out:
     // 2048 -> 8192, 3 tokens 24.8 us, so 19.0.)
     const long long passes = n_active == 1 ? (p.meta[1] + NT - 1) / NT : (cw[n_active] + 9) / 10;
-    int boxes = 1;                                           // eight rows each
-    while (boxes < C::WARPS && passes * ((p.n_out + 8 * boxes - 1) / (8 * boxes)) > gridDim.x) boxes <<= 1;
-    const int chunk_rows = 8 * boxes;
-    auto span = pass_span<C::THREADS, NT, 16>(cw, n_active, (p.n_out + chunk_rows - 1) / chunk_rows);
+    int log_rows = 3;                                        // boxes of eight rows each
+    while (8 * C::WARPS >> log_rows > 1 && passes * ((p.n_out + (1 << log_rows) - 1) >> log_rows) > gridDim.x) ++log_rows;
+    const int chunk_rows = 1 << log_rows, boxes = chunk_rows / 8;
+    auto span = pass_span<C::THREADS, NT, 16>(cw, n_active, (p.n_out + chunk_rows - 1) >> log_rows);
 
     if (warp == C::WARPS) {
         // ---------------------------------------------------------------- weight producer

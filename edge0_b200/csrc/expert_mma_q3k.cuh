@@ -48,8 +48,13 @@ struct Q3kCfg {
     static constexpr int PITCH = K + 16;                      // of an activation row
     static constexpr int SB = K / 256;
     static constexpr int FULL = 4 + NTG;       // work of a full pass (q3k_work)
+    // A pass's activation rows come by bulk copies, one to a row; rows of up to 512 bytes by the threads, whose loads do not queue up: 256 -> 256,
+    // 50 rows to each of 16 experts, 18.4 us with copies and 16.5 without (whole call), 512 -> 768, 8000 rows over 128 experts 70 and 68; pieces of
+    // 768 do not divide by the threads.
+    static constexpr bool WIDE_ACTS = K > 512;
     static constexpr size_t SMEM = (size_t) WARPS * STAGES * TILE + (size_t) TOK * PITCH;
     static_assert(TILE % 32 == 0 && PITCH % 128 == 16, "halves of a tile are multiples of 16 bytes; fragment loads fall on different banks");
+    static_assert(WIDE_ACTS || (THREADS % (K / 16) == 0 && TOK % (THREADS / (K / 16)) == 0), "every thread moves as many pieces of the activation rows");
     static_assert(SMEM + 4096 <= 227 * 1024, "one CTA fits an SM");
 };
 
@@ -68,6 +73,7 @@ __device__ __forceinline__ void q3k_mma_body(const GemvParams & p) {
     uint8_t * const tiles = acts + (size_t) C::TOK * C::PITCH;   // [WARPS][STAGES][16 rows]
     __shared__ uint2 s_prod[64];                              // six-bit scale v -> bytes (32 - v) * (c - 4), c = 0..7
     __shared__ float s_dx[C::TOK][SB];
+    __shared__ int s_row[C::TOK];                             // the pass's routed rows
     __shared__ uint64_t full[C::WARPS][C::STAGES], act_full;
     __shared__ volatile int s_abort;
 
@@ -93,22 +99,20 @@ __device__ __forceinline__ void q3k_mma_body(const GemvParams & p) {
     // a tile for each warp to a chunk; while there are items for less than every CTA, as few as leaves one to a CTA
     const int n_tiles = (p.n_out + C::FEAT - 1) / C::FEAT;
     const long long passes = (cw[n_active] + 4) / 5;
-    int per = 1;
-    while (per < C::WARPS && passes * ((n_tiles + per - 1) / per) > gridDim.x) per = min(C::WARPS, 2 * per);
-    auto span = pass_span<C::THREADS, C::TOK, C::FULL>(cw, n_active, (n_tiles + per - 1) / per);
+    int log_per = 0;
+    while (C::WARPS >> log_per > 1 && passes * ((n_tiles + (1 << log_per) - 1) >> log_per) > gridDim.x) ++log_per;
+    const int per = 1 << log_per;
+    auto span = pass_span<C::THREADS, C::TOK, C::FULL>(cw, n_active, (n_tiles + per - 1) >> log_per);
 
     // raw rows of the warp's tile of an item, if it has one
     auto has_tile = [&](int ch) { return warp < per && ch * per + warp < n_tiles; };
     uint8_t * const my_tiles = tiles + (size_t) warp * C::STAGES * C::TILE;
     auto pre = span;
-    int pre_at = -1, pre_e = 0, pre_n = 0, pre_stage = 0;
+    int pre_stage = 0;
     auto fetch = [&] {                                        // of the next item that has one
         while (pre.more()) {
-            if (pre.a != pre_at) {
-                pre_at = pre.a;
-                pre_e = p.active[pre_at];
-                pre_n = p.offsets[pre_e + 1] - p.offsets[pre_e];
-            }
+            // (asked for again for every item: held in registers they spilled the chains, 2048 -> 768, 1001 tokens, whole layer 545 us, so 526)
+            const int pre_e = p.active[pre.a], pre_n = p.offsets[pre_e + 1] - p.offsets[pre_e];
             const int ch = pre.ch;
             pre.next(pre_n);
             if (!has_tile(ch)) continue;
@@ -150,23 +154,45 @@ __device__ __forceinline__ void q3k_mma_body(const GemvParams & p) {
         }
         const int t0 = C::TOK * span.ps, n = min(C::TOK, n_e - t0);
         if (loaded != span.ps) {
-            __syncthreads();                                  // everybody is done with the rows that give way
-            if (warp == 0) {
-                if (lane == 0) mbar_arrive_expect_tx(&act_full, (uint32_t) (n * K));
-                __syncwarp();
-                if (lane < n) {
-                    const int r = p.perm[row_beg + t0 + lane];
-                    const int arow = (r / p.n_ids) * p.ne11 + (r % p.n_ids) % p.ne11;
-                    bulk_g2s(acts + (size_t) lane * C::PITCH, p.act.q + (size_t) arow * K, K, &act_full);
+            auto act_row = [&](int r) { return (int) ((r / p.n_ids) * p.ne11 + (r % p.n_ids) % p.ne11); };
+            const int * const rows = p.perm + row_beg + t0;
+            if constexpr (C::WIDE_ACTS) {
+                __syncthreads();                              // everybody is done with the rows that give way
+                if (warp == 0) {
+                    if (lane == 0) mbar_arrive_expect_tx(&act_full, (uint32_t) (n * K));
+                    __syncwarp();
+                    if (lane < n) {
+                        const int r = rows[lane];
+                        bulk_g2s(acts + (size_t) lane * C::PITCH, p.act.q + (size_t) act_row(r) * K, K, &act_full);
+                    }
+                }
+                if (tid < n) s_row[tid] = rows[tid];
+                for (int i = tid; i < n * SB; i += C::THREADS) s_dx[i / SB][i % SB] = p.act.d[(size_t) act_row(rows[i / SB]) * SB + i % SB];
+                wait_or_abort(&act_full, act_parity, &s_abort, p.err);
+                act_parity ^= 1u;
+            } else {
+                constexpr int PIECES = K / 16, STEP = C::THREADS / PIECES;     // a thread moves its piece of every STEP-th row
+                const int piece = tid % PIECES, first = tid / PIECES;
+                uint4 v[C::TOK / STEP];
+                int r[C::TOK / STEP];
+                float d[C::TOK / STEP];
+#pragma unroll
+                for (int i = 0; i < C::TOK / STEP; ++i) r[i] = rows[min(first + i * STEP, n - 1)];
+#pragma unroll
+                for (int i = 0; i < C::TOK / STEP; ++i) {
+                    const size_t row = act_row(r[i]);
+                    v[i] = reinterpret_cast<const uint4 *>(p.act.q + row * K)[piece];
+                    d[i] = p.act.d[row * SB + piece / 16];
+                }
+                __syncthreads();                              // everybody is done with the rows that give way
+#pragma unroll
+                for (int i = 0; i < C::TOK / STEP; ++i) {
+                    const int t = first + i * STEP;
+                    reinterpret_cast<uint4 *>(acts + (size_t) t * C::PITCH)[piece] = v[i];
+                    if (piece % 16 == 0) s_dx[t][piece / 16] = d[i];
+                    if (piece == 0) s_row[t] = r[i];
                 }
             }
-            for (int i = tid; i < n * SB; i += C::THREADS) {
-                const int r = p.perm[row_beg + t0 + i / SB];
-                const int arow = (r / p.n_ids) * p.ne11 + (r % p.n_ids) % p.ne11;
-                s_dx[i / SB][i % SB] = p.act.d[(size_t) arow * SB + i % SB];
-            }
-            wait_or_abort(&act_full, act_parity, &s_abort, p.err);
-            act_parity ^= 1u;
             __syncthreads();
             loaded = span.ps;
         }
@@ -266,7 +292,7 @@ __device__ __forceinline__ void q3k_mma_body(const GemvParams & p) {
                 for (int c = 0; c < 2; ++c) {
                     const int t = 8 * i + 2 * q + c;
                     if (t >= n) continue;
-                    float * orow = p.out + (size_t) p.perm[row_beg + t0 + t] * p.n_out + f0;
+                    float * orow = p.out + (size_t) s_row[t] * p.n_out + f0;
                     if (DUAL) {
                         orow[g] = __fmul_rn(ggml_silu(__fmul_rn(v[0][c], sc0)), __fmul_rn(v[1][c], sc1));
                     } else {
