@@ -470,11 +470,17 @@ bool q3k_on_mma(int wtype, int64_t rows, int n_groups) { return wtype == TYPE_Q3
 // Rows of one or two tokens: the integer kernel that takes them one by one, unless there are so few groups that Q3_K is on passes of 32.
 bool few_rows(int wtype, int64_t rows, int n_groups) { return rows <= 16 && !q3k_on_mma(wtype, rows, n_groups); }
 
-// Indexed products whose rows share experts, two to each or more, leave the kernel of few rows where it would read and decode more than this,
-// an expert's rows once for each of them; the line lies where the last of the shapes crosses.  Few rows and grouped, us: 2048 -> 2048, 16 rows
-// over 2 experts, Q3_K (28 MB) 19 and 19, NVFP4 (36 MB) 25 and 30; 2048 -> 4096 over 2, 12 rows, Q3_K (41 MB) 27 and 19, NVFP4 (54 MB) 35 and
-// 29; 256 -> 16384 over 4, 16 rows, NVFP4 (36 MB) 31 and 21; 768 -> 65536 over 2, 4 rows, Q3_K (82 MB) 58 and 35.
-constexpr int64_t INDEXED_FEW_BYTES = 40 << 20;
+// Indexed products leave the kernel of few rows where it would read and decode more than this, a row at a time from one wave of CTAs to the
+// next without a ring.  Few rows and grouped, 16 rows with an expert each, us, by what they read: NVFP4, 62 MB, 768 columns 32 and 36,
+// 2048 34 and 33, 4096 40 and 42; 90 MB 46 and 41, 50 and 43, 60 and 43 (and 57 on the kernel before this one).  Q3_K, 52 MB, 512 and 768 columns
+// 35 and 41, 36 and 38; 90 MB 58 and 57, 61 and 55; 120 MB 256 and 2048 columns 71 and 84, 64 and 63; 220 MB 127 and 140, 114 and 103.
+// With two rows or more to an expert the grouped kernels share what they read: 2048 -> 2048, 16 rows over 2 experts, Q3_K (28 MB) 19 and 19,
+// NVFP4 (36 MB) 25 and 30; 2048 -> 4096 over 2, 12 rows, Q3_K (41 MB) 27 and 19, NVFP4 (54 MB) 35 and 29; 256 -> 16384 over 4, 16 rows, NVFP4
+// (36 MB) 31 and 21; 768 -> 65536 over 2, 4 rows, Q3_K (82 MB) 58 and 35.
+bool indexed_few(int wtype, int64_t k, int64_t n_out, int rows, int n_as) {
+    const int64_t mb = rows >= 2 * n_as ? 40 : wtype == TYPE_NVFP4 ? 64 : k == 512 || k == 768 ? 72 : 140;
+    return few_rows(wtype, rows, n_as) && rows * n_out * weight_row_bytes(wtype, k) <= mb << 20;
+}
 
 // the integer product of grouped rows: `rows` routed rows in up to n_groups groups
 template <bool DUAL>
@@ -1612,7 +1618,7 @@ int b200moe_mul_mat_id(b200moe_ctx * ctx, int wtype, const void * as, int64_t ne
     if (rc) return rc;
     Plan & p = ctx->plan;
     const int rows = (int) (T * n_ids);
-    const bool few = few_rows(wtype, rows, (int) n_as) && (rows < 2 * n_as || rows * ne01 * weight_row_bytes(wtype, ne00) <= INDEXED_FEW_BYTES);
+    const bool few = indexed_few(wtype, ne00, ne01, rows, (int) n_as);
     const OverlapScope scope = layer_overlap(ctx, rows, (int) n_as);
     if (!few) CUDA_TRY(ctx, cudaMemsetAsync(p.groups.counts, 0, sizeof(int) * n_as, st));
     // activations: T*ne11 rows of ne00; plan.hq holds T*k rows of width n_ff (= ne00 here), ne11 <= k
