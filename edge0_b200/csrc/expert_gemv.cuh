@@ -362,7 +362,8 @@ __device__ __forceinline__ PassSpan<PT> pass_span(const int * cw, int n_active, 
 //   feature), which share the activations and the thread's fixed work.
 // A chain per thread over the whole K, 16 rows to a four-warp CTA, chunks looked up in the group tables: one token, 2048 -> 768, top-8
 // of 128, gate/up and down 12.1 and 9.8 us (Q3_K 9.9 and 8.6), so 10.4 and 8.3 (8.8 and 8.3).  16 features of gate and up to a CTA 11.1, eight
-// segments 12.1; a segment's bytes behind a barrier of their own gained nothing.
+// segments 12.1 (and of K = 4096, whose four leave a thread 255 registers and none spilled: 1024 features, 8 rows 15.3 and 13.8, 2048 27.5 and
+// 24.4); a segment's bytes behind a barrier of their own gained nothing.
 template <int WT, int K, bool DUAL>
 struct FewCfg {
     static constexpr int PAIRS = DUAL ? 8 : 16;               // row pairs of a CTA
@@ -372,7 +373,7 @@ struct FewCfg {
     static constexpr int TPR = WT == TYPE_NVFP4 ? 4 : 8;      // threads of a row pair
     static constexpr int GROUPS = PAIRS * TPR / 32;           // warps of a segment
     static constexpr int STEPS = WT == TYPE_NVFP4 ? K / 32 : K / 256;   // of a chain
-    static constexpr int SEG = WT == TYPE_NVFP4 ? (K == 4096 ? 8 : 4) : STEPS == 8 ? 4 : STEPS;
+    static constexpr int SEG = WT == TYPE_NVFP4 ? 4 : STEPS == 8 ? 4 : STEPS;
     static constexpr int U = STEPS / SEG;                     // steps of a segment
     static constexpr int THREADS = GROUPS * SEG * 32;
     static constexpr int ACT_D = WT == TYPE_NVFP4 ? K / 32 : K / 256;
