@@ -966,15 +966,13 @@ int dense_matvec(b200moe_ctx * ctx, int wtype, const void * w, const float * sca
 }
 
 // The values of h [rows][n] whose rounding is in doubt, onto `list` (requant_mark_kernel).  MARK_ROWS rows to a warp where that still
-// leaves half of the warps the GPU can hold, else one: 4096 tokens (32768 x 768 values, 49152 warps of four rows) 69 us with one row
-// and 37 with four, 777 tokens (9324 warps) 15 and 10; the two
-// lists of 64 tokens of a latent layer over 512 experts (1280 warps and 128) 8.0 and 9.9: one wave of blocks, which several rows make longer.
+// leaves half of the warps the GPU can hold (4736), else one: 4096 tokens (32768 x 768 values, 49152 warps of four rows) 69 us with one
+// row and 37 with four, 777 tokens (9324 warps) 15 and 10; the two lists of 64 tokens of a latent layer over 512 experts (1280 warps and 128) 8.0 and 9.9: one wave of blocks, which several rows make longer.
 constexpr int MARK_ROWS = 4;
-constexpr int64_t MARK_FULL_WARPS = 148 * 32;
 int launch_mark(b200moe_ctx * ctx, const float * h, int rows, int n, float step_margin, float rel_margin, const FixList & list, cudaStream_t st) {
     const int * perm = ctx->plan.groups.perm, * meta = ctx->plan.groups.meta;
     const int64_t chunks = n / 128, several = (rows + MARK_ROWS - 1) / MARK_ROWS * chunks;
-    if (several >= MARK_FULL_WARPS)
+    if (several >= (int64_t) ctx->sm_count * 32)
         launch_k(ctx, requant_mark_kernel<MARK_ROWS>, dim3((unsigned) ((several + 7) / 8)), dim3(256), 0, st, h, perm, meta, rows, n, step_margin, rel_margin, list);
     else
         launch_k(ctx, requant_mark_kernel<1>, dim3((unsigned) ((rows * chunks + 7) / 8)), dim3(256), 0, st, h, perm, meta, rows, n, step_margin, rel_margin, list);
