@@ -90,8 +90,8 @@ def physical_cores() -> int:
     return os.cpu_count() or 1
 
 
-# DRAM bytes per algorithmic byte of the gate/up expert kernel, from the ncu capture summarised in profiles/ (626.88 MB / 598.08 MB)
-NCU_TRAFFIC_PER_ALGORITHMIC_BYTE = 1.0482
+# DRAM bytes per algorithmic byte of the gate/up expert kernel, from the ncu capture summarised in profiles/ (618.63 MB / 598.08 MB)
+NCU_TRAFFIC_PER_ALGORITHMIC_BYTE = 1.0344
 
 
 class ClockSampler:
@@ -337,7 +337,7 @@ def single_layer_extras(ctx, dev, args, peak, peaks):
                                 "peak_bf16_measured": bf16_peak, "frac_of_bf16_measured": tf / bf16_peak,
                                 "peak_fp4_measured": f4, "peak_fp4_measured_how": f4_how, "frac_of_fp4_measured": tf / f4 if f4 else None,
                                 "peak_fp4_vendor_dense": FP4_VENDOR_TFLOPS, "frac_of_fp4_vendor": tf / FP4_VENDOR_TFLOPS,
-                                "engine": "tcgen05 kind::f16 (activations as fp16 hi + lo: 2 x the useful flop issued) + exact re-quantisation fix-up"}
+                                "engine": "tcgen05 kind::mxf4nvf4 (activations as six digit planes: 6 x the useful flop issued) + exact re-quantisation fix-up"}
         out["c3_nvfp4_prefill T=4096"] = r
     except Exception as ex:
         out["c3_nvfp4_prefill T=4096"] = {"error": repr(ex)[:300]}
@@ -508,7 +508,7 @@ def run_c5_arm(args):
                              "achieved": gu_b / (gu_us * 1e-6) / 1e9 if gu_us else 0.0, "peak": peak, "unit": "GB/s",
                              "frac": gu_b / (gu_us * 1e-6) / 1e9 / peak if gu_us else 0.0, "traffic": gu_b * NCU_TRAFFIC_PER_ALGORITHMIC_BYTE,
                              "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of this kernel in the ncu capture of the one-GPU step "
-                                               "(profiles/expert_gemm_fp4_c5_latent_T256.md: 626.88 MB for 598.08 MB algorithmic), scaled by the "
+                                               "(profiles/expert_gemm_fp4_c5_latent_T256.md: 618.63 MB for 598.08 MB algorithmic), scaled by the "
                                                "experts this rank holds", "peak_source": peak_kind,
                              "algorithmic_bytes_per_launch": gu_b, "avg_launch_us": gu_us, "experts_touched_on_rank0": U_local,
                              "down_kernel": {"achieved": dn_b / (dn_us * 1e-6) / 1e9 if dn_us else 0.0, "avg_launch_us": dn_us,

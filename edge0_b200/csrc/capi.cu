@@ -413,7 +413,7 @@ int launch_few_rows(b200moe_ctx * ctx, const GemvParams & p, int rows, cudaStrea
     return check_launch(ctx, "expert_few_rows");
 }
 
-// NVFP4, more than a few rows: n_mats matrices behind one another (one when every group shares it)
+// NVFP4, more than a few rows: p.n_as matrices behind one another, or one that every group shares (p.w_stride = 0)
 template <int K, bool DUAL>
 int launch_gemv_nvfp4(b200moe_ctx * ctx, const GemvParams & p, cudaStream_t st) {
     using C = Nvfp4GemvCfg<K, DUAL>;
@@ -967,7 +967,8 @@ int dense_matvec(b200moe_ctx * ctx, int wtype, const void * w, const float * sca
 
 // The values of h [rows][n] whose rounding is in doubt, onto `list` (requant_mark_kernel).  MARK_ROWS rows to a warp where that still
 // leaves half of the warps the GPU can hold (4736), else one: 4096 tokens (32768 x 768 values, 49152 warps of four rows) 69 us with one
-// row and 37 with four, 777 tokens (9324 warps) 15 and 10; the two lists of 64 tokens of a latent layer over 512 experts (1280 warps and 128) 8.0 and 9.9: one wave of blocks, which several rows make longer.
+// row and 37 with four, 777 tokens (9324 warps) 15 and 10; the two lists of 64 tokens of a latent layer over 512 experts (1280 warps and 128)
+// 8.0 and 9.9: one wave of blocks, which several rows make longer.
 constexpr int MARK_ROWS = 4;
 int launch_mark(b200moe_ctx * ctx, const float * h, int rows, int n, float step_margin, float rel_margin, const FixList & list, cudaStream_t st) {
     const int * perm = ctx->plan.groups.perm, * meta = ctx->plan.groups.meta;

@@ -373,7 +373,7 @@ expert_gemm_fp4_kernel(const Fp4Params p, const __grid_constant__ CUtensorMap ma
     const int my_stages = n_units > (int) blockIdx.x ? (n_units - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x * KC : 0;
     // weight stage: [A0][A1]; activation stage: [B][SFB]
     constexpr uint32_t OFF_A1 = C::A_TILE, OFF_SFB = C::B_TILE;
-    // 768 threads leave 80 registers to a thread.  With the small tile producers and issuer give theirs to the epilogue, which spilled without
+    // 768 threads leave 80 registers to a thread.  With the small tile producers and issuer give theirs to the epilogue, which spilled without (4 to 8 bytes are left)
     // (40 + 2 x 104 + 3 x 72 = 464 of the launch's 480 per 128 threads; 64 tokens over 128 experts: gate/up 51.7 us, so 49.9, down 29.4 and 27.0).
     // The large one loses with it (4096 tokens, down: 244 us, 283 so); what kept a short K from spilling there is that the loops over
     // K = 256 pieces stay loops (K = 512, 1024 tokens x 32768 features: 111 us unrolled, so 98).

@@ -17,11 +17,11 @@
 // brings the two low code bits of its group in place, one the high bits of both groups, and a byte permute picks four of the eight products
 // of a (row, sub-block) by the codes packed to a selector.  No operand tile in shared memory, no barrier between super-blocks: a warp fetches
 // its own raw rows and meets the others only when the routed rows change.  The code is separate for each number of token groups: with a test
-// between them nothing was scheduled across (1001 tokens, gate/up: 430 us, so 308).
+// between them nothing was scheduled across (1001 tokens, gate/up: 430 us, then 308).
 // What bounds it is the half-rate integer unit and, with 32 routed rows to a pass, its own dependences at two warps per scheduler (255
-// registers; IPC 0.58 per scheduler).  Decoding 64 x 64 tiles through shared memory, a barrier to a super-block (IPC 0.32), and a thread per
-// reference lane with dp4a took, 2048 -> 768 of 128 experts, us: gate/up of 32 tokens 130 and of 1001 tokens 537, down 71 and 311; so 73 and
-// 308, 45 and 196.
+// registers, a few values spilled beside the loops; IPC 0.56 per scheduler).  Decoding 64 x 64 tiles through shared memory, a barrier to a super-block (IPC 0.32), and a thread per
+// reference lane with dp4a took, 2048 -> 768 of 128 experts, us: gate/up of 32 tokens 130 and of 1001 tokens 537, down 71 and 311; so 75 and
+// 289, 42 and 174.
 // Activation rows are K + 16 bytes apart, which makes the 16-byte fragment loads conflict-free.
 #pragma once
 #include "common.cuh"
@@ -315,6 +315,7 @@ __device__ __forceinline__ void q3k_mma_body(const GemvParams & p) {
     __syncthreads();
 }
 
+// passes of 16 routed rows, for few rows per expert, and of 32 (Q3K_MMA_MIN_ROWS)
 template <int K, bool DUAL>
 __global__ void __launch_bounds__(Q3kCfg<K, DUAL, 2>::THREADS, 1) q3k_expert_gemv_kernel(const GemvParams p) {
     q3k_mma_body<K, DUAL, 2>(p);

@@ -195,7 +195,7 @@ class Context:
         return int(c.kernel_launches)
 
     def set_expert_path(self, path: int):
-        """0 automatic, 1 integer GEMV always, 2 tensor-core grouped GEMM whenever the shape allows."""
+        """0 automatic, 1 integer kernels always, 2 tensor-core grouped GEMM whenever the shape allows."""
         self.check(self.lib.b200moe_set_expert_path(self.handle, path))
 
     def set_launch_overlap(self, enable: bool) -> None:
